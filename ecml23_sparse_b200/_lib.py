@@ -144,6 +144,25 @@ def load(rebuild_if_stale: bool = True):
     return lib
 
 
+_binding = None
+
+
+def binding():
+    """The native binding module (``_native.so``), built first when its source is newer (needs a compiler)."""
+    global _binding
+    if _binding is None:
+        load()
+        try:
+            _build.build_binding()
+        except Exception as exc:  # no compiler on this machine: use the shipped module if there is one
+            if not os.path.exists(_build.BINDING_PATH):
+                raise ImportError(f"_native.so is missing and could not be built: {exc}") from exc
+        from . import _native
+
+        _binding = _native
+    return _binding
+
+
 def check(status: int) -> None:
     if status != FFI_OK:
         raise FFIError(status, load().ffi_last_error().decode("utf-8", "replace"))

@@ -1,7 +1,8 @@
-"""Builds the CUDA library ``libffi_b200.so`` in-tree for sm_100a with nvcc.
+"""Builds, in-tree, the CUDA library ``libffi_b200.so`` for sm_100a with nvcc and ``_native.so``, the
+binding of its hot entry points over torch tensors, with the host compiler.
 
-``python -m ecml23_sparse_b200.build`` or :func:`build`.  The library is rebuilt when a
-source file is newer than it.  nvcc cross-compiles without a GPU.
+``python -m ecml23_sparse_b200.build`` or :func:`build`.  Each is rebuilt when a source file is newer
+than it.  nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -16,6 +17,8 @@ ROOT = os.path.dirname(PKG_DIR)
 CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIB_PATH = os.path.join(PKG_DIR, "libffi_b200.so")
+BINDING_SRC = os.path.join(CSRC, "binding.cpp")
+BINDING_PATH = os.path.join(PKG_DIR, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -82,6 +85,37 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     return LIB_PATH
 
 
+def _binding_stale() -> bool:
+    if not os.path.exists(BINDING_PATH):
+        return True
+    deps = [BINDING_SRC, os.path.join(INCLUDE, "ffi_b200.h")]
+    return any(os.path.getmtime(d) > os.path.getmtime(BINDING_PATH) for d in deps)
+
+
+def build_binding(force: bool = False, verbose: bool = False) -> str:
+    """Compiles ``_native.so`` against the torch this interpreter imports and the CUDA library beside it."""
+    if not force and not _binding_stale():
+        return BINDING_PATH
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    build()
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include"), INCLUDE]
+    libs = [p for p in cpp_extension.library_paths()]
+    cmd = [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-isystem{i}" for i in includes),
+           BINDING_SRC, "-o", BINDING_PATH, f"-L{PKG_DIR}", "-lffi_b200", "-Wl,-rpath,$ORIGIN",
+           *(f"-L{p}" for p in libs), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    subprocess.run(cmd, check=True)
+    return BINDING_PATH
+
+
 if __name__ == "__main__":
     extra = ["-Xptxas", "-v"] if "--ptxas" in sys.argv else None
     print(build(force=True, verbose=True, extra=extra))
+    print(build_binding(force=True, verbose=True))

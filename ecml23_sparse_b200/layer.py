@@ -59,8 +59,8 @@ class FFILayer(nn.Module):
     def forward(self, inputs: torch.Tensor) -> torch.Tensor:
         if inputs.dim() != 2 or inputs.shape[1] != self.in_features:
             raise ValueError(f"expected input of shape [B, {self.in_features}], got {tuple(inputs.shape)}")
-        tp_in = inputs.t().contiguous()  # custom_layer.py:48
-        return ops.ffi_matmul_tp(tp_in, self.lookup(), self.weights(), self.bias).contiguous()
+        # one autograd node: the transposition of custom_layer.py:48, the op on the reshaped vectors, the bias
+        return ops._native().layer_forward(inputs, self.kernel_indices, self.kernel_weights, self.bias, self.units, self.fan_in)
 
     # ---- rewiring (sparse/layer.py:62-86,236-237; sparse/custom_layer.py:20-43) -----------------
     def rewire_candidates(self, fraction: float = 0.01) -> torch.Tensor:

@@ -9,8 +9,9 @@ Same function names, argument order and return values as the reference's wrapper
 * ``fan_in_sparse_matmul_grad_tp(...)`` likewise for the transposed layout
 
 and the gradient wiring of fixed_fan_in_ops.py:31-40 (``[feature_grad, None, weight_grad]``)
-as :class:`torch.autograd.Function` objects behind ``ffi_matmul`` / ``ffi_matmul_tp``.
-Every call goes through the C ABI of ``libffi_b200.so``; there is no CPU path.
+as an autograd node behind ``ffi_matmul`` / ``ffi_matmul_tp``.
+Every call goes through the C ABI of ``libffi_b200.so``; there is no CPU path.  The hot entry points are one native
+call each (``csrc/binding.cpp``: checks, output and scratch allocation, launch, autograd node); the rest goes over ctypes.
 """
 from __future__ import annotations
 
@@ -29,6 +30,15 @@ _PLAN_CACHE_MAX = 8
 
 def _stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def _native():
+    """The native binding; its autograd node asks this module for a table's plan."""
+    global _native
+    mod = _lib.binding()
+    mod.set_get_plan(get_plan)
+    _native = lambda: mod  # noqa: E731
+    return mod
 
 
 def _workspace(device, nbytes: int) -> Optional[torch.Tensor]:
@@ -65,17 +75,6 @@ def _as_index(lookup: torch.Tensor) -> torch.Tensor:
     return lookup
 
 
-def _shapes(features, lookup, weights, transposed):
-    if lookup.shape != weights.shape:
-        raise ValueError(f"lookup {tuple(lookup.shape)} and weights {tuple(weights.shape)} must have equal shapes")
-    if transposed:
-        N, B = features.shape
-    else:
-        B, N = features.shape
-    L, K = lookup.shape
-    return B, N, L, K
-
-
 class FFIPlan:
     """Transposed (CSR-by-input) index of one lookup table; owns device memory.
 
@@ -92,6 +91,7 @@ class FFIPlan:
             _lib.check(_lib.load().ffi_plan_create(lookup.data_ptr(), self.L, self.K, self.N,
                                                    _stream_ptr(self.device), ctypes.byref(handle)))
         self._handle = handle
+        self.address = handle.value
         self.builds = 1
         self._finalizer = weakref.finalize(self, _lib.load().ffi_plan_destroy, handle)
 
@@ -137,7 +137,7 @@ def get_plan(lookup: torch.Tensor, n_in: int) -> FFIPlan:
     keeps a reference to the table so that its address cannot be handed to another tensor while
     the entry lives (at most 8 tables are kept).
     """
-    key = (lookup.data_ptr(), tuple(lookup.shape), int(n_in), lookup.device.index)
+    key = (lookup.data_ptr(), lookup.shape, n_in, lookup.get_device())
     hit = _plan_cache.get(key)
     if hit is not None and hit[0] == lookup._version:
         return hit[1]
@@ -156,42 +156,11 @@ def get_plan(lookup: torch.Tensor, n_in: int) -> FFIPlan:
 def clear_caches():
     _plan_cache.clear()
     _workspaces.clear()
-
-
-_STORAGE_DTYPES = (torch.float32, torch.bfloat16)
-
-
-def _storage_dtype(features, weights) -> int:
-    """x and W share one storage type: fp32, or bf16 (accumulation, y and all gradients stay fp32)."""
-    if features.dtype != weights.dtype:
-        raise TypeError(f"features ({features.dtype}) and weights ({weights.dtype}) must have the same dtype")
-    return _lib.FFI_BF16 if features.dtype == torch.bfloat16 else _lib.FFI_F32
+    _native().clear_scratch()
 
 
 def _forward(features, lookup, weights, bias, transposed: bool) -> torch.Tensor:
-    features = _check_cuda("features", features, _STORAGE_DTYPES)
-    weights = _check_cuda("weights", weights, _STORAGE_DTYPES)
-    dtype = _storage_dtype(features, weights)
-    lookup = _as_index(lookup)
-    B, N, L, K = _shapes(features, lookup, weights, transposed)
-    lib = _lib.load()
-    dev = features.device
-    if bias is not None:
-        if bias.shape != (L,) or bias.dtype != torch.float32 or not bias.is_cuda:
-            raise ValueError("bias must be a float32 CUDA tensor of shape [L]")
-        bias = bias.contiguous()
-    out = torch.empty((B, L), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        ws_bytes = lib.ffi_forward_workspace_bytes(B, N, L, K, int(transposed), dtype)
-        ws = _workspace(dev, ws_bytes + 256 if ws_bytes else 0)
-        ws_ptr, ws_len = None, 0
-        if ws is not None:
-            off = (-ws.data_ptr()) % 256
-            ws_ptr, ws_len = ws.data_ptr() + off, ws.numel() - off
-        _lib.check(lib.ffi_forward(features.data_ptr(), lookup.data_ptr(), weights.data_ptr(),
-                                   bias.data_ptr() if bias is not None else None, out.data_ptr(),
-                                   B, N, L, K, int(transposed), dtype, ws_ptr, ws_len, _stream_ptr(dev)))
-    return out
+    return _native().forward(features, lookup, weights, bias, transposed)
 
 
 def _backward(features, lookup, weights, out_grad, transposed: bool, plan: Optional[FFIPlan] = None,
@@ -200,55 +169,13 @@ def _backward(features, lookup, weights, out_grad, transposed: bool, plan: Optio
     """grad_is_transposed: `out_grad` is gT[L][ldg] (from forward_bce / transpose_gradient), not g[B,L].
     feature_grad_out: a contiguous float32 tensor with the number of elements of `features` that
     receives grad_x instead of a fresh allocation (e.g. a slot of a peer-visible buffer)."""
-    features = _check_cuda("features", features, _STORAGE_DTYPES)
-    weights = _check_cuda("weights", weights, _STORAGE_DTYPES)
-    dtype = _storage_dtype(features, weights)
-    out_grad = _check_cuda("out_grad", out_grad, (torch.float32,))
-    lookup = _as_index(lookup)
-    B, N, L, K = _shapes(features, lookup, weights, transposed)
-    if grad_is_transposed:
-        if out_grad.shape[0] != L or out_grad.shape[1] < B:
-            raise ValueError(f"transposed out_grad has shape {tuple(out_grad.shape)}, expected [{L}, >= {B}]")
-    elif tuple(out_grad.shape) != (B, L):
-        raise ValueError(f"out_grad has shape {tuple(out_grad.shape)}, expected {(B, L)}")
-    lib = _lib.load()
-    dev = features.device
     if want_feature_grad and plan is None:
-        plan = get_plan(lookup, N)
-    gx = None
-    if want_feature_grad:
-        if feature_grad_out is not None:
-            if (feature_grad_out.dtype != torch.float32 or not feature_grad_out.is_contiguous()
-                    or feature_grad_out.numel() != features.numel() or feature_grad_out.device != dev):
-                raise ValueError("feature_grad_out must be a contiguous float32 tensor of features' size on its device")
-            gx = feature_grad_out.view(features.shape)
-        else:
-            gx = torch.empty(features.shape, dtype=torch.float32, device=dev)
-    gw = torch.empty(weights.shape, dtype=torch.float32, device=dev) if want_weight_grad else None
-    gb = torch.empty((L,), dtype=torch.float32, device=dev) if want_bias_grad else None
-    with torch.cuda.device(dev):
-        handle = plan.handle if plan is not None else None
-        ws_bytes = lib.ffi_backward_workspace_bytes(handle, B, N, L, K, int(transposed), dtype,
-                                                    int(want_feature_grad), int(want_weight_grad or want_bias_grad))
-        ws = _workspace(dev, ws_bytes + 256 if ws_bytes else 0)
-        ws_ptr = None
-        ws_len = 0
-        if ws is not None:
-            off = (-ws.data_ptr()) % 256
-            ws_ptr = ws.data_ptr() + off
-            ws_len = ws.numel() - off
-        outs = (gx.data_ptr() if gx is not None else None, gw.data_ptr() if gw is not None else None,
-                gb.data_ptr() if gb is not None else None)
-        if grad_is_transposed:
-            _lib.check(lib.ffi_backward_from_transposed(features.data_ptr(), lookup.data_ptr(), weights.data_ptr(),
-                                                        out_grad.data_ptr(), out_grad.shape[1], handle, *outs,
-                                                        B, N, L, K, int(transposed), dtype, ws_ptr, ws_len,
-                                                        _stream_ptr(dev)))
-        else:
-            _lib.check(lib.ffi_backward(features.data_ptr(), lookup.data_ptr(), weights.data_ptr(), out_grad.data_ptr(),
-                                        handle, *outs, B, N, L, K, int(transposed), dtype, ws_ptr, ws_len,
-                                        _stream_ptr(dev)))
-    return gx, gw, gb
+        plan = get_plan(lookup.contiguous(), features.shape[0 if transposed else 1])
+    return _native().backward(features, lookup, weights, out_grad, transposed, plan.address if plan is not None else 0,
+                              want_feature_grad, want_weight_grad, want_bias_grad, grad_is_transposed, feature_grad_out)
+
+
+_LOSS_KINDS = {"bce": _lib.FFI_LOSS_BCE, "squared_hinge": _lib.FFI_LOSS_SQUARED_HINGE, "hinge": _lib.FFI_LOSS_HINGE}
 
 
 def forward_bce(features, lookup, weights, bias, row_ptr, labels, transposed: bool, total_labels=None,
@@ -259,35 +186,8 @@ def forward_bce(features, lookup, weights, bias, row_ptr, labels, transposed: bo
 
     The logits are never materialised.  `loss_out` (optional, one fp32 element on the device) receives the
     loss scalar in place, e.g. a slot of the buffer a label-sharded step exchanges."""
-    features = _check_cuda("features", features, _STORAGE_DTYPES)
-    weights = _check_cuda("weights", weights, _STORAGE_DTYPES)
-    dtype = _storage_dtype(features, weights)
-    lookup = _as_index(lookup)
-    B, N, L, K = _shapes(features, lookup, weights, transposed)
-    dev = features.device
-    lib = _lib.load()
-    row_ptr = row_ptr.to(device=dev, dtype=torch.int32).contiguous()
-    labels = labels.to(device=dev, dtype=torch.int32).contiguous()
-    if row_ptr.numel() != B + 1:
-        raise ValueError("row_ptr must have B+1 entries")
-    ldg = int(lib.ffi_transposed_gradient_stride(B))
-    gT = torch.empty((L, ldg), dtype=torch.float32, device=dev)
-    if loss_out is None:
-        loss_out = torch.empty((), dtype=torch.float32, device=dev)
-    elif loss_out.dtype != torch.float32 or loss_out.numel() != 1 or loss_out.device != dev:
-        raise ValueError("loss_out must be one fp32 element on the features' device")
-    with torch.cuda.device(dev):
-        ws_bytes = lib.ffi_forward_bce_workspace_bytes(B, N, L, K, int(transposed), dtype)
-        ws = _workspace(dev, ws_bytes + 256)
-        off = (-ws.data_ptr()) % 256
-        kind = {"bce": _lib.FFI_LOSS_BCE, "squared_hinge": _lib.FFI_LOSS_SQUARED_HINGE, "hinge": _lib.FFI_LOSS_HINGE}[loss]
-        _lib.check(lib.ffi_forward_loss(kind, features.data_ptr(), lookup.data_ptr(), weights.data_ptr(),
-                                        bias.data_ptr() if bias is not None else None, row_ptr.data_ptr(),
-                                        labels.data_ptr() if labels.numel() else row_ptr.data_ptr(), gT.data_ptr(),
-                                        loss_out.data_ptr(), B, N, L, K, total_labels or L, label_offset,
-                                        int(transposed), dtype, ws.data_ptr() + off, ws.numel() - off,
-                                        _stream_ptr(dev)))
-    return loss_out, gT
+    return _native().forward_loss(_LOSS_KINDS[loss], features, lookup, weights, bias, row_ptr, labels, transposed,
+                                  total_labels or 0, label_offset, loss_out)
 
 
 def forward_topk(features, lookup, weights, bias, k: int, transposed: bool, label_offset: int = 0):
@@ -295,24 +195,7 @@ def forward_topk(features, lookup, weights, bias, k: int, transposed: bool, labe
     of tf.nn.top_k, without materialising the logits: what PrecisionAtK (sparse/metrics.py:9-70)
     consumes.  With a sharded label dimension call it per shard (`label_offset` = first label of the
     shard) and merge the candidates with `merge_topk`."""
-    features = _check_cuda("features", features, (torch.float32, torch.bfloat16))
-    weights = _check_cuda("weights", weights, (features.dtype,))
-    lookup = _as_index(lookup)
-    B, N, L, K = _shapes(features, lookup, weights, transposed)
-    dev = features.device
-    lib = _lib.load()
-    dtype = _lib.FFI_BF16 if features.dtype == torch.bfloat16 else _lib.FFI_F32
-    top_val = torch.empty((B, k), dtype=torch.float32, device=dev)
-    top_idx = torch.empty((B, k), dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
-        ws_bytes = lib.ffi_forward_topk_workspace_bytes(B, N, L, K, int(transposed), dtype)
-        ws = _workspace(dev, ws_bytes + 256)
-        off = (-ws.data_ptr()) % 256
-        _lib.check(lib.ffi_forward_topk(features.data_ptr(), lookup.data_ptr(), weights.data_ptr(),
-                                        bias.data_ptr() if bias is not None else None, top_val.data_ptr(),
-                                        top_idx.data_ptr(), k, B, N, L, K, label_offset, int(transposed),
-                                        dtype, ws.data_ptr() + off, ws.numel() - off, _stream_ptr(dev)))
-    return top_val, top_idx
+    return _native().forward_topk(features, lookup, weights, bias, k, transposed, label_offset)
 
 
 def merge_topk(candidates, k: int):
@@ -375,29 +258,11 @@ def fan_in_sparse_matmul_grad_tp(features, lookup, weights, out_grad):
 
 # ---- gradient registration (sparse/ops/fixed_fan_in_ops.py:31-40) ---------------------
 
-class _FanInSparseMatmul(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, features, lookup, weights, bias, transposed):
-        ctx.save_for_backward(features, lookup, weights)
-        ctx.transposed = transposed
-        ctx.has_bias = bias is not None
-        return _forward(features, lookup, weights, bias, transposed)
-
-    @staticmethod
-    def backward(ctx, grad):
-        features, lookup, weights = ctx.saved_tensors
-        need_x, _, need_w = ctx.needs_input_grad[:3]
-        need_b = ctx.has_bias and ctx.needs_input_grad[3]
-        gx, gw, gb = _backward(features, lookup, weights, grad.contiguous(), ctx.transposed,
-                               want_feature_grad=need_x, want_weight_grad=need_w, want_bias_grad=need_b)
-        return gx, None, gw, gb, None
-
-
 def ffi_matmul(features, lookup, weights, bias=None):
     """Differentiable FanInSparseMatmul (+ optional fused bias)."""
-    return _FanInSparseMatmul.apply(features, lookup, weights, bias, False)
+    return _native().matmul(features, lookup, weights, bias, False)
 
 
 def ffi_matmul_tp(features, lookup, weights, bias=None):
     """Differentiable FanInSparseMatmulTp (features given as [N,B]) (+ optional fused bias)."""
-    return _FanInSparseMatmul.apply(features, lookup, weights, bias, True)
+    return _native().matmul(features, lookup, weights, bias, True)

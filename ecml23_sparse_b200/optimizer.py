@@ -10,8 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
-from .ops import _stream_ptr
+from . import ops
 
 
 class FusedAdam:
@@ -28,20 +27,13 @@ class FusedAdam:
     def step(self, grads=None):
         """Applies one update; `grads` defaults to each parameter's `.grad`."""
         self.iterations += 1
-        lib = _lib.load()
+        adam_step = ops._native().adam_step
         for j, p in enumerate(self.params):
             g = grads[j] if grads is not None else p.grad
             if g is None:
                 continue
-            g = g.contiguous()
-            if g.dtype != torch.float32 or g.shape != p.shape:
-                raise ValueError("gradient must be float32 with the parameter's shape")
-            dtype = _lib.FFI_BF16 if p.dtype == torch.bfloat16 else _lib.FFI_F32
-            data = p.data if isinstance(p, torch.nn.Parameter) else p
-            with torch.cuda.device(p.device):
-                _lib.check(lib.ffi_adam_step(data.data_ptr(), self.m[j].data_ptr(), self.v[j].data_ptr(), g.data_ptr(),
-                                             p.numel(), self.lr, self.beta_1, self.beta_2, self.epsilon,
-                                             self.iterations, dtype, _stream_ptr(p.device)))
+            adam_step(p.data if isinstance(p, torch.nn.Parameter) else p, self.m[j], self.v[j], g, self.lr, self.beta_1,
+                      self.beta_2, self.epsilon, self.iterations)
 
     def zero_moments(self, index: int, locations: torch.Tensor):
         """Zero m and v of parameter `index` at flat positions `locations`."""
