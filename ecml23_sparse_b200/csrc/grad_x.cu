@@ -230,51 +230,74 @@ __global__ void reduce_partials_kernel(const float* __restrict__ partial, float*
 
 // One warp per (input i, batch tile of 32*VEC): walks row i of the canonical index and gathers
 // one row of the transposed gradient gT[L][ldg] per entry.
+//
+// What bounds it: 4*B*L*K gathered bytes through the L2-to-SM fabric (20 TB/s for 512-byte rows that hit L2, 9 TB/s for
+// a table of three times L2, by a bare gather loop), so the rows have to hit L2.  All resident warps start at output 0
+// and walk their rows, sorted by output, at about the same pace, so the part of gT they touch at any time is a moving
+// window; the more warps are resident (64 per SM, two gathers each) and the fewer columns a row has (one batch tile at a
+// time), the better the window fits.  B=256, N=65,536, L=501,070, K=32: 1.03 ms (16 TB/s) against 1.53 ms with the tiles
+// of an input side by side at 48 warps per SM; B=512, N=100,000, L=83,762, K=72: 0.72 against 1.31 ms; B=128, N=32,768,
+// L=670,091: 0.69 against 0.71 ms.  Cutting the walk into segments of outputs that fit L2, one launch each, measured
+// slower (1.16 ms): carrying the sums through memory and the launch tails cost more than the hits gain.
+struct GxWideParams {
+    const float* gT;
+    const int* rowptr;
+    const int* perm;
+    float* gx;
+    long long ldg;
+    int B, N, K, x_transposed;
+};
+
 template <int VEC, typename TW>
-__global__ void __launch_bounds__(256) ffi_grad_x_wide_kernel(const TW* __restrict__ W,
-                                                              const float* __restrict__ gT,
-                                                              const int* __restrict__ rowptr,
-                                                              const int* __restrict__ perm,
-                                                              float* __restrict__ gx, int B, int N,
-                                                              int K, long long ldg, int x_transposed) {
+__global__ void __launch_bounds__(256, 8) ffi_grad_x_wide_kernel(const TW* __restrict__ W, GxWideParams p) {
     using V = typename Vec<VEC>::type;
-    constexpr int BTW = 32 * VEC;
+    constexpr int kGroup = 2;  // gathers in flight per warp
     const int lane = threadIdx.x & 31;
-    const long long wid = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int nBT = static_cast<int>(ldg / BTW);
-    if (wid >= static_cast<long long>(N) * nBT) return;
-    const int i = static_cast<int>(wid / nBT);
-    const int bt = static_cast<int>(wid - static_cast<long long>(i) * nBT);
-    const V* gTv = reinterpret_cast<const V*>(gT + bt * BTW) + lane;
-    const size_t ldv = static_cast<size_t>(ldg / VEC);
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= p.N) return;
+    const V* gTv = reinterpret_cast<const V*>(p.gT + blockIdx.y * (32 * VEC)) + lane;
+    const unsigned ldv = static_cast<unsigned>(p.ldg / VEC);
     float acc[VEC];
 #pragma unroll
     for (int q = 0; q < VEC; ++q) acc[q] = 0.f;
-    const int s = rowptr[i], t = rowptr[i + 1];
-    for (int base = s; base < t; base += 32) {
-        const int e = base + lane;
-        int o = 0;
-        float w = 0.f;
-        if (e < t) {
-            const int pos = __ldg(perm + e);
-            o = pos / K;
-            w = widen(W[pos]);
+    int e = p.rowptr[i];
+    const int t = p.rowptr[i + 1];
+    // 32 entries at a time sit in the lanes as (output o, weight w); the flat positions of the next 32 are requested
+    // before the current ones are worked on
+    int pos = e + lane < t ? __ldg(p.perm + e + lane) : 0;
+    while (e < t) {
+        const int cnt = min(32, t - e);
+        const int o = pos / p.K;
+        const float w = lane < cnt ? widen(W[pos]) : 0.f;
+        e += 32;
+        if (e + lane < t) pos = __ldg(p.perm + e + lane);
+        int u = 0;
+#pragma unroll 1
+        for (; u + kGroup <= cnt; u += kGroup) {
+            V v[kGroup];
+#pragma unroll
+            for (int j = 0; j < kGroup; ++j) v[j] = __ldg(gTv + static_cast<size_t>(__shfl_sync(0xffffffffu, o, u + j)) * ldv);
+#pragma unroll
+            for (int j = 0; j < kGroup; ++j) {
+                const float wu = __shfl_sync(0xffffffffu, w, u + j);
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) acc[q] = fmaf(wu, vec_get(v[j], q), acc[q]);
+            }
         }
-        const int cnt = min(32, t - base);
-        for (int u = 0; u < cnt; ++u) {
-            const int ou = __shfl_sync(0xffffffffu, o, u);
+#pragma unroll 1
+        for (; u < cnt; ++u) {
+            const V v = __ldg(gTv + static_cast<size_t>(__shfl_sync(0xffffffffu, o, u)) * ldv);
             const float wu = __shfl_sync(0xffffffffu, w, u);
-            const V v = __ldg(gTv + static_cast<size_t>(ou) * ldv);
 #pragma unroll
             for (int q = 0; q < VEC; ++q) acc[q] = fmaf(wu, vec_get(v, q), acc[q]);
         }
     }
-    const int b = bt * BTW + lane * VEC;
+    const int b = blockIdx.y * (32 * VEC) + lane * VEC;
 #pragma unroll
     for (int q = 0; q < VEC; ++q) {
-        if (b + q < B) {
-            if (x_transposed) gx[static_cast<size_t>(i) * B + b + q] = acc[q];
-            else gx[static_cast<size_t>(b + q) * N + i] = acc[q];
+        if (b + q < p.B) {
+            if (p.x_transposed) p.gx[static_cast<size_t>(i) * p.B + b + q] = acc[q];
+            else p.gx[static_cast<size_t>(b + q) * p.N + i] = acc[q];
         }
     }
 }
@@ -481,20 +504,14 @@ int launch_grad_x(const GradXArgs& a, cudaStream_t stream) {
         return FFI_OK;
     }
 
-    // Wide inputs: one warp per (input, batch tile) over the canonical index.
+    // Wide inputs: one warp per (input, batch tile) over the canonical index, batch tile by batch tile.
     const int vec = a.ldg % 128 == 0 ? 4 : (a.ldg % 64 == 0 ? 2 : 1);
-    const long long warps = static_cast<long long>(a.N) * (a.ldg / (32 * vec));
-    const unsigned blocks = static_cast<unsigned>(ceil_div(warps, 8));
+    const GxWideParams p{a.gT, plan->rowptr, plan->perm, a.gx, a.ldg, a.B, a.N, a.K, a.x_transposed};
+    const dim3 grid(static_cast<unsigned>(ceil_div(a.N, 8)), static_cast<unsigned>(ceil_div(a.B, 32 * vec)));
     auto launch_wide = [&](auto w_typed) {
-        if (vec == 4)
-            ffi_grad_x_wide_kernel<4><<<blocks, 256, 0, stream>>>(w_typed, a.gT, plan->rowptr, plan->perm, a.gx, a.B, a.N,
-                                                                  a.K, a.ldg, a.x_transposed);
-        else if (vec == 2)
-            ffi_grad_x_wide_kernel<2><<<blocks, 256, 0, stream>>>(w_typed, a.gT, plan->rowptr, plan->perm, a.gx, a.B, a.N,
-                                                                  a.K, a.ldg, a.x_transposed);
-        else
-            ffi_grad_x_wide_kernel<1><<<blocks, 256, 0, stream>>>(w_typed, a.gT, plan->rowptr, plan->perm, a.gx, a.B, a.N,
-                                                                  a.K, a.ldg, a.x_transposed);
+        if (vec == 4) ffi_grad_x_wide_kernel<4><<<grid, 256, 0, stream>>>(w_typed, p);
+        else if (vec == 2) ffi_grad_x_wide_kernel<2><<<grid, 256, 0, stream>>>(w_typed, p);
+        else ffi_grad_x_wide_kernel<1><<<grid, 256, 0, stream>>>(w_typed, p);
     };
     if (a.w_bf16) launch_wide(static_cast<const __nv_bfloat16*>(a.W));
     else launch_wide(static_cast<const float*>(a.W));
