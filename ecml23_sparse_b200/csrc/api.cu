@@ -72,6 +72,7 @@ int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const v
                         bool* handled);
 int forward_bf16_warps(int64_t B, int64_t N, int64_t K, bool loss_epilogue);
 int launch_transpose_pad_bf16(const void* src, void* dst, int rows, int cols, int64_t ld_dst, cudaStream_t stream);
+int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int64_t ld_dst, int esize, cudaStream_t stream);
 
 bool forward_uses_smem_x(int B, int N, int K, int* bpl_out);
 int launch_widen_bf16(const void* src, float* dst, int64_t n, cudaStream_t stream);
@@ -114,19 +115,24 @@ XPlan plan_x(bool smem_path, int64_t B, int64_t N, int x_transposed) {
     return xp;
 }
 
+// An [N,B] x whose rows already are what the padded copy would hold (a batch of whole 128-column tiles) needs no copy.
+bool padded_in_place(const XPlan& xp, const void* x, int64_t B, int x_transposed) {
+    return x_transposed && xp.ld == B && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+}
+
 int stage_x(const XPlan& xp, const float* x, float* ws, int64_t B, int64_t N, int x_transposed,
             cudaStream_t stream, const float** xT) {
     if (!xp.copy) {
         *xT = x;
         return FFI_OK;
     }
-    if (x_transposed) {
-        if (xp.ld != B) FFI_CUDA_CHECK(cudaMemsetAsync(ws, 0, static_cast<size_t>(N) * xp.ld * 4, stream));
-        FFI_CUDA_CHECK(cudaMemcpy2DAsync(ws, xp.ld * 4, x, B * 4, B * 4, N, cudaMemcpyDeviceToDevice, stream));
-    } else {
-        int rc = launch_transpose_pad(x, ws, static_cast<int>(B), static_cast<int>(N), xp.ld, stream);
-        if (rc != FFI_OK) return rc;
+    if (padded_in_place(xp, x, B, x_transposed)) {
+        *xT = x;
+        return FFI_OK;
     }
+    const int rc = x_transposed ? launch_pad_rows(x, ws, N, B, xp.ld, 4, stream)
+                                : launch_transpose_pad(x, ws, static_cast<int>(B), static_cast<int>(N), xp.ld, stream);
+    if (rc != FFI_OK) return rc;
     *xT = ws;
     return FFI_OK;
 }
@@ -171,13 +177,13 @@ int stage_x_any(const XPlan& xp, const void* x, void* ws, int64_t B, int64_t N, 
         *xT = x;
         return FFI_OK;
     }
-    if (x_transposed) {
-        if (xp.ld != B) FFI_CUDA_CHECK(cudaMemsetAsync(ws, 0, static_cast<size_t>(N) * xp.ld * esize, stream));
-        FFI_CUDA_CHECK(cudaMemcpy2DAsync(ws, xp.ld * esize, x, B * esize, B * esize, N, cudaMemcpyDeviceToDevice, stream));
-    } else {
-        const int rc = launch_transpose_pad_bf16(x, ws, static_cast<int>(B), static_cast<int>(N), xp.ld, stream);
-        if (rc != FFI_OK) return rc;
+    if (padded_in_place(xp, x, B, x_transposed)) {
+        *xT = x;
+        return FFI_OK;
     }
+    const int rc = x_transposed ? launch_pad_rows(x, ws, N, B, xp.ld, static_cast<int>(esize), stream)
+                                : launch_transpose_pad_bf16(x, ws, static_cast<int>(B), static_cast<int>(N), xp.ld, stream);
+    if (rc != FFI_OK) return rc;
     *xT = ws;
     return FFI_OK;
 }
@@ -398,7 +404,7 @@ static int backward_impl(const void* x, const int32_t* idx, const void* W, const
     if (gT_in) {
         if (ldg_in < B || ldg_in % 32 != 0 || reinterpret_cast<uintptr_t>(gT_in) % 16 != 0)
             return fail(FFI_ERR_INVALID_ARGUMENT, "gT needs a row stride that is a multiple of 32 and >= B, 16-byte aligned");
-        if (grad_bias && !fused) {  // the fused backward sums grad_bias from the g tiles it loads
+        if (grad_bias && !fused && !grad_w) {  // a grad_W kernel sums grad_bias from the rows of gT it reads anyway
             rc = launch_bias_grad_rows(gT_in, ldg_in, L, grad_bias, stream);
             if (rc != FFI_OK) return rc;
             bias_done = true;

@@ -252,7 +252,38 @@ __global__ void transpose_pad_any_kernel(const T* __restrict__ src, T* __restric
     }
 }
 
+// src [rows][cols] -> dst [rows][ld_dst], zero padded; one thread per 16 bytes of dst (ld_dst a multiple of 16 bytes)
+template <typename T>
+__global__ void pad_rows_kernel(const T* __restrict__ src, uint4* __restrict__ dst, long long rows, int cols, int vecs) {
+    constexpr int E = 16 / sizeof(T);
+    const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (id >= rows * vecs) return;
+    const long long r = id / vecs;
+    const int c0 = static_cast<int>(id - r * vecs) * E;
+    union {
+        T t[E];
+        uint4 v;
+    } u;
+#pragma unroll
+    for (int j = 0; j < E; ++j) u.t[j] = c0 + j < cols ? src[r * cols + c0 + j] : T(0);
+    dst[id] = u.v;
+}
+
 }  // namespace
+
+// x [N,B] -> [N][ld_dst], zero padded in the batch (esize 2 or 4; ld_dst a multiple of 8)
+int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int64_t ld_dst, int esize, cudaStream_t stream) {
+    const int vecs = static_cast<int>(ld_dst * esize / 16);
+    const unsigned blocks = static_cast<unsigned>(ceil_div(rows * vecs, 256));
+    if (esize == 2)
+        pad_rows_kernel<<<blocks, 256, 0, stream>>>(static_cast<const unsigned short*>(src), static_cast<uint4*>(dst), rows,
+                                                    static_cast<int>(cols), vecs);
+    else
+        pad_rows_kernel<<<blocks, 256, 0, stream>>>(static_cast<const unsigned*>(src), static_cast<uint4*>(dst), rows,
+                                                    static_cast<int>(cols), vecs);
+    FFI_LAUNCH_CHECK("pad_rows_kernel");
+    return FFI_OK;
+}
 
 // x [B,N] bf16 -> xT [N][ld_dst] bf16, zero padded
 int launch_transpose_pad_bf16(const void* src, void* dst, int rows, int cols, int64_t ld_dst, cudaStream_t stream) {
