@@ -75,6 +75,12 @@ int launch_transpose_pad_bf16(const void* src, void* dst, int rows, int cols, in
 int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int64_t ld_dst, int esize, cudaStream_t stream);
 
 bool forward_uses_smem_x(int B, int N, int K, int* bpl_out);
+bool forward_small_applicable(int64_t B, int64_t N, int64_t K);
+int launch_forward_small(const void* x, int x_transposed, const int32_t* idx, const void* W, bool bf16, const float* bias,
+                         float* y, int64_t B, int64_t N, int64_t L, int64_t K, cudaStream_t stream, bool* handled);
+size_t topk_rows_list_bytes(int64_t B, int64_t L);
+int launch_topk_rows(const float* y, int64_t B, int64_t L, uint2* lists, int kk, int label_offset, float* top_val, int* top_idx,
+                     cudaStream_t stream);
 int launch_widen_bf16(const void* src, float* dst, int64_t n, cudaStream_t stream);
 bool grad_w_uses_smem_x(int B, int N, int K, int* bpl_out);
 
@@ -234,6 +240,11 @@ extern "C" int ffi_forward(const void* x, const int32_t* idx, const void* W, con
     if (debug_bounds_enabled()) {
         rc = check_index_range(idx, L * K, N, stream);
         if (rc != FFI_OK) return rc;
+    }
+    if (dtype == FFI_F32 || dtype == FFI_BF16) {
+        bool handled = false;
+        rc = launch_forward_small(x, x_transposed, idx, W, dtype == FFI_BF16, bias, y, B, N, L, K, stream, &handled);
+        if (rc != FFI_OK || handled) return rc;
     }
     if (dtype == FFI_BF16) {
         // native bf16 kernel (x tile and W rows stay bf16 in shared memory) where the shape allows it
@@ -656,7 +667,10 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
 
 extern "C" size_t ffi_forward_topk_workspace_bytes(int64_t B, int64_t N, int64_t L, int64_t K, int x_transposed,
                                                    int dtype) {
-    return ffi_forward_workspace_bytes(B, N, L, K, x_transposed, dtype) + kAlign + align_up(forward_topk_workspace_bytes(B));
+    const size_t batched = ffi_forward_workspace_bytes(B, N, L, K, x_transposed, dtype) + kAlign + align_up(forward_topk_workspace_bytes(B));
+    if (B <= 0 || L <= 0 || !forward_small_applicable(B, N, K)) return batched;
+    const size_t small = align_up(topk_rows_list_bytes(B, L)) + static_cast<size_t>(B) * L * 4;
+    return small > batched ? small : batched;
 }
 
 extern "C" int ffi_forward_topk(const void* x, const int32_t* idx, const void* W, const float* bias, float* top_val,
@@ -677,6 +691,16 @@ extern "C" int ffi_forward_topk(const void* x, const int32_t* idx, const void* W
     if (!workspace || reinterpret_cast<uintptr_t>(workspace) % kAlign != 0 || workspace_bytes < need)
         return fail(FFI_ERR_WORKSPACE, "ffi_forward_topk needs %zu bytes of %zu-byte aligned workspace", need, kAlign);
     const bool bf16 = dtype == FFI_BF16;
+    if (k >= 1 && k <= kTopK && forward_small_applicable(B, N, K)) {
+        // a few samples: their logits fit the scratch (4*B*L bytes) and the selection reads them back from L2
+        float* y = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + align_up(topk_rows_list_bytes(B, L)));
+        bool handled = false;
+        rc = launch_forward_small(x, x_transposed, idx, W, bf16, bias, y, B, N, L, K, stream, &handled);
+        if (rc != FFI_OK) return rc;
+        if (handled)
+            return launch_topk_rows(y, B, L, static_cast<uint2*>(workspace), k, static_cast<int>(label_offset), top_val, top_idx,
+                                    stream);
+    }
     if (bf16 && !bf16_takes_tiled_forward(B, N, K)) {
         // narrow inputs in bf16 storage: widened (exactly) into the workspace, then the fp32 kernels
         const float *x32 = nullptr, *W32 = nullptr;
