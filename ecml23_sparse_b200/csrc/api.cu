@@ -357,11 +357,11 @@ static int backward_impl(const void* x, const int32_t* idx, const void* W, const
         rc = check_index_range(idx, L * K, N, static_cast<cudaStream_t>(stream_v));
         if (rc != FFI_OK) return rc;
     }
-    // bf16 storage: the group kernel (one pass, batch <= 128) and the kernels for wide inputs read bf16 x and W
+    // bf16 storage: the one-pass kernel and the kernels for wide inputs read bf16 x and W
     // themselves; for the other shapes both are widened (exactly) into the workspace and the fp32 kernels run.
     bool bf16 = false;
     if (dtype == FFI_BF16) {
-        const bool one_pass = grad_x && grad_w && plan && backward_fused_takes_bf16(plan, B);
+        const bool one_pass = grad_x && grad_w && plan && backward_fused_applicable(plan, B);
         const bool w_native = !(grad_w || grad_bias) ||
                               !grad_w_stream_applicable(static_cast<int>(B), static_cast<int>(N), static_cast<int>(K), idx);
         const bool x_native = !grad_x || (plan && !plan->has_chunks);

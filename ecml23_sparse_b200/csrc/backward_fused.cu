@@ -1,27 +1,22 @@
-// grad_x and grad_W of the fixed-fan-in sparse layer in ONE pass over the transposed index
-// (narrow inputs, batch <= 128):
+// grad_x and grad_W of the fixed-fan-in sparse layer in ONE pass over the transposed index (narrow inputs):
 //   grad_x[b,i] = sum over entries (o,k) with idx[o,k]==i of W[o,k] * g[b,o]
 //   grad_W[o,k] = sum_b g[b,o] * x[b, idx[o,k]]
 //
 // Replaces, for that case, both halves of the reference's grad functor
 // (tfsparse/cc/kernels/backward.cu:112-133: feature_grad_launch_vector_tp + the
 // weight_grad launch).  Walking the entries grouped by input i means x[:, i] is the same for a
-// whole run of entries, so it sits in registers and grad_W needs NO gather of its own: the
+// whole run of entries, so grad_W needs NO gather of its own: the
 // g[:, o] vector gathered for grad_x is multiplied by x[:, i] and reduced over the lanes.  This
 // removes the B*L*K shared-memory gathers of a separate grad_W pass.
 //
-// Structure (per CTA = range of chunks x slice of 16*NI inputs; warp = NI inputs):
-//   * grad_x accumulators and x[:, i] of the warp's inputs live in registers (NI x BPL each, as
-//     packed fp32 pairs: the axpy and the dot use the two-wide fp32 FMA of sm_100);
-//   * per chunk: the g tile comes from gT by cp.async into XOR-swizzled granules; the NEXT chunk's
-//     entries are staged meanwhile (double buffer) as (W, code) pairs, code = byte offset of the
-//     entry's g row with its swizzle key | k << 18, the weights gathered by 4-byte cp.async that
-//     complete behind the walk;
-//   * per entry: one broadcast LDS.64 (entry), one XOR for the lane's address, one gathered LDS.128
-//     (g), the FMAs, one STS of the lane's partial grad_W dot into a per-warp 16 x 32 buffer; every
-//     16 entries two lanes per entry add the buffer rows (fixed order) and store grad_W[o,k].
-// grad_x partials are flushed every few chunks and added in fp64 in a fixed order.
-// No atomics on floating-point data: results are bit-reproducible.
+// A launch covers up to 128 batch columns; larger batches run one launch per tile of 128 (grad_W of a later tile adds to
+// what the tile before stored: one addition per element and launch, in tile order).  At B=256, N=512, L=65,536, K=64
+// two launches take 0.335 ms (bf16 storage, no widening) against 0.54 + 0.02 ms of the separate kernels for grad_x and
+// grad_W.
+//
+// Structure (per CTA = range of chunks x slice of 16*ni inputs; warp = ni inputs): see the comment at
+// ffi_bwd_pairs_kernel.  grad_x partials are flushed every few chunks, one per range, and the ranges are added in fp64 in
+// a fixed order.  Results are bit-reproducible.
 #include <cuda.h>
 
 #include <type_traits>
@@ -37,7 +32,6 @@ __device__ long long g_wait_limit = 4000000000ll;  // clock64 ticks a wait may l
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kSlots = 16;            // entries buffered per warp before the lane reduction
 constexpr int kDRow = 36;             // row stride of the per-warp dot buffer: 16-byte rows, conflict-free
 constexpr int kStageUnroll = 4;       // staged entries per thread kept in flight
 constexpr int kKShift = 18;           // entry code = byte offset of the g row (with its swizzle key) | k << 18
@@ -63,62 +57,6 @@ __device__ __forceinline__ u64 mul2(u64 a, u64 b) {
     return d;
 }
 
-// The BPL batch elements one lane holds of a vector over the batch (a g row, x[:, i], a grad_x sum).
-template <int BPL>
-struct LaneVec;
-template <>
-struct LaneVec<4> {
-    u64 a, b;
-    __device__ __forceinline__ void zero() { a = b = 0ull; }
-    __device__ __forceinline__ void set(const float* v) { a = pack2(v[0], v[1]), b = pack2(v[2], v[3]); }
-    __device__ __forceinline__ void get(float* v) const { unpack2(a, v[0], v[1]), unpack2(b, v[2], v[3]); }
-    __device__ __forceinline__ void load_shared(const unsigned char* ptr) {
-        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(ptr);
-        a = t.x, b = t.y;
-    }
-    // this += w * g
-    __device__ __forceinline__ void axpy(float w, const LaneVec& g) {
-        const u64 ww = pack2(w, w);
-        a = fma2(ww, g.a, a), b = fma2(ww, g.b, b);
-    }
-    __device__ __forceinline__ float dot(const LaneVec& g) const {
-        float lo, hi;
-        unpack2(fma2(g.b, b, mul2(g.a, a)), lo, hi);
-        return lo + hi;
-    }
-};
-template <>
-struct LaneVec<2> {
-    u64 a;
-    __device__ __forceinline__ void zero() { a = 0ull; }
-    __device__ __forceinline__ void set(const float* v) { a = pack2(v[0], v[1]); }
-    __device__ __forceinline__ void get(float* v) const { unpack2(a, v[0], v[1]); }
-    __device__ __forceinline__ void load_shared(const unsigned char* ptr) { a = *reinterpret_cast<const u64*>(ptr); }
-    __device__ __forceinline__ void axpy(float w, const LaneVec& g) { a = fma2(pack2(w, w), g.a, a); }
-    __device__ __forceinline__ float dot(const LaneVec& g) const {
-        float lo, hi;
-        unpack2(mul2(g.a, a), lo, hi);
-        return lo + hi;
-    }
-};
-template <>
-struct LaneVec<1> {
-    float a;
-    __device__ __forceinline__ void zero() { a = 0.f; }
-    __device__ __forceinline__ void set(const float* v) { a = v[0]; }
-    __device__ __forceinline__ void get(float* v) const { v[0] = a; }
-    __device__ __forceinline__ void load_shared(const unsigned char* ptr) { a = *reinterpret_cast<const float*>(ptr); }
-    __device__ __forceinline__ void axpy(float w, const LaneVec& g) { a = fmaf(w, g.a, a); }
-    __device__ __forceinline__ float dot(const LaneVec& g) const { return g.a * a; }
-};
-
-template <int BPL>
-__device__ __forceinline__ void store_zero_vec(float* dst) {
-    if constexpr (BPL == 4) *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-    else if constexpr (BPL == 2) *reinterpret_cast<float2*>(dst) = make_float2(0.f, 0.f);
-    else *dst = 0.f;
-}
-
 struct BwdFusedParams {
     const void* W;   // fp32; the group kernel also takes bf16 (its TX)
     const float* gT;
@@ -127,7 +65,7 @@ struct BwdFusedParams {
     long long ldx;
     const int* cperm;
     const int* cptr;
-    float* partial;  // [R*S][N][Bpad]
+    float* partial;  // [R][N][Bpad]
     float* gW;
     float* gbias;  // pair kernel only: grad_bias[o] = sum_b gT[o][b], from the g tiles it holds anyway
     int B, N, L, K;
@@ -138,232 +76,11 @@ struct BwdFusedParams {
     int Bpad;
     int entCap;
     int segChunks;  // chunks per flushed partial
-    int S;          // partial slots per range
+    int ni;         // inputs per warp
 };
 
-template <int NI, int BPL>
-__global__ void __launch_bounds__(kThreads, 1) ffi_bwd_fused_kernel(BwdFusedParams p) {
-    constexpr int BT = 32 * BPL;
-    constexpr int GR = BPL;
-    constexpr int SW = 32 / GR - 1;
-    constexpr int CPN = kWarps * NI + 1;
-    constexpr unsigned kRowMask = (1u << kKShift) - 1u;
-    using LV = LaneVec<BPL>;
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-
-    const int T = p.T, K = p.K, L = p.L, N = p.N;
-    float* g_s = reinterpret_cast<float*>(smem_raw);                                    // [T][BT] swizzled
-    uint2* ent_s = reinterpret_cast<uint2*>(g_s + static_cast<size_t>(T) * BT);         // [2][entCap]
-    float* dbuf_s = reinterpret_cast<float*>(ent_s + 2 * p.entCap);                     // [warps][kSlots][kDRow]
-    int* cp_s = reinterpret_cast<int*>(dbuf_s + kWarps * kSlots * kDRow);               // [2][CPN]
-
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int warp = tid >> 5;
-    const int r = blockIdx.x;
-    const int i_lo = blockIdx.y * (kWarps * NI);
-    const int i_hi = min(N, i_lo + kWarps * NI);
-    const long long c_begin = p.nChunks * r / p.R;
-    const long long c_end = p.nChunks * (r + 1) / p.R;
-
-    LV acc[NI], xr[NI];
-#pragma unroll
-    for (int j = 0; j < NI; ++j) {
-        const int i = i_lo + warp * NI + j;
-        float xv[BPL];
-#pragma unroll
-        for (int q = 0; q < BPL; ++q) {
-            const int b = lane * BPL + q;
-            xv[q] = (i < N && b < p.B) ? __ldg(static_cast<const float*>(p.xT) + static_cast<size_t>(i) * p.ldx + b) : 0.f;
-        }
-        acc[j].zero();
-        xr[j].set(xv);
-    }
-
-    // First entry and entry count of the slice in a chunk (two words of the plan's offset table);
-    // fetched one chunk ahead of the staging that needs them.
-    auto slice_bounds = [&](long long c, int& e_lo, int& cnt) {
-        const int* cptr_c = p.cptr + c * (N + 1);
-        e_lo = __ldg(cptr_c + i_lo);
-        cnt = __ldg(cptr_c + i_hi) - e_lo;
-    };
-
-    // Entries (W, code) and run offsets of the slice in chunk c -> buffer buf.  The codes are stored
-    // at once; the weights are gathered by 4-byte cp.async straight into the entries, so that their
-    // latency runs behind whatever the caller does next (the caller commits and waits).
-    // (The plan guarantees that a slice never holds more than entCap entries.)
-    auto stage = [&](long long c, int buf, int e_lo, int cnt) {
-        const int* cptr_c = p.cptr + c * (N + 1);
-        for (int t = tid; t < CPN; t += kThreads) cp_s[buf * CPN + t] = __ldg(cptr_c + min(i_lo + t, i_hi)) - e_lo;
-        const int* cperm_c = p.cperm + c * static_cast<long long>(T) * K + e_lo;
-        const int pos0 = static_cast<int>(c * T) * K;  // flat position of the chunk's first row
-        uint2* dst = ent_s + buf * p.entCap;
-        for (int e0 = tid; e0 < cnt; e0 += kThreads * kStageUnroll) {
-            int pos[kStageUnroll];
-#pragma unroll
-            for (int u = 0; u < kStageUnroll; ++u) {
-                const int e = e0 + u * kThreads;
-                pos[u] = e < cnt ? __ldg(cperm_c + e) : -1;
-            }
-#pragma unroll
-            for (int u = 0; u < kStageUnroll; ++u) {
-                if (pos[u] >= 0) {
-                    uint2* d = dst + e0 + u * kThreads;
-                    __pipeline_memcpy_async(&d->x, static_cast<const float*>(p.W) + pos[u], 4);
-                    const int rel = pos[u] - pos0;
-                    const int ol = p.kShift >= 0 ? (rel >> p.kShift) : rel / K;
-                    const int k = rel - ol * K;
-                    d->y = static_cast<unsigned>(ol * (BT * 4) + (ol & SW) * (GR * 4)) |
-                           (static_cast<unsigned>(k) << kKShift);
-                }
-            }
-        }
-    };
-
-    int nb_lo = 0, nb_cnt = 0;  // bounds of the chunk to be staged next
-    if (c_begin < c_end) {
-        slice_bounds(c_begin, nb_lo, nb_cnt);
-        stage(c_begin, 0, nb_lo, nb_cnt);
-        if (c_begin + 1 < c_end) slice_bounds(c_begin + 1, nb_lo, nb_cnt);
-    }
-    __pipeline_commit();
-    __pipeline_wait_prior(0);
-    float* dbuf = dbuf_s + warp * (kSlots * kDRow);
-    // address of this lane's granule of row `code & kRowMask`: one XOR with the lane's byte offset
-    const unsigned char* gs_bytes = reinterpret_cast<const unsigned char*>(g_s);
-    const unsigned laneOff = static_cast<unsigned>(lane) * (GR * 4);
-
-    for (long long c = c_begin; c < c_end; ++c) {
-        const int buf = static_cast<int>(c - c_begin) & 1;
-        const long long o0 = c * T;
-        const int nrows = static_cast<int>(min(static_cast<long long>(T), static_cast<long long>(L) - o0));
-        __syncthreads();  // previous chunk's walk is done; buffer `buf` is staged
-
-        {
-            // thread = (granule gl of a row, rows warp, warp + 16, ...)
-            const int gl = lane;
-            const float* src = p.gT + static_cast<size_t>(o0 + warp) * p.ldg + gl * GR;
-            const size_t srcStep = static_cast<size_t>(kWarps) * p.ldg;
-#pragma unroll 4
-            for (int ol = warp; ol < T; ol += kWarps, src += srcStep) {
-                float* dst = g_s + ol * BT + ((gl ^ (ol & SW)) * GR);
-                if (ol < nrows) __pipeline_memcpy_async(dst, src, 4 * GR);
-                else store_zero_vec<BPL>(dst);
-            }
-        }
-        __pipeline_commit();
-        if (c + 1 < c_end) {  // its index loads overlap the tile copy, its weight gathers the walk
-            stage(c + 1, buf ^ 1, nb_lo, nb_cnt);
-            if (c + 2 < c_end) slice_bounds(c + 2, nb_lo, nb_cnt);
-        }
-        __pipeline_commit();
-        __pipeline_wait_prior(1);  // the tile has landed; the staged weights may still be in flight
-        __syncthreads();
-
-
-        // ---- walk the runs of this warp's inputs -------------------------------------------
-        const uint2* ent = ent_s + buf * p.entCap;
-        const int* cp = cp_s + buf * CPN + warp * NI;
-        int slot = 0;
-        int eblk = cp[0];  // entry held by slot 0 of the dot buffer
-
-        // Adds the buffered per-lane dots of `n` entries (two lanes per entry, fixed order) and stores
-        // grad_W[o,k] of those entries.
-        auto reduce_slots = [&](int n) {
-            __syncwarp();
-            const int sl = lane >> 1, h = lane & 1;
-            const float4* row = reinterpret_cast<const float4*>(dbuf + sl * kDRow + h * 16);
-            const float4 q0 = row[0], q1 = row[1], q2 = row[2], q3 = row[3];
-            float sum = (((q0.x + q0.y) + (q0.z + q0.w)) + ((q1.x + q1.y) + (q1.z + q1.w))) +
-                        (((q2.x + q2.y) + (q2.z + q2.w)) + ((q3.x + q3.y) + (q3.z + q3.w)));
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            if (h == 0 && sl < n && p.gW) {
-                const unsigned code = ent[eblk + sl].y;
-                const unsigned ol = (code & kRowMask) / (BT * 4);
-                p.gW[(static_cast<size_t>(o0) + ol) * K + (code >> kKShift)] = sum;
-            }
-            __syncwarp();
-        };
-
-#pragma unroll
-        for (int j = 0; j < NI; ++j) {
-            const int t = cp[j + 1];
-            int e = cp[j];
-            // groups of four entries: all loads of a group are issued before its stores (the
-            // compiler cannot move loads across the shared-memory stores by itself)
-            for (; e + 4 <= t; e += 4) {
-                uint2 en[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) en[u] = ent[e + u];
-                if (slot + 4 > kSlots) {
-                    reduce_slots(slot);
-                    eblk = e;
-                    slot = 0;
-                }
-                LV v[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) v[u].load_shared(gs_bytes + ((en[u].y & kRowMask) ^ laneOff));
-                float* drow = dbuf + slot * kDRow + lane;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    acc[j].axpy(__uint_as_float(en[u].x), v[u]);
-                    drow[u * kDRow] = xr[j].dot(v[u]);
-                }
-                slot += 4;
-            }
-            for (; e < t; ++e) {
-                if (slot == kSlots) {
-                    reduce_slots(slot);
-                    eblk = e;
-                    slot = 0;
-                }
-                const uint2 en = ent[e];
-                LV v;
-                v.load_shared(gs_bytes + ((en.y & kRowMask) ^ laneOff));
-                acc[j].axpy(__uint_as_float(en.x), v);
-                dbuf[slot * kDRow + lane] = xr[j].dot(v);
-                ++slot;
-            }
-        }
-        if (slot > 0) reduce_slots(slot);
-
-        __pipeline_wait_prior(0);  // this thread's staged weights of the next chunk are in place
-
-        // Every segChunks chunks the running grad_x sums go out as one partial and restart from zero.
-        const long long done = c - c_begin + 1;
-        if (done % p.segChunks == 0 || c + 1 == c_end) {
-            const int seg = static_cast<int>((done - 1) / p.segChunks);
-#pragma unroll
-            for (int j = 0; j < NI; ++j) {
-                const int i = i_lo + warp * NI + j;
-                if (i < N) {
-                    float* dst = p.partial + ((static_cast<size_t>(r) * p.S + seg) * N + i) * p.Bpad + lane * BPL;
-                    float out[BPL];
-                    acc[j].get(out);
-#pragma unroll
-                    for (int q = 0; q < BPL; ++q) dst[q] = out[q];
-                    acc[j].zero();
-                }
-            }
-        }
-    }
-
-    // Segments a range never reached hold zeros (ranges differ by at most one chunk).
-    for (int seg = static_cast<int>((c_end - c_begin + p.segChunks - 1) / p.segChunks); seg < p.S; ++seg) {
-#pragma unroll
-        for (int j = 0; j < NI; ++j) {
-            const int i = i_lo + warp * NI + j;
-            if (i < N) {
-                float* dst = p.partial + ((static_cast<size_t>(r) * p.S + seg) * N + i) * p.Bpad + lane * BPL;
-#pragma unroll
-                for (int q = 0; q < BPL; ++q) dst[q] = 0.f;
-            }
-        }
-    }
-}
-
 // =====================================================================================
-// Batch 65..128: two entries per warp step, accumulators and x parked in tensor memory.
+// Two entries per warp step, accumulators and x parked in tensor memory (shown for 65..128 batch columns).
 //
 // A half warp covers the 128 batch columns of one entry (lane q of a half holds columns 4q..4q+3
 // and 64+4q..64+4q+3: two LDS.128, conflict-free without any swizzle), so the two halves of a
@@ -603,13 +320,16 @@ struct LaneOf<4> {
 // With VPL = 4 an input's state is 8 TMEM columns instead of 16, so a warp owns 16 inputs, a CTA 256, and three
 // slices per range instead of six fetch each g tile.
 //
+// FULL: all NI inputs of a warp are in use (a run-time count costs 1 to 2 %: 940 -> 951 us at the headline shape).
+// ACC: a batch tile after the first (as a run-time flag it cost 5 %), whose grad_W and grad_bias add to what the tiles
+// before stored.
 // TX is the storage type of x and W.  bf16 x is widened (exactly) on its way into tensor memory.  A bf16
 // weight is fetched as the aligned 4-byte word that holds it (cp.async copies at least 4 bytes) and turned
 // into its fp32 bit pattern by the thread that fetched it once the copy has landed (the entry's code tells
 // which half: the chunk's first position is even, so the parity of the position within the chunk is the
 // parity of the flat position).
 //
-template <int NI, int THREADS, int SLOTS, int G, typename TX, int VPL = 8>
+template <int NI, int THREADS, int SLOTS, int G, typename TX, int VPL, bool ACC, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
     ffi_bwd_pairs_kernel(BwdFusedParams p, const __grid_constant__ CUtensorMap g_map) {
     constexpr bool kBf16 = !std::is_same<TX, float>::value;
@@ -619,8 +339,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     constexpr int BT = VPL * LG;  // batch columns of the tile
     constexpr int HALF = 2 * BT;  // bytes between a lane's two 16-byte pieces of a tile row (VPL = 8)
     constexpr int COLS = 2 * VPL; // TMEM columns of one input: its sums and its x values
-    constexpr int kThreads = THREADS, kWarps = THREADS / 32, kSlots = SLOTS;  // shadow the file-wide values
-    constexpr int CPN = kWarps * NI + 1;
+    constexpr int kThreads = THREADS, kWarps = THREADS / 32, kSlots = SLOTS;
+    const int ni = FULL ? NI : p.ni;  // inputs per warp: the slices of a range split the inputs evenly
+    const int CPN = kWarps * ni + 1;
     constexpr unsigned kRowMask = (1u << kKShift) - 1u;
     static_assert((THREADS / 128) * NI * COLS <= kTmemCols, "the warps of a lane quarter share the TMEM columns");
     static_assert(SLOTS * G == 32, "the lane reduction maps the 32 lanes to (buffered step, group)");
@@ -641,8 +362,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int grp = lane / LG;  // which entry of a step this lane works on
     const int q = lane % LG;
     const int r = blockIdx.x;
-    const int i_lo = blockIdx.y * (kWarps * NI);
-    const int i_hi = min(N, i_lo + kWarps * NI);
+    const int i_lo = blockIdx.y * (kWarps * ni);
+    const int i_hi = min(N, i_lo + kWarps * ni);
     const long long c_begin = p.nChunks * r / p.R;
     const long long c_end = p.nChunks * (r + 1) / p.R;
 
@@ -657,8 +378,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                             static_cast<unsigned>(warp >> 2) * (NI * COLS);
 
     if constexpr (VPL == 8) {
-        for (int j = 0; j < NI; ++j) {
-            const int i = i_lo + warp * NI + j;
+        for (int j = 0; j < ni; ++j) {
+            const int i = i_lo + warp * ni + j;
             unsigned xv[8], zero[8];
     #pragma unroll
             for (int m = 0; m < 8; ++m) {
@@ -670,8 +391,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             tmem_store8(taddr0 + j * 16 + 8, xv);
         }
     } else {
-        for (int j = 0; j < NI; ++j) {
-            const int i = i_lo + warp * NI + j;
+        for (int j = 0; j < ni; ++j) {
+            const int i = i_lo + warp * ni + j;
             unsigned xv[VPL], zero[VPL];
     #pragma unroll
             for (int m = 0; m < VPL; ++m) {
@@ -811,13 +532,13 @@ __global__ void __launch_bounds__(THREADS, 1)
                 float sum = v.sum();
 #pragma unroll
                 for (int off = LG / 2; off >= 1; off /= 2) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-                if (q == 0 && o0 + rr < p.L) p.gbias[o0 + rr] = sum;
+                if (q == 0 && o0 + rr < p.L) p.gbias[o0 + rr] = ACC ? p.gbias[o0 + rr] + sum : sum;
             }
         }
 
         // ---- walk the runs of this warp's inputs, G entries per step ---------------------------
         const uint2* ent = ent_s + buf * p.entCap + grp;  // this group's entry of a step
-        const int* cp = cp_s + buf * CPN + warp * NI;
+        const int* cp = cp_s + buf * CPN + warp * ni;
         float* gWc = p.gW ? p.gW + static_cast<size_t>(o0) * K : nullptr;
         // Row of the dot buffer the next step fills: 32 per-lane dots, then the codes of its G entries.
         // dptr points at this lane's column of that row; the code of the lane's entry goes to
@@ -839,14 +560,18 @@ __global__ void __launch_bounds__(THREADS, 1)
                 sum = ((q0.x + q0.y) + (q0.z + q0.w)) + ((q1.x + q1.y) + (q1.z + q1.w));
             }
             const unsigned code = *dmine;
-            if (myrow < rows && code != kPadCode && gWc) gWc[code >> kKShift] = sum;
+            if (myrow < rows && code != kPadCode && gWc) {
+                // batch tiles after the first add to what the tile before stored: one addition per element and launch
+                if (ACC) atomicAdd(gWc + (code >> kKShift), sum);
+                else gWc[code >> kKShift] = sum;
+            }
             __syncwarp();
             dptr = dlane;
         };
 
         int e = cp[0];
 #pragma unroll 1
-        for (int j = 0; j < NI; ++j) {
+        for (int j = 0; j < ni; ++j) {
             const int t = cp[j + 1];
             if (e >= t) continue;
             LaneT acc, xr;
@@ -905,8 +630,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (done % p.segChunks == 0 || c + 1 == c_end) {
             const int seg = static_cast<int>((done - 1) / p.segChunks);
             if constexpr (VPL == 8) {
-                for (int j = 0; j < NI; ++j) {
-                    const int i = i_lo + warp * NI + j;
+                for (int j = 0; j < ni; ++j) {
+                    const int i = i_lo + warp * ni + j;
                     unsigned av[8], zero[8];
                     tmem_load8(taddr0 + j * 16, av);
     #pragma unroll
@@ -936,8 +661,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                 }
             } else {
-                for (int j = 0; j < NI; ++j) {
-                    const int i = i_lo + warp * NI + j;
+                for (int j = 0; j < ni; ++j) {
+                    const int i = i_lo + warp * ni + j;
                     unsigned av[VPL], zero[VPL];
     #pragma unroll
                     for (int m = 0; m < VPL; ++m) zero[m] = 0u;
@@ -973,8 +698,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     // A range without chunks still owns a partial: zeros.
     if (c_begin >= c_end) {
-        for (int j = 0; j < NI; ++j) {
-            const int i = i_lo + warp * NI + j;
+        for (int j = 0; j < ni; ++j) {
+            const int i = i_lo + warp * ni + j;
             if (i < N && grp == 0) {
                 float* dst = p.partial + (static_cast<size_t>(r) * N + i) * p.Bpad + 4 * q;
                 *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -992,27 +717,25 @@ __global__ void __launch_bounds__(THREADS, 1)
 }
 
 struct FusedConfig {
-    int bpl, ni, iparts, Bpad, R, entCap, segChunks, S;
-    int groups;  // lane groups per warp of the group kernel (2: batch 33..128, 4: batch <= 32), 0: ffi_bwd_fused_kernel
-    int vpl;     // batch elements per lane of the group kernel: 8 (batch 65..128) or 4
+    int ni, iparts, Bpad, R, entCap, segChunks;
+    int groups;  // lane groups per warp (2: batch 33..128, 4: batch <= 32)
+    int vpl;     // batch elements per lane: 8 (batch 65..128) or 4
     size_t smem;
 };
 
-constexpr int kGroupThreads = 512, kGroupNI = 8;  // (1024 threads x 4 inputs was measured: 10 % slower)
+constexpr int kGroupThreads = 512;  // (1024 threads x 4 inputs was measured: 10 % slower)
 
+// For one tile of at most 128 batch columns.
 bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedConfig* c) {
     if (!plan || !plan->has_chunks || B > 128) return false;
-    if (plan->K >= (1 << (32 - kKShift))) return false;  // k shares the entry's code word with the row offset
-    // the group kernel's entry code holds the position within the chunk in 14 bits
-    const bool group_kernel = static_cast<long long>(plan->chunk_rows) * plan->K <= (1 << (32 - kKShift));
-    c->groups = group_kernel ? (B > 32 ? 2 : 4) : 0;
-    c->vpl = group_kernel && B <= 64 ? 4 : 8;
-    c->bpl = group_kernel ? (B > 64 ? 4 : 2) : (B <= 32 ? 1 : (B <= 64 ? 2 : 4));
-    // ffi_bwd_fused_kernel: 32 accumulator + 32 x registers per lane; the group kernel: 512 TMEM columns per lane quarter
-    c->ni = group_kernel ? (c->vpl == 4 ? 2 * kGroupNI : kGroupNI) : 32 / c->bpl;
-    const int BT = group_kernel ? c->vpl * (32 / c->groups) : 32 * c->bpl;
-    const int width = kWarps * c->ni;  // inputs per slice: 128, 256 or 512
-    c->iparts = static_cast<int>(ceil_div(plan->N, width));
+    // the entry code holds the position within the chunk in 14 bits
+    if (static_cast<long long>(plan->chunk_rows) * plan->K > (1 << (32 - kKShift))) return false;
+    c->groups = B > 32 ? 2 : 4;
+    c->vpl = B <= 64 ? 4 : 8;
+    const int BT = c->vpl * (32 / c->groups);
+    const FusedSlices sl = fused_slices(plan->N, c->vpl == 4);
+    c->ni = sl.ni;
+    c->iparts = sl.parts;
     c->Bpad = BT;
     int R = dev.sm_count / c->iparts;
     if (R < 1) R = 1;
@@ -1023,24 +746,23 @@ bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedC
     int seg = static_cast<int>(256.0 / (per_chunk > 1.0 ? per_chunk : 1.0));
     if (seg < 1) seg = 1;
     c->segChunks = seg;
-    // the group kernel adds its segments into one partial per range; the register kernel keeps one per segment
-    c->S = group_kernel ? 1 : static_cast<int>(ceil_div(ceil_div(plan->n_chunks, R), seg));
-    const int stat = width <= 128 ? 0 : (width <= 256 ? 1 : 2);
-    const size_t cap = static_cast<size_t>((plan->max_slice_entries[stat] + 7) / 8 * 8 + 8);
+    const size_t cap = static_cast<size_t>((plan->max_slice_entries[c->vpl == 4] + 7) / 8 * 8 + 8);
     const size_t T = static_cast<size_t>(plan->chunk_rows);
     if (T * BT * 4 > (size_t{1} << kKShift)) return false;
-    // the group kernel buffers 32 / groups steps per warp; + its barrier, TMEM slot and alignment slack
-    const size_t slots = group_kernel ? 32 / c->groups : kSlots;
-    const size_t total = T * BT * 4 + 2 * cap * 8 + static_cast<size_t>(kWarps) * slots * kDRow * 4 +
-                         2 * (kWarps * c->ni + 1) * 4 + 16 + (group_kernel ? 1024 : 0);
+    // a warp buffers 32 / groups steps; + the barrier, the TMEM slot and alignment slack
+    const size_t total = T * BT * 4 + 2 * cap * 8 + static_cast<size_t>(kWarps) * (32 / c->groups) * kDRow * 4 +
+                         2 * (kWarps * c->ni + 1) * 4 + 16 + 1024;
     if (total > static_cast<size_t>(dev.max_smem_optin)) return false;  // unusually dense slice or large K: separate kernels
     c->entCap = static_cast<int>(cap);
     c->smem = total;
     return true;
 }
 
+// Columns of the batch tile that starts at b0.
+int64_t tile_columns(int64_t B, int64_t b0) { return B - b0 < 128 ? B - b0 : 128; }
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (the library does not link libcuda).
-int encode_g_map(CUtensorMap* map, const float* gT, int64_t L, int64_t ldg, int chunk_rows, int BT) {
+int encode_g_map(CUtensorMap* map, const float* gT, int64_t L, int64_t ldg, int64_t cols, int chunk_rows, int BT) {
     using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1056,7 +778,7 @@ int encode_g_map(CUtensorMap* map, const float* gT, int64_t L, int64_t ldg, int 
         return fail(FFI_ERR_INVALID_ARGUMENT, "transposed gradient must be 16-byte aligned, chunks at most 256 rows");
     // the stored rows may be narrower than the tile (batch <= 32 keeps 32 columns): the box's columns past them
     // are filled with zeros, like its rows past L
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(ldg < BT ? ldg : BT), static_cast<cuuint64_t>(L)};
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols < BT ? cols : BT), static_cast<cuuint64_t>(L)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ldg) * 4};
     const cuuint32_t box[2] = {static_cast<cuuint32_t>(BT), static_cast<cuuint32_t>(chunk_rows)};
     const cuuint32_t elem[2] = {1, 1};
@@ -1067,72 +789,53 @@ int encode_g_map(CUtensorMap* map, const float* gT, int64_t L, int64_t ldg, int 
     return FFI_OK;
 }
 
-template <int NI, int BPL>
-int launch_fused_t(const BwdFusedParams& p, const FusedConfig& c, cudaStream_t stream) {
-    auto kern = ffi_bwd_fused_kernel<NI, BPL>;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(c.smem)));
-    dim3 grid(static_cast<unsigned>(c.R), static_cast<unsigned>(c.iparts), 1);
-    kern<<<grid, kThreads, c.smem, stream>>>(p);
-    FFI_LAUNCH_CHECK("ffi_bwd_fused_kernel");
-    return FFI_OK;
-}
-
 }  // namespace
 
 bool backward_fused_applicable(const ffi_plan* plan, int64_t B) {
     DeviceInfo dev;
     if (get_device_info(&dev) != FFI_OK) return false;
     FusedConfig c;
-    return fused_config(plan, B, dev, &c);
-}
-
-// True when the one-pass backward of this shape is the group kernel, which also reads bf16 x and W.
-bool backward_fused_takes_bf16(const ffi_plan* plan, int64_t B) {
-    DeviceInfo dev;
-    if (get_device_info(&dev) != FFI_OK) return false;
-    FusedConfig c;
-    return fused_config(plan, B, dev, &c) && c.groups != 0;
+    const int64_t first = tile_columns(B, 0), last = B - (B - 1) / 128 * 128;
+    return fused_config(plan, first, dev, &c) && fused_config(plan, last, dev, &c);
 }
 
 size_t backward_fused_workspace_bytes(const ffi_plan* plan, int64_t B) {
     DeviceInfo dev;
     if (get_device_info(&dev) != FFI_OK) return 0;
-    FusedConfig c;
-    if (!fused_config(plan, B, dev, &c)) return 0;
-    return static_cast<size_t>(c.R) * c.S * plan->N * c.Bpad * 4;
+    size_t most = 0;
+    for (int64_t cols : {tile_columns(B, 0), B - (B - 1) / 128 * 128}) {
+        FusedConfig c;
+        if (!fused_config(plan, cols, dev, &c)) return 0;
+        const size_t need = static_cast<size_t>(c.R) * plan->N * c.Bpad * 4;
+        if (need > most) most = need;
+    }
+    return most;
 }
 
-int reduce_range_partials(const float* partial, float* gx, int R, int N, int B, int Bpad, int x_transposed,
+int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int B, int x_transposed,
                           cudaStream_t stream);
 
-// grad_x (always), grad_W (when gW != nullptr) and grad_bias (when gbias != nullptr, from gT) in one
-// kernel (grad_bias by a separate pass over gT where the pair kernel does not apply).  xT is x as [N][ldx].
+// grad_x (always), grad_W (when gW != nullptr) and grad_bias (when gbias != nullptr, from gT).  xT is x as [N][ldx].
 int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float* gW, float* gbias,
                           cudaStream_t stream) {
     DeviceInfo dev;
     int rc = get_device_info(&dev);
     if (rc != FFI_OK) return rc;
-    FusedConfig c;
-    if (!fused_config(a.plan, a.B, dev, &c)) return fail(FFI_ERR_UNSUPPORTED, "fused backward does not cover this shape");
-    const size_t need = static_cast<size_t>(c.R) * c.S * a.N * c.Bpad * 4;
+    const size_t need = backward_fused_workspace_bytes(a.plan, a.B);
     if (!a.workspace || a.workspace_bytes < need || reinterpret_cast<uintptr_t>(a.workspace) % 16 != 0)
         return fail(FFI_ERR_WORKSPACE, "fused backward needs %zu bytes of 16-byte aligned workspace", need);
-    // the group kernel's tile copy fills the columns past a narrower stored row with zeros
-    const int64_t min_ldg = c.groups ? round_up(a.B, 32) : c.Bpad;
-    if (!a.gT || a.ldg < min_ldg || a.ldg % 32 != 0 || !xT)
+    // the tile copy fills the columns past a narrower stored row with zeros
+    if (!a.gT || a.ldg < round_up(a.B, 32) || a.ldg % 32 != 0 || !xT)
         return fail(FFI_ERR_INVALID_ARGUMENT, "fused backward needs gT and xT");
     BwdFusedParams p;
     p.W = a.W;
-    p.gT = a.gT;
     p.ldg = a.ldg;
-    p.xT = xT;
     p.ldx = ldx;
     p.cperm = a.plan->cperm;
     p.cptr = a.plan->cptr;
     p.partial = static_cast<float*>(a.workspace);
     p.gW = gW;
-    p.gbias = nullptr;
-    p.B = a.B;
+    p.gbias = gbias;
     p.N = a.N;
     p.L = a.L;
     p.K = a.K;
@@ -1141,22 +844,21 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         if ((1 << sh) == a.K) p.kShift = sh;
     p.T = a.plan->chunk_rows;
     p.nChunks = a.plan->n_chunks;
-    p.R = c.R;
-    p.Bpad = c.Bpad;
-    p.entCap = c.entCap;
-    p.segChunks = c.segChunks;
-    p.S = c.S;
-    const bool pairs = c.groups != 0;
-    if (a.w_bf16 && !pairs) return fail(FFI_ERR_UNSUPPORTED, "this fused backward kernel reads fp32 x and W");
-    if (gbias && !pairs) {  // the other kernels leave grad_bias to a pass over gT
-        rc = launch_bias_grad_rows(a.gT, a.ldg, a.L, gbias, stream);
-        if (rc != FFI_OK) return rc;
-    }
-    if (pairs) {
-        p.gbias = gbias;
+    for (int64_t b0 = 0; b0 < a.B; b0 += 128) {
+        const int cols = static_cast<int>(tile_columns(a.B, b0));
+        FusedConfig c;
+        if (!fused_config(a.plan, cols, dev, &c)) return fail(FFI_ERR_UNSUPPORTED, "fused backward does not cover this shape");
+        p.gT = a.gT + b0;
+        p.xT = static_cast<const unsigned char*>(xT) + b0 * (a.w_bf16 ? 2 : 4);
+        p.B = cols;
+        p.R = c.R;
+        p.Bpad = c.Bpad;
+        p.entCap = c.entCap;
+        p.segChunks = c.segChunks;
+        p.ni = c.ni;
         // gT as a 2-D tensor [L rows][BT columns] with row pitch ldg; one box = the g tile of a chunk
         CUtensorMap g_map;
-        rc = encode_g_map(&g_map, a.gT, a.L, a.ldg, a.plan->chunk_rows, c.Bpad);
+        rc = encode_g_map(&g_map, p.gT, a.L, a.ldg, a.ldg - b0, a.plan->chunk_rows, c.Bpad);
         if (rc != FFI_OK) return rc;
         dim3 grid(static_cast<unsigned>(c.R), static_cast<unsigned>(c.iparts), 1);
         auto launch_group = [&](auto kern) -> int {
@@ -1164,21 +866,28 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
             kern<<<grid, kGroupThreads, c.smem, stream>>>(p, g_map);
             return FFI_OK;
         };
-        if (c.groups == 2 && c.vpl == 8 && !a.w_bf16) rc = launch_group(ffi_bwd_pairs_kernel<kGroupNI, kGroupThreads, 16, 2, float>);
-        else if (c.groups == 2 && c.vpl == 8) rc = launch_group(ffi_bwd_pairs_kernel<kGroupNI, kGroupThreads, 16, 2, __nv_bfloat16>);
-        else if (c.groups == 2 && c.vpl == 4 && !a.w_bf16) rc = launch_group(ffi_bwd_pairs_kernel<2 * kGroupNI, kGroupThreads, 16, 2, float, 4>);
-        else if (c.groups == 2 && c.vpl == 4) rc = launch_group(ffi_bwd_pairs_kernel<2 * kGroupNI, kGroupThreads, 16, 2, __nv_bfloat16, 4>);
-        else if (!a.w_bf16) rc = launch_group(ffi_bwd_pairs_kernel<2 * kGroupNI, kGroupThreads, 8, 4, float, 4>);
-        else rc = launch_group(ffi_bwd_pairs_kernel<2 * kGroupNI, kGroupThreads, 8, 4, __nv_bfloat16, 4>);
+        auto launch_typed = [&](auto tx, auto acc) -> int {
+            using TX = decltype(tx);
+            constexpr bool ACC = decltype(acc)::value;
+            constexpr int NI8 = kFusedNI, NI4 = 2 * kFusedNI, TH = kGroupThreads;
+            if (!ACC && c.ni == (c.vpl == 8 ? NI8 : NI4)) {
+                if (c.vpl == 8) return launch_group(ffi_bwd_pairs_kernel<NI8, TH, 16, 2, TX, 8, false, true>);
+                if (c.groups == 2) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 16, 2, TX, 4, false, true>);
+                return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 8, 4, TX, 4, false, true>);
+            }
+            if (c.vpl == 8) return launch_group(ffi_bwd_pairs_kernel<NI8, TH, 16, 2, TX, 8, ACC, false>);
+            if (c.groups == 2) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 16, 2, TX, 4, ACC, false>);
+            return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 8, 4, TX, 4, ACC, false>);
+        };
+        auto launch_tile = [&](auto acc) { return a.w_bf16 ? launch_typed(__nv_bfloat16{}, acc) : launch_typed(float{}, acc); };
+        rc = b0 > 0 ? launch_tile(std::true_type{}) : launch_tile(std::false_type{});
         if (rc != FFI_OK) return rc;
         FFI_LAUNCH_CHECK("ffi_bwd_pairs_kernel");
-        rc = FFI_OK;
+        rc = reduce_range_partials(p.partial, a.gx + (a.x_transposed ? b0 : b0 * a.N), c.R, a.N, cols, c.Bpad, a.B,
+                                   a.x_transposed, stream);
+        if (rc != FFI_OK) return rc;
     }
-    else if (c.bpl == 4) rc = launch_fused_t<8, 4>(p, c, stream);
-    else if (c.bpl == 2) rc = launch_fused_t<16, 2>(p, c, stream);
-    else rc = launch_fused_t<32, 1>(p, c, stream);
-    if (rc != FFI_OK) return rc;
-    return reduce_range_partials(p.partial, a.gx, c.R * c.S, a.N, a.B, c.Bpad, a.x_transposed, stream);
+    return FFI_OK;
 }
 
 }  // namespace ffi

@@ -236,8 +236,8 @@ struct ffi_plan {
     int chunk_rows = 0;     // T: outputs per chunk of the chunked lists
     int64_t n_chunks = 0;   // ceil(L / T)
     bool has_chunks = false;
-    // largest number of entries any (chunk, slice of w consecutive inputs) holds, for w = 128, 256, 512, 1024
-    int max_slice_entries[4] = {0, 0, 0, 0};
+    // largest number of entries any (chunk, slice) holds, for the slicings fused_slices(N, 0 / 1)
+    int max_slice_entries[2] = {0, 0};
     int32_t* rowptr = nullptr;  // [N+1]   canonical CSR-by-input
     int32_t* perm = nullptr;    // [L*K]   positions sorted by (idx[p], p)
     int32_t* cperm = nullptr;   // [L*K]   chunk-major: chunk c holds its T*K positions sorted by (idx[p], p)
@@ -270,10 +270,20 @@ size_t grad_x_workspace_bytes(const ffi_plan* plan, int64_t B);
 bool grad_x_narrow_applicable(const ffi_plan* plan, int64_t B);
 int launch_grad_x(const GradXArgs& a, cudaStream_t stream);
 
-// grad_x and grad_W in one pass over the transposed index (narrow inputs, batch <= 128).
+// How the one-pass backward splits the inputs: `parts` slices of 16 warps x `ni` inputs, as even as possible; at most
+// kFusedNI inputs per warp with a batch tile of 65..128 columns, twice that with up to 64 (narrow).
+constexpr int kFusedNI = 8;
+struct FusedSlices {
+    int parts, ni;
+};
+inline FusedSlices fused_slices(int64_t N, bool narrow) {
+    const int64_t parts = ceil_div(N, 16 * kFusedNI * (narrow ? 2 : 1));
+    return {static_cast<int>(parts), static_cast<int>(ceil_div(N, 16 * parts))};
+}
+
+// grad_x and grad_W in one pass over the transposed index (narrow inputs).
 bool backward_fused_applicable(const ffi_plan* plan, int64_t B);
 size_t backward_fused_workspace_bytes(const ffi_plan* plan, int64_t B);
-bool backward_fused_takes_bf16(const ffi_plan* plan, int64_t B);
 // xT (x as [N][ldx]) has the element type of a.W: fp32, or bf16 when a.w_bf16 is set.
 int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float* gW, float* gbias,
                           cudaStream_t stream);

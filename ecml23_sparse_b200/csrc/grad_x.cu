@@ -211,19 +211,36 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_grad_x_narrow_kernel(GxNarrow
     }
 }
 
-// gx = sum over ranges of partial[r][i][b], in range order; writes [B,N] or [N,B].
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ gx,
-                                       int R, int N, int B, int Bpad, int x_transposed) {
-    const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (id >= static_cast<long long>(N) * Bpad) return;
+// gx = sum over the R partials [r][i][b] (Bpad columns each, `cols` of them used), in fp64 and a fixed order; writes rows
+// of [N][B] or [B][N].  A block takes 32 columns; its 8 warps each add every eighth partial with four loads in flight and
+// the 8 sums are added in warp order.  (One thread per column with a chain of R loads took 13 us at R=148, N=128; this 4.)
+__global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ gx,
+                                                              int R, int N, int cols, int Bpad, int B, int x_transposed) {
+    __shared__ double part[8][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long id = static_cast<long long>(blockIdx.x) * 32 + lane;  // Bpad is a multiple of 32: no tail
+    const size_t stride = static_cast<size_t>(N) * Bpad;
+    double acc = 0.0;  // the range partials are large next to a small total: add them in fp64
+    int r = warp;
+    for (; r + 24 < R; r += 32) {
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __ldg(partial + (r + 8 * u) * stride + id);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc += static_cast<double>(v[u]);
+    }
+    for (; r < R; r += 8) acc += static_cast<double>(__ldg(partial + r * stride + id));
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp != 0) return;
+    double s = part[0][lane];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += part[w][lane];
     const int i = static_cast<int>(id / Bpad);
     const int b = static_cast<int>(id - static_cast<long long>(i) * Bpad);
-    if (b >= B) return;
-    double acc = 0.0;  // the range partials are large next to a small total: add them in fp64
-    for (int r = 0; r < R; ++r) acc += static_cast<double>(partial[(static_cast<size_t>(r) * N + i) * Bpad + b]);
-    const float s = static_cast<float>(acc);
-    if (x_transposed) gx[static_cast<size_t>(i) * B + b] = s;
-    else gx[static_cast<size_t>(b) * N + i] = s;
+    if (b >= cols) return;
+    if (x_transposed) gx[static_cast<size_t>(i) * B + b] = static_cast<float>(s);
+    else gx[static_cast<size_t>(b) * N + i] = static_cast<float>(s);
 }
 
 // ---- wide inputs -------------------------------------------------------------------
@@ -455,6 +472,15 @@ size_t grad_x_min_workspace_bytes(const ffi_plan* plan, int64_t B) {
     return 0;
 }
 
+// Shared with the one-pass backward: see reduce_partials_kernel.
+int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int B, int x_transposed,
+                          cudaStream_t stream) {
+    const long long blocks = static_cast<long long>(N) * Bpad / 32;
+    reduce_partials_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(partial, gx, R, N, cols, Bpad, B, x_transposed);
+    FFI_LAUNCH_CHECK("reduce_partials_kernel");
+    return FFI_OK;
+}
+
 int launch_grad_x(const GradXArgs& a, cudaStream_t stream) {
     DeviceInfo dev;
     int rc = get_device_info(&dev);
@@ -497,11 +523,7 @@ int launch_grad_x(const GradXArgs& a, cudaStream_t stream) {
         else if (c.bpl == 2) rc = launch_narrow_t<32, 2>(p, c.smem, c.iparts, c.nBT, stream);
         else rc = launch_narrow_t<64, 1>(p, c.smem, c.iparts, c.nBT, stream);
         if (rc != FFI_OK) return rc;
-        const long long total = static_cast<long long>(a.N) * c.Bpad;
-        reduce_partials_kernel<<<static_cast<unsigned>(ceil_div(total, 256)), 256, 0, stream>>>(
-            p.partial, a.gx, c.R * c.S, a.N, a.B, c.Bpad, a.x_transposed);
-        FFI_LAUNCH_CHECK("reduce_partials_kernel");
-        return FFI_OK;
+        return reduce_range_partials(p.partial, a.gx, c.R * c.S, a.N, a.B, c.Bpad, a.B, a.x_transposed, stream);
     }
 
     // Wide inputs: one warp per (input, batch tile) over the canonical index, batch tile by batch tile.
@@ -605,15 +627,3 @@ extern "C" int ffi_grad_x_static(const float* W, const float* gT, int64_t ldg, c
     a.workspace_bytes = kStaticScratchBytes;
     return launch_grad_x(a, static_cast<cudaStream_t>(stream_v));
 }
-
-namespace ffi {
-// Shared with the fused backward kernel: grad_x = sum over ranges of partial[r][i][b], range order.
-int reduce_range_partials(const float* partial, float* gx, int R, int N, int B, int Bpad, int x_transposed,
-                          cudaStream_t stream) {
-    const long long total = static_cast<long long>(N) * Bpad;
-    reduce_partials_kernel<<<static_cast<unsigned>(ceil_div(total, 256)), 256, 0, stream>>>(partial, gx, R, N, B, Bpad,
-                                                                                           x_transposed);
-    FFI_LAUNCH_CHECK("reduce_partials_kernel");
-    return FFI_OK;
-}
-}  // namespace ffi

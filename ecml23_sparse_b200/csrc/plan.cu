@@ -14,6 +14,7 @@
 // Concatenating, for each input i, its runs over the chunks in chunk order gives back
 // exactly row i of the canonical form (chunks are ascending ranges of p).
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 
 #include "ffi_common.cuh"
@@ -266,14 +267,14 @@ __global__ void chunk_fill_kernel(const int* __restrict__ perm, const int* __res
     }
 }
 
-// stats[j] = max over chunks c and slices s of (entries of chunk c whose input lies in
-// [s*w, (s+1)*w)), w = 128 << j.  Integer max is order independent.
-__global__ void slice_stats_kernel(const int* __restrict__ cptr, int N, long long nChunks, int* __restrict__ stats) {
+// stats[j] = max over chunks c and slices s of the entries of chunk c whose input lies in slice s (w0 or w1 inputs wide).
+// Integer max is order independent.
+__global__ void slice_stats_kernel(const int* __restrict__ cptr, int N, long long nChunks, int w0, int w1, int* __restrict__ stats) {
     const long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (c >= nChunks) return;
     const int* row = cptr + c * (N + 1);
-    for (int j = 0; j < 4; ++j) {
-        const int w = 128 << j;
+    for (int j = 0; j < 2; ++j) {
+        const int w = j ? w1 : w0;
         int best = 0;
         for (int lo = 0; lo < N; lo += w) best = max(best, row[min(N, lo + w)] - row[lo]);
         atomicMax(stats + j, best);
@@ -329,13 +330,30 @@ struct DeviceBuffer {
 
 }  // namespace
 
-// Rows per chunk of the chunked lists: the grad_x kernel keeps, per chunk, a g tile of
-// T x 128 floats and up to T*K staged (weight, row) pairs in shared memory.
-int plan_chunk_rows(int64_t K) {
-    const int64_t budget = 200 * 1024;
-    int64_t T = budget / (512 + 8 * K);
-    if (T > 256) T = 256;
-    T = T / 8 * 8;
+// Rows per chunk of the chunked lists: the one-pass backward keeps, per chunk, a g tile of T x 128 floats and twice the
+// (weight, code) pairs of a slice of the inputs in shared memory, and a chunk's positions fit 14 bits.
+//   * T is the largest multiple of 8 up to 256 for which that fits (long runs per input and chunk are cheap runs);
+//   * it is lowered until the chunks fill the SMs: the kernel runs R = SMs / slices ranges of chunks, so the chunks are cut
+//     to a whole number per range; a short L (down to 16 rows per chunk) is cut to one chunk per range, or two where they
+//     keep 64 rows, for the ranges of a batch of 64 are twice as many.  Before, a table of fewer than R * 256 rows left most
+//     SMs idle: 513 rows ran on 3 of 148 (B=127, N=254, K=73: backward 73 -> 18 us).
+int plan_chunk_rows(int64_t L, int64_t K, int64_t N) {
+    DeviceInfo dev;
+    const int64_t sms = get_device_info(&dev) == FFI_OK ? dev.sm_count : 148;
+    const FusedSlices sl = fused_slices(N, false);
+    const double share = sl.parts > 1 ? 16.0 * sl.ni / static_cast<double>(N) : 1.0;
+    int64_t T = 256;
+    for (; T > 8; T -= 8) {
+        const double entries = static_cast<double>(T) * K * share;
+        const double spread = sl.parts > 1 ? 5.0 * std::sqrt(entries) : 0.0;  // a random table's fullest slice
+        if (T * K <= 16384 && T * 512 + 16 * (entries + spread + 16) <= 186.0 * 1024) break;
+    }
+    if (T * K > 16384) return 0;  // K in the thousands: no chunked lists
+    const int64_t R = sms / sl.parts > 0 ? sms / sl.parts : 1;
+    const int64_t n = ceil_div(L, T);
+    const int64_t want = n > R ? round_up(n, R) : (L >= 2 * R * 64 ? 2 * R : R);
+    const int64_t even = round_up(ceil_div(L, want), 8);
+    if (even < T) T = even < 16 ? (T < 16 ? T : 16) : even;
     return static_cast<int>(T);
 }
 
@@ -364,7 +382,7 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     g.n = L * K;
     g.nTiles = ceil_div(g.n, kTile);
     g.scan_segs = ceil_div(256 * g.nTiles > N + 1 ? 256 * g.nTiles : N + 1, kScanSeg);
-    g.T = plan_chunk_rows(K);
+    g.T = plan_chunk_rows(L, K, N);
     g.nChunks = ceil_div(L, g.T > 0 ? g.T : 1);
     g.cptrBytes = g.nChunks * (N + 1) * 4;
     g.chunks = g.T >= 8 && N <= kNarrowMaxN && g.cptrBytes <= (512LL << 20) && static_cast<long long>(g.T) * K <= 65536;
@@ -446,9 +464,9 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
         // slice statistics for the kernels that stage one slice of a chunk in shared memory
         FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, 4 * sizeof(int), stream));
         slice_stats_kernel<<<static_cast<unsigned>(ceil_div(g.nChunks, 256)), 256, 0, stream>>>(
-            plan->cptr, static_cast<int>(N), g.nChunks, stats);
+            plan->cptr, static_cast<int>(N), g.nChunks, 16 * fused_slices(N, false).ni, 16 * fused_slices(N, true).ni, stats);
         FFI_LAUNCH_CHECK("slice_stats_kernel");
-        FFI_CUDA_CHECK(cudaMemcpyAsync(plan->max_slice_entries, stats, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+        FFI_CUDA_CHECK(cudaMemcpyAsync(plan->max_slice_entries, stats, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
         plan->chunk_rows = g.T;
         plan->n_chunks = g.nChunks;
         plan->has_chunks = true;
