@@ -59,17 +59,12 @@ int check_plan_device(const ffi_plan* plan) {
     return FFI_OK;
 }
 
-struct Bf16LossEpilogue {
-    float* gT;
-    long long ldg;
-    float scale;
-    double* loss_partials;
-    int loss_kind;
-    int* ctas;
-};
 int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const void* W, const float* bias, float* y,
                         int64_t B, int64_t N, int64_t L, int64_t K, const Bf16LossEpilogue* loss, cudaStream_t stream,
                         bool* handled);
+bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss);
+int launch_forward_dense(const void* xT, int64_t ldx, const int32_t* idx, const void* W, const float* bias, float* y, int64_t B,
+                         int64_t N, int64_t L, int64_t K, const Bf16LossEpilogue* loss, cudaStream_t stream);
 int forward_bf16_warps(int64_t B, int64_t N, int64_t K, bool loss_epilogue);
 int launch_transpose_pad_bf16(const void* src, void* dst, int rows, int cols, int64_t ld_dst, cudaStream_t stream);
 int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int64_t ld_dst, int esize, cudaStream_t stream);
@@ -247,6 +242,13 @@ extern "C" int ffi_forward(const void* x, const int32_t* idx, const void* W, con
         if (rc != FFI_OK || handled) return rc;
     }
     if (dtype == FFI_BF16) {
+        if (forward_dense_applicable(B, N, L, K, false)) {  // tensor cores on densified tiles of W
+            const void* xT = nullptr;
+            int64_t ldx = 0;
+            rc = stage_x_bf16(x, workspace, workspace_bytes, B, N, x_transposed, stream, &xT, &ldx);
+            if (rc != FFI_OK) return rc;
+            return launch_forward_dense(xT, ldx, idx, W, bias, y, B, N, L, K, nullptr, stream);
+        }
         // native bf16 kernel (x tile and W rows stay bf16 in shared memory) where the shape allows it
         if (forward_bf16_warps(B, N, K, false) >= 4) {
             const void* xT = nullptr;
@@ -576,8 +578,9 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
         return fail(FFI_ERR_WORKSPACE, "ffi_forward_loss needs %zu bytes of %zu-byte aligned workspace",
                     ffi_forward_bce_workspace_bytes(B, N, L, K, x_transposed, dtype), kAlign);
     unsigned char* ws = static_cast<unsigned char*>(workspace);
-    const bool bf16_tiled = dtype == FFI_BF16 && forward_bf16_warps(B, N, K, true) < 4 && bf16_takes_tiled_forward(B, N, K);
-    if (dtype == FFI_BF16 && forward_bf16_warps(B, N, K, true) < 4 && !bf16_tiled) {
+    const bool dense = dtype == FFI_BF16 && forward_dense_applicable(B, N, L, K, true);
+    const bool bf16_tiled = !dense && dtype == FFI_BF16 && forward_bf16_warps(B, N, K, true) < 4 && bf16_takes_tiled_forward(B, N, K);
+    if (dtype == FFI_BF16 && !dense && forward_bf16_warps(B, N, K, true) < 4 && !bf16_tiled) {
         // no native kernel for this shape: x and W are widened (exactly) at the front of the workspace
         const float *x32 = nullptr, *W32 = nullptr;
         void* rest = nullptr;
@@ -624,9 +627,10 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
         int ctas_b = 0;
         bool handled_b = false;
         Bf16LossEpilogue e{gT, ldg, scale, partials, loss_kind, &ctas_b};
-        rc = launch_forward_bf16(xTb, ldxb, idx, W, bias, nullptr, B, N, L, K, &e, stream, &handled_b);
+        rc = dense ? launch_forward_dense(xTb, ldxb, idx, W, bias, nullptr, B, N, L, K, &e, stream)
+                   : launch_forward_bf16(xTb, ldxb, idx, W, bias, nullptr, B, N, L, K, &e, stream, &handled_b);
         if (rc != FFI_OK) return rc;
-        if (!handled_b) return fail(FFI_ERR_UNSUPPORTED, "ffi_forward_loss: unaligned bf16 W or idx");
+        if (!dense && !handled_b) return fail(FFI_ERR_UNSUPPORTED, "ffi_forward_loss: unaligned bf16 W or idx");
         if (static_cast<size_t>(ctas_b) * sizeof(double) > kBcePartialBytes)
             return fail(FFI_ERR_UNSUPPORTED, "too many loss partials (%d)", ctas_b);
         return launch_bce_positive_fix(xTb, ldxb, idx, W, bias, row_ptr, labels, gT, ldg, loss, partials, ctas_b,

@@ -26,6 +26,8 @@
 namespace ffi {
 int peer_wait_timeouts(int* out);  // peer_reduce.cu
 int set_peer_wait_limit(long long ticks);
+int dense_forward_timeouts(int* out);  // forward_dense.cu
+int set_dense_forward_wait_limit(long long ticks);
 namespace {
 __device__ int g_wait_timeouts = 0;  // bounded waits of this file's kernels that gave up
 __device__ long long g_wait_limit = 4000000000ll;  // clock64 ticks a wait may last (about two seconds)
@@ -898,7 +900,8 @@ extern "C" int ffi_set_wait_limit_ticks(int64_t ticks) {
     if (ticks < 1000) return ffi::fail(FFI_ERR_INVALID_ARGUMENT, "the wait limit must be at least 1000 ticks");
     const long long t = ticks;
     FFI_CUDA_CHECK(cudaMemcpyToSymbol(ffi::g_wait_limit, &t, sizeof(t)));
-    return ffi::set_peer_wait_limit(t);
+    const int rc = ffi::set_dense_forward_wait_limit(t);
+    return rc != FFI_OK ? rc : ffi::set_peer_wait_limit(t);
 }
 
 // Number of bounded device-side waits that gave up since the library was loaded (0 in a healthy
@@ -910,5 +913,9 @@ extern "C" int ffi_wait_timeouts(int* out) {
     const int rc = ffi::peer_wait_timeouts(&peers);
     if (rc != FFI_OK) return rc;
     *out += peers;
+    int dense = 0;
+    const int rd = ffi::dense_forward_timeouts(&dense);
+    if (rd != FFI_OK) return rd;
+    *out += dense;
     return FFI_OK;
 }

@@ -198,6 +198,16 @@ struct FwdArgs {
 };
 int launch_forward(const FwdArgs& a, cudaStream_t stream);
 
+// Loss epilogue of the bf16 forward kernels; *ctas receives the number of loss partials written.
+struct Bf16LossEpilogue {
+    float* gT;
+    long long ldg;
+    float scale;
+    double* loss_partials;
+    int loss_kind;
+    int* ctas;
+};
+
 struct GradWArgs {
     const void* xT;  // fp32, or bf16 when `bf16` is set (tiled kernel only)
     bool bf16 = false;

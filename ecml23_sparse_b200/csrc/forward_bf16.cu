@@ -308,15 +308,6 @@ int forward_bf16_warps(int64_t B, int64_t N, int64_t K, bool loss_epilogue) {
     return static_cast<int>(warps);
 }
 
-struct Bf16LossEpilogue {
-    float* gT;
-    long long ldg;
-    float scale;
-    double* loss_partials;
-    int loss_kind;
-    int* ctas;
-};
-
 // xT: bf16 [N][ldx]; W: bf16 [L][K].  *handled = false when the shape needs another path.
 int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const void* W, const float* bias, float* y,
                         int64_t B, int64_t N, int64_t L, int64_t K, const Bf16LossEpilogue* loss, cudaStream_t stream,

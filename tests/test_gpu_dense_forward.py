@@ -1,0 +1,62 @@
+"""The tensor-core forward for bf16 storage (densified tiles of 64 outputs): ragged last tiles and panels, batches of one
+and several tiles, fan-ins of one and two entries per lane, repeated inputs in a row (few: the list; many: further rounds of
+a tile), zero weights, both epilogues."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from ecml23_sparse_b200 import ops, synth
+from cases import ATOL, RTOL, assert_close, config_style_inputs, to_cuda
+
+pytestmark = pytest.mark.gpu
+
+
+def bf16_case(dev, B, N, L, K, seed, repeats):
+    x, idx, W, _ = config_style_inputs(B, N, L, K, seed=seed)
+    if repeats == "some":
+        idx = synth.indices_with_replacement(seed, 12, L, K, N).numpy()
+    elif repeats == "all":
+        idx[:, :] = idx[:, :1]           # a row reads one input K times
+    W[::7, ::3] = 0.0
+    xd, Wd = to_cuda(x, dev).to(torch.bfloat16), to_cuda(W, dev).to(torch.bfloat16)
+    return xd, to_cuda(idx, dev), Wd, xd.float().cpu().numpy(), idx, Wd.float().cpu().numpy()
+
+
+@pytest.mark.parametrize("shape", [(65, 128, 64, 32), (128, 768, 1_001, 32), (100, 300, 130, 40), (256, 512, 777, 64),
+                                   (130, 129, 20_003, 8), (33, 64, 1, 4), (97, 700, 300, 31)],
+                         ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
+@pytest.mark.parametrize("repeats", ["none", "some", "all"])
+def test_dense_forward_matches_the_oracle(cuda_device, shape, repeats):
+    dev = cuda_device
+    B, N, L, K = shape
+    xd, idd, Wd, x, idx, W = bf16_case(dev, B, N, L, K, 31, repeats)
+    bias = synth.normal(31, 40, (L,), std=0.5).numpy()
+    ref = oracle.forward_f64(x, idx, W, bias=bias)
+    for transposed in (False, True):
+        xin = xd.t().contiguous() if transposed else xd
+        y = ops._forward(xin, idd, Wd, to_cuda(bias, dev), transposed)
+        assert_close(y.cpu().numpy(), ref, RTOL, ATOL, "y")
+        assert torch.equal(y, ops._forward(xin, idd, Wd, to_cuda(bias, dev), transposed))
+
+
+@pytest.mark.parametrize("shape", [(65, 128, 64, 32), (128, 768, 1_001, 32), (100, 300, 130, 40), (256, 512, 777, 64)],
+                         ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
+@pytest.mark.parametrize("repeats", ["none", "some"])
+@pytest.mark.parametrize("loss_name", ["bce", "squared_hinge"])
+def test_dense_forward_loss_matches_the_oracle(cuda_device, shape, repeats, loss_name):
+    dev = cuda_device
+    B, N, L, K = shape
+    xd, idd, Wd, x, idx, W = bf16_case(dev, B, N, L, K, 37, repeats)
+    bias = synth.normal(37, 40, (L,), std=0.5).numpy()
+    row_ptr, labels = synth.multi_hot_targets(37, 41, B, L)
+    loss, gT = ops.forward_bce(xd, idd, Wd, to_cuda(bias, dev), row_ptr, labels, False, loss=loss_name)
+    z = oracle.forward_f64(x, idx, W, bias=bias).astype(np.float32)
+    if loss_name == "bce":
+        loss_ref, g_ref = oracle.bce_f64(z, row_ptr.numpy(), labels.numpy())
+        assert_close(gT[:, :B].t().cpu().numpy(), g_ref, 5e-5, 2e-7 / (B * L), "gradient")
+    else:
+        loss_ref, g_ref = oracle.hinge_f64(z, row_ptr.numpy(), labels.numpy(), squared=True)
+        assert np.abs(gT[:, :B].t().cpu().numpy() - g_ref).max() <= 4e-5 / (B * L) * max(1.0, np.abs(z).max())
+    assert abs(float(loss) - loss_ref) <= 2e-5 * abs(loss_ref) + 1e-7
+    assert not gT[:, B:].any()
