@@ -38,7 +38,7 @@ EXPORTED_SYMBOLS = (
     "ffi_backward_from_transposed", "ffi_forward_bce_workspace_bytes", "ffi_forward_bce", "ffi_forward_loss", "ffi_wait_timeouts",
     "ffi_set_wait_limit_ticks",
     "ffi_forward_topk_workspace_bytes", "ffi_forward_topk", "ffi_peer_sum",
-    "ffi_bce_workspace_bytes", "ffi_bce_grad", "ffi_adam_step",
+    "ffi_bce_workspace_bytes", "ffi_bce_grad", "ffi_adam_step", "ffi_adam_step_group",
     "ffi_rewire_workspace_bytes", "ffi_rewire",
 )
 
@@ -116,6 +116,8 @@ def _declare(lib):
     lib.ffi_rewire_workspace_bytes.argtypes = []
     lib.ffi_rewire.restype = i32
     lib.ffi_rewire.argtypes = [vp, vp, vp, vp, i64, i64, i64, ctypes.c_uint64, vp, vp, vp, sz, vp]
+    lib.ffi_adam_step_group.restype = i32
+    lib.ffi_adam_step_group.argtypes = [vp, i32, f32, f32, f32, f32, i64, vp]
     lib.ffi_adam_step.restype = i32
     lib.ffi_adam_step.argtypes = [vp, vp, vp, vp, i64, f32, f32, f32, f32, i64, i32, vp]
 

@@ -49,6 +49,40 @@ int get_device_info(DeviceInfo* info) {
     return FFI_OK;
 }
 
+cudaError_t prepare_kernel(const void* kern, int threads, size_t smem, int* occ) {
+    struct Entry {
+        const void* kern = nullptr;
+        int dev = -1, threads = 0, occ = 0;
+        size_t smem = 0;
+    };
+    static thread_local Entry cache[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    Entry& c = cache[((reinterpret_cast<uintptr_t>(kern) >> 4) * 31 + smem / 64 + threads) % 64];
+    if (c.kern != kern || c.dev != dev || c.threads != threads || c.smem != smem) {
+        // the most the device allows, so that no later call with less takes it away from a remembered one
+        cudaFuncAttributes a;
+        DeviceInfo info;
+        if (get_device_info(&info) != FFI_OK) return cudaErrorInvalidDevice;
+        e = cudaFuncGetAttributes(&a, kern);
+        if (e != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 info.max_smem_optin - static_cast<int>(a.sharedSizeBytes));
+        if (e != cudaSuccess) return e;
+        int n = 0;
+        if (threads > 0) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem);
+        if (e != cudaSuccess) return e;
+        c.kern = kern;
+        c.dev = dev;
+        c.threads = threads;
+        c.smem = smem;
+        c.occ = n;
+    }
+    if (occ) *occ = c.occ;
+    return cudaSuccess;
+}
+
 // A plan's index arrays live on the GPU it was built on: a call made with another GPU current would
 // hand its kernels pointers into that other GPU's memory.
 int check_plan_device(const ffi_plan* plan) {
@@ -544,7 +578,7 @@ int launch_bce_positive_fix(const void* xT, int64_t ldx, const int* idx, const v
                             const int* row_ptr, const int* labels, float* gT, int64_t ldg, float* loss,
                             const double* partials, int nPartials, double* pos_partials, float scale, int B,
                             int64_t L, int K, int64_t label_offset, int loss_kind, bool bf16, cudaStream_t stream);
-constexpr size_t kBcePartialBytes = 1024 * sizeof(double);  // >= one partial per CTA of the forward kernel
+constexpr size_t kBcePartialBytes = (kMaxLossPartials + 1) * sizeof(double);  // one partial per CTA of the forward kernel, the ticket
 }  // namespace ffi
 
 extern "C" size_t ffi_forward_bce_workspace_bytes(int64_t B, int64_t N, int64_t L, int64_t K, int x_transposed,
@@ -631,7 +665,7 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
                    : launch_forward_bf16(xTb, ldxb, idx, W, bias, nullptr, B, N, L, K, &e, stream, &handled_b);
         if (rc != FFI_OK) return rc;
         if (!dense && !handled_b) return fail(FFI_ERR_UNSUPPORTED, "ffi_forward_loss: unaligned bf16 W or idx");
-        if (static_cast<size_t>(ctas_b) * sizeof(double) > kBcePartialBytes)
+        if (static_cast<size_t>(ctas_b) * sizeof(double) > kMaxLossPartials * sizeof(double))
             return fail(FFI_ERR_UNSUPPORTED, "too many loss partials (%d)", ctas_b);
         return launch_bce_positive_fix(xTb, ldxb, idx, W, bias, row_ptr, labels, gT, ldg, loss, partials, ctas_b,
                                        pos_partials, scale, static_cast<int>(B), L, static_cast<int>(K), label_offset,
@@ -662,7 +696,7 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
         rc = launch_forward_loss_tile(a, gT, ldg, scale, partials, &ctas, loss_kind, stream);
         if (rc != FFI_OK) return rc;
     }
-    if (static_cast<size_t>(ctas) * sizeof(double) > kBcePartialBytes)
+    if (static_cast<size_t>(ctas) * sizeof(double) > kMaxLossPartials * sizeof(double))
         return fail(FFI_ERR_UNSUPPORTED, "too many loss partials (%d)", ctas);
     return launch_bce_positive_fix(xT, xp.ld, idx, a.W, bias, row_ptr, labels, gT, ldg, loss, partials, ctas,
                                    pos_partials, scale, static_cast<int>(B), L, static_cast<int>(K), label_offset, loss_kind,

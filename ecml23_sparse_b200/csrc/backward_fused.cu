@@ -379,32 +379,29 @@ __global__ void __launch_bounds__(THREADS, 1)
     const unsigned taddr0 = tmem_base + ((static_cast<unsigned>(warp & 3) * 32u) << 16) +
                             static_cast<unsigned>(warp >> 2) * (NI * COLS);
 
-    if constexpr (VPL == 8) {
-        for (int j = 0; j < ni; ++j) {
-            const int i = i_lo + warp * ni + j;
-            unsigned xv[8], zero[8];
-    #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                const int b = (m < 4 ? 0 : BT / 2) + 4 * q + (m & 3);
-                xv[m] = __float_as_uint((i < N && b < p.B) ? widen(xTt[static_cast<size_t>(i) * p.ldx + b]) : 0.f);
-                zero[m] = 0u;
-            }
-            tmem_store8(taddr0 + j * 16, zero);
-            tmem_store8(taddr0 + j * 16 + 8, xv);
-        }
-    } else {
-        for (int j = 0; j < ni; ++j) {
-            const int i = i_lo + warp * ni + j;
-            unsigned xv[VPL], zero[VPL];
-    #pragma unroll
+    // x of the warp's inputs: all loads of four inputs are under way before the first is stored (one input at a time, this
+    // prologue took a third of a small launch)
+    for (int j0 = 0; j0 < ni; j0 += 4) {
+        unsigned xv[4][VPL];
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+            const int i = i_lo + warp * ni + j0 + jj;
+#pragma unroll
             for (int m = 0; m < VPL; ++m) {
                 const int b = (m < 4 ? 0 : BT / 2) + 4 * q + (m & 3);
-                xv[m] = __float_as_uint((i < N && b < p.B) ? widen(xTt[static_cast<size_t>(i) * p.ldx + b]) : 0.f);
-                zero[m] = 0u;
+                xv[jj][m] = __float_as_uint(
+                    (j0 + jj < ni && i < N && b < p.B) ? widen(xTt[static_cast<size_t>(i) * p.ldx + b]) : 0.f);
             }
-            tmem_store_cols<VPL>(taddr0 + j * COLS, zero);
-            tmem_store_cols<VPL>(taddr0 + j * COLS + VPL, xv);
         }
+        unsigned zero[VPL];
+#pragma unroll
+        for (int m = 0; m < VPL; ++m) zero[m] = 0u;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+            if (j0 + jj < ni) {
+                tmem_store_cols<VPL>(taddr0 + (j0 + jj) * COLS, zero);
+                tmem_store_cols<VPL>(taddr0 + (j0 + jj) * COLS + VPL, xv[jj]);
+            }
     }
     tmem_wait_store();
 
@@ -864,7 +861,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         if (rc != FFI_OK) return rc;
         dim3 grid(static_cast<unsigned>(c.R), static_cast<unsigned>(c.iparts), 1);
         auto launch_group = [&](auto kern) -> int {
-            FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(c.smem)));
+            FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, c.smem, nullptr));
             kern<<<grid, kGroupThreads, c.smem, stream>>>(p, g_map);
             return FFI_OK;
         };

@@ -11,12 +11,14 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
+#include <pybind11/stl.h>
 
 #include <list>
 #include <memory>
 #include <mutex>
 #include <optional>
 #include <tuple>
+#include <vector>
 
 #include "ffi_b200.h"
 
@@ -260,16 +262,31 @@ std::tuple<Tensor, Tensor> forward_topk(const Tensor& features, const Tensor& lo
     return {val, lab};
 }
 
-void adam_step(const Tensor& p, const Tensor& m, const Tensor& v, const Tensor& grad, double lr, double beta1, double beta2,
+void adam_step(const std::vector<std::tuple<Tensor, Tensor, Tensor, Tensor>>& params, double lr, double beta1, double beta2,
                double eps, int64_t step) {
-    const Tensor g = grad.contiguous();
-    if (g.scalar_type() != at::kFloat || g.sizes() != p.sizes() || !g.is_cuda())
-        throw py::value_error("gradient must be float32 with the parameter's shape");
-    const c10::cuda::CUDAGuard guard(p.device());
-    check(ffi_adam_step(p.data_ptr(), m.data_ptr<float>(), v.data_ptr<float>(), g.const_data_ptr<float>(), p.numel(),
-                        static_cast<float>(lr), static_cast<float>(beta1), static_cast<float>(beta2), static_cast<float>(eps),
-                        step, p.scalar_type() == at::kBFloat16 ? FFI_BF16 : FFI_F32,
-                        c10::cuda::getCurrentCUDAStream(p.device().index())));
+    std::vector<ffi_adam_tensor> group;
+    std::vector<Tensor> held;  // contiguous copies live until the launch
+    at::Device dev(at::kCUDA, 0);
+    const auto flush = [&] {
+        if (group.empty()) return;
+        const c10::cuda::CUDAGuard guard(dev);
+        check(ffi_adam_step_group(group.data(), static_cast<int>(group.size()), static_cast<float>(lr), static_cast<float>(beta1),
+                                  static_cast<float>(beta2), static_cast<float>(eps), step,
+                                  c10::cuda::getCurrentCUDAStream(dev.index())));
+        group.clear();
+    };
+    for (const auto& [p, m, v, grad] : params) {
+        const Tensor g = grad.contiguous();
+        if (g.scalar_type() != at::kFloat || g.sizes() != p.sizes() || !g.is_cuda())
+            throw py::value_error("gradient must be float32 with the parameter's shape");
+        if (dev != p.device()) flush();
+        dev = p.device();
+        held.push_back(g);
+        if (p.numel() > 0)
+            group.push_back({p.data_ptr(), m.data_ptr<float>(), v.data_ptr<float>(), g.const_data_ptr<float>(), p.numel(),
+                             p.scalar_type() == at::kBFloat16 ? FFI_BF16 : FFI_F32});
+    }
+    flush();
 }
 
 // ---- autograd (gradient registration of sparse/ops/fixed_fan_in_ops.py:31-40: [feature_grad, None, weight_grad]) ----

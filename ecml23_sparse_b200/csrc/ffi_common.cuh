@@ -56,6 +56,10 @@ struct DeviceInfo {
 };
 int get_device_info(DeviceInfo* info);
 
+// Lets `kern` use `smem` bytes of dynamic shared memory on the current device and, with occ, tells how many CTAs of
+// `threads` threads an SM holds.  The answers are kept per thread of the host (the two driver calls cost 1 to 2 us a launch).
+cudaError_t prepare_kernel(const void* kern, int threads, size_t smem, int* occ);
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
 
@@ -163,6 +167,14 @@ __device__ __forceinline__ void loss_for_negative(int kind, float z, float& valu
         value = kind == 1 ? h * h : h;
         grad = kind == 1 ? 2.f * h : (h > 0.f ? 1.f : 0.f);
     }
+}
+
+// Scratch of the fused loss: one partial per CTA of the forward kernel, then a ticket counter that the forward kernel clears
+// and the kernel after it draws from.
+constexpr int kMaxLossPartials = 1024;
+__host__ __device__ inline unsigned* loss_ticket(double* partials) { return reinterpret_cast<unsigned*>(partials + kMaxLossPartials); }
+__device__ __forceinline__ void clear_loss_ticket(double* partials) {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *loss_ticket(partials) = 0u;
 }
 
 // Top-k epilogues of the forward kernels (evaluation: P@1, P@3, P@5 need 5 candidates per sample).

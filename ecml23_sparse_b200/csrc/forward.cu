@@ -257,6 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_kernel(FwdKernelParams p)
         double* red = reinterpret_cast<double*>(smem_raw);
         if (lane == 0) red[warp] = v;
         __syncthreads();
+        clear_loss_ticket(p.loss_partials);
         if (tid == 0) {
             double t = 0.0;
             for (int w = 0; w < kWarps; ++w) t += red[w];
@@ -304,25 +305,21 @@ int pick_TO(size_t budget, int N, int bpl, bool xsmem, int Kp) {
     return static_cast<int>(to / 16 * 16);
 }
 
-constexpr int kMaxLossPartialsTile = 1024;  // doubles the caller's scratch holds for the per-CTA loss sums
-
 template <int BPL, bool XSMEM, int MODE, typename TX>
 int launch_fwd_t(const FwdKernelParams& p, size_t smem, int nBT, const DeviceInfo& dev,
                  cudaStream_t stream, int* ctas_out) {
     constexpr bool LOSS = MODE == 1;
     auto kern = ffi_fwd_kernel<BPL, XSMEM, MODE, TX>;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
     int occ = 0;
-    FFI_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "forward kernel does not fit on an SM (smem %zu)", smem);
     if (MODE == 2) occ = 1;  // the scratch for the top-k lists is sized for one CTA per SM
     int per_bt = dev.sm_count * occ / nBT;
     if (per_bt < 1) per_bt = 1;
     dim3 grid(static_cast<unsigned>(min(p.numTiles, per_bt)), static_cast<unsigned>(nBT));
-    if (LOSS && static_cast<long long>(grid.x) * grid.y > kMaxLossPartialsTile)
+    if (LOSS && static_cast<long long>(grid.x) * grid.y > kMaxLossPartials)
         return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %d per-CTA partials; this batch needs %u",
-                    kMaxLossPartialsTile, grid.x * grid.y);
+                    kMaxLossPartials, grid.x * grid.y);
     if (ctas_out) *ctas_out = static_cast<int>(grid.x * grid.y);
     kern<<<grid, kThreads, smem, stream>>>(p);
     FFI_LAUNCH_CHECK("ffi_fwd_kernel");
@@ -413,15 +410,18 @@ static int launch_forward_tile(const FwdArgs& a, const TileLossEpilogue* loss, c
         // wide inputs: the per-warp gather kernel where fan-in and alignment allow it
         bool handled = false;
         rc = launch_forward_gather(a, bpl, loss ? loss->gT : nullptr, loss ? loss->ldg : 0, loss ? loss->scale : 0.f,
-                                   loss ? loss->loss_partials : nullptr, loss ? loss->loss_kind : 0, kMaxLossPartialsTile,
+                                   loss ? loss->loss_partials : nullptr, loss ? loss->loss_kind : 0, kMaxLossPartials,
                                    loss ? loss->ctas : nullptr, stream, &handled);
         if (rc != FFI_OK || handled) return rc;
     }
     p.TO = pick_TO(dev.max_smem_optin, a.N, bpl, xsmem, p.Kp);
     if (p.TO < 16) return fail(FFI_ERR_UNSUPPORTED, "fan-in K=%d too large for the staged tiles", a.K);
+    const int nBT = static_cast<int>(ceil_div(a.B, 32 * bpl));
+    // a short table is cut into smaller tiles, so that every SM gets one (513 rows in tiles of 128 ran on 5 SMs: 17 us)
+    const int64_t per_sm = round_up(ceil_div(a.L, dev.sm_count / nBT > 0 ? dev.sm_count / nBT : 1), 16);
+    if (per_sm < p.TO) p.TO = static_cast<int>(per_sm);
     p.numTiles = static_cast<int>(ceil_div(a.L, p.TO));
     const size_t smem = fwd_smem_bytes(a.N, bpl, xsmem, p.TO, p.Kp);
-    const int nBT = static_cast<int>(ceil_div(a.B, 32 * bpl));
     if (!xsmem) {
         // The global-memory gather reads whole lane vectors: rows must be padded and aligned.
         if (a.ldx % (32 * bpl) != 0 || a.ldx < static_cast<int64_t>(nBT) * 32 * bpl ||

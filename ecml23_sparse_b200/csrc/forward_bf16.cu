@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
         double* red = reinterpret_cast<double*>(smem_raw);
         if (lane == 0) red[warp] = v;
         __syncthreads();
+        clear_loss_ticket(p.loss_partials);
         if (tid == 0) {
             double t = 0.0;
             for (int w = 0; w < nwarps; ++w) t += red[w];
@@ -342,12 +343,12 @@ int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const v
     *handled = true;
     if (loss) {
         auto kern = ffi_fwd_bf16_kernel<1>;
-        FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
         *loss->ctas = static_cast<int>(grid);
         kern<<<grid, warps * 32, smem, stream>>>(p);
     } else {
         auto kern = ffi_fwd_bf16_kernel<0>;
-        FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
         kern<<<grid, warps * 32, smem, stream>>>(p);
     }
     FFI_LAUNCH_CHECK("ffi_fwd_bf16_kernel");

@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
         double* red = reinterpret_cast<double*>(smem);
         if (lane == 0) red[warp] = v;
         __syncthreads();
+        clear_loss_ticket(p.loss_partials);
         if (tid == 0) {
             double s = 0.0;
             for (int w = 0; w < kEmitWarps; ++w) s += red[w];
@@ -470,7 +471,7 @@ int launch_forward_dense(const void* xT, int64_t ldx, const int32_t* idx, const 
     const dim3 grid(static_cast<unsigned>(tiles < per_bt ? tiles : per_bt), static_cast<unsigned>(nBT));
     if (loss) *loss->ctas = static_cast<int>(grid.x * grid.y);
     auto go = [&](auto kern) -> int {
-        FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
         kern<<<grid, kThreads, smem, stream>>>(p);
         FFI_LAUNCH_CHECK("ffi_fwd_dense_kernel");
         return FFI_OK;

@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
         double* red = reinterpret_cast<double*>(smem_raw);
         if (lane == 0) red[warp] = v;
         __syncthreads();
+        clear_loss_ticket(p.loss_partials);
         if (threadIdx.x == 0) {
             double t = 0.0;
             for (int w = 0; w < kWarps; ++w) t += red[w];
@@ -208,9 +209,8 @@ int launch_fwd_gather_t(const FwdGatherParams& p, int nBT, int max_partials, con
     auto kern = ffi_fwd_gather_kernel<BPL, MODE, TX>;
     const size_t warpWords = 2 * static_cast<size_t>(p.K / WPE + p.K) + (MODE == 0 ? kRows * (BT + 4) : 0);
     const size_t smem = kWarps * warpWords * 4;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int occ = 0;
-    FFI_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "forward gather kernel does not fit on an SM (smem %zu)", smem);
     const long long want = ceil_div(ceil_div(p.L, kRows), kWarps);
     long long per_bt = static_cast<long long>(dev.sm_count) * occ / nBT;

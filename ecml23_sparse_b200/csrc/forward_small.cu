@@ -130,9 +130,8 @@ __global__ void __launch_bounds__(kThreads) ffi_fwd_small_kernel(SmallParams p) 
 template <int BP, typename TX>
 int launch_small_t(const SmallParams& p, size_t smem, const DeviceInfo& dev, cudaStream_t stream) {
     auto kern = ffi_fwd_small_kernel<BP, TX>;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int occ = 0;
-    FFI_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "small-batch forward kernel does not fit on an SM (smem %zu)", smem);
     const int tileRows = (BP <= 4 ? 4 : 2) * (32 >> p.lgG);
     const int64_t want = ceil_div(ceil_div(p.L, tileRows), kWarps), cap = static_cast<int64_t>(dev.sm_count) * occ;

@@ -50,8 +50,6 @@ __device__ __forceinline__ float floor_value(int k) {
     return k == kFloorNone ? -INFINITY : __int_as_float(k >= 0 ? k : k ^ 0x7fffffff);
 }
 
-constexpr size_t kMaxLossPartials = 1024;  // doubles the caller's scratch holds for the per-CTA loss sums
-
 // A HALF warp covers the batch tile (16 lanes x VPL batch elements) and the two halves of a warp
 // work on the two rows of a row pair at once.  The fetch of a row's W and idx values is then one
 // shared-memory access for both rows (two addresses, one per half) instead of a warp-uniform access
@@ -296,6 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
         double* red = reinterpret_cast<double*>(smem_raw);
         if (lane == 0) red[warp] = v;
         __syncthreads();
+        clear_loss_ticket(p.loss_partials);
         if (tid == 0) {
             double t = 0.0;
             for (int w = 0; w < kWarps; ++w) t += red[w];
@@ -308,9 +307,8 @@ template <int VPL, int MODE>
 int launch_pair_t(const FwdStreamParams& p, size_t smem, int nBT, const DeviceInfo& dev, cudaStream_t stream,
                   int* ctas_out) {
     auto kern = ffi_fwd_pair_kernel<VPL, MODE>;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int occ = 0;
-    FFI_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "streaming forward kernel does not fit on an SM (smem %zu)", smem);
     // The epilogue variants write one record per CTA (loss partial, top-k lists) into scratch that is
     // sized for one CTA per SM, whatever occupancy the kernel would allow.
@@ -320,8 +318,8 @@ int launch_pair_t(const FwdStreamParams& p, size_t smem, int nBT, const DeviceIn
     const long long numQuads = (static_cast<long long>(p.L) + 3) / 4;
     const long long want = (numQuads + kWarps - 1) / kWarps;
     dim3 grid(static_cast<unsigned>(want < per_bt ? want : per_bt), static_cast<unsigned>(nBT));
-    if (MODE == 1 && static_cast<size_t>(grid.x) * grid.y > kMaxLossPartials)
-        return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %zu per-CTA partials; this batch needs %u",
+    if (MODE == 1 && static_cast<size_t>(grid.x) * grid.y > static_cast<size_t>(kMaxLossPartials))
+        return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %d per-CTA partials; this batch needs %u",
                     kMaxLossPartials, grid.x * grid.y);
     if (ctas_out) *ctas_out = static_cast<int>(grid.x * grid.y);
     kern<<<grid, kThreads, smem, stream>>>(p);

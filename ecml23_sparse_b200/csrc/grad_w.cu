@@ -257,10 +257,8 @@ int gw_pick_TO(size_t budget, int N, int bpl, bool xsmem, int Kp) {
 template <int BPL, int G, bool XSMEM, typename TX>
 int launch_gw_t(GradWKernelParams p, size_t smem, int nBT, const DeviceInfo& dev, cudaStream_t stream) {
     auto kern = ffi_grad_w_kernel<BPL, G, XSMEM, TX>;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
     int occ = 0;
-    FFI_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "grad_W kernel does not fit on an SM (smem %zu)", smem);
     const unsigned grid = static_cast<unsigned>(min(p.numTiles, dev.sm_count * occ));
     // Batch tiles run as consecutive launches so that tile t adds to what tile t-1 wrote.

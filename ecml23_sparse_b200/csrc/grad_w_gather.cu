@@ -141,9 +141,8 @@ template <int BPL, typename TX>
 int launch_gather_t(GatherParams p, int nBT, const DeviceInfo& dev, cudaStream_t stream) {
     auto kern = ffi_grad_w_gather_kernel<BPL, TX>;
     const size_t smem = static_cast<size_t>(kWarps) * (32 * kRow + 2 * p.K) * 4;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int occ = 0;
-    FFI_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "grad_W gather kernel does not fit on an SM (smem %zu)", smem);
     const long long want = ceil_div(p.L, kWarps);
     const long long cap = static_cast<long long>(dev.sm_count) * occ;

@@ -192,9 +192,8 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_grad_w_stream_kernel(GradWStr
 template <int BPL, int G>
 int launch_gws_t(GradWStreamParams p, size_t smem, int nBT, const DeviceInfo& dev, cudaStream_t stream) {
     auto kern = ffi_grad_w_stream_kernel<BPL, G>;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int occ = 0;
-    FFI_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "streaming grad_W kernel does not fit on an SM (smem %zu)", smem);
     const long long numQuads = (static_cast<long long>(p.L) + 3) / 4;
     const long long want = (numQuads + kWarps - 1) / kWarps;

@@ -322,8 +322,7 @@ __global__ void __launch_bounds__(256, 8) ffi_grad_x_wide_kernel(const TW* __res
 template <int NI, int BPL>
 int launch_narrow_t(const GxNarrowParams& p, size_t smem, int iparts, int nBT, cudaStream_t stream) {
     auto kern = ffi_grad_x_narrow_kernel<NI, BPL>;
-    FFI_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
     dim3 grid(static_cast<unsigned>(p.R), static_cast<unsigned>(iparts), static_cast<unsigned>(nBT));
     kern<<<grid, kThreads, smem, stream>>>(p);
     FFI_LAUNCH_CHECK("ffi_grad_x_narrow_kernel");

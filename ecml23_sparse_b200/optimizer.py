@@ -2,7 +2,7 @@
 
 Mirror of ``SparseAdam`` (sparse/optimizer.py:9-23), i.e. ``keras.optimizers.Adam`` with its
 defaults as used at run.py:126 (lr 1e-3, beta 0.9/0.999, epsilon 1e-7, no amsgrad): one fused
-kernel per parameter instead of Keras' chain of elementwise ops.  ``zero_moments`` is the
+launch for all parameters instead of Keras' chain of elementwise ops.  ``zero_moments`` is the
 moment reset that ``SparseAdam.update_sparse`` performs at rewired positions
 (custom_layer.py:20-30).
 """
@@ -27,13 +27,13 @@ class FusedAdam:
     def step(self, grads=None):
         """Applies one update; `grads` defaults to each parameter's `.grad`."""
         self.iterations += 1
-        adam_step = ops._native().adam_step
+        todo = []
         for j, p in enumerate(self.params):
             g = grads[j] if grads is not None else p.grad
-            if g is None:
-                continue
-            adam_step(p.data if isinstance(p, torch.nn.Parameter) else p, self.m[j], self.v[j], g, self.lr, self.beta_1,
-                      self.beta_2, self.epsilon, self.iterations)
+            if g is not None:
+                todo.append((p.data if isinstance(p, torch.nn.Parameter) else p, self.m[j], self.v[j], g))
+        if todo:
+            ops._native().adam_step(todo, self.lr, self.beta_1, self.beta_2, self.epsilon, self.iterations)
 
     def zero_moments(self, index: int, locations: torch.Tensor):
         """Zero m and v of parameter `index` at flat positions `locations`."""

@@ -310,6 +310,18 @@ int ffi_bce_grad(const float* z, const int32_t* row_ptr, const int32_t* labels, 
 int ffi_adam_step(void* w, float* m, float* v, const float* grad, int64_t n, float lr, float beta1,
                   float beta2, float eps, int64_t step, int dtype, void* stream);
 
+/* The same step for several parameters (a layer's weights and bias) in one launch per eight of them. */
+typedef struct ffi_adam_tensor {
+    void* w;           /* fp32 or bf16 */
+    float* m;
+    float* v;
+    const float* grad;
+    int64_t n;
+    int dtype;
+} ffi_adam_tensor;
+int ffi_adam_step_group(const ffi_adam_tensor* tensors, int count, float lr, float beta1, float beta2, float eps,
+                        int64_t step, void* stream);
+
 /* --------------------------------------------------------------- rewiring ---- */
 
 /*

@@ -56,3 +56,24 @@ def test_topk_of_fewer_rows_than_k(cuda_device):
     W = torch.tensor([[1.0], [3.0], [2.0]], device=cuda_device).expand(3, 4).contiguous()
     vals, lab = ops.forward_topk(x, idx, W, None, 5, True)
     assert lab.tolist() == [[1, 2, 0, -1, -1]] * 2 and vals[:, :3].tolist() == [[12.0, 8.0, 4.0]] * 2
+
+
+def test_adam_step_of_several_parameters_matches_one_by_one(cuda_device):
+    """One launch for all parameters: sizes with and without a remainder, unaligned views, both storage types, more than
+    one group of eight."""
+    dev = cuda_device
+    sizes = [1, 3, 4, 1_001, 70_001, 8, 2_000_003, 17, 5]
+    base = [synth.normal(3, j, (n + 1,)).to(dev) for j, n in enumerate(sizes)]
+    def params():
+        return [(b[1:].clone() if j % 3 == 0 else b.clone()[1:]).to(torch.bfloat16 if j % 2 else torch.float32)
+                for j, b in enumerate(base)]
+    grads = [synth.normal(4, j, (n,)).to(dev) for j, n in enumerate(sizes)]
+    together = ffi.FusedAdam(params())
+    for _ in range(2):
+        together.step(grads)
+    for j in range(len(sizes)):
+        alone = ffi.FusedAdam([params()[j]])
+        for _ in range(2):
+            alone.step([grads[j]])
+        assert torch.equal(alone.params[0], together.params[j])
+        assert torch.equal(alone.m[0], together.m[j]) and torch.equal(alone.v[0], together.v[j])
