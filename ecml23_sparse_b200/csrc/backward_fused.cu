@@ -158,6 +158,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+// The same box into L2 only.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -504,6 +508,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             fence_proxy_async();
             mbar_expect_tx(g_bar, tileBytes);
             tma_load_2d(g_s, &g_map, 0, static_cast<int>(o0), g_bar);
+            // the next tile on its way from DRAM to L2 meanwhile; the slices of the range take turns
+            if (c + 1 < c_end && static_cast<int>((c + 1) % gridDim.y) == static_cast<int>(blockIdx.y))
+                tma_prefetch_2d(&g_map, 0, static_cast<int>(o0 + T));
         }
         pending = c;
         const int staged_cnt = c + 1 < c_end ? pl_cnt : 0;  // entries of chunk c + 1 going into the other buffer
