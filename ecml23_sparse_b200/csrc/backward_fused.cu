@@ -79,6 +79,7 @@ struct BwdFusedParams {
     int entCap;
     int segChunks;  // chunks per flushed partial
     int ni;         // inputs per warp
+    int boxes;      // TMA boxes per tile (at most 256 rows each)
 };
 
 // =====================================================================================
@@ -500,17 +501,20 @@ __global__ void __launch_bounds__(THREADS, 1)
             break;
         }
 
-        // The g tile of the chunk: one TMA box [T rows][BT columns] of gT (rows past L and columns past the
-        // stored row arrive as zeros).
+        // The g tile of the chunk: one TMA box [T rows][BT columns] of gT, or two of half the rows where T > 256
+        // (rows past L and columns past the stored row arrive as zeros).
         // (A second tile buffer filled one chunk ahead was measured: it needs T <= 168 to fit, and the
         // shorter runs cost more than the hidden copy saves.)
         if (tid == 0) {
             fence_proxy_async();
             mbar_expect_tx(g_bar, tileBytes);
-            tma_load_2d(g_s, &g_map, 0, static_cast<int>(o0), g_bar);
+            for (int h = 0; h < p.boxes; ++h) {
+                const int rows = T / p.boxes;
+                tma_load_2d(g_s + static_cast<size_t>(h) * rows * BT, &g_map, 0, static_cast<int>(o0) + h * rows, g_bar);
+            }
             // the next tile on its way from DRAM to L2 meanwhile; the slices of the range take turns
             if (c + 1 < c_end && static_cast<int>((c + 1) % gridDim.y) == static_cast<int>(blockIdx.y))
-                tma_prefetch_2d(&g_map, 0, static_cast<int>(o0 + T));
+                for (int h = 0; h < p.boxes; ++h) tma_prefetch_2d(&g_map, 0, static_cast<int>(o0) + T + h * (T / p.boxes));
         }
         pending = c;
         const int staged_cnt = c + 1 < c_end ? pl_cnt : 0;  // entries of chunk c + 1 going into the other buffer
@@ -850,6 +854,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         if ((1 << sh) == a.K) p.kShift = sh;
     p.T = a.plan->chunk_rows;
     p.nChunks = a.plan->n_chunks;
+    p.boxes = p.T > 256 ? 2 : 1;
     for (int64_t b0 = 0; b0 < a.B; b0 += 128) {
         const int cols = static_cast<int>(tile_columns(a.B, b0));
         FusedConfig c;
@@ -864,7 +869,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         p.ni = c.ni;
         // gT as a 2-D tensor [L rows][BT columns] with row pitch ldg; one box = the g tile of a chunk
         CUtensorMap g_map;
-        rc = encode_g_map(&g_map, p.gT, a.L, a.ldg, a.ldg - b0, a.plan->chunk_rows, c.Bpad);
+        rc = encode_g_map(&g_map, p.gT, a.L, a.ldg, a.ldg - b0, p.T / p.boxes, c.Bpad);
         if (rc != FFI_OK) return rc;
         dim3 grid(static_cast<unsigned>(c.R), static_cast<unsigned>(c.iparts), 1);
         auto launch_group = [&](auto kern) -> int {

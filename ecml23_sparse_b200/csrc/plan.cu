@@ -332,7 +332,10 @@ struct DeviceBuffer {
 
 // Rows per chunk of the chunked lists: the one-pass backward keeps, per chunk, a g tile of T x 128 floats and twice the
 // (weight, code) pairs of a slice of the inputs in shared memory, and a chunk's positions fit 14 bits.
-//   * T is the largest multiple of 8 up to 256 for which that fits (long runs per input and chunk are cheap runs);
+//   * T is the largest multiple of 8 for which that fits (long runs per input and chunk are cheap runs) into what leaves
+//     60 KB of L1 to the gathers of W: with 28 KB the kernel slows down by a tenth (B=128, N=768, K=32: 903 us with T=264,
+//     917 with 256, 995 with 288).  Where the runs would be shorter than six entries their length counts for more, and the
+//     whole shared memory is used (N=1024, K=8: 322 us with T=352, 352 with 296; N=2000, K=32: 223 and 235).
 //   * it is lowered until the chunks fill the SMs: the kernel runs R = SMs / slices ranges of chunks, so the chunks are cut
 //     to a whole number per range; a short L (down to 16 rows per chunk) is cut to one chunk per range, or two where they
 //     keep 64 rows, for the ranges of a batch of 64 are twice as many.  Before, a table of fewer than R * 256 rows left most
@@ -342,11 +345,12 @@ int plan_chunk_rows(int64_t L, int64_t K, int64_t N) {
     const int64_t sms = get_device_info(&dev) == FFI_OK ? dev.sm_count : 148;
     const FusedSlices sl = fused_slices(N, false);
     const double share = sl.parts > 1 ? 16.0 * sl.ni / static_cast<double>(N) : 1.0;
-    int64_t T = 256;
+    int64_t T = 512;
+    const double budget = 264.0 * K >= 6.0 * N ? 160700.0 : 190464.0;
     for (; T > 8; T -= 8) {
         const double entries = static_cast<double>(T) * K * share;
-        const double spread = sl.parts > 1 ? 5.0 * std::sqrt(entries) : 0.0;  // a random table's fullest slice
-        if (T * K <= 16384 && T * 512 + 16 * (entries + spread + 16) <= 186.0 * 1024) break;
+        const double spread = sl.parts > 1 ? 4.0 * std::sqrt(entries) : 0.0;  // a random table's fullest slice
+        if (T * K <= 16384 && T * 512 + 16 * (entries + spread + 16) <= budget) break;
     }
     if (T * K > 16384) return 0;  // K in the thousands: no chunked lists
     const int64_t R = sms / sl.parts > 0 ? sms / sl.parts : 1;
