@@ -90,9 +90,16 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_kernel(FwdKernelParams p)
             int i = e / BT;
             int bl = e - i * BT;
             int b = b0 + bl;
-            float v = b < p.B ? widen(xT[static_cast<size_t>(i) * p.ldx + b]) : 0.f;
-            x_s[i * BT + (bl & 31) * BPL + (bl >> 5)] = v;
+            float* dst = x_s + i * BT + (bl & 31) * BPL + (bl >> 5);
+            if constexpr (kBf16) {
+                *dst = b < p.B ? widen(xT[static_cast<size_t>(i) * p.ldx + b]) : 0.f;
+            } else {  // asynchronous copies, all of a thread's in flight at once (the zero-filled ones read nothing)
+                const bool in = b < p.B;
+                __pipeline_memcpy_async(dst, in ? xT + static_cast<size_t>(i) * p.ldx + b : xT, 4, in ? 0 : 4);
+            }
         }
+        __pipeline_commit();
+        __pipeline_wait_prior(0);
     }
     __syncthreads();
 

@@ -434,12 +434,12 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
 // Where launch_forward_dense is the faster kernel.  Its time hardly depends on K or the batch, the gather kernels' is
 // proportional to K and (in steps of 32 to 128 columns) to the batch:
 //   * more than 32 samples (writing y; 64: 238 against 277 us, 32 with few rows: 25 against 21 us at L=20,000) or 64 (loss
-//     gradient: no gain at 64, 249 against 284 us at 128);
+//     gradient: no gain at 64 and N=768, 249 against 284 us at 128; with N <= 256 it gains at any batch);
 //   * with the loss epilogue a fan-in of at least 24 (16: 247 against 214 us);
 //   * a fan-in of at most 64 (registers of the building warps) and a quarter of the inputs: beyond, repeated inputs in a row
 //     are so frequent that their list overflows (N=150, K=40 drawn with replacement: 602 against 215 us).
 bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss) {
-    return N <= 64 * kMaxPanels && K <= 64 && 4 * K <= N && (loss ? B > 64 && K >= 24 : B > 32) && L > 0;
+    return N <= 64 * kMaxPanels && K <= 64 && 4 * K <= N && (loss ? (B > 64 || N <= 256) && K >= 24 : B > 32) && L > 0;
 }
 
 // y (or, with `loss`, the loss gradient and one loss partial per CTA) from bf16 x as [N][ldx] and bf16 W.

@@ -384,23 +384,26 @@ bool narrow_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, Narro
 // offsets (L is odd in practice), so a 256-byte row segment costs one extra 32-byte sector.
 // The launcher picks `tro` so that the blocks fill a whole number of waves over the GPU: with 64 outputs
 // per block a short L (a shard of the label dimension) leaves the last wave nearly empty.
+// BS is the batch slab: 128 columns, or the whole row of a batch of at most 64 or 32 (a slab of 128 left three threads in
+// four idle there: 69 us for 32 x 670,091, 40 us with a slab of its own).
 constexpr int kTrO = 64;        // most outputs per block
 constexpr int kTrResident = 4;  // blocks per SM (launch bound)
+template <int BS>
 __global__ void __launch_bounds__(256, kTrResident) transpose_g_kernel(const float* __restrict__ g, float* __restrict__ gT,
                                                                     float* __restrict__ gbias, int B, long long L,
                                                                     long long ldg, int tro) {
-    __shared__ float tile[128][kTrO + 1];
+    __shared__ float tile[BS][kTrO + 1];
     const int tid = threadIdx.x;
     const int tx = tid & (kTrO - 1), ty = tid / kTrO;  // load: tx = output, ty = batch row within a group of 4
-    const int bx = tid & 127, oy0 = tid >> 7;           // store: bx = batch column, oy0 = first output row
+    const int bx = tid & (BS - 1), oy0 = tid / BS;     // store: bx = batch column, oy0 = first output row
     const long long o0 = static_cast<long long>(blockIdx.x) * tro;
     const int nrows = static_cast<int>(L - o0 < tro ? L - o0 : tro);  // outputs of this block
     const bool ocol = tx < nrows;
     float colsum = 0.f;
-    for (long long bb = 0; bb < ldg; bb += 128) {
+    for (long long bb = 0; bb < ldg; bb += BS) {
         const float* src = g + static_cast<size_t>(bb + ty) * L + o0 + tx;
-#pragma unroll 16
-        for (int u = 0; u < 32; ++u) {
+#pragma unroll (BS < 64 ? BS / 4 : 16)
+        for (int u = 0; u < BS / 4; ++u) {
             const long long b = bb + ty + 4 * u;
             const float v = (ocol && b < B) ? __ldcs(src + static_cast<size_t>(4 * u) * L) : 0.f;
             tile[ty + 4 * u][tx] = v;
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(256, kTrResident) transpose_g_kernel(const flo
         if (bb + bx < ldg) {
             float* dst = gT + static_cast<size_t>(o0) * ldg + bb + bx;
 #pragma unroll 8
-            for (int oy = oy0; oy < nrows; oy += 2) dst[static_cast<size_t>(oy) * ldg] = tile[bx][oy];
+            for (int oy = oy0; oy < nrows; oy += 256 / BS) dst[static_cast<size_t>(oy) * ldg] = tile[bx][oy];
         }
         __syncthreads();
     }
@@ -441,7 +444,8 @@ int launch_transpose_g(const float* g, float* gT, float* gbias, int B, int64_t L
     tro = tro < 8 ? 8 : (tro > kTrO ? kTrO : tro);
     const long long blocks_o = ceil_div(L, tro);
     if (blocks_o > 2147483647LL) return fail(FFI_ERR_UNSUPPORTED, "L too large");
-    transpose_g_kernel<<<static_cast<unsigned>(blocks_o), 256, 0, stream>>>(g, gT, gbias, B, L, ldg, static_cast<int>(tro));
+    auto kern = ldg == 32 ? transpose_g_kernel<32> : (ldg == 64 ? transpose_g_kernel<64> : transpose_g_kernel<128>);
+    kern<<<static_cast<unsigned>(blocks_o), 256, 0, stream>>>(g, gT, gbias, B, L, ldg, static_cast<int>(tro));
     FFI_LAUNCH_CHECK("transpose_g_kernel");
     return FFI_OK;
 }
