@@ -34,10 +34,13 @@ struct FwdStreamParams {
     // top-k epilogue: every warp keeps, per batch element of the tile, the kTopK best logits of the
     // rows it computed; lists [tile][cta][warp][batch][kTopK] of (value, row) go to `topk_lists`
     uint2* topk_lists;
-    // per batch column, the highest kTopK-th best value any warp has seen so far (order_key): no final list holds less, so a
-    // warp skips what lies below.  Without it every warp sorts its own first few hundred rows' worth of insertions, a
-    // seventh of the kernel (0.60 -> 0.51 ms at B=128, N=768, L=670,091, K=32).  nullptr: few rows per warp, no sharing.
+    // per batch column and group of warps (one in kTopK), the highest logit seen so far (order_key).  The lowest of a column's
+    // kTopK groups is a bound: that many logits reach it, so a row pair whose logits all lie below it is done with.  Without
+    // it every warp sorts its own few hundred rows (0.60 ms at B=128, N=768, L=670,091, K=32); with the best kTopK-th value
+    // of any warp as the bound, which two logits in a thousand still pass, 0.51 ms; with this one, passed by about twenty per
+    // column in all, 0.48 ms.  nullptr: few rows per warp, no sharing.
     int* topk_floor;
+    int topk_stride;  // columns per group
 };
 
 // Order-preserving map of floats to signed integers; the memset value kFloorNone decodes to "no bound yet".
@@ -148,11 +151,28 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
     for (int m = 0; m < TM; ++m)
 #pragma unroll
         for (int j = 0; j < kTopK; ++j) tv[m][j] = -INFINITY, ti[m][j] = 0x7fffffff;
-    for (; qd < numQuads; qd += GW) {
-        int fl[TM];  // the shared bounds, requested ahead of their use
-        if constexpr (MODE == 2) {
+    int fq[VPL];  // MODE 2: bounds of the columns this lane computes
 #pragma unroll
-            for (int m = 0; m < TM; ++m) fl[m] = p.topk_floor ? __ldcg(p.topk_floor + b0 + lane + 32 * m) : kFloorNone;
+    for (int j = 0; j < VPL; ++j) fq[j] = kFloorNone;
+    int turn = 0;
+    for (; qd < numQuads; qd += GW) {
+        if constexpr (MODE == 2) {
+            if (p.topk_floor && (turn++ & 7) == 0) {  // the shared bounds of this lane's columns, now and then
+#pragma unroll
+                for (int j = 0; j < VPL; ++j) fq[j] = 0x7fffffff;
+#pragma unroll
+                for (int g = 0; g < kTopK; ++g) {
+                    const int* src = p.topk_floor + g * p.topk_stride + b0;
+#pragma unroll
+                    for (int j = 0; j < VPL; j += 2) {
+                        const int2 t = __ldcg(reinterpret_cast<const int2*>(src + pair_column<VPL>(q, j)));
+                        fq[j] = min(fq[j], t.x), fq[j + 1] = min(fq[j + 1], t.y);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < VPL; ++j)  // nothing passes in the padded columns
+                    if (b0 + pair_column<VPL>(q, j) >= p.B) fq[j] = order_key(INFINITY);
+            }
         }
 #pragma unroll
         for (int half = 0; half < 2; ++half, ++s) {
@@ -227,34 +247,32 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
                             else *reinterpret_cast<float2*>(dst) = make_float2(gv[0], gv[1]);
                         }
                     }
+                } else if constexpr (MODE == 2) {
+                    bool hit = p.topk_floor == nullptr;
+#pragma unroll
+                    for (int j = 0; j < VPL; ++j) hit |= acc[j] + bias >= floor_value(fq[j]);
+                    if (__any_sync(0xffffffffu, hit)) {
+                        float* yrow = ys + h * S;
+#pragma unroll
+                        for (int j = 0; j < VPL; ++j) yrow[pair_column<VPL>(q, j)] = acc[j] + bias;
+                        __syncwarp();
+#pragma unroll
+                        for (int m = 0; m < TM; ++m) {
+                            const int bl = lane + 32 * m;
+                            if (bl < BT && b0 + bl < p.B) {
+                                const float best = tv[m][0];
+#pragma unroll
+                                for (int oo = 0; oo < 2; ++oo)
+                                    if (oA + oo < L) topk_insert(tv[m], ti[m], ys[oo * S + bl], static_cast<int>(oA) + oo);
+                                if (p.topk_floor && tv[m][0] > best)
+                                    atomicMax(p.topk_floor + (gw % kTopK) * p.topk_stride + b0 + bl, order_key(tv[m][0]));
+                            }
+                        }
+                    }
                 } else {
                     float* yrow = ys + (2 * half + h) * S;
 #pragma unroll
                     for (int j = 0; j < VPL; ++j) yrow[pair_column<VPL>(q, j)] = acc[j] + bias;
-                }
-            }
-            __syncwarp();
-        }
-        if constexpr (MODE == 2) {
-            const long long oq = 4 * qd;
-#pragma unroll
-            for (int m = 0; m < TM; ++m) {
-                const int bl = lane + 32 * m;
-                if (bl < BT && b0 + bl < p.B) {
-                    const float fv = floor_value(fl[m]);
-                    bool grown = false;
-#pragma unroll
-                    for (int oo = 0; oo < 4; ++oo) {
-                        const float v = ys[oo * S + bl];
-                        if (oq + oo < L && v >= fv && topk_better(v, static_cast<int>(oq + oo), tv[m][kTopK - 1], ti[m][kTopK - 1])) {
-                            topk_insert(tv[m], ti[m], v, static_cast<int>(oq + oo));
-                            grown = true;
-                        }
-                    }
-                    if (grown && p.topk_floor) {
-                        const float kth = tv[m][kTopK - 1];  // (the kk-th would need a run-time index into registers)
-                        if (kth > fv) atomicMax(p.topk_floor + b0 + bl, order_key(kth));
-                    }
                 }
             }
             __syncwarp();
@@ -342,7 +360,7 @@ struct TopkEpilogue {
     uint2* lists;  // scratch from forward_topk_workspace_bytes
     int* ctas_x;   // out: CTAs per batch tile
     int* bt;       // out: batch tile width
-    int* floor;    // [batch padded to whole tiles] shared bounds, cleared by the launcher
+    int* floor;    // [kTopK][batch padded to whole tiles] shared bounds, cleared by the launcher
 };
 
 static int launch_forward_stream_impl(const FwdArgs& a, const BceEpilogue* bce, const TopkEpilogue* topk,
@@ -380,6 +398,7 @@ static int launch_forward_stream_impl(const FwdArgs& a, const BceEpilogue* bce, 
     p.loss_kind = bce ? bce->loss_kind : 0;
     p.topk_lists = topk ? topk->lists : nullptr;
     p.topk_floor = nullptr;
+    p.topk_stride = 0;
     const int nBT = static_cast<int>(ceil_div(a.B, 32 * bpl));
     *handled = true;
     // same tile sizes and shared-memory footprint: BT = 32 * bpl = 16 * VPL
@@ -387,7 +406,8 @@ static int launch_forward_stream_impl(const FwdArgs& a, const BceEpilogue* bce, 
         int ctas = 0;
         // sharing pays once a warp sees more rows than its list has room for a few times over
         if (a.L >= 8 * kTopK * kWarps * dev.sm_count / nBT) {
-            FFI_CUDA_CHECK(cudaMemsetAsync(topk->floor, 0x80, static_cast<size_t>(nBT) * 32 * bpl * sizeof(int), stream));
+            p.topk_stride = nBT * 32 * bpl;
+            FFI_CUDA_CHECK(cudaMemsetAsync(topk->floor, 0x80, kTopK * static_cast<size_t>(p.topk_stride) * sizeof(int), stream));
             p.topk_floor = topk->floor;
         }
         if (bpl == 4) rc = launch_pair_t<8, 2>(p, smem, nBT, dev, stream, &ctas);
@@ -434,7 +454,7 @@ static size_t topk_list_bytes(int64_t B) {
     const size_t lists = static_cast<size_t>(dev.sm_count + ceil_div(B, 32)) * kWarps;
     return lists * 128 * kTopK * sizeof(uint2);
 }
-size_t forward_topk_workspace_bytes(int64_t B) { return topk_list_bytes(B) + round_up(B, 128) * sizeof(int); }
+size_t forward_topk_workspace_bytes(int64_t B) { return topk_list_bytes(B) + kTopK * round_up(B, 128) * sizeof(int); }
 
 // Forward whose epilogue keeps the best logits per batch element instead of writing y; top_val/top_idx
 // [B][kk] receive them in tf.nn.top_k order (row + label_offset as the index).  *handled as above.
