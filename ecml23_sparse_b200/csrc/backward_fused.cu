@@ -768,6 +768,12 @@ bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedC
     return true;
 }
 
+// Whether a tile of `cols` columns has the ranges and row width of configuration c.
+bool fused_same_layout(const ffi_plan* plan, int64_t cols, const DeviceInfo& dev, const FusedConfig& c) {
+    FusedConfig o;
+    return fused_config(plan, cols, dev, &o) && o.R == c.R && o.Bpad == c.Bpad;
+}
+
 // Columns of the batch tile that starts at b0.
 int64_t tile_columns(int64_t B, int64_t b0) { return B - b0 < 128 ? B - b0 : 128; }
 
@@ -812,18 +818,17 @@ bool backward_fused_applicable(const ffi_plan* plan, int64_t B) {
 size_t backward_fused_workspace_bytes(const ffi_plan* plan, int64_t B) {
     DeviceInfo dev;
     if (get_device_info(&dev) != FFI_OK) return 0;
-    size_t most = 0;
-    for (int64_t cols : {tile_columns(B, 0), B - (B - 1) / 128 * 128}) {
+    size_t total = 0;  // the partials of every batch tile, summed by one launch at the end
+    for (int64_t b0 = 0; b0 < B; b0 += 128) {
         FusedConfig c;
-        if (!fused_config(plan, cols, dev, &c)) return 0;
-        const size_t need = static_cast<size_t>(c.R) * plan->N * c.Bpad * 4;
-        if (need > most) most = need;
+        if (!fused_config(plan, tile_columns(B, b0), dev, &c)) return 0;
+        total += static_cast<size_t>(c.R) * plan->N * c.Bpad * 4;
     }
-    return most;
+    return total;
 }
 
-int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int B, int x_transposed,
-                          cudaStream_t stream);
+int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int tiles, int B,
+                          int x_transposed, cudaStream_t stream);
 
 // grad_x (always), grad_W (when gW != nullptr) and grad_bias (when gbias != nullptr, from gT).  xT is x as [N][ldx].
 int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float* gW, float* gbias,
@@ -855,6 +860,8 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
     p.T = a.plan->chunk_rows;
     p.nChunks = a.plan->n_chunks;
     p.boxes = p.T > 256 ? 2 : 1;
+    const float* partials = p.partial;  // of the tiles not summed yet
+    int tiles = 1;
     for (int64_t b0 = 0; b0 < a.B; b0 += 128) {
         const int cols = static_cast<int>(tile_columns(a.B, b0));
         FusedConfig c;
@@ -894,9 +901,19 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         rc = b0 > 0 ? launch_tile(std::true_type{}) : launch_tile(std::false_type{});
         if (rc != FFI_OK) return rc;
         FFI_LAUNCH_CHECK("ffi_bwd_pairs_kernel");
-        rc = reduce_range_partials(p.partial, a.gx + (a.x_transposed ? b0 : b0 * a.N), c.R, a.N, cols, c.Bpad, a.B,
-                                   a.x_transposed, stream);
-        if (rc != FFI_OK) return rc;
+        // tiles of the same layout (all of 65..128 columns) are summed together, a narrower last one by itself
+        const bool last = b0 + 128 >= a.B;
+        if (!last && fused_same_layout(a.plan, tile_columns(a.B, b0 + 128), dev, c)) {
+            ++tiles;
+        } else {
+            const int64_t first = b0 - 128 * (tiles - 1);
+            rc = reduce_range_partials(partials, a.gx + (a.x_transposed ? first : first * a.N), c.R, a.N,
+                                       static_cast<int>(b0 + cols - first), c.Bpad, tiles, a.B, a.x_transposed, stream);
+            if (rc != FFI_OK) return rc;
+            partials = p.partial + static_cast<size_t>(c.R) * a.N * c.Bpad;
+            tiles = 1;
+        }
+        p.partial += static_cast<size_t>(c.R) * a.N * c.Bpad;
     }
     return FFI_OK;
 }

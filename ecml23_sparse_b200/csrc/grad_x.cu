@@ -216,6 +216,9 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_grad_x_narrow_kernel(GxNarrow
 // the 8 sums are added in warp order.  (One thread per column with a chain of R loads took 13 us at R=148, N=128; this 4.)
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ gx,
                                                               int R, int N, int cols, int Bpad, int B, int x_transposed) {
+    // blockIdx.y: batch tile, each with R partials of its own and `cols` columns (the last one what is left of them)
+    partial += static_cast<size_t>(blockIdx.y) * R * N * Bpad;
+    const int b0 = blockIdx.y * Bpad;
     __shared__ double part[8][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long id = static_cast<long long>(blockIdx.x) * 32 + lane;  // Bpad is a multiple of 32: no tail
@@ -238,9 +241,9 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
     for (int w = 1; w < 8; ++w) s += part[w][lane];
     const int i = static_cast<int>(id / Bpad);
     const int b = static_cast<int>(id - static_cast<long long>(i) * Bpad);
-    if (b >= cols) return;
-    if (x_transposed) gx[static_cast<size_t>(i) * B + b] = static_cast<float>(s);
-    else gx[static_cast<size_t>(b) * N + i] = static_cast<float>(s);
+    if (b0 + b >= cols) return;
+    if (x_transposed) gx[static_cast<size_t>(i) * B + b0 + b] = static_cast<float>(s);
+    else gx[static_cast<size_t>(b0 + b) * N + i] = static_cast<float>(s);
 }
 
 // ---- wide inputs -------------------------------------------------------------------
@@ -476,10 +479,10 @@ size_t grad_x_min_workspace_bytes(const ffi_plan* plan, int64_t B) {
 }
 
 // Shared with the one-pass backward: see reduce_partials_kernel.
-int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int B, int x_transposed,
-                          cudaStream_t stream) {
-    const long long blocks = static_cast<long long>(N) * Bpad / 32;
-    reduce_partials_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(partial, gx, R, N, cols, Bpad, B, x_transposed);
+int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int tiles, int B,
+                          int x_transposed, cudaStream_t stream) {
+    const dim3 grid(static_cast<unsigned>(static_cast<long long>(N) * Bpad / 32), static_cast<unsigned>(tiles));
+    reduce_partials_kernel<<<grid, 256, 0, stream>>>(partial, gx, R, N, cols, Bpad, B, x_transposed);
     FFI_LAUNCH_CHECK("reduce_partials_kernel");
     return FFI_OK;
 }
@@ -526,7 +529,7 @@ int launch_grad_x(const GradXArgs& a, cudaStream_t stream) {
         else if (c.bpl == 2) rc = launch_narrow_t<32, 2>(p, c.smem, c.iparts, c.nBT, stream);
         else rc = launch_narrow_t<64, 1>(p, c.smem, c.iparts, c.nBT, stream);
         if (rc != FFI_OK) return rc;
-        return reduce_range_partials(p.partial, a.gx, c.R * c.S, a.N, a.B, c.Bpad, a.B, a.x_transposed, stream);
+        return reduce_range_partials(p.partial, a.gx, c.R * c.S, a.N, a.B, c.Bpad, 1, a.B, a.x_transposed, stream);
     }
 
     // Wide inputs: one warp per (input, batch tile) over the canonical index, batch tile by batch tile.
