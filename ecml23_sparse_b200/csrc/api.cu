@@ -348,6 +348,14 @@ extern "C" int ffi_forward(const void* x, const int32_t* idx, const void* W, con
     return launch_forward(a, stream);
 }
 
+extern "C" int ffi_transpose_features(const float* x, float* xT, int64_t B, int64_t N, void* stream_v) {
+    FFI_TRACE("ffi_transpose_features");
+    if (!x || !xT) return fail(FFI_ERR_INVALID_ARGUMENT, "NULL tensor passed to ffi_transpose_features");
+    const int rc = check_shape(B, N, 1, 1);
+    if (rc != FFI_OK) return rc;
+    return launch_transpose_pad(x, xT, static_cast<int>(B), static_cast<int>(N), B, static_cast<cudaStream_t>(stream_v));
+}
+
 extern "C" int64_t ffi_transposed_gradient_stride(int64_t B) { return B > 0 ? transposed_g_stride(B) : 0; }
 
 extern "C" int ffi_transpose_gradient(const float* g, float* gT, float* grad_bias, int64_t B, int64_t L,

@@ -102,6 +102,14 @@ Tensor cuda_matrix(const char* name, const Tensor& t, bool float_only) {
     return t.contiguous();
 }
 
+// units, fan_in >= 0: the table or the weights come as a layer's flat vector of that many connections.
+Tensor flat_vector(const char* name, const Tensor& t, int64_t units, int64_t fan_in) {
+    if (!t.is_cuda()) throw py::value_error(std::string(name) + " must be a CUDA tensor: this library has no CPU path");
+    if (t.dim() != 1 || t.size(0) != units * fan_in)
+        throw py::value_error(std::string(name) + " must be a vector of units * fan_in elements, got shape " + shape_text(t));
+    return t.contiguous();
+}
+
 Tensor index_matrix(const Tensor& t) {
     if (!t.is_cuda()) throw py::value_error("lookup must be a CUDA tensor: this library has no CPU path");
     if (t.scalar_type() != at::kInt && t.scalar_type() != at::kUInt32)
@@ -117,21 +125,24 @@ struct Operands {
     const int32_t* idx_ptr() const { return static_cast<const int32_t*>(idx.const_data_ptr()); }
 };
 
-Operands operands(const Tensor& features, const Tensor& lookup, const Tensor& weights, bool transposed) {
+Operands operands(const Tensor& features, const Tensor& lookup, const Tensor& weights, bool transposed, int64_t units = -1,
+                  int64_t fan_in = -1) {
     Operands o;
+    const bool flat = units >= 0;
     o.x = cuda_matrix("features", features, false);
-    o.W = cuda_matrix("weights", weights, false);
+    o.W = flat ? flat_vector("weights", weights, units, fan_in) : cuda_matrix("weights", weights, false);
     if (o.x.scalar_type() != o.W.scalar_type())
         throw py::type_error(std::string("features (") + c10::toString(o.x.scalar_type()) + ") and weights (" +
                              c10::toString(o.W.scalar_type()) + ") must have the same dtype");
     o.dtype = o.x.scalar_type() == at::kBFloat16 ? FFI_BF16 : FFI_F32;
-    o.idx = index_matrix(lookup);
+    if (flat && lookup.scalar_type() != at::kInt) throw py::type_error("the layer's table must be int32");
+    o.idx = flat ? flat_vector("lookup", lookup, units, fan_in) : index_matrix(lookup);
     if (o.idx.sizes() != o.W.sizes())
         throw py::value_error("lookup " + shape_text(o.idx) + " and weights " + shape_text(o.W) + " must have equal shapes");
     o.B = o.x.size(transposed ? 1 : 0);
     o.N = o.x.size(transposed ? 0 : 1);
-    o.L = o.W.size(0);
-    o.K = o.W.size(1);
+    o.L = flat ? units : o.W.size(0);
+    o.K = flat ? fan_in : o.W.size(1);
     return o;
 }
 
@@ -149,8 +160,7 @@ OptTensor checked_bias(const OptTensor& bias, int64_t L) {
 }
 
 // ---- the operations ----------------------------------------------------------------------------------------
-Tensor forward(const Tensor& features, const Tensor& lookup, const Tensor& weights, const OptTensor& bias_in, bool transposed) {
-    const Operands o = operands(features, lookup, weights, transposed);
+Tensor run_forward(const Operands& o, const OptTensor& bias_in, bool transposed) {
     const OptTensor bias = checked_bias(bias_in, o.L);
     const c10::cuda::CUDAGuard guard(o.x.device());
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream(o.x.device().index());
@@ -163,11 +173,13 @@ Tensor forward(const Tensor& features, const Tensor& lookup, const Tensor& weigh
     return out;
 }
 
-std::tuple<OptTensor, OptTensor, OptTensor> backward(const Tensor& features, const Tensor& lookup, const Tensor& weights,
-                                                     const Tensor& out_grad, bool transposed, uintptr_t plan_handle,
-                                                     bool want_x, bool want_w, bool want_b, bool grad_is_transposed,
-                                                     const OptTensor& gx_out) {
-    const Operands o = operands(features, lookup, weights, transposed);
+Tensor forward(const Tensor& features, const Tensor& lookup, const Tensor& weights, const OptTensor& bias, bool transposed) {
+    return run_forward(operands(features, lookup, weights, transposed), bias, transposed);
+}
+
+std::tuple<OptTensor, OptTensor, OptTensor> run_backward(const Operands& o, const Tensor& out_grad, bool transposed,
+                                                         uintptr_t plan_handle, bool want_x, bool want_w, bool want_b,
+                                                         bool grad_is_transposed, const OptTensor& gx_out) {
     const Tensor g = cuda_matrix("out_grad", out_grad, true);
     if (grad_is_transposed) {
         if (g.size(0) != o.L || g.size(1) < o.B)
@@ -208,6 +220,14 @@ std::tuple<OptTensor, OptTensor, OptTensor> backward(const Tensor& features, con
                                       o.L, o.K, transposed, o.dtype, ws, len, stream);
         }));
     return {gx, gw, gb};
+}
+
+std::tuple<OptTensor, OptTensor, OptTensor> backward(const Tensor& features, const Tensor& lookup, const Tensor& weights,
+                                                     const Tensor& out_grad, bool transposed, uintptr_t plan_handle,
+                                                     bool want_x, bool want_w, bool want_b, bool grad_is_transposed,
+                                                     const OptTensor& gx_out) {
+    return run_backward(operands(features, lookup, weights, transposed), out_grad, transposed, plan_handle, want_x, want_w,
+                        want_b, grad_is_transposed, gx_out);
 }
 
 Tensor device_int32(const Tensor& t, const at::Device& dev) {
@@ -314,41 +334,40 @@ struct PlanRef {
 struct FanInSparseMatmul : public torch::autograd::Function<FanInSparseMatmul> {
     static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& features, const Tensor& lookup,
                           const Tensor& weights, const OptTensor& bias, bool transposed, bool layer, int64_t units, int64_t fan_in) {
-        const Tensor x = layer ? features.t().contiguous() : features;
-        const Tensor idx = layer ? lookup.view({units, fan_in}) : lookup;
-        const Tensor W = layer ? weights.view({units, fan_in}) : weights;
-        ctx->saved_data["transposed"] = transposed;
-        ctx->saved_data["layer"] = layer;
-        ctx->saved_data["bias"] = bias && bias->defined();
-        if (layer) {
-            // x is this node's own transposed copy; table and weights are saved as the caller's tensors, so that an
-            // in-place change between forward and backward is noticed
-            ctx->saved_data["units"] = units;
-            ctx->saved_data["fan_in"] = fan_in;
-        }
+        const Tensor x = layer ? turned(features) : features;
+        ctx->saved_data["flags"] = static_cast<int64_t>(transposed) | (layer ? 2 : 0) | (bias && bias->defined() ? 4 : 0);
+        // of a layer x is this node's own transposed copy; table and weights are saved as the caller's tensors, so that an
+        // in-place change between forward and backward is noticed
         ctx->save_for_backward({x, lookup, weights});
-        return ::forward(x, idx, W, bias, transposed);
+        return run_forward(operands(x, lookup, weights, transposed, layer ? units : -1, fan_in), bias, transposed);
     }
 
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
         const auto saved = ctx->get_saved_variables();
-        const bool transposed = ctx->saved_data["transposed"].toBool(), layer = ctx->saved_data["layer"].toBool();
+        const int64_t flags = ctx->saved_data["flags"].toInt();
+        const bool transposed = flags & 1, layer = flags & 2;
         const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(2);
-        const bool need_b = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(3);
-        Tensor idx = saved[1], W = saved[2];
-        if (layer) {
-            const int64_t units = ctx->saved_data["units"].toInt(), fan_in = ctx->saved_data["fan_in"].toInt();
-            idx = idx.view({units, fan_in});
-            W = W.detach().view({units, fan_in});
-        }
+        const bool need_b = (flags & 4) && ctx->needs_input_grad(3);
+        const int64_t units = layer ? grads[0].size(1) : -1, fan_in = layer ? saved[2].numel() / units : -1;
         std::optional<PlanRef> plan;
-        if (need_x) plan.emplace(idx, saved[0].size(transposed ? 0 : 1));
-        auto [gx, gw, gb] = ::backward(saved[0], idx, W, grads[0], transposed, plan ? plan->handle : 0, need_x, need_w, need_b,
-                                       false, std::nullopt);
+        if (need_x) plan.emplace(layer ? saved[1].view({units, fan_in}) : saved[1], saved[0].size(transposed ? 0 : 1));
+        auto [gx, gw, gb] = run_backward(operands(saved[0], saved[1], saved[2], transposed, units, fan_in), grads[0], transposed,
+                                         plan ? plan->handle : 0, need_x, need_w, need_b, false, std::nullopt);
         torch::autograd::variable_list out(8);
         if (gx) out[0] = layer ? gx->t() : *gx;
         if (gw) out[2] = layer ? gw->view({-1}) : *gw;
         if (gb) out[3] = *gb;
+        return out;
+    }
+
+    // [B,N] -> a contiguous [N,B] (sparse/custom_layer.py:48)
+    static Tensor turned(const Tensor& x) {
+        if (!x.is_cuda() || x.scalar_type() != at::kFloat || x.dim() != 2 || !x.is_contiguous() || x.numel() == 0)
+            return x.t().contiguous();
+        const c10::cuda::CUDAGuard guard(x.device());
+        Tensor out = f32({x.size(1), x.size(0)}, x.device());
+        check(ffi_transpose_features(x.const_data_ptr<float>(), out.data_ptr<float>(), x.size(0), x.size(1),
+                                     c10::cuda::getCurrentCUDAStream(x.device().index())));
         return out;
     }
 };

@@ -80,6 +80,12 @@ int ffi_forward(const void* x, const int32_t* idx, const void* W, const float* b
                 int64_t B, int64_t N, int64_t L, int64_t K, int x_transposed, int dtype,
                 void* workspace, size_t workspace_bytes, void* stream);
 
+/*
+ * x[B,N] -> xT[N,B] (fp32): the transposition in front of the transposed op in the reference's layer
+ * (sparse/custom_layer.py:48).
+ */
+int ffi_transpose_features(const float* x, float* xT, int64_t B, int64_t N, void* stream);
+
 /* ------------------------------------------------------------------- plan ---- */
 
 /*
