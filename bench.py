@@ -764,11 +764,10 @@ def run_ours(args):
         "backward_fused": (4 * B * Ls + (4 + esize) * Ls * K + 4 * Ls * K + (4 + esize) * B * N, 2 * fma_pass),
     }
     narrow = N <= 2048  # the plan holds the chunked index the one-pass backward walks; x tiles fit shared memory
-    names = {"forward": ("ffi_fwd_bf16_kernel" if args.storage == "bf16" and B <= 128 and K % 8 == 0 else
-                         "ffi_fwd_pair_kernel") if narrow else "ffi_fwd_kernel",
+    names = {"forward": ("ffi_fwd_dense_kernel" if args.storage == "bf16" else "ffi_fwd_pair_kernel") if narrow
+             else "ffi_fwd_gather_kernel",
              "transpose_g": "transpose_g_kernel",
-             "backward_fused": ("ffi_bwd_pairs_kernel" if B > 64 else "ffi_bwd_fused_kernel") if narrow
-             else "ffi_grad_w_kernel + ffi_grad_x_wide_kernel"}
+             "backward_fused": "ffi_bwd_pairs_kernel" if narrow else "ffi_grad_w_gather_kernel + ffi_grad_x_wide_kernel"}
     kernels = {}
     for name, ms in kernel_ms.items():
         nbytes, fmas = work[name]

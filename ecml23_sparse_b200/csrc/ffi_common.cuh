@@ -260,6 +260,7 @@ struct ffi_plan {
     bool has_chunks = false;
     // largest number of entries any (chunk, slice) holds, for the slicings fused_slices(N, 0 / 1)
     int max_slice_entries[2] = {0, 0};
+    void* arrays = nullptr;     // the allocation that holds the four index arrays
     int32_t* rowptr = nullptr;  // [N+1]   canonical CSR-by-input
     int32_t* perm = nullptr;    // [L*K]   positions sorted by (idx[p], p)
     int32_t* cperm = nullptr;   // [L*K]   chunk-major: chunk c holds its T*K positions sorted by (idx[p], p)

@@ -543,19 +543,22 @@ extern "C" int ffi_plan_create(const int32_t* idx, int64_t L, int64_t K, int64_t
     FFI_CUDA_CHECK(cudaGetDevice(&plan->device));
     const PlanLayout g = plan_layout(L, K, N);
 
-    if (cudaMalloc(&plan->rowptr, (N + 1) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&plan->perm, g.n * sizeof(int)) != cudaSuccess) {
+    // the index arrays are one allocation: a cudaMalloc and a cudaFree of this size take about a millisecond each
+    const size_t rowptr_at = 0, perm_at = rowptr_at + scratch_up((N + 1) * sizeof(int)), cptr_at = perm_at + scratch_up(g.n * 4);
+    const size_t cperm_at = cptr_at + (g.chunks ? scratch_up(g.cptrBytes) : 0), total = cperm_at + (g.chunks ? scratch_up(g.n * 4) : 0);
+    if (cudaMalloc(&plan->arrays, total) != cudaSuccess) {
         cudaGetLastError();
+        plan->arrays = nullptr;
         return fail(FFI_ERR_ALLOC, "cudaMalloc of the transposed index failed");
     }
-    plan->device_bytes = (N + 1) * sizeof(int) + g.n * sizeof(int);
+    unsigned char* base = static_cast<unsigned char*>(plan->arrays);
+    plan->rowptr = reinterpret_cast<int32_t*>(base + rowptr_at);
+    plan->perm = reinterpret_cast<int32_t*>(base + perm_at);
     if (g.chunks) {
-        if (cudaMalloc(&plan->cptr, g.cptrBytes) != cudaSuccess || cudaMalloc(&plan->cperm, g.n * 4) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(FFI_ERR_ALLOC, "cudaMalloc of the chunked index failed");
-        }
-        plan->device_bytes += g.cptrBytes + g.n * 4;
+        plan->cptr = reinterpret_cast<int32_t*>(base + cptr_at);
+        plan->cperm = reinterpret_cast<int32_t*>(base + cperm_at);
     }
+    plan->device_bytes = total;
     DeviceBuffer scratch;
     if (scratch.alloc(g.total) != cudaSuccess) {
         cudaGetLastError();
@@ -587,10 +590,7 @@ extern "C" int ffi_plan_rebuild(ffi_plan* plan, const int32_t* idx, void* stream
 
 extern "C" int ffi_plan_destroy(ffi_plan* plan) {
     if (!plan) return FFI_OK;
-    if (plan->rowptr) cudaFree(plan->rowptr);
-    if (plan->perm) cudaFree(plan->perm);
-    if (plan->cperm) cudaFree(plan->cperm);
-    if (plan->cptr) cudaFree(plan->cptr);
+    if (plan->arrays) cudaFree(plan->arrays);
     if (plan->build_scratch) cudaFree(plan->build_scratch);
     delete plan;
     return FFI_OK;
