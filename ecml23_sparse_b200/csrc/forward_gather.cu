@@ -20,7 +20,7 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-// rows of results a warp collects before it writes y (fewer for the widest lanes, whose rows are twice as long)
+// rows of results a warp collects before it writes y, at most (fewer for the widest lanes, whose rows are twice as long)
 template <int BPL>
 struct ResultRows {
     static constexpr int value = BPL == 8 ? 4 : 8;
@@ -34,6 +34,7 @@ struct FwdGatherParams {
     const float* bias;
     float* y;
     int B, N, L, K;
+    int row_bits;  // log2 of the rows a warp takes at a time
     // loss epilogue (MODE 1), as in the tiled kernel: gT[o][b] = scale * dloss/dz for target 0, zero in the padded
     // batch columns up to ldg, and one partial sum of the loss values per CTA
     float* gT;
@@ -64,13 +65,20 @@ __device__ __forceinline__ void fma_lane(float (&acc)[BPL], float w, const typen
     }
 }
 
-template <int BPL, int MODE, typename TX>
+// Words of a staged W row.  ODD: the rows do not start on 16-byte boundaries (K % 4 != 0, K % 8 != 0 for bf16, or a ragged
+// base) and are copied word by word; a bf16 row may start in the upper half of its first word.
+template <typename TX, bool ODD>
+__host__ __device__ constexpr int staged_w_words(int K) {
+    if (!ODD) return std::is_same<TX, float>::value ? K : K / 2;
+    return ((std::is_same<TX, float>::value ? K : K / 2 + 1) + 3) & ~3;
+}
+
+template <int BPL, int MODE, typename TX, bool ODD>
 __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherParams p) {
     constexpr int BT = 32 * BPL;
     constexpr int S = BT + 4;  // row stride of the result tile
     constexpr int kRows = ResultRows<BPL>::value;
     constexpr bool kBf16 = !std::is_same<TX, float>::value;
-    constexpr int WPE = kBf16 ? 2 : 1;  // weights per 32-bit word of a staged W row
     using V = typename Vec<BPL>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
@@ -78,8 +86,8 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
     const int K = p.K, L = p.L;
     const int b0 = blockIdx.y * BT;
     // per warp: two (W row, idx row) buffers, then the result tile (MODE 0)
-    const int wWords = K / WPE;
-    const int rowWords = wWords + K;
+    const int wWords = staged_w_words<TX, ODD>(K);
+    const int rowWords = wWords + (ODD ? (K + 3) & ~3 : K);
     const int warpWords = 2 * rowWords + (MODE == 0 ? kRows * S : 0);
     unsigned* wbuf = reinterpret_cast<unsigned*>(smem_raw) + static_cast<size_t>(warp) * warpWords;
     float* ys = reinterpret_cast<float*>(wbuf + 2 * rowWords);
@@ -87,13 +95,28 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
     const TX* xg = static_cast<const TX*>(p.xT) + b0;
     const size_t ldv = static_cast<size_t>(p.ldx / BPL);
     const long long GW = static_cast<long long>(gridDim.x) * kWarps;
-    // a warp takes blocks of kRows consecutive rows, so that its results leave as runs along o
-    const long long numBlocks = (static_cast<long long>(L) + kRows - 1) / kRows;
+    const int rows = 1 << p.row_bits;
+    // a warp takes blocks of `rows` consecutive rows, so that its results leave as runs along o
+    const long long numBlocks = (static_cast<long long>(L) + rows - 1) >> p.row_bits;
     long long blk = static_cast<long long>(blockIdx.x) * kWarps + warp;
 
     auto issue = [&](long long row, int buf) {
         if (row < L) {
             unsigned* dst = wbuf + buf * rowWords;
+            if constexpr (ODD) {
+                const long long e0 = row * K;
+                if constexpr (kBf16) {  // the words that hold elements e0 .. e0 + K - 1, none of them past the end of W
+                    const unsigned* wsrc = static_cast<const unsigned*>(p.W) + e0 / 2;
+                    const int n = static_cast<int>((e0 + K + 1) / 2 - e0 / 2);
+                    const bool cut = row + 1 == L && ((e0 + K) & 1);
+                    for (int c = lane; c < n; c += 32) __pipeline_memcpy_async(dst + c, wsrc + c, 4, cut && c == n - 1 ? 2 : 0);
+                } else {
+                    for (int c = lane; c < K; c += 32) __pipeline_memcpy_async(dst + c, static_cast<const unsigned*>(p.W) + e0 + c, 4);
+                }
+                for (int c = lane; c < K; c += 32) __pipeline_memcpy_async(dst + wWords + c, p.idx + e0 + c, 4);
+                __pipeline_commit();
+                return;
+            }
             const unsigned* wsrc = reinterpret_cast<const unsigned*>(static_cast<const TX*>(p.W) + row * K);
             for (int c = lane; c < wWords / 4; c += 32) __pipeline_memcpy_async(dst + 4 * c, wsrc + 4 * c, 16);
             for (int c = lane; c < K / 4; c += 32)
@@ -112,20 +135,21 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
 
     float loss_local = 0.f;
     int s = 0;
-    if (blk < numBlocks) issue(blk * kRows, 0);
+    if (blk < numBlocks) issue(blk << p.row_bits, 0);
     for (; blk < numBlocks; blk += GW) {
-        const long long o0 = blk * kRows;
+        const long long o0 = blk << p.row_bits;
 #pragma unroll 1
-        for (int r = 0; r < kRows; ++r, s ^= 1) {
+        for (int r = 0; r < rows; ++r, s ^= 1) {
             const long long o = o0 + r;
             // the row after this one: the next of the block, or the first row of the warp's next block
-            const long long next = r + 1 < kRows ? o + 1 : (blk + GW) * kRows;
+            const long long next = r + 1 < rows ? o + 1 : (blk + GW) << p.row_bits;
             issue(next, s ^ 1);
             __pipeline_wait_prior(1);
             __syncwarp();
             if (o < L) {
                 const unsigned* wr = wbuf + s * rowWords;
                 const int* ir = reinterpret_cast<const int*>(wr + wWords);
+                const int w0 = ODD && kBf16 ? static_cast<int>((o * K) & 1) : 0;  // element of the first word that the row starts with
                 float acc[BPL];
 #pragma unroll
                 for (int j = 0; j < BPL; ++j) acc[j] = 0.f;
@@ -138,17 +162,21 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
 #pragma unroll
                     for (int u = 0; u < 8; ++u) v[u] = load_lane_vec<BPL>(xg, static_cast<size_t>(ii[u]) * ldv + lane);
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) fma_lane<BPL>(acc, weight(wr, k + u), v[u]);
+                    for (int u = 0; u < 8; ++u) fma_lane<BPL>(acc, weight(wr, k + u + w0), v[u]);
                 }
-                if (k < K) {  // four entries left
+                if (ODD ? k + 4 <= K : k < K) {
                     const int4 i0 = *reinterpret_cast<const int4*>(ir + k);
                     const int ii[4] = {i0.x, i0.y, i0.z, i0.w};
                     V v[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) v[u] = load_lane_vec<BPL>(xg, static_cast<size_t>(ii[u]) * ldv + lane);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) fma_lane<BPL>(acc, weight(wr, k + u), v[u]);
+                    for (int u = 0; u < 4; ++u) fma_lane<BPL>(acc, weight(wr, k + u + w0), v[u]);
+                    k += 4;
                 }
+                if constexpr (ODD)
+                    for (; k < K; ++k)
+                        fma_lane<BPL>(acc, weight(wr, k + w0), load_lane_vec<BPL>(xg, static_cast<size_t>(ir[k]) * ldv + lane));
                 const float bias = p.bias ? __ldg(p.bias + o) : 0.f;
                 if constexpr (MODE == 1) {
                     float gv[BPL];
@@ -172,12 +200,11 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
             __syncwarp();
         }
         if constexpr (MODE == 0) {
-            // kRows consecutive lanes write the kRows outputs of one batch row: 32- or 16-byte runs along o
-            const int rows = static_cast<int>(L - o0 < kRows ? L - o0 : kRows);
-            const int oo = lane & (kRows - 1);
+            // `rows` consecutive lanes write the outputs of one batch row: 32- or 16-byte runs along o
+            const int oo = lane & (rows - 1);
 #pragma unroll 4
-            for (int bl = lane / kRows; bl < BT; bl += 32 / kRows)
-                if (b0 + bl < p.B && oo < rows) p.y[static_cast<size_t>(b0 + bl) * L + o0 + oo] = ys[oo * S + bl];
+            for (int bl = lane >> p.row_bits; bl < BT; bl += 32 >> p.row_bits)
+                if (b0 + bl < p.B && o0 + oo < L) p.y[static_cast<size_t>(b0 + bl) * L + o0 + oo] = ys[oo * S + bl];
             __syncwarp();
         }
     }
@@ -200,21 +227,24 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
     }
 }
 
-template <int BPL, int MODE, typename TX>
-int launch_fwd_gather_t(const FwdGatherParams& p, int nBT, int max_partials, const DeviceInfo& dev, cudaStream_t stream,
+template <int BPL, int MODE, typename TX, bool ODD>
+int launch_fwd_gather_t(FwdGatherParams p, int nBT, int max_partials, const DeviceInfo& dev, cudaStream_t stream,
                         int* ctas_out) {
     constexpr int BT = 32 * BPL;
     constexpr int kRows = ResultRows<BPL>::value;
-    constexpr int WPE = std::is_same<TX, float>::value ? 1 : 2;
-    auto kern = ffi_fwd_gather_kernel<BPL, MODE, TX>;
-    const size_t warpWords = 2 * static_cast<size_t>(p.K / WPE + p.K) + (MODE == 0 ? kRows * (BT + 4) : 0);
+    auto kern = ffi_fwd_gather_kernel<BPL, MODE, TX, ODD>;
+    const size_t warpWords = 2 * static_cast<size_t>(staged_w_words<TX, ODD>(p.K) + (ODD ? (p.K + 3) & ~3 : p.K)) + (MODE == 0 ? kRows * (BT + 4) : 0);
     const size_t smem = kWarps * warpWords * 4;
     int occ = 0;
     FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "forward gather kernel does not fit on an SM (smem %zu)", smem);
-    const long long want = ceil_div(ceil_div(p.L, kRows), kWarps);
     long long per_bt = static_cast<long long>(dev.sm_count) * occ / nBT;
     if (per_bt < 1) per_bt = 1;
+    // a table too short for every warp to get kRows rows is spread over more of them: the rows of a warp are a serial chain
+    // of trips to L2 (B=85, N=24,896, L=728, K=40 bf16: 27.6 us with eight rows each, 5.4 with one)
+    p.row_bits = 0;
+    while ((2 << p.row_bits) <= kRows && (p.L >> (p.row_bits + 1)) >= per_bt * kWarps) ++p.row_bits;
+    const long long want = ceil_div(ceil_div(p.L, 1 << p.row_bits), kWarps);
     dim3 grid(static_cast<unsigned>(want < per_bt ? want : per_bt), static_cast<unsigned>(nBT));
     if (MODE == 1 && static_cast<long long>(grid.x) * grid.y > max_partials)
         return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %d per-CTA partials; this batch needs %u",
@@ -225,18 +255,27 @@ int launch_fwd_gather_t(const FwdGatherParams& p, int nBT, int max_partials, con
     return FFI_OK;
 }
 
-template <int MODE, typename TX>
+template <int MODE, typename TX, bool ODD>
 int launch_fwd_gather_b(const FwdGatherParams& p, int bpl, int nBT, int max_partials, const DeviceInfo& dev,
                         cudaStream_t stream, int* ctas_out) {
-    if (bpl == 4) return launch_fwd_gather_t<4, MODE, TX>(p, nBT, max_partials, dev, stream, ctas_out);
-    if (bpl == 2) return launch_fwd_gather_t<2, MODE, TX>(p, nBT, max_partials, dev, stream, ctas_out);
-    return launch_fwd_gather_t<1, MODE, TX>(p, nBT, max_partials, dev, stream, ctas_out);
+    if constexpr (!std::is_same<TX, float>::value)
+        if (bpl == 8) return launch_fwd_gather_t<8, MODE, TX, ODD>(p, nBT, max_partials, dev, stream, ctas_out);
+    if (bpl == 4) return launch_fwd_gather_t<4, MODE, TX, ODD>(p, nBT, max_partials, dev, stream, ctas_out);
+    if (bpl == 2) return launch_fwd_gather_t<2, MODE, TX, ODD>(p, nBT, max_partials, dev, stream, ctas_out);
+    return launch_fwd_gather_t<1, MODE, TX, ODD>(p, nBT, max_partials, dev, stream, ctas_out);
+}
+
+template <int MODE, typename TX>
+int launch_fwd_gather_m(const FwdGatherParams& p, bool odd, int bpl, int nBT, int max_partials, const DeviceInfo& dev,
+                        cudaStream_t stream, int* ctas_out) {
+    if (odd) return launch_fwd_gather_b<MODE, TX, true>(p, bpl, nBT, max_partials, dev, stream, ctas_out);
+    return launch_fwd_gather_b<MODE, TX, false>(p, bpl, nBT, max_partials, dev, stream, ctas_out);
 }
 
 }  // namespace
 
-// Takes the shapes the tiled kernel would gather from L2 for (x too wide for shared memory) when K is a multiple
-// of 4 (8 for bf16 storage) and the rows are aligned; *handled tells the caller.  With gT set it writes the loss
+// Takes the shapes the tiled kernel would gather from L2 for (x too wide for shared memory) when the rows of
+// x are aligned and W starts on a word; *handled tells the caller.  With gT set it writes the loss
 // gradient and per-CTA loss partials (at most max_partials; *ctas receives their number) instead of y.
 int launch_forward_gather(const FwdArgs& a, int bpl, float* gT, int64_t ldg, float scale, double* loss_partials,
                           int loss_kind, int max_partials, int* ctas, cudaStream_t stream, bool* handled) {
@@ -249,13 +288,15 @@ int launch_forward_gather(const FwdArgs& a, int bpl, float* gT, int64_t ldg, flo
     if (a.bf16 && bpl == 4 && a.B > 128 && a.ldx % 256 == 0 && (!gT || ldg % 256 == 0)) bpl = 8;
     const int BT = 32 * bpl;
     const int nBT = static_cast<int>(ceil_div(a.B, BT));
-    const int kq = a.bf16 ? 8 : 4;
-    if (a.K % kq != 0 || reinterpret_cast<uintptr_t>(a.idx) % 16 != 0 || reinterpret_cast<uintptr_t>(a.W) % 16 != 0 ||
-        a.ldx % BT != 0 || a.ldx < static_cast<int64_t>(nBT) * BT || reinterpret_cast<uintptr_t>(a.xT) % 16 != 0)
+    const bool odd = a.K % (a.bf16 ? 8 : 4) != 0 || reinterpret_cast<uintptr_t>(a.idx) % 16 != 0 || reinterpret_cast<uintptr_t>(a.W) % 16 != 0;
+    if (reinterpret_cast<uintptr_t>(a.W) % 4 != 0 || a.ldx % BT != 0 || a.ldx < static_cast<int64_t>(nBT) * BT || reinterpret_cast<uintptr_t>(a.xT) % 16 != 0)
         return FFI_OK;
     if (gT && (ldg % bpl != 0 || ldg > static_cast<int64_t>(nBT) * BT || reinterpret_cast<uintptr_t>(gT) % 16 != 0 ||
                (ldg * 4) % 16 != 0))
         return FFI_OK;
+    // sixteen warps' buffers have to fit an SM (fan-ins up to about six hundred)
+    const int Kp = static_cast<int>(round_up(a.K, 4)) + 4;
+    if (static_cast<size_t>(kWarps) * (4 * Kp + (gT ? 0 : 8 * (BT + 4))) * 4 > static_cast<size_t>(dev.max_smem_optin)) return FFI_OK;
     FwdGatherParams p;
     p.xT = a.xT;
     p.ldx = a.ldx;
@@ -273,16 +314,12 @@ int launch_forward_gather(const FwdArgs& a, int bpl, float* gT, int64_t ldg, flo
     p.loss_partials = loss_partials;
     p.loss_kind = loss_kind;
     *handled = true;
-    if (bpl == 8) {
-        if (gT) return launch_fwd_gather_t<8, 1, __nv_bfloat16>(p, nBT, max_partials, dev, stream, ctas);
-        return launch_fwd_gather_t<8, 0, __nv_bfloat16>(p, nBT, max_partials, dev, stream, ctas);
-    }
     if (a.bf16) {
-        if (gT) return launch_fwd_gather_b<1, __nv_bfloat16>(p, bpl, nBT, max_partials, dev, stream, ctas);
-        return launch_fwd_gather_b<0, __nv_bfloat16>(p, bpl, nBT, max_partials, dev, stream, ctas);
+        if (gT) return launch_fwd_gather_m<1, __nv_bfloat16>(p, odd, bpl, nBT, max_partials, dev, stream, ctas);
+        return launch_fwd_gather_m<0, __nv_bfloat16>(p, odd, bpl, nBT, max_partials, dev, stream, ctas);
     }
-    if (gT) return launch_fwd_gather_b<1, float>(p, bpl, nBT, max_partials, dev, stream, ctas);
-    return launch_fwd_gather_b<0, float>(p, bpl, nBT, max_partials, dev, stream, ctas);
+    if (gT) return launch_fwd_gather_m<1, float>(p, odd, bpl, nBT, max_partials, dev, stream, ctas);
+    return launch_fwd_gather_m<0, float>(p, odd, bpl, nBT, max_partials, dev, stream, ctas);
 }
 
 }  // namespace ffi

@@ -1,5 +1,5 @@
 // Forward of the fixed-fan-in sparse layer, barrier-free variant for the common case
-// (x tile resident in shared memory, K a multiple of 4, 16-byte aligned W and idx).
+// (fp32 storage, x tile resident in shared memory).
 //
 // Same arithmetic as ffi_fwd_kernel (forward.cu), but every warp is its own pipeline: it owns a private double buffer for the W/idx rows of
 // the next row pair (filled by the warp's own cp.async: 2 rows x (W + idx) of K=32 are
@@ -23,6 +23,7 @@ struct FwdStreamParams {
     const float* bias;
     float* y;
     int B, N, L, K;
+    int Kp;  // K rounded up to a multiple of 4: row stride in the warps' buffers
     // fused sigmoid-BCE epilogue (BCE variant): instead of y the kernel writes the loss gradient,
     // already transposed, gT[o][b] = scale * sigmoid(z[b,o]) (positives are corrected afterwards),
     // and one partial sum of softplus(z) per CTA
@@ -67,7 +68,12 @@ __device__ __forceinline__ int pair_column(int q, int j) {
 
 // (Keeping the indices as 16-bit values in the warp's buffer, four per 8-byte access, was measured:
 // the repacking on the way in costs more than the narrower fetch saves, 0.50 vs 0.48 ms.)
-template <int VPL, int MODE>
+//
+// ODD: K is not a multiple of 4, or W or idx not 16-byte aligned.  The rows are then copied with 4-byte cp.async into the same
+// 16-byte aligned rows of the buffer (K/8 copies per lane and row pair, a tenth of the instructions of a pair), so the loop
+// reads them four entries at a time all the same; the K % 4 last ones singly, for a padding entry of weight 0 would still
+// turn an infinite x into a NaN.  Such shapes went to the kernel with CTA-wide tiles before.
+template <int VPL, int MODE, bool ODD>
 __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamParams p) {
     constexpr bool BCE = MODE == 1;  // 0: write y; 1: loss epilogue; 2: running top-k of the logits
     constexpr int BT = 16 * VPL;
@@ -80,13 +86,13 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
     const int h = lane >> 4;  // which row of a pair
     const int q = lane & 15;
     const int b0 = blockIdx.y * BT;
-    const int K = p.K, L = p.L;
+    const int K = p.K, L = p.L, Kp = ODD ? p.Kp : p.K;
 
     float* x_s = reinterpret_cast<float*>(smem_raw);
-    const int regionWords = 8 * K + 4 * S;
+    const int regionWords = 8 * Kp + 4 * S;
     float* region = x_s + static_cast<size_t>(p.N) * BT + static_cast<size_t>(warp) * regionWords;
     float* wi = region;
-    float* ys = region + 8 * K;
+    float* ys = region + 8 * Kp;
 
     const float* xs_lane = x_s + (VPL == 8 ? 4 : VPL) * q;
     const long long numQuads = (static_cast<long long>(L) + 3) / 4;
@@ -96,7 +102,18 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
     const int nChunks = 2 * chunksPerRow;
 
     auto issue = [&](long long pr, int buf) {
-        float* dstbuf = wi + buf * 4 * K;
+        float* dstbuf = wi + buf * 4 * Kp;
+        if constexpr (ODD) {
+            const long long e0 = 2 * pr * K;
+            const int n = 2 * pr + 1 < L ? 2 * K : K;  // both rows, or the one row left of an odd L
+            for (int c = lane; c < n; c += 32) {
+                float* dst = dstbuf + c + (c >= K ? 2 * Kp - K : 0);
+                __pipeline_memcpy_async(dst, p.W + e0 + c, 4);
+                __pipeline_memcpy_async(dst + Kp, p.idx + e0 + c, 4);
+            }
+            __pipeline_commit();
+            return;
+        }
         for (int c = lane; c < nChunks; c += 32) {
             const int row = c / chunksPerRow;
             const int within = c - row * chunksPerRow;
@@ -192,9 +209,9 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
             if (oA < L) {
                 const bool mine = oA + h < L;       // false only for the missing second row of an odd L
                 const long long o = mine ? oA + h : oA;
-                const float* row = wi + buf * 4 * K + (mine ? h : 0) * 2 * K;
+                const float* row = wi + buf * 4 * Kp + (mine ? h : 0) * 2 * Kp;
                 const float4* wr = reinterpret_cast<const float4*>(row);
-                const int4* ir = reinterpret_cast<const int4*>(row + K);
+                const int4* ir = reinterpret_cast<const int4*>(row + Kp);
                 const float bias = p.bias ? __ldg(p.bias + o) : 0.f;
                 float acc[VPL];
 #pragma unroll
@@ -226,6 +243,23 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
 #pragma unroll
                         for (int j = 0; j < VPL; ++j) acc[j] = fmaf(ww[u], a[u][j], acc[j]);
                 }
+                if constexpr (ODD) {
+                    for (int k = K & ~3; k < K; ++k) {
+                        const float w = row[k];
+                        const float* src = xs_lane + __float_as_int(row[Kp + k]) * BT;
+                        if constexpr (VPL == 2) {
+                            const float2 t = *reinterpret_cast<const float2*>(src);
+                            acc[0] = fmaf(w, t.x, acc[0]), acc[1] = fmaf(w, t.y, acc[1]);
+                        } else {
+#pragma unroll
+                            for (int v = 0; v < VPL / 4; ++v) {
+                                const float4 t = *reinterpret_cast<const float4*>(src + 64 * v);
+                                acc[4 * v] = fmaf(w, t.x, acc[4 * v]), acc[4 * v + 1] = fmaf(w, t.y, acc[4 * v + 1]);
+                                acc[4 * v + 2] = fmaf(w, t.z, acc[4 * v + 2]), acc[4 * v + 3] = fmaf(w, t.w, acc[4 * v + 3]);
+                            }
+                        }
+                    }
+                }
                 if constexpr (BCE) {
                     // a lane holds runs of 4 (or 2) consecutive batch elements of its row: vector stores
 #pragma unroll
@@ -247,6 +281,9 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
                             else *reinterpret_cast<float2*>(dst) = make_float2(gv[0], gv[1]);
                         }
                     }
+                    if (mine && blockIdx.y + 1 == gridDim.y)  // the last tile clears the columns past it, too
+                        for (long long b = b0 + BT + 4 * q; b < p.ldg; b += 64)
+                            *reinterpret_cast<float4*>(p.gT + static_cast<size_t>(o) * p.ldg + b) = make_float4(0.f, 0.f, 0.f, 0.f);
                 } else if constexpr (MODE == 2) {
                     bool hit = p.topk_floor == nullptr;
 #pragma unroll
@@ -321,10 +358,10 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
     }
 }
 
-template <int VPL, int MODE>
+template <int VPL, int MODE, bool ODD>
 int launch_pair_t(const FwdStreamParams& p, size_t smem, int nBT, const DeviceInfo& dev, cudaStream_t stream,
                   int* ctas_out) {
-    auto kern = ffi_fwd_pair_kernel<VPL, MODE>;
+    auto kern = ffi_fwd_pair_kernel<VPL, MODE, ODD>;
     int occ = 0;
     FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "streaming forward kernel does not fit on an SM (smem %zu)", smem);
@@ -343,6 +380,13 @@ int launch_pair_t(const FwdStreamParams& p, size_t smem, int nBT, const DeviceIn
     kern<<<grid, kThreads, smem, stream>>>(p);
     FFI_LAUNCH_CHECK("ffi_fwd_pair_kernel");
     return FFI_OK;
+}
+
+template <int MODE, bool ODD>
+int launch_pair(const FwdStreamParams& p, size_t smem, int nBT, int bpl, const DeviceInfo& dev, cudaStream_t stream, int* ctas_out) {
+    if (bpl == 4) return launch_pair_t<8, MODE, ODD>(p, smem, nBT, dev, stream, ctas_out);
+    if (bpl == 2) return launch_pair_t<4, MODE, ODD>(p, smem, nBT, dev, stream, ctas_out);
+    return launch_pair_t<2, MODE, ODD>(p, smem, nBT, dev, stream, ctas_out);
 }
 
 }  // namespace
@@ -370,14 +414,24 @@ static int launch_forward_stream_impl(const FwdArgs& a, const BceEpilogue* bce, 
     int rc = get_device_info(&dev);
     if (rc != FFI_OK) return rc;
     if (a.bf16) return FFI_OK;  // this kernel reads fp32 only
-    if (a.K % 4 != 0 || reinterpret_cast<uintptr_t>(a.W) % 16 != 0 || reinterpret_cast<uintptr_t>(a.idx) % 16 != 0)
-        return FFI_OK;
-    int bpl = a.B <= 32 ? 1 : (a.B <= 64 ? 2 : 4);
+    const int Kp = static_cast<int>(round_up(a.K, 4));
+    const bool odd = a.K % 4 != 0 || reinterpret_cast<uintptr_t>(a.W) % 16 != 0 || reinterpret_cast<uintptr_t>(a.idx) % 16 != 0;
+    // Width of the batch tiles: the one with the least work for the busiest warp, counted in accesses of the shared-memory
+    // pipe per row pair (per four entries the gathers, W and idx and their copies; the results; about 20 for the rest) times
+    // its rounds over the table.  A long table takes the widest tile that fits; a short one, whose row quads do not fill the
+    // warps, narrower ones: B=127, N=254, L=513, K=73 had 9 CTAs of 128 columns (13.8 us with CTA-wide tiles), now 36 of 32
+    // (7.7 us); B=418, N=228, L=2,578, K=16 15.3 -> 8.7 us in tiles of 64.  A narrower tile has to promise a tenth, for it
+    // fetches W and idx more often (B=152, L=31,964, K=8: promised 5 %, 22 -> 25 us).
+    int bpl = 0;
     size_t smem = 0;
-    for (; bpl >= 1; bpl /= 2) {
-        const size_t BT = 32 * bpl;
-        smem = static_cast<size_t>(a.N) * BT * 4 + static_cast<size_t>(kWarps) * (8 * a.K + 4 * (BT + 8)) * 4;
-        if (smem <= static_cast<size_t>(dev.max_smem_optin)) break;
+    double least = 0;
+    for (int c = a.B <= 32 ? 1 : (a.B <= 64 ? 2 : 4); c >= 1; c /= 2) {
+        const size_t BT = 32 * c;
+        const size_t need = static_cast<size_t>(a.N) * BT * 4 + static_cast<size_t>(kWarps) * (8 * Kp + 4 * (BT + 8)) * 4;
+        if (need > static_cast<size_t>(dev.max_smem_optin)) continue;
+        const int64_t per_bt = dev.sm_count / ceil_div(a.B, BT) > 0 ? dev.sm_count / ceil_div(a.B, BT) : 1;
+        const double cost = ((BT / 4 + 2.5) * Kp / 4 + BT / 4 + 20) * static_cast<double>(ceil_div(ceil_div(a.L, 4), per_bt * kWarps) * ceil_div(ceil_div(a.B, BT) * per_bt, dev.sm_count));
+        if (bpl == 0 || cost < 0.9 * least) bpl = c, smem = need, least = cost;
     }
     if (bpl < 1) return FFI_OK;
     FwdStreamParams p;
@@ -391,6 +445,7 @@ static int launch_forward_stream_impl(const FwdArgs& a, const BceEpilogue* bce, 
     p.N = a.N;
     p.L = a.L;
     p.K = a.K;
+    p.Kp = Kp;
     p.gT = bce ? bce->gT : nullptr;
     p.ldg = bce ? bce->ldg : 0;
     p.scale = bce ? bce->scale : 0.f;
@@ -410,21 +465,14 @@ static int launch_forward_stream_impl(const FwdArgs& a, const BceEpilogue* bce, 
             FFI_CUDA_CHECK(cudaMemsetAsync(topk->floor, 0x80, kTopK * static_cast<size_t>(p.topk_stride) * sizeof(int), stream));
             p.topk_floor = topk->floor;
         }
-        if (bpl == 4) rc = launch_pair_t<8, 2>(p, smem, nBT, dev, stream, &ctas);
-        else if (bpl == 2) rc = launch_pair_t<4, 2>(p, smem, nBT, dev, stream, &ctas);
-        else rc = launch_pair_t<2, 2>(p, smem, nBT, dev, stream, &ctas);
+        rc = odd ? launch_pair<2, true>(p, smem, nBT, bpl, dev, stream, &ctas) : launch_pair<2, false>(p, smem, nBT, bpl, dev, stream, &ctas);
         *topk->ctas_x = ctas / nBT;
         *topk->bt = 32 * bpl;
         return rc;
     }
-    if (bce) {
-        if (bpl == 4) return launch_pair_t<8, 1>(p, smem, nBT, dev, stream, bce->ctas);
-        if (bpl == 2) return launch_pair_t<4, 1>(p, smem, nBT, dev, stream, bce->ctas);
-        return launch_pair_t<2, 1>(p, smem, nBT, dev, stream, bce->ctas);
-    }
-    if (bpl == 4) return launch_pair_t<8, 0>(p, smem, nBT, dev, stream, nullptr);
-    if (bpl == 2) return launch_pair_t<4, 0>(p, smem, nBT, dev, stream, nullptr);
-    return launch_pair_t<2, 0>(p, smem, nBT, dev, stream, nullptr);
+    if (bce)
+        return odd ? launch_pair<1, true>(p, smem, nBT, bpl, dev, stream, bce->ctas) : launch_pair<1, false>(p, smem, nBT, bpl, dev, stream, bce->ctas);
+    return odd ? launch_pair<0, true>(p, smem, nBT, bpl, dev, stream, nullptr) : launch_pair<0, false>(p, smem, nBT, bpl, dev, stream, nullptr);
 }
 
 // Launches the barrier-free kernel when the shape allows it; *handled tells the caller.

@@ -35,6 +35,7 @@ struct GatherParams {
     float* gW;
     float* gbias;
     int B, N, L, K;
+    int vec16;       // idx rows can be copied 16 bytes at a time (otherwise, K % 4 != 0 or a ragged base, 4 bytes)
     int b0;          // first batch element of this launch's batch tile
     int accumulate;  // add to gW / gbias instead of overwriting (batch tiles after the first)
 };
@@ -45,9 +46,9 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_grad_w_gather_kernel(GatherPa
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int K = p.K, L = p.L;
+    const int K = p.K, L = p.L, Kp = (p.K + 3) & ~3;
     // per warp: 32 buffered entries, then two idx rows
-    float* dbuf = reinterpret_cast<float*>(smem_raw) + static_cast<size_t>(warp) * (32 * kRow + 2 * K);
+    float* dbuf = reinterpret_cast<float*>(smem_raw) + static_cast<size_t>(warp) * (32 * kRow + 2 * Kp);
     int* ibuf = reinterpret_cast<int*>(dbuf + 32 * kRow);
 
     const TX* xg = static_cast<const TX*>(p.xT) + p.b0;
@@ -56,9 +57,13 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_grad_w_gather_kernel(GatherPa
     long long o = static_cast<long long>(blockIdx.x) * kWarps + warp;
 
     auto issue = [&](long long row, int buf) {
-        if (row < L)
-            for (int c = lane; c < K / 4; c += 32)
-                __pipeline_memcpy_async(ibuf + buf * K + 4 * c, p.idx + row * K + 4 * c, 16);
+        if (row < L) {
+            if (p.vec16)
+                for (int c = lane; c < K / 4; c += 32)
+                    __pipeline_memcpy_async(ibuf + buf * Kp + 4 * c, p.idx + row * K + 4 * c, 16);
+            else
+                for (int c = lane; c < K; c += 32) __pipeline_memcpy_async(ibuf + buf * Kp + c, p.idx + row * K + c, 4);
+        }
         __pipeline_commit();
     };
 
@@ -82,9 +87,9 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_grad_w_gather_kernel(GatherPa
         }
         __pipeline_wait_prior(1);
         __syncwarp();
-        const int* ir = ibuf + s * K;
+        const int* ir = ibuf + s * Kp;
         for (int kg = 0; kg < K; kg += 32) {
-            const int n = min(32, K - kg);  // a multiple of 4
+            const int n = min(32, K - kg);
             int k = 0;
             for (; k + 8 <= n; k += 8) {
                 const int4 i0 = *reinterpret_cast<const int4*>(ir + kg + k);
@@ -101,7 +106,7 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_grad_w_gather_kernel(GatherPa
                     dbuf[(k + u) * kRow + lane] = a;
                 }
             }
-            if (k < n) {  // four entries left
+            if (k + 4 <= n) {
                 const int4 i0 = *reinterpret_cast<const int4*>(ir + kg + k);
                 const int ii[4] = {i0.x, i0.y, i0.z, i0.w};
                 V v[4];
@@ -114,6 +119,14 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_grad_w_gather_kernel(GatherPa
                     for (int j = 0; j < BPL; ++j) a = fmaf(gv[j], vec_get(v[u], j), a);
                     dbuf[(k + u) * kRow + lane] = a;
                 }
+                k += 4;
+            }
+            for (; k < n; ++k) {  // K % 4 entries left
+                const V v = load_lane_vec<BPL>(xg, static_cast<size_t>(ir[kg + k]) * ldv + lane);
+                float a = 0.f;
+#pragma unroll
+                for (int j = 0; j < BPL; ++j) a = fmaf(gv[j], vec_get(v, j), a);
+                dbuf[k * kRow + lane] = a;
             }
             __syncwarp();
             if (lane < n) {
@@ -140,7 +153,7 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_grad_w_gather_kernel(GatherPa
 template <int BPL, typename TX>
 int launch_gather_t(GatherParams p, int nBT, const DeviceInfo& dev, cudaStream_t stream) {
     auto kern = ffi_grad_w_gather_kernel<BPL, TX>;
-    const size_t smem = static_cast<size_t>(kWarps) * (32 * kRow + 2 * p.K) * 4;
+    const size_t smem = static_cast<size_t>(kWarps) * (32 * kRow + 2 * round_up(p.K, 4)) * 4;
     int occ = 0;
     FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "grad_W gather kernel does not fit on an SM (smem %zu)", smem);
@@ -160,7 +173,7 @@ int launch_gather_t(GatherParams p, int nBT, const DeviceInfo& dev, cudaStream_t
 }  // namespace
 
 // Takes the shapes the tiled kernel would gather from L2 for (x too wide for shared memory) when the transposed
-// gradient is at hand, K is a multiple of 4 and the rows are aligned; *handled tells the caller.
+// gradient is at hand and the rows of x and gT are aligned; *handled tells the caller.
 int launch_grad_w_gather(const GradWArgs& a, int bpl, cudaStream_t stream, bool* handled) {
     *handled = false;
     DeviceInfo dev;
@@ -171,11 +184,11 @@ int launch_grad_w_gather(const GradWArgs& a, int bpl, cudaStream_t stream, bool*
     if (a.bf16 && bpl == 4 && a.B > 128 && a.ldx % 256 == 0 && a.ldg % 256 == 0) bpl = 8;
     const int BT = 32 * bpl;
     const int nBT = static_cast<int>(ceil_div(a.B, BT));
-    if (!a.gT || a.K % 4 != 0 || reinterpret_cast<uintptr_t>(a.idx) % 16 != 0 || a.ldg % 4 != 0 ||
+    if (!a.gT || a.ldg % 4 != 0 ||
         a.ldg < static_cast<int64_t>(nBT) * BT || reinterpret_cast<uintptr_t>(a.gT) % 16 != 0 || a.ldx % BT != 0 ||
         a.ldx < static_cast<int64_t>(nBT) * BT || reinterpret_cast<uintptr_t>(a.xT) % 16 != 0)
         return FFI_OK;
-    const size_t smem = static_cast<size_t>(kWarps) * (32 * kRow + 2 * a.K) * 4;
+    const size_t smem = static_cast<size_t>(kWarps) * (32 * kRow + 2 * round_up(a.K, 4)) * 4;
     if (smem > static_cast<size_t>(dev.max_smem_optin)) return FFI_OK;
     GatherParams p;
     p.xT = a.xT;
@@ -189,6 +202,7 @@ int launch_grad_w_gather(const GradWArgs& a, int bpl, cudaStream_t stream, bool*
     p.N = a.N;
     p.L = a.L;
     p.K = a.K;
+    p.vec16 = a.K % 4 == 0 && reinterpret_cast<uintptr_t>(a.idx) % 16 == 0;
     p.b0 = 0;
     p.accumulate = 0;
     *handled = true;
