@@ -106,8 +106,9 @@ int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int6
 bool forward_uses_smem_x(int B, int N, int K, int* bpl_out);
 bool forward_small_applicable(int64_t B, int64_t N, int64_t K);
 int launch_forward_small(const void* x, int x_transposed, const int32_t* idx, const void* W, bool bf16, const float* bias,
-                         float* y, int64_t B, int64_t N, int64_t L, int64_t K, cudaStream_t stream, bool* handled);
+                         float* y, int64_t B, int64_t N, int64_t L, int64_t K, unsigned* tickets, cudaStream_t stream, bool* handled);
 size_t topk_rows_list_bytes(int64_t B, int64_t L);
+unsigned* topk_rows_tickets(void* lists, int64_t B, int64_t L);
 int launch_topk_rows(const float* y, int64_t B, int64_t L, uint2* lists, int kk, int label_offset, float* top_val, int* top_idx,
                      cudaStream_t stream);
 int launch_widen_bf16(const void* src, float* dst, int64_t n, cudaStream_t stream);
@@ -272,7 +273,7 @@ extern "C" int ffi_forward(const void* x, const int32_t* idx, const void* W, con
     }
     if (dtype == FFI_F32 || dtype == FFI_BF16) {
         bool handled = false;
-        rc = launch_forward_small(x, x_transposed, idx, W, dtype == FFI_BF16, bias, y, B, N, L, K, stream, &handled);
+        rc = launch_forward_small(x, x_transposed, idx, W, dtype == FFI_BF16, bias, y, B, N, L, K, nullptr, stream, &handled);
         if (rc != FFI_OK || handled) return rc;
     }
     if (dtype == FFI_BF16) {
@@ -741,7 +742,7 @@ extern "C" int ffi_forward_topk(const void* x, const int32_t* idx, const void* W
         // a few samples: their logits fit the scratch (4*B*L bytes) and the selection reads them back from L2
         float* y = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + align_up(topk_rows_list_bytes(B, L)));
         bool handled = false;
-        rc = launch_forward_small(x, x_transposed, idx, W, bf16, bias, y, B, N, L, K, stream, &handled);
+        rc = launch_forward_small(x, x_transposed, idx, W, bf16, bias, y, B, N, L, K, topk_rows_tickets(workspace, B, L), stream, &handled);
         if (rc != FFI_OK) return rc;
         if (handled)
             return launch_topk_rows(y, B, L, static_cast<uint2*>(workspace), k, static_cast<int>(label_offset), top_val, top_idx,

@@ -180,6 +180,13 @@ __device__ __forceinline__ void clear_loss_ticket(double* partials) {
 // Top-k epilogues of the forward kernels (evaluation: P@1, P@3, P@5 need 5 candidates per sample).
 constexpr int kTopK = 8;  // capacity of a top-k list
 
+// Order-preserving map of floats to signed integers, and back.
+__device__ __forceinline__ int order_key(float v) {
+    const int i = __float_as_int(v);
+    return i >= 0 ? i : i ^ 0x7fffffff;
+}
+__device__ __forceinline__ float order_value(int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7fffffff); }
+
 // Sorted (value descending, row ascending) insertion; `better` orders candidates the way
 // tf.nn.top_k does: higher value first, lower index on ties.
 __device__ __forceinline__ bool topk_better(float v, int i, float v2, int i2) { return v > v2 || (v == v2 && i < i2); }

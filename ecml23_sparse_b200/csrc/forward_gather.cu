@@ -114,13 +114,12 @@ __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherPa
                     for (int c = lane; c < K; c += 32) __pipeline_memcpy_async(dst + c, static_cast<const unsigned*>(p.W) + e0 + c, 4);
                 }
                 for (int c = lane; c < K; c += 32) __pipeline_memcpy_async(dst + wWords + c, p.idx + e0 + c, 4);
-                __pipeline_commit();
-                return;
+            } else {
+                const unsigned* wsrc = reinterpret_cast<const unsigned*>(static_cast<const TX*>(p.W) + row * K);
+                for (int c = lane; c < wWords / 4; c += 32) __pipeline_memcpy_async(dst + 4 * c, wsrc + 4 * c, 16);
+                for (int c = lane; c < K / 4; c += 32)
+                    __pipeline_memcpy_async(dst + wWords + 4 * c, p.idx + row * K + 4 * c, 16);
             }
-            const unsigned* wsrc = reinterpret_cast<const unsigned*>(static_cast<const TX*>(p.W) + row * K);
-            for (int c = lane; c < wWords / 4; c += 32) __pipeline_memcpy_async(dst + 4 * c, wsrc + 4 * c, 16);
-            for (int c = lane; c < K / 4; c += 32)
-                __pipeline_memcpy_async(dst + wWords + 4 * c, p.idx + row * K + 4 * c, 16);
         }
         __pipeline_commit();
     };

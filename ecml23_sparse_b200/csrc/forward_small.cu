@@ -7,7 +7,7 @@
 // idx), gathers the operands of all samples from shared memory (x_s[N][BP], 4*BP bytes per entry) and the G partial sums
 // are added with shuffles.  What bounds it is the stream of W and idx from HBM (8 bytes per entry) up to four samples, and
 // the shared-memory gathers (random rows: about 2.6 to 3.5 conflicts per phase) from eight on.  At N=768, L=670,091,
-// K=32, fp32, writing y: 34 / 36 / 50 / 107 us for 1 / 2 / 4 / 8 samples (5.0 TB/s at one), against 148 us of the batched
+// K=32, fp32, writing y: 34 / 36 / 50 / 90 us for 1 / 2 / 4 / 8 samples (5.0 TB/s at one), against 148 us of the batched
 // kernel for any batch up to 32; with 16 samples per entry it took 258 us, so the batched kernel has that.
 #include <type_traits>
 
@@ -28,16 +28,28 @@ struct SmallParams {
     float* y;
     int B, N, L, K;
     int lgG;  // log2 of the lanes per row
+    unsigned* tickets;  // nullable, [B]: cleared for the top-k selection that follows
 };
 
+// x_s[i][b].  The rows of eight samples swap their halves in every other group of four rows: a phase of a 16-byte gather then
+// spreads over all eight bank groups, not over the four that hold the same half of every row (B=8, N=768, L=670,091, K=32: 107 ->
+// 90 us).
 template <int BP>
-__device__ __forceinline__ void load_samples(const float* src, float (&out)[BP]) {
-    if constexpr (BP >= 4) {
-#pragma unroll
-        for (int c = 0; c < BP / 4; ++c) {
-            const float4 t = reinterpret_cast<const float4*>(src)[c];
-            out[4 * c] = t.x, out[4 * c + 1] = t.y, out[4 * c + 2] = t.z, out[4 * c + 3] = t.w;
-        }
+__device__ __forceinline__ int sample_at(int i, int b) {
+    return BP == 8 ? i * 8 + (b ^ (i & 4)) : i * BP + b;
+}
+
+template <int BP>
+__device__ __forceinline__ void load_samples(const float* x_s, int i, float (&out)[BP]) {
+    const float* src = x_s + sample_at<BP>(i, 0);
+    if constexpr (BP == 8) {
+        const float4 t = *reinterpret_cast<const float4*>(src);
+        const float4 t2 = *reinterpret_cast<const float4*>(x_s + (sample_at<BP>(i, 0) ^ 4));
+        out[0] = t.x, out[1] = t.y, out[2] = t.z, out[3] = t.w;
+        out[4] = t2.x, out[5] = t2.y, out[6] = t2.z, out[7] = t2.w;
+    } else if constexpr (BP == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(src);
+        out[0] = t.x, out[1] = t.y, out[2] = t.z, out[3] = t.w;
     } else if constexpr (BP == 2) {
         const float2 t = *reinterpret_cast<const float2*>(src);
         out[0] = t.x, out[1] = t.y;
@@ -64,15 +76,16 @@ __global__ void __launch_bounds__(kThreads) ffi_fwd_small_kernel(SmallParams p) 
 #pragma unroll 4
         for (int e = threadIdx.x; e < total; e += kThreads) {
             const int i = e / BP, b = e - i * BP;
-            x_s[e] = b < p.B ? widen(x[i * p.x_si + b]) : 0.f;
+            x_s[sample_at<BP>(i, b)] = b < p.B ? widen(x[i * p.x_si + b]) : 0.f;
         }
     } else {
 #pragma unroll 4
         for (int e = threadIdx.x; e < total; e += kThreads) {
             const int b = e / p.N, i = e - b * p.N;
-            x_s[i * BP + b] = b < p.B ? widen(x[b * p.x_sb + i]) : 0.f;
+            x_s[sample_at<BP>(i, b)] = b < p.B ? widen(x[b * p.x_sb + i]) : 0.f;
         }
     }
+    if (p.tickets && blockIdx.x == 0 && threadIdx.x < p.B) p.tickets[threadIdx.x] = 0;
     __syncthreads();
 
     const int tileRows = U * rpw;
@@ -105,7 +118,7 @@ __global__ void __launch_bounds__(kThreads) ffi_fwd_small_kernel(SmallParams p) 
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     float v[BP];
-                    load_samples<BP>(x_s + ii[c] * BP, v);
+                    load_samples<BP>(x_s, ii[c], v);
 #pragma unroll
                     for (int b = 0; b < BP; ++b) acc[u][b] = fmaf(w[u][c], v[b], acc[u][b]);
                 }
@@ -163,7 +176,7 @@ bool forward_small_applicable(int64_t B, int64_t N, int64_t K) {
 // y for a batch of at most kSmallMaxB, x in either layout and storage type; *handled = false where another kernel has to run
 // (fan-in not a multiple of four, unaligned rows, x too wide for shared memory).
 int launch_forward_small(const void* x, int x_transposed, const int32_t* idx, const void* W, bool bf16, const float* bias,
-                         float* y, int64_t B, int64_t N, int64_t L, int64_t K, cudaStream_t stream, bool* handled) {
+                         float* y, int64_t B, int64_t N, int64_t L, int64_t K, unsigned* tickets, cudaStream_t stream, bool* handled) {
     *handled = false;
     if (!forward_small_applicable(B, N, K) || reinterpret_cast<uintptr_t>(W) % (bf16 ? 8 : 16) != 0 ||
         reinterpret_cast<uintptr_t>(idx) % 16 != 0)
@@ -180,6 +193,7 @@ int launch_forward_small(const void* x, int x_transposed, const int32_t* idx, co
     p.W = W;
     p.bias = bias;
     p.y = y;
+    p.tickets = tickets;
     p.B = static_cast<int>(B);
     p.N = static_cast<int>(N);
     p.L = static_cast<int>(L);

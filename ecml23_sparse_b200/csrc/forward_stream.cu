@@ -44,14 +44,10 @@ struct FwdStreamParams {
     int topk_stride;  // columns per group
 };
 
-// Order-preserving map of floats to signed integers; the memset value kFloorNone decodes to "no bound yet".
+// Bounds are kept as order_key; the memset value kFloorNone decodes to "no bound yet".
 constexpr int kFloorNone = static_cast<int>(0x80808080u);
-__device__ __forceinline__ int order_key(float v) {
-    const int i = __float_as_int(v);
-    return i >= 0 ? i : i ^ 0x7fffffff;
-}
 __device__ __forceinline__ float floor_value(int k) {
-    return k == kFloorNone ? -INFINITY : __int_as_float(k >= 0 ? k : k ^ 0x7fffffff);
+    return k == kFloorNone ? -INFINITY : order_value(k);
 }
 
 // A HALF warp covers the batch tile (16 lanes x VPL batch elements) and the two halves of a warp
@@ -111,19 +107,18 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamPara
                 __pipeline_memcpy_async(dst, p.W + e0 + c, 4);
                 __pipeline_memcpy_async(dst + Kp, p.idx + e0 + c, 4);
             }
-            __pipeline_commit();
-            return;
-        }
-        for (int c = lane; c < nChunks; c += 32) {
-            const int row = c / chunksPerRow;
-            const int within = c - row * chunksPerRow;
-            const bool isIdx = within >= K / 4;
-            const int kc = isIdx ? within - K / 4 : within;
-            const long long o = 2 * pr + row;
-            if (o < L) {
-                const void* src = isIdx ? static_cast<const void*>(p.idx + o * K + 4 * kc)
-                                        : static_cast<const void*>(p.W + o * K + 4 * kc);
-                __pipeline_memcpy_async(dstbuf + row * 2 * K + (isIdx ? K : 0) + 4 * kc, src, 16);
+        } else {
+            for (int c = lane; c < nChunks; c += 32) {
+                const int row = c / chunksPerRow;
+                const int within = c - row * chunksPerRow;
+                const bool isIdx = within >= K / 4;
+                const int kc = isIdx ? within - K / 4 : within;
+                const long long o = 2 * pr + row;
+                if (o < L) {
+                    const void* src = isIdx ? static_cast<const void*>(p.idx + o * K + 4 * kc)
+                                            : static_cast<const void*>(p.W + o * K + 4 * kc);
+                    __pipeline_memcpy_async(dstbuf + row * 2 * K + (isIdx ? K : 0) + 4 * kc, src, 16);
+                }
             }
         }
         __pipeline_commit();
