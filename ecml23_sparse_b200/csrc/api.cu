@@ -99,7 +99,7 @@ int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const v
 bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss);
 int launch_forward_dense(const void* xT, int64_t ldx, const int32_t* idx, const void* W, const float* bias, float* y, int64_t B,
                          int64_t N, int64_t L, int64_t K, const Bf16LossEpilogue* loss, cudaStream_t stream);
-int forward_bf16_warps(int64_t B, int64_t N, int64_t K, bool loss_epilogue);
+bool forward_bf16_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss_epilogue);
 int launch_transpose_pad_bf16(const void* src, void* dst, int rows, int cols, int64_t ld_dst, cudaStream_t stream);
 int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int64_t ld_dst, int esize, cudaStream_t stream);
 
@@ -285,7 +285,7 @@ extern "C" int ffi_forward(const void* x, const int32_t* idx, const void* W, con
             return launch_forward_dense(xT, ldx, idx, W, bias, y, B, N, L, K, nullptr, stream);
         }
         // native bf16 kernel (x tile and W rows stay bf16 in shared memory) where the shape allows it
-        if (forward_bf16_warps(B, N, K, false) >= 4) {
+        if (forward_bf16_applicable(B, N, L, K, false)) {
             const void* xT = nullptr;
             int64_t ldx = 0;
             rc = stage_x_bf16(x, workspace, workspace_bytes, B, N, x_transposed, stream, &xT, &ldx);
@@ -622,8 +622,10 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
                     ffi_forward_bce_workspace_bytes(B, N, L, K, x_transposed, dtype), kAlign);
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     const bool dense = dtype == FFI_BF16 && forward_dense_applicable(B, N, L, K, true);
-    const bool bf16_tiled = !dense && dtype == FFI_BF16 && forward_bf16_warps(B, N, K, true) < 4 && bf16_takes_tiled_forward(B, N, K);
-    if (dtype == FFI_BF16 && !dense && forward_bf16_warps(B, N, K, true) < 4 && !bf16_tiled) {
+    const bool bf16_native = dtype == FFI_BF16 && forward_bf16_applicable(B, N, L, K, true) &&
+                             reinterpret_cast<uintptr_t>(W) % 16 == 0 && reinterpret_cast<uintptr_t>(idx) % 16 == 0;
+    const bool bf16_tiled = !dense && dtype == FFI_BF16 && !bf16_native && bf16_takes_tiled_forward(B, N, K);
+    if (dtype == FFI_BF16 && !dense && !bf16_native && !bf16_tiled) {
         // no native kernel for this shape: x and W are widened (exactly) at the front of the workspace
         const float *x32 = nullptr, *W32 = nullptr;
         void* rest = nullptr;

@@ -7,7 +7,8 @@
 // What bf16 storage buys: the kernel is bound by the shared-memory pipe (one gathered operand per FMA), and
 // a bf16 operand is half an fp32 one.  The whole batch tile of x, [N][128] bf16, fits shared memory (192 KB
 // at N = 768), a HALF warp covers the 128 batch columns of a row with ONE 16-byte load per lane and entry
-// (8 batch elements per lane), and the two halves of a warp work on the two rows of a row pair.  Per
+// (8 batch elements per lane; smaller batches and wider inputs take tiles of 64 or 32 columns, 4 or 2 per lane: B=64,
+// N=768, L=670,091, K=32 with the loss epilogue 268 -> 183 us, B=32 268 -> 152), and the two halves of a warp work on the two rows of a row pair.  Per
 // (row, k, 128 batch) that is 2 shared-memory wavefronts instead of the 4 (plus a second fetch of W and idx
 // for the second batch tile) of the fp32 kernel.  Widening happens in the multiply: the two bf16 halves of a
 // 32-bit word feed the mixed-precision FMA of sm_100 (`fma.rn.f32.bf16`: bf16 x bf16 + fp32, the product of
@@ -22,8 +23,7 @@
 namespace ffi {
 namespace {
 
-constexpr int BT = 128;  // batch columns of the x tile
-constexpr int S = BT + 8;  // result-tile row stride (floats)
+__host__ __device__ constexpr int result_stride(int BT) { return BT + 8; }  // floats per row of a warp's result tile
 
 struct FwdBf16Params {
     const __nv_bfloat16* xT;  // [N][ldx]
@@ -54,10 +54,30 @@ __device__ __forceinline__ void loss_negative_bf(int kind, float z, float& value
     }
 }
 
+// VPL bf16 of one lane, as 32-bit words
+template <int VPL>
+struct LaneWords;
+template <>
+struct LaneWords<8> {
+    using type = uint4;
+};
+template <>
+struct LaneWords<4> {
+    using type = uint2;
+};
+template <>
+struct LaneWords<2> {
+    using type = unsigned;
+};
+
 // Row record in a warp's buffer: K int32 indices, then K bf16 weights (6 K bytes; K % 8 == 0 keeps both parts
 // 16-byte aligned).
-template <int MODE>
+// VPL batch elements per lane, so a batch tile has 16 * VPL columns: 128, 64 or 32.
+template <int MODE, int VPL>
 __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
+    constexpr int BT = 16 * VPL;
+    constexpr int S = result_stride(BT);
+    using XV = typename LaneWords<VPL>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -66,6 +86,7 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
     const int h = lane >> 4;  // which row of a pair
     const int q = lane & 15;
     const int K = p.K, L = p.L;
+    const int b0 = blockIdx.y * BT;
 
     __nv_bfloat16* x_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);
     const int rowBytes = 6 * K;
@@ -80,7 +101,7 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
         const int total = p.N * vecPerRow;
         for (int e = tid; e < total; e += blockDim.x) {
             const int i = e / vecPerRow;
-            const int b = (e - i * vecPerRow) * 8;
+            const int bl = (e - i * vecPerRow) * 8, b = b0 + bl;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (b + 8 <= p.B) {
                 v = *reinterpret_cast<const uint4*>(p.xT + static_cast<size_t>(i) * p.ldx + b);
@@ -92,19 +113,24 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
                 auto two = [](unsigned short lo, unsigned short hi) { return static_cast<unsigned>(lo) | (static_cast<unsigned>(hi) << 16); };
                 v = make_uint4(two(t[0], t[1]), two(t[2], t[3]), two(t[4], t[5]), two(t[6], t[7]));
             }
-            *reinterpret_cast<uint4*>(x_s + static_cast<size_t>(i) * BT + b) = v;
+            *reinterpret_cast<uint4*>(x_s + static_cast<size_t>(i) * BT + bl) = v;
         }
     } else {
-        const int total = p.N * BT;
+        // ragged rows: two-byte loads, many of a thread's in flight (B=59, N=455, L=2,973, K=72: of 33 us about 20 were this fill)
+        const unsigned short* xg = reinterpret_cast<const unsigned short*>(p.xT);
+        const int total = p.N * (BT / 2);
+#pragma unroll 12
         for (int e = tid; e < total; e += blockDim.x) {
-            const int i = e / BT;
-            const int b = e - i * BT;
-            x_s[e] = b < p.B ? p.xT[static_cast<size_t>(i) * p.ldx + b] : __ushort_as_bfloat16(0);
+            const int i = e / (BT / 2);
+            const int b = b0 + 2 * (e - i * (BT / 2));
+            const unsigned short* src = xg + static_cast<size_t>(i) * p.ldx + b;
+            const unsigned lo = b < p.B ? __ldg(src) : 0u, hi = b + 1 < p.B ? __ldg(src + 1) : 0u;
+            reinterpret_cast<unsigned*>(x_s)[e] = lo | hi << 16;
         }
     }
     __syncthreads();
 
-    const unsigned char* xs_lane = reinterpret_cast<const unsigned char*>(x_s) + q * 16;
+    const unsigned char* xs_lane = reinterpret_cast<const unsigned char*>(x_s) + q * (2 * VPL);
     const long long numQuads = (static_cast<long long>(L) + 3) / 4;
     const long long gw = static_cast<long long>(blockIdx.x) * nwarps + warp;
     const long long GW = static_cast<long long>(gridDim.x) * nwarps;
@@ -156,52 +182,68 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
                 const int4* ir = reinterpret_cast<const int4*>(row);
                 const uint4* wr = reinterpret_cast<const uint4*>(row + 4 * K);
                 const float bias = p.bias ? __ldg(p.bias + o) : 0.f;
-                float zz[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                float z[VPL];
+#pragma unroll
+                for (int j = 0; j < VPL; ++j) z[j] = 0.f;
                 for (int k8 = 0; k8 < K / 8; ++k8) {
                     const int4 ia = ir[2 * k8], ib = ir[2 * k8 + 1];
                     const uint4 w8 = wr[k8];
                     const int ii[8] = {ia.x, ia.y, ia.z, ia.w, ib.x, ib.y, ib.z, ib.w};
                     const unsigned ww[4] = {w8.x, w8.y, w8.z, w8.w};
-                    uint4 xv[8];
+                    XV xv[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) xv[u] = *reinterpret_cast<const uint4*>(xs_lane + ii[u] * (BT * 2));
+                    for (int u = 0; u < 8; ++u) xv[u] = *reinterpret_cast<const XV*>(xs_lane + ii[u] * (BT * 2));
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
                         unsigned short wl, wh;
                         asm("mov.b32 {%0, %1}, %2;" : "=h"(wl), "=h"(wh) : "r"(ww[u >> 1]));
                         const unsigned short w16 = (u & 1) ? wh : wl;
-                        const unsigned words[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w};
+                        unsigned words[VPL / 2];
+                        if constexpr (VPL == 8) words[0] = xv[u].x, words[1] = xv[u].y, words[2] = xv[u].z, words[3] = xv[u].w;
+                        else if constexpr (VPL == 4) words[0] = xv[u].x, words[1] = xv[u].y;
+                        else words[0] = xv[u];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
+                        for (int j = 0; j < VPL / 2; ++j) {
                             unsigned short xl, xh;
                             asm("mov.b32 {%0, %1}, %2;" : "=h"(xl), "=h"(xh) : "r"(words[j]));
-                            asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(zz[2 * j]) : "h"(xl), "h"(w16));
-                            asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(zz[2 * j + 1]) : "h"(xh), "h"(w16));
+                            asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(z[2 * j]) : "h"(xl), "h"(w16));
+                            asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(z[2 * j + 1]) : "h"(xh), "h"(w16));
                         }
                     }
                 }
-                float z[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) z[j] = zz[j];
                 if constexpr (MODE == 1) {
-                    float gv[8];
+                    float gv[VPL];
+                    const int b = b0 + VPL * q;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const bool live = 8 * q + j < p.B;
+                    for (int j = 0; j < VPL; ++j) {
+                        const bool live = b + j < p.B;
                         float v, g;
                         loss_negative_bf(p.loss_kind, z[j] + bias, v, g);
                         if (live && mine) loss_local += v;
                         gv[j] = live ? p.scale * g : 0.f;
                     }
-                    if (mine && 8 * q < p.ldg) {
-                        float* dst = p.gT + static_cast<size_t>(o) * p.ldg + 8 * q;
-                        *reinterpret_cast<float4*>(dst) = make_float4(gv[0], gv[1], gv[2], gv[3]);
-                        *reinterpret_cast<float4*>(dst + 4) = make_float4(gv[4], gv[5], gv[6], gv[7]);
+                    float* grow = p.gT + static_cast<size_t>(o) * p.ldg;
+                    if (mine && b < p.ldg) {
+                        if constexpr (VPL == 2) {
+                            *reinterpret_cast<float2*>(grow + b) = make_float2(gv[0], gv[1]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < VPL; j += 4)
+                                *reinterpret_cast<float4*>(grow + b + j) = make_float4(gv[j], gv[j + 1], gv[j + 2], gv[j + 3]);
+                        }
                     }
+                    if (mine && blockIdx.y + 1 == gridDim.y)  // the last tile clears the columns past it, too
+                        for (long long c = b0 + BT + 4 * q; c < p.ldg; c += 64)
+                            *reinterpret_cast<float4*>(grow + c) = make_float4(0.f, 0.f, 0.f, 0.f);
                 } else {
-                    float* yrow = ys + (2 * half + h) * S + 8 * q;
-                    *reinterpret_cast<float4*>(yrow) = make_float4(z[0] + bias, z[1] + bias, z[2] + bias, z[3] + bias);
-                    *reinterpret_cast<float4*>(yrow + 4) = make_float4(z[4] + bias, z[5] + bias, z[6] + bias, z[7] + bias);
+                    float* yrow = ys + (2 * half + h) * S + VPL * q;
+                    if constexpr (VPL == 2) {
+                        *reinterpret_cast<float2*>(yrow) = make_float2(z[0] + bias, z[1] + bias);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < VPL; j += 4)
+                            *reinterpret_cast<float4*>(yrow + j) = make_float4(z[j] + bias, z[j + 1] + bias, z[j + 2] + bias, z[j + 3] + bias);
+                    }
                 }
             }
             __syncwarp();
@@ -212,7 +254,7 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
             for (int it = 0; it < BT * 4 / 32; ++it) {
                 const int id = it * 32 + lane;
                 const int bl = id >> 2, oo = id & 3;
-                if (bl < p.B && oq + oo < L) p.y[static_cast<size_t>(bl) * L + oq + oo] = ys[oo * S + bl];
+                if (b0 + bl < p.B && oq + oo < L) p.y[static_cast<size_t>(b0 + bl) * L + oq + oo] = ys[oo * S + bl];
             }
             __syncwarp();
         }
@@ -231,7 +273,7 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
         if (tid == 0) {
             double t = 0.0;
             for (int w = 0; w < nwarps; ++w) t += red[w];
-            p.loss_partials[blockIdx.x] = t;
+            p.loss_partials[static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x] = t;
         }
     }
 }
@@ -296,17 +338,52 @@ int launch_transpose_pad_bf16(const void* src, void* dst, int rows, int cols, in
     return FFI_OK;
 }
 
-// Warps per CTA the native bf16 forward can run with for this shape (0: not applicable).
-int forward_bf16_warps(int64_t B, int64_t N, int64_t K, bool loss_epilogue) {
+// Warps per CTA with batch tiles of BT columns, at most 16.
+static int bf16_warps(const DeviceInfo& dev, int64_t BT, int64_t N, int64_t K, bool loss) {
+    const int64_t tile = N * BT * 2, region = 4 * 6 * K + (loss ? 0 : 4 * result_stride(static_cast<int>(BT)) * 4);
+    const int64_t warps = (dev.max_smem_optin - tile) / region;
+    return static_cast<int>(tile >= dev.max_smem_optin ? 0 : (warps > 16 ? 16 : warps));
+}
+
+// Batch columns of a tile (0: another kernel has to run) and warps per CTA.  As in the fp32 kernel the width is the one with
+// the least work for the busiest SM, in accesses of the shared-memory pipe: eight entries of a row pair cost BT/4 gathers and
+// about 4 for W, idx and their copies.  A narrower tile than the widest that fits has to promise a tenth.
+static int bf16_tile(const DeviceInfo& dev, int64_t B, int64_t N, int64_t L, int64_t K, bool loss, int* warps_out) {
+    if (K % 8 != 0 || K <= 0) return 0;
+    int best = 0;
+    double least = 0;
+    for (int64_t BT = B <= 32 ? 32 : (B <= 64 ? 64 : 128); BT >= 32; BT /= 2) {
+        const int warps = bf16_warps(dev, BT, N, K, loss);
+        if (warps < (BT == 128 && B <= 128 ? 4 : 8)) continue;
+        const int64_t nBT = ceil_div(B, BT), per_bt = dev.sm_count / nBT > 0 ? dev.sm_count / nBT : 1;
+        const double cost = ((BT / 4 + 4) * K / 8.0 + BT / 4 + 20) * warps *
+                            static_cast<double>(ceil_div(ceil_div(L, 4), per_bt * warps) * ceil_div(nBT * per_bt, dev.sm_count));
+        if (best == 0 || cost < 0.9 * least) best = static_cast<int>(BT), least = cost, *warps_out = warps;
+    }
+    return best;
+}
+
+// Whether the native bf16 forward takes this shape (its rows of W and idx on 16-byte boundaries).
+bool forward_bf16_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss_epilogue) {
     DeviceInfo dev;
-    if (get_device_info(&dev) != FFI_OK) return 0;
-    if (B > BT || K % 8 != 0 || K <= 0) return 0;
-    const size_t tile = static_cast<size_t>(N) * BT * 2;
-    const size_t region = 4 * 6 * static_cast<size_t>(K) + (loss_epilogue ? 0 : 4 * S * 4);
-    if (tile + 4 * region > static_cast<size_t>(dev.max_smem_optin)) return 0;
-    size_t warps = (dev.max_smem_optin - tile) / region;
-    if (warps > 16) warps = 16;
-    return static_cast<int>(warps);
+    int warps = 0;
+    return get_device_info(&dev) == FFI_OK && bf16_tile(dev, B, N, L, K, loss_epilogue, &warps) > 0;
+}
+
+template <int MODE, int VPL>
+static int launch_bf16_t(const FwdBf16Params& p, dim3 grid, int warps, size_t smem, cudaStream_t stream) {
+    auto kern = ffi_fwd_bf16_kernel<MODE, VPL>;
+    FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
+    kern<<<grid, warps * 32, smem, stream>>>(p);
+    FFI_LAUNCH_CHECK("ffi_fwd_bf16_kernel");
+    return FFI_OK;
+}
+
+template <int MODE>
+static int launch_bf16_m(const FwdBf16Params& p, int BT, dim3 grid, int warps, size_t smem, cudaStream_t stream) {
+    if (BT == 128) return launch_bf16_t<MODE, 8>(p, grid, warps, smem, stream);
+    if (BT == 64) return launch_bf16_t<MODE, 4>(p, grid, warps, smem, stream);
+    return launch_bf16_t<MODE, 2>(p, grid, warps, smem, stream);
 }
 
 // xT: bf16 [N][ldx]; W: bf16 [L][K].  *handled = false when the shape needs another path.
@@ -317,8 +394,9 @@ int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const v
     DeviceInfo dev;
     int rc = get_device_info(&dev);
     if (rc != FFI_OK) return rc;
-    const int warps = forward_bf16_warps(B, N, K, loss != nullptr);
-    if (warps < 4 || reinterpret_cast<uintptr_t>(W) % 16 != 0 || reinterpret_cast<uintptr_t>(idx) % 16 != 0) return FFI_OK;
+    int warps = 0;
+    const int BT = bf16_tile(dev, B, N, L, K, loss != nullptr, &warps);
+    if (BT == 0 || reinterpret_cast<uintptr_t>(W) % 16 != 0 || reinterpret_cast<uintptr_t>(idx) % 16 != 0) return FFI_OK;
     FwdBf16Params p;
     p.xT = static_cast<const __nv_bfloat16*>(xT);
     p.ldx = ldx;
@@ -335,24 +413,16 @@ int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const v
     p.scale = loss ? loss->scale : 0.f;
     p.loss_partials = loss ? loss->loss_partials : nullptr;
     p.loss_kind = loss ? loss->loss_kind : 0;
-    const size_t region = 4 * 6 * static_cast<size_t>(K) + (loss ? 0 : 4 * S * 4);
+    const size_t region = 4 * 6 * static_cast<size_t>(K) + (loss ? 0 : 4 * result_stride(BT) * 4);
     const size_t smem = static_cast<size_t>(N) * BT * 2 + static_cast<size_t>(warps) * region;
-    const long long numQuads = (L + 3) / 4;
-    const long long want = (numQuads + warps - 1) / warps;
-    const unsigned grid = static_cast<unsigned>(want < dev.sm_count ? want : dev.sm_count);
+    const int64_t want = ceil_div(ceil_div(L, 4), warps), nBT = ceil_div(B, BT), per_bt = dev.sm_count / nBT > 0 ? dev.sm_count / nBT : 1;
+    const dim3 grid(static_cast<unsigned>(want < per_bt ? want : per_bt), static_cast<unsigned>(nBT));
+    if (loss && static_cast<long long>(grid.x) * grid.y > kMaxLossPartials)
+        return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %d per-CTA partials; this batch needs %u", kMaxLossPartials,
+                    grid.x * grid.y);
     *handled = true;
-    if (loss) {
-        auto kern = ffi_fwd_bf16_kernel<1>;
-        FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
-        *loss->ctas = static_cast<int>(grid);
-        kern<<<grid, warps * 32, smem, stream>>>(p);
-    } else {
-        auto kern = ffi_fwd_bf16_kernel<0>;
-        FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
-        kern<<<grid, warps * 32, smem, stream>>>(p);
-    }
-    FFI_LAUNCH_CHECK("ffi_fwd_bf16_kernel");
-    return FFI_OK;
+    if (loss) *loss->ctas = static_cast<int>(grid.x * grid.y);
+    return loss ? launch_bf16_m<1>(p, BT, grid, warps, smem, stream) : launch_bf16_m<0>(p, BT, grid, warps, smem, stream);
 }
 
 }  // namespace ffi

@@ -431,15 +431,16 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
 
 }  // namespace
 
-// Where launch_forward_dense is the faster kernel.  Its time hardly depends on K or the batch, the gather kernels' is
-// proportional to K and (in steps of 32 to 128 columns) to the batch:
-//   * more than 32 samples (writing y; 64: 238 against 277 us, 32 with few rows: 25 against 21 us at L=20,000) or 64 (loss
-//     gradient: no gain at 64 and N=768, 249 against 284 us at 128; with N <= 256 it gains at any batch);
-//   * with the loss epilogue a fan-in of at least 24 (16: 247 against 214 us);
+// Where launch_forward_dense is the faster kernel.  Its time hardly depends on K or the batch, the gather kernel's
+// (forward_bf16.cu) is proportional to K and, in tiles of 32, 64 or 128 columns, to the batch:
+//   * more than 64 samples (128: y 236 against 370 us and loss gradient 242 against 272 at N=768, L=670,091, K=32, y 30 against
+//     53 at N=256, L=100,000; 64: 87 against 58 and 31 against 32);
+//   * a fan-in of at least 16 for y and 24 for the loss gradient (16: 43 against 51 and 50 against 47 us at B=256, N=512,
+//     L=65,536; 8: y 45 against 41);
 //   * a fan-in of at most 64 (registers of the building warps) and a quarter of the inputs: beyond, repeated inputs in a row
 //     are so frequent that their list overflows (N=150, K=40 drawn with replacement: 602 against 215 us).
 bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss) {
-    return N <= 64 * kMaxPanels && K <= 64 && 4 * K <= N && (loss ? (B > 64 || N <= 256) && K >= 24 : B > 32) && L > 0;
+    return N <= 64 * kMaxPanels && K <= 64 && 4 * K <= N && B > 64 && K >= (loss ? 24 : 16) && L > 0;
 }
 
 // y (or, with `loss`, the loss gradient and one loss partial per CTA) from bf16 x as [N][ldx] and bf16 W.
