@@ -34,7 +34,8 @@ __device__ long long g_wait_limit = 4000000000ll;  // clock64 ticks a wait may l
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kDRow = 36;             // row stride of the per-warp dot buffer: 16-byte rows, conflict-free
+// row stride of the per-warp dot buffer (32 dots, the codes of the step's entries): 16-byte rows, conflict-free
+__host__ __device__ constexpr int dot_row(int groups) { return groups <= 4 ? 36 : 32 + groups; }
 constexpr int kStageUnroll = 4;       // staged entries per thread kept in flight
 constexpr int kKShift = 18;           // entry code = byte offset of the g row (with its swizzle key) | k << 18
 
@@ -323,7 +324,11 @@ struct LaneOf<4> {
 // columns of one entry, so a warp step works on G consecutive entries of a run.
 //   batch 65..128: G = 2, VPL = 8 (the case described above; two 16-byte pieces of a tile row per lane);
 //   batch 33..64:  G = 2, VPL = 4 (one 16-byte piece per lane, the tile is [T][64]);
-//   batch <= 32:   G = 4, VPL = 4 (a quarter warp per entry, the tile is [T][32]).
+//   batch 17..32:  G = 4, VPL = 4 (a quarter warp per entry, the tile is [T][32]);
+//   batch 9..16:   G = 8, VPL = 4 (tile [T][16]); batch <= 8: G = 16 (tile [T][8]).  The walk's steps
+//                  take about the same time whatever they hold: backward with the transposition at N=768,
+//                  L=670,091, K=32 577 us for 17..32 samples, 504 for 9..16, 458 for up to 8 (577 before); N=205,
+//                  L=71,169, K=48: 83, 67 and 61 us.
 // With VPL = 4 an input's state is 8 TMEM columns instead of 16, so a warp owns 16 inputs, a CTA 256, and three
 // slices per range instead of six fetch each g tile.
 //
@@ -346,7 +351,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     constexpr int BT = VPL * LG;  // batch columns of the tile
     constexpr int HALF = 2 * BT;  // bytes between a lane's two 16-byte pieces of a tile row (VPL = 8)
     constexpr int COLS = 2 * VPL; // TMEM columns of one input: its sums and its x values
-    constexpr int kThreads = THREADS, kWarps = THREADS / 32, kSlots = SLOTS;
+    constexpr int kThreads = THREADS, kWarps = THREADS / 32, kSlots = SLOTS, kDRow = dot_row(G);
     const int ni = FULL ? NI : p.ni;  // inputs per warp: the slices of a range split the inputs evenly
     const int CPN = kWarps * ni + 1;
     constexpr unsigned kRowMask = (1u << kKShift) - 1u;
@@ -484,7 +489,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const float* dlast1 = dlane + (kSlots - 1) * kDRow;           // last row a single step may fill
     const float* dlast2 = dlane + (kSlots - 2) * kDRow;           // last row a double step may start at
     const int myrow = lane / G, myent = lane % G;                 // the (buffered step, entry) this lane reduces
-    const float4* drow = reinterpret_cast<const float4*>(dbuf + myrow * kDRow + myent * LG);
+    const float* dots = dbuf + myrow * kDRow + myent * LG;
     const unsigned* dmine = reinterpret_cast<const unsigned*>(dbuf) + myrow * kDRow + 32 + myent;
     const unsigned char* gs_lane = reinterpret_cast<const unsigned char*>(g_s) + q * 16;
     const unsigned tileBytes = static_cast<unsigned>(T) * (BT * 4);
@@ -536,13 +541,15 @@ __global__ void __launch_bounds__(THREADS, 1)
 
         // grad_bias of the chunk's rows: the slices of a range take turns, each row is one group's sum
         if (p.gbias && static_cast<int>(c % gridDim.y) == static_cast<int>(blockIdx.y)) {
-            for (int rr = G * warp + grp; rr < T; rr += G * kWarps) {
+            for (int r0 = G * warp; r0 < T; r0 += G * kWarps) {  // (a warp stays together: T is a multiple of 8 only)
+                const int rr = r0 + grp;
                 LaneT v;
-                v.template load_shared<HALF>(gs_lane + rr * (BT * 4));
+                v.zero();
+                if (G <= 8 || rr < T) v.template load_shared<HALF>(gs_lane + rr * (BT * 4));
                 float sum = v.sum();
 #pragma unroll
                 for (int off = LG / 2; off >= 1; off /= 2) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-                if (q == 0 && o0 + rr < p.L) p.gbias[o0 + rr] = ACC ? p.gbias[o0 + rr] + sum : sum;
+                if (q == 0 && (G <= 8 || rr < T) && o0 + rr < p.L) p.gbias[o0 + rr] = ACC ? p.gbias[o0 + rr] + sum : sum;
             }
         }
 
@@ -560,8 +567,14 @@ __global__ void __launch_bounds__(THREADS, 1)
         auto reduce_slots = [&]() {
             __syncwarp();
             const int rows = static_cast<int>(dptr - dlane) / kDRow;
+            const float4* drow = reinterpret_cast<const float4*>(dots);
             float sum;
-            if constexpr (LG == 16) {
+            if constexpr (LG == 2) {
+                const float2 q0 = *reinterpret_cast<const float2*>(dots);
+                sum = q0.x + q0.y;
+            } else if constexpr (LG == 4) {
+                sum = (drow[0].x + drow[0].y) + (drow[0].z + drow[0].w);
+            } else if constexpr (LG == 16) {
                 const float4 q0 = drow[0], q1 = drow[1], q2 = drow[2], q3 = drow[3];
                 sum = (((q0.x + q0.y) + (q0.z + q0.w)) + ((q1.x + q1.y) + (q1.z + q1.w))) +
                       (((q2.x + q2.y) + (q2.z + q2.w)) + ((q3.x + q3.y) + (q3.z + q3.w)));
@@ -728,7 +741,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 struct FusedConfig {
     int ni, iparts, Bpad, R, entCap, segChunks;
-    int groups;  // lane groups per warp (2: batch 33..128, 4: batch <= 32)
+    int groups;  // lane groups per warp (2: batch 33..128, 4, 8, 16: batch <= 32, 16, 8)
     int vpl;     // batch elements per lane: 8 (batch 65..128) or 4
     size_t smem;
 };
@@ -740,7 +753,7 @@ bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedC
     if (!plan || !plan->has_chunks || B > 128) return false;
     // the entry code holds the position within the chunk in 14 bits
     if (static_cast<long long>(plan->chunk_rows) * plan->K > (1 << (32 - kKShift))) return false;
-    c->groups = B > 32 ? 2 : 4;
+    c->groups = B > 32 ? 2 : (B > 16 ? 4 : (B > 8 ? 8 : 16));
     c->vpl = B <= 64 ? 4 : 8;
     const int BT = c->vpl * (32 / c->groups);
     const FusedSlices sl = fused_slices(plan->N, c->vpl == 4);
@@ -760,7 +773,7 @@ bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedC
     const size_t T = static_cast<size_t>(plan->chunk_rows);
     if (T * BT * 4 > (size_t{1} << kKShift)) return false;
     // a warp buffers 32 / groups steps; + the barrier, the TMEM slot and alignment slack
-    const size_t total = T * BT * 4 + 2 * cap * 8 + static_cast<size_t>(kWarps) * (32 / c->groups) * kDRow * 4 +
+    const size_t total = T * BT * 4 + 2 * cap * 8 + static_cast<size_t>(kWarps) * (32 / c->groups) * dot_row(c->groups) * 4 +
                          2 * (kWarps * c->ni + 1) * 4 + 16 + 1024;
     if (total > static_cast<size_t>(dev.max_smem_optin)) return false;  // unusually dense slice or large K: separate kernels
     c->entCap = static_cast<int>(cap);
@@ -790,7 +803,7 @@ int encode_g_map(CUtensorMap* map, const float* gT, int64_t L, int64_t ldg, int6
         if (q != cudaDriverEntryPointSuccess || !fn) return fail(FFI_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
         encode = reinterpret_cast<EncodeFn>(fn);
     }
-    if (reinterpret_cast<uintptr_t>(gT) % 16 != 0 || chunk_rows > 256 || (BT != 32 && BT != 64 && BT != 128))
+    if (reinterpret_cast<uintptr_t>(gT) % 16 != 0 || chunk_rows > 256 || (BT != 8 && BT != 16 && BT != 32 && BT != 64 && BT != 128))
         return fail(FFI_ERR_INVALID_ARGUMENT, "transposed gradient must be 16-byte aligned, chunks at most 256 rows");
     // the stored rows may be narrower than the tile (batch <= 32 keeps 32 columns): the box's columns past them
     // are filled with zeros, like its rows past L
@@ -891,11 +904,15 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
             if (!ACC && c.ni == (c.vpl == 8 ? NI8 : NI4)) {
                 if (c.vpl == 8) return launch_group(ffi_bwd_pairs_kernel<NI8, TH, 16, 2, TX, 8, false, true>);
                 if (c.groups == 2) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 16, 2, TX, 4, false, true>);
-                return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 8, 4, TX, 4, false, true>);
+                if (c.groups == 4) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 8, 4, TX, 4, false, true>);
+                if (c.groups == 8) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 4, 8, TX, 4, false, true>);
+                return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 2, 16, TX, 4, false, true>);
             }
             if (c.vpl == 8) return launch_group(ffi_bwd_pairs_kernel<NI8, TH, 16, 2, TX, 8, ACC, false>);
             if (c.groups == 2) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 16, 2, TX, 4, ACC, false>);
-            return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 8, 4, TX, 4, ACC, false>);
+            if (c.groups == 4) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 8, 4, TX, 4, ACC, false>);
+            if (c.groups == 8) return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 4, 8, TX, 4, ACC, false>);
+            return launch_group(ffi_bwd_pairs_kernel<NI4, TH, 2, 16, TX, 4, ACC, false>);
         };
         auto launch_tile = [&](auto acc) { return a.w_bf16 ? launch_typed(__nv_bfloat16{}, acc) : launch_typed(float{}, acc); };
         rc = b0 > 0 ? launch_tile(std::true_type{}) : launch_tile(std::false_type{});

@@ -221,8 +221,10 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
     const int b0 = blockIdx.y * Bpad;
     __shared__ double part[8][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long id = static_cast<long long>(blockIdx.x) * 32 + lane;  // Bpad is a multiple of 32: no tail
     const size_t stride = static_cast<size_t>(N) * Bpad;
+    // (a tail only where Bpad is 8 or 16: its lanes read the last element and write nothing)
+    const long long mine = static_cast<long long>(blockIdx.x) * 32 + lane, end = static_cast<long long>(stride);
+    const long long id = mine < end ? mine : end - 1;
     double acc = 0.0;  // the range partials are large next to a small total: add them in fp64
     int r = warp;
     for (; r + 24 < R; r += 32) {
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
     for (int w = 1; w < 8; ++w) s += part[w][lane];
     const int i = static_cast<int>(id / Bpad);
     const int b = static_cast<int>(id - static_cast<long long>(i) * Bpad);
-    if (b0 + b >= cols) return;
+    if (b0 + b >= cols || mine >= end) return;
     if (x_transposed) gx[static_cast<size_t>(i) * B + b0 + b] = static_cast<float>(s);
     else gx[static_cast<size_t>(b0 + b) * N + i] = static_cast<float>(s);
 }
@@ -481,7 +483,7 @@ size_t grad_x_min_workspace_bytes(const ffi_plan* plan, int64_t B) {
 // Shared with the one-pass backward: see reduce_partials_kernel.
 int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int tiles, int B,
                           int x_transposed, cudaStream_t stream) {
-    const dim3 grid(static_cast<unsigned>(static_cast<long long>(N) * Bpad / 32), static_cast<unsigned>(tiles));
+    const dim3 grid(static_cast<unsigned>(ceil_div(static_cast<long long>(N) * Bpad, 32)), static_cast<unsigned>(tiles));
     reduce_partials_kernel<<<grid, 256, 0, stream>>>(partial, gx, R, N, cols, Bpad, B, x_transposed);
     FFI_LAUNCH_CHECK("reduce_partials_kernel");
     return FFI_OK;
