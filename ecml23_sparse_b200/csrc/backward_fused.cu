@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const float* dlast1 = dlane + (kSlots - 1) * kDRow;           // last row a single step may fill
     const float* dlast2 = dlane + (kSlots - 2) * kDRow;           // last row a double step may start at
     const int myrow = lane / G, myent = lane % G;                 // the (buffered step, entry) this lane reduces
-    const float* dots = dbuf + myrow * kDRow + myent * LG;
+    const float4* drow = reinterpret_cast<const float4*>(dbuf + myrow * kDRow + myent * LG);  // (8-byte aligned where LG = 2)
     const unsigned* dmine = reinterpret_cast<const unsigned*>(dbuf) + myrow * kDRow + 32 + myent;
     const unsigned char* gs_lane = reinterpret_cast<const unsigned char*>(g_s) + q * 16;
     const unsigned tileBytes = static_cast<unsigned>(T) * (BT * 4);
@@ -541,10 +541,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 
         // grad_bias of the chunk's rows: the slices of a range take turns, each row is one group's sum
         if (p.gbias && static_cast<int>(c % gridDim.y) == static_cast<int>(blockIdx.y)) {
-            for (int r0 = G * warp; r0 < T; r0 += G * kWarps) {  // (a warp stays together: T is a multiple of 8 only)
-                const int rr = r0 + grp;
+            // (T is a multiple of 8: with more groups the last rows leave some of a warp's lanes without one)
+            for (int rr = G * warp + grp; G <= 8 ? rr < T : rr - grp < T; rr += G * kWarps) {
                 LaneT v;
-                v.zero();
+                if constexpr (G > 8) v.zero();
                 if (G <= 8 || rr < T) v.template load_shared<HALF>(gs_lane + rr * (BT * 4));
                 float sum = v.sum();
 #pragma unroll
@@ -567,10 +567,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         auto reduce_slots = [&]() {
             __syncwarp();
             const int rows = static_cast<int>(dptr - dlane) / kDRow;
-            const float4* drow = reinterpret_cast<const float4*>(dots);
             float sum;
             if constexpr (LG == 2) {
-                const float2 q0 = *reinterpret_cast<const float2*>(dots);
+                const float2 q0 = *reinterpret_cast<const float2*>(drow);
                 sum = q0.x + q0.y;
             } else if constexpr (LG == 4) {
                 sum = (drow[0].x + drow[0].y) + (drow[0].z + drow[0].w);
