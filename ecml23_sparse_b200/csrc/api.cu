@@ -703,7 +703,7 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
     bool handled = false;
     rc = launch_forward_bce_stream(a, gT, ldg, scale, partials, &ctas, loss_kind, stream, &handled);
     if (rc != FFI_OK) return rc;
-    if (!handled) {  // wide inputs or K % 4 != 0: the CTA-tile kernel with the same epilogue
+    if (!handled) {  // wide inputs: the gather or the CTA-tile kernel with the same epilogue
         rc = launch_forward_loss_tile(a, gT, ldg, scale, partials, &ctas, loss_kind, stream);
         if (rc != FFI_OK) return rc;
     }

@@ -453,7 +453,7 @@ static int launch_forward_tile(const FwdArgs& a, const TileLossEpilogue* loss, c
 
 int launch_forward(const FwdArgs& a, cudaStream_t stream) {
     if (!a.bf16) {
-        // Preferred: the barrier-free kernel (x tile in shared memory, K % 4 == 0, aligned rows).
+        // Preferred: the barrier-free kernel (x tile in shared memory).
         bool handled = false;
         int rc = launch_forward_stream(a, stream, &handled);
         if (rc != FFI_OK || handled) return rc;
@@ -462,7 +462,7 @@ int launch_forward(const FwdArgs& a, cudaStream_t stream) {
 }
 
 // Forward with the loss gradient in the epilogue for the shapes the barrier-free kernel does not take
-// (wide inputs, K not a multiple of 4): same outputs as launch_forward_bce_stream.
+// (wide inputs, bf16 storage): same outputs as launch_forward_bce_stream.
 int launch_forward_loss_tile(const FwdArgs& a, float* gT, int64_t ldg, float scale, double* loss_partials, int* ctas,
                              int loss_kind, cudaStream_t stream) {
     TileLossEpilogue e{gT, ldg, scale, loss_partials, loss_kind, ctas};

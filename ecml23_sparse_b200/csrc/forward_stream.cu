@@ -510,7 +510,7 @@ int launch_forward_topk_stream(const FwdArgs& a, void* scratch, float* top_val, 
     int rc = launch_forward_stream_impl(a, nullptr, &e, stream, handled);
     if (rc != FFI_OK) return rc;
     int lists_per_tile = ctas_x * kWarps;
-    if (!*handled) {  // wide inputs, K not a multiple of 4, bf16 storage: the CTA-tile kernel's top-k epilogue
+    if (!*handled) {  // wide inputs, bf16 storage: the CTA-tile kernel's top-k epilogue
         rc = launch_forward_topk_tile(a, scratch, &lists_per_tile, &bt, stream);
         if (rc != FFI_OK) return rc;
         *handled = true;

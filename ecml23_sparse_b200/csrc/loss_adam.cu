@@ -127,6 +127,9 @@ __global__ void __launch_bounds__(256) bce_positive_fix_kernel(
     for (int e = lo + warp; e < hi; e += nwarps) {
         const long long o = static_cast<long long>(labels[e]) - label_offset;
         if (o < 0 || o >= L) continue;
+        // what the end needs is requested with the row: this kernel is a chain of trips to memory
+        float* cell = gT + static_cast<size_t>(o) * ldg + b;
+        const float bias_o = bias ? __ldg(bias + o) : 0.f, negative = loss_kind == 0 ? *cell : 0.f;
         float z = 0.f;
         for (int k = lane; k < K; k += 32) {
             const int i = idx[o * K + k];
@@ -135,19 +138,19 @@ __global__ void __launch_bounds__(256) bce_positive_fix_kernel(
 #pragma unroll
         for (int off = 16; off >= 1; off /= 2) z += __shfl_xor_sync(0xffffffffu, z, off);
         if (lane == 0) {
-            z += bias ? bias[o] : 0.f;
+            z += bias_o;
             // possum collects loss(target 1) - loss(target 0) of this logit
             if (loss_kind == 0) {
                 possum -= static_cast<double>(z);
-                gT[static_cast<size_t>(o) * ldg + b] -= scale;
+                *cell = negative - scale;
             } else {
                 const float hp = fmaxf(1.f - z, 0.f), hn = fmaxf(1.f + z, 0.f);
                 if (loss_kind == 1) {
                     possum += static_cast<double>(hp * hp) - static_cast<double>(hn * hn);
-                    gT[static_cast<size_t>(o) * ldg + b] = -2.f * hp * scale;
+                    *cell = -2.f * hp * scale;
                 } else {
                     possum += static_cast<double>(hp) - static_cast<double>(hn);
-                    gT[static_cast<size_t>(o) * ldg + b] = hp > 0.f ? -scale : 0.f;
+                    *cell = hp > 0.f ? -scale : 0.f;
                 }
             }
         }
