@@ -6,7 +6,9 @@
 // Why densify: the gather kernels move one operand per multiplication through shared memory (2.7 GFMA x 2 bytes at the
 // headline shape, 0.28 ms), while a row of 32 entries among 768 inputs costs the tensor core 24 times the multiplications
 // at 60 times the rate.  The products of bf16 values are exact in fp32 and the accumulator is fp32, so nothing is lost
-// against the gather; zeros add nothing.
+// against the gather; zeros add nothing to finite inputs.  An infinite or NaN x[i,b] would turn them into NaN in every row,
+// so the tensor core is given +-1 in its place, and the rows that read input i get w * x[i,b] added in fp32 (the sum then
+// holds +-|w| and the infinity or NaN itself: what a plain sum over the row's entries holds).
 //
 // Dataflow (one persistent CTA per SM and batch tile of 128):
 //   * the batch tile of x is the A operand and stays in tensor memory, lane = sample, 32-bit column = two inputs
@@ -78,6 +80,11 @@ __device__ __forceinline__ float bce_negative16(float (&z)[16]) {
     return sum + __logf(prod);
 }
 
+constexpr unsigned kBf16One = 0x3f80u;
+__device__ __forceinline__ bool bf16_finite(unsigned low_half) { return (low_half & 0x7f80u) != 0x7f80u; }
+__device__ __forceinline__ __nv_bfloat162 as_bf162(unsigned w) { return *reinterpret_cast<const __nv_bfloat162*>(&w); }
+__device__ __forceinline__ unsigned as_word(__nv_bfloat162 v) { return *reinterpret_cast<const unsigned*>(&v); }
+
 constexpr int kExtras = 19;  // per building warp and tile (8 rows): the shared memory that N = 768 leaves
 
 struct DenseBarriers {
@@ -90,7 +97,28 @@ struct DenseBarriers {
     int extras[2][kBuildWarps];    // entries in the lists below
     uint2 extra[2][kBuildWarps][kExtras];  // (input | row of the tile << 16, weight) of repeated inputs
     int bad;                       // a wait gave up: everybody runs through without waiting
+    unsigned nonfinite[2 * kMaxPanels];  // inputs with a sample of this tile that is infinite or NaN
 };
+
+// z plus the products of row o with the infinite and NaN inputs of sample b.  Called by whole warps, where a tile has any.
+__device__ __forceinline__ float add_nonfinite(const DenseFwdParams& p, const unsigned* flags, long long o, int b, float z) {
+    const int lane = threadIdx.x & 31;
+    for (int k0 = 0; k0 < p.K; k0 += 32) {
+        const int k = k0 + lane;
+        const unsigned i = k < p.K ? static_cast<unsigned>(__ldg(p.idx + o * p.K + k)) : 0xffffffffu;
+        const unsigned w = k < p.K ? static_cast<unsigned>(__ldg(p.W + o * p.K + k)) << 16 : 0u;
+        unsigned todo = __ballot_sync(0xffffffffu, i < static_cast<unsigned>(p.N) && (flags[i >> 5] >> (i & 31) & 1u));
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const unsigned ib = __shfl_sync(0xffffffffu, i, src);
+            const float wb = __uint_as_float(__shfl_sync(0xffffffffu, w, src));
+            const float x = b < p.B ? widen(p.xT[static_cast<size_t>(ib) * p.ldx + b]) : 0.f;
+            if (!isfinite(x)) z = fmaf(wb, x, z);
+        }
+    }
+    return z;
+}
 
 // MODE 0 writes y, 1 the loss gradient.  KG: entries of a row per lane (K <= 32 * KG).
 template <int MODE, int KG>
@@ -114,6 +142,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
         }
         *bad = 0;
     }
+    if (tid < 2 * kMaxPanels) bars->nonfinite[tid] = 0;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -150,6 +179,20 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     r[j] = xl[(2 * (c + j)) * 128] | (static_cast<unsigned>(xl[(2 * (c + j) + 1) * 128]) << 16);
+                // zero times an infinity or a NaN is NaN: one sum tells whether any of the sixteen values is not finite
+                __nv_bfloat162 zeros = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) zeros = __hfma2(as_bf162(r[j]), __floats2bfloat162_rn(0.f, 0.f), zeros);
+                if ((as_word(zeros) & 0x7fff7fffu) != 0) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const bool lo = !bf16_finite(r[j]), hi = !bf16_finite(r[j] >> 16);
+                        const int i = 2 * (c + j);
+                        if (lo | hi) atomicOr(bars->nonfinite + (i >> 5), (static_cast<unsigned>(lo) | static_cast<unsigned>(hi) << 1) << (i & 31));
+                        if (lo) r[j] = (r[j] & 0xffff8000u) | kBf16One;
+                        if (hi) r[j] = (r[j] & 0x8000ffffu) | kBf16One << 16;
+                    }
+                }
                 tc::store8(tmem + lane_base + c, r);
             }
             tc::wait_store();
@@ -332,6 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
         const int b = b0 + q * 32 + lane;
         float* sq = ys + warp * 512;  // its [32 samples][16 outputs] square, rows rotated (conflict-free both ways)
         auto sq_at = [&](int row, int col) -> float& { return sq[row * 16 + ((col + (row >> 1)) & 15)]; };
+        const bool nonfinite = __any_sync(0xffffffffu, lane < 2 * kMaxPanels && bars->nonfinite[lane] != 0);
         int it = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
             const int buf = it & 1;
@@ -345,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
             tc::fence_before_sync();
             // repeated inputs of these 16 outputs (two building warps)
             const int n0 = bars->extras[buf][(c0 >> 3)], n1 = bars->extras[buf][(c0 >> 3) + 1];
-            const bool extra = n0 + n1 > 0;
+            const bool extra = n0 + n1 > 0 || nonfinite;
             if (MODE == 0 || extra) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) sq_at(lane, j) = v[j];
@@ -356,6 +400,11 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                     const float xv = b < p.B ? widen(p.xT[static_cast<size_t>(x.x & 0xffffu) * p.ldx + b]) : 0.f;
                     float& z = sq_at(lane, static_cast<int>(x.x >> 16) - c0);
                     z = fmaf(__uint_as_float(x.y), xv, z);
+                }
+                if (nonfinite) {
+#pragma unroll 1
+                    for (int j = 0; j < 16 && o0 + j < L; ++j)
+                        sq_at(lane, j) = add_nonfinite(p, bars->nonfinite, o0 + j, b, sq_at(lane, j));
                 }
             }
             __syncwarp();

@@ -60,3 +60,32 @@ def test_dense_forward_loss_matches_the_oracle(cuda_device, shape, repeats, loss
         assert np.abs(gT[:, :B].t().cpu().numpy() - g_ref).max() <= 4e-5 / (B * L) * max(1.0, np.abs(z).max())
     assert abs(float(loss) - loss_ref) <= 2e-5 * abs(loss_ref) + 1e-7
     assert not gT[:, B:].any()
+
+
+@pytest.mark.parametrize("shape", [(65, 128, 64, 32), (130, 768, 1_001, 32), (100, 300, 130, 40)],
+                         ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
+@pytest.mark.parametrize("repeats", ["none", "some", "all"])
+def test_non_finite_inputs_reach_only_the_rows_that_read_them(cuda_device, shape, repeats):
+    """Infinities and NaN in single inputs, an all-NaN sample: every logit is what the sum over its row's own entries is."""
+    dev = cuda_device
+    B, N, L, K = shape
+    xd, idd, Wd, clean, idx, W = bf16_case(dev, B, N, L, K, 43, repeats)
+    bad = clean.copy()
+    bad[3, [0, 6, N - 1]] = np.inf, -np.inf, np.nan
+    bad[4, 7] = -np.inf
+    bad[B - 1, :] = np.nan
+    xd = to_cuda(bad, dev).to(torch.bfloat16)
+    bias = synth.normal(43, 40, (L,), std=0.5).numpy()
+    with np.errstate(invalid="ignore"):
+        ref = np.stack([(W.astype(np.float64) * row[idx]).sum(-1) for row in bad.astype(np.float64)]) + bias
+    assert np.isfinite(ref[:B - 1]).any(axis=1).all() and not np.isfinite(ref).all()
+    for transposed in (False, True):
+        y = ops._forward(xd.t().contiguous() if transposed else xd, idd, Wd, to_cuda(bias, dev), transposed).cpu().numpy()
+        finite = np.isfinite(ref)
+        assert np.array_equal(np.isnan(y), np.isnan(ref)) and np.array_equal(y[~finite], ref[~finite].astype(np.float32), equal_nan=True)
+        assert_close(y[finite], ref[finite], RTOL, ATOL, "y")
+
+    row_ptr, labels = synth.multi_hot_targets(43, 41, B, L)
+    _, gT = ops.forward_bce(xd, idd, Wd, to_cuda(bias, dev), row_ptr, labels, False)
+    _, g_ref = oracle.bce_f64(np.where(finite, ref, 0.0).astype(np.float32), row_ptr.numpy(), labels.numpy())
+    assert_close(gT[:, :B].t().cpu().numpy()[finite], g_ref[finite], 5e-5, 2e-7 / (B * L), "gradient")
