@@ -402,15 +402,16 @@ static int backward_impl(const void* x, const int32_t* idx, const void* W, const
         rc = check_index_range(idx, L * K, N, static_cast<cudaStream_t>(stream_v));
         if (rc != FFI_OK) return rc;
     }
-    // bf16 storage: the one-pass kernel and the kernels for wide inputs read bf16 x and W
-    // themselves; for the other shapes both are widened (exactly) into the workspace and the fp32 kernels run.
+    // bf16 storage: the one-pass kernel (W on a word boundary: it is copied in words) and the kernels for wide inputs read
+    // bf16 x and W themselves; else both are widened (exactly) into the workspace and the fp32 kernels run.
     bool bf16 = false;
     if (dtype == FFI_BF16) {
         const bool one_pass = grad_x && grad_w && plan && backward_fused_applicable(plan, B);
+        const bool words = reinterpret_cast<uintptr_t>(W) % 4 == 0;
         const bool w_native = !(grad_w || grad_bias) ||
                               !grad_w_stream_applicable(static_cast<int>(B), static_cast<int>(N), static_cast<int>(K), idx);
         const bool x_native = !grad_x || (plan && !plan->has_chunks);
-        bf16 = one_pass || (w_native && x_native && !(grad_x && grad_w && plan && backward_fused_applicable(plan, B)));
+        bf16 = one_pass ? words : w_native && x_native;
         if (!bf16) {
             const float *x32 = nullptr, *W32 = nullptr;
             void* rest = nullptr;

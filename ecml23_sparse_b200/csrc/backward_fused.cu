@@ -81,6 +81,7 @@ struct BwdFusedParams {
     int segChunks;  // chunks per flushed partial
     int ni;         // inputs per warp
     int boxes;      // TMA boxes per tile (at most 256 rows each)
+    int lastHalf;   // bf16 W of an odd number of elements: position of the last one, which has no whole word; else -1
 };
 
 // =====================================================================================
@@ -339,7 +340,7 @@ struct LaneOf<4> {
 // weight is fetched as the aligned 4-byte word that holds it (cp.async copies at least 4 bytes) and turned
 // into its fp32 bit pattern by the thread that fetched it once the copy has landed (the entry's code tells
 // which half: the chunk's first position is even, so the parity of the position within the chunk is the
-// parity of the flat position).
+// parity of the flat position).  W has to start on a word; of the last element of an odd number two bytes are copied.
 //
 template <int NI, int THREADS, int SLOTS, int G, typename TX, int VPL, bool ACC, bool FULL>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (tid < CPN) cpv = __ldg(p.cptr + c * (N + 1) + min(i_lo + tid, i_hi)) - e_lo;
     };
     auto emit_one = [&](uint2* d, int ps, int pos0) {
-        if constexpr (kBf16) __pipeline_memcpy_async(&d->x, static_cast<const unsigned*>(p.W) + (ps >> 1), 4);
+        if constexpr (kBf16) __pipeline_memcpy_async(&d->x, static_cast<const unsigned*>(p.W) + (ps >> 1), 4, ps == p.lastHalf ? 2 : 0);
         else __pipeline_memcpy_async(&d->x, static_cast<const float*>(p.W) + ps, 4);
         const int rel = ps - pos0;
         const int ol = p.kShift >= 0 ? (rel >> p.kShift) : rel / K;
@@ -872,6 +873,9 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
     p.T = a.plan->chunk_rows;
     p.nChunks = a.plan->n_chunks;
     p.boxes = p.T > 256 ? 2 : 1;
+    p.lastHalf = a.w_bf16 && (a.plan->L * a.plan->K) % 2 != 0 ? static_cast<int>(a.plan->L * a.plan->K - 1) : -1;
+    if (a.w_bf16 && reinterpret_cast<uintptr_t>(a.W) % 4 != 0)
+        return fail(FFI_ERR_INVALID_ARGUMENT, "fused backward copies bf16 weights word by word: W must be 4-byte aligned");
     const float* partials = p.partial;  // of the tiles not summed yet
     int tiles = 1;
     for (int64_t b0 = 0; b0 < a.B; b0 += 128) {

@@ -33,3 +33,21 @@ def test_one_pass_backward_matches_the_oracle(cuda_device, shape, bf16):
         assert_close(b.cpu().numpy(), oracle.grad_bias_f64(g), RTOL, ATOL * max(1.0, B ** 0.5 / 4), "grad_bias")
     info = ops.get_plan(idd, N).info()
     assert info["chunk_rows"] % 8 == 0 and 8 <= info["chunk_rows"] <= 512
+
+
+@pytest.mark.parametrize("shape", [(130, 300, 999, 33), (40, 64, 7, 12), (200, 768, 4_111, 24), (5, 254, 513, 73)],
+                         ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
+def test_bf16_weights_off_the_word_boundary(cuda_device, shape):
+    """W starts one element into its storage: the 4-byte copies of the one-pass kernel cannot read it."""
+    dev = cuda_device
+    B, N, L, K = shape
+    x, idx, W, g = config_style_inputs(B, N, L, K, seed=29)
+    xd, Wd = to_cuda(x, dev).to(torch.bfloat16), to_cuda(W, dev).to(torch.bfloat16)
+    off = torch.cat([Wd.new_zeros(1), Wd.reshape(-1)])[1:].view(L, K)
+    assert off.data_ptr() % 4 == 2
+    idd, gd = to_cuda(idx, dev), to_cuda(g, dev)
+    gx, gw, gb = ops._backward(xd, idd, off, gd, False, want_bias_grad=True)
+    x, W = xd.float().cpu().numpy(), Wd.float().cpu().numpy()
+    assert_close(gw.cpu().numpy(), oracle.grad_w_f64(x, idx, g), RTOL, ATOL * max(1.0, B ** 0.5 / 8), "grad_W")
+    assert_close(gx.cpu().numpy(), oracle.grad_x_f64(idx, W, g, N), RTOL, gx_atol(L, K, N), "grad_x")
+    assert_close(gb.cpu().numpy(), oracle.grad_bias_f64(g), RTOL, ATOL * max(1.0, B ** 0.5 / 4), "grad_bias")
