@@ -37,6 +37,7 @@ namespace {
 
 __device__ int g_dense_timeouts = 0;                // bounded waits of this kernel that gave up
 __device__ long long g_dense_limit = 4000000000ll;  // clock64 ticks a wait may last (about two seconds)
+constexpr long long kDrainLimit = 4000000000ll;     // ... and the last one, for MMAs that are under way, whatever that is set to
 
 constexpr int kEmitWarps = 16, kBuildWarps = 8;  // warps 0..15 write results, 16..23 build tiles, 24 issues the MMAs
 constexpr int kMmaWarp = kEmitWarps + kBuildWarps;
@@ -92,11 +93,12 @@ struct DenseBarriers {
     unsigned long long done[2];    // its MMAs are done: the tile buffer is free
     unsigned long long ready[2];   // ... and no further round follows: D is complete
     unsigned long long dfree[2];   // D has been read (one arrival per emitting warp)
+    unsigned long long idle;       // all MMAs of the CTA are done
     unsigned tmem;
     int more[2];                   // another round of this tile follows
     int extras[2][kBuildWarps];    // entries in the lists below
     uint2 extra[2][kBuildWarps][kExtras];  // (input | row of the tile << 16, weight) of repeated inputs
-    int bad;                       // a wait gave up: everybody runs through without waiting
+    int bad;                       // a wait gave up: everybody runs through without waiting, the results are void
     unsigned nonfinite[2 * kMaxPanels];  // inputs with a sample of this tile that is infinite or NaN
 };
 
@@ -140,8 +142,13 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
             tc::bar_init(bars->ready + i, 1);
             tc::bar_init(bars->dfree + i, kEmitWarps);
         }
+        tc::bar_init(&bars->idle, 1);
         *bad = 0;
     }
+    // After a wait that gave up the lists are read before or while they are written: what stands there is always a list.
+    for (unsigned e = tid; e < sizeof(bars->extra) / 4; e += kThreads) reinterpret_cast<unsigned*>(bars->extra)[e] = 0;
+    if (tid < 2 * kBuildWarps) bars->extras[0][tid] = 0;
+    if (tid < 2) bars->more[tid] = 0;
     if (tid < 2 * kMaxPanels) bars->nonfinite[tid] = 0;
     tc::fence_before_sync();
     __syncthreads();
@@ -207,11 +214,11 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
     const int tiles = (L + kRows - 1) / kRows;
     const long long limit = g_dense_limit;
     auto await = [&](unsigned long long* bar, unsigned parity) {
-        if (*bad) return;
-        if (!tc::bar_wait(bar, parity, limit)) {
+        if (!*bad && !tc::bar_wait(bar, parity, limit)) {
             atomicAdd(&g_dense_timeouts, 1);
             *bad = 1;
         }
+        __syncwarp();  // a lane may have given up by itself
     };
     float loss_local = 0.f;
 
@@ -225,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                 await(bars->full + buf, full_ph[buf]);
                 full_ph[buf] ^= 1u;
                 if (first && it >= 2) await(bars->dfree + buf, ((it >> 1) - 1) & 1);
-                const bool more = *static_cast<volatile int*>(&bars->more[buf]) != 0 && !*bad;
+                const bool more = __shfl_sync(0xffffffffu, *static_cast<volatile int*>(&bars->more[buf]) != 0 && !*bad, 0);
                 if (lane == 0) {
                     tc::fence_after_sync();
                     const unsigned base = tc::smem_addr(smem) + buf * tileBytes;
@@ -239,8 +246,10 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                 if (!more) break;
             }
         }
-        // the CTA's memory is given back only after the last MMAs have read it
-        for (int k = 0; k < 2 && k < it; ++k) await(bars->ready + ((it - 1 - k) & 1), ((it - 1 - k) >> 1) & 1);
+        // the CTA's memory is given back only after the last MMAs have read it, also when some wait has given up
+        if (lane == 0) tc::commit(&bars->idle);
+        __syncwarp();
+        if (!tc::bar_wait(&bars->idle, 0, kDrainLimit)) atomicAdd(&g_dense_timeouts, 1);
     } else if (warp >= kEmitWarps) {
         // ---- tiles of Wd -------------------------------------------------------------------------------------------------
         const int bw = warp - kEmitWarps;
@@ -349,13 +358,13 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                     "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\n"
                     "barrier.cta.red.or.pred q, 1, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
                     : "=r"(again)
-                    : "r"(static_cast<unsigned>(left)), "n"(32 * kBuildWarps)
+                    : "r"(static_cast<unsigned>(left && !*bad)), "n"(32 * kBuildWarps)
                     : "memory");
                 if (lane == 0) {
                     if (bw == 0) *static_cast<volatile int*>(&bars->more[buf]) = static_cast<int>(again);
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_addr(bars->full + buf)) : "memory");
                 }
-                if (!again || *bad) break;
+                if (!again) break;  // one answer for the eight warps, which meet at the barrier above
             }
             const int next = t + static_cast<int>(gridDim.x);
             if (next < tiles) fetch(next);

@@ -89,3 +89,37 @@ def test_non_finite_inputs_reach_only_the_rows_that_read_them(cuda_device, shape
     _, gT = ops.forward_bce(xd, idd, Wd, to_cuda(bias, dev), row_ptr, labels, False)
     _, g_ref = oracle.bce_f64(np.where(finite, ref, 0.0).astype(np.float32), row_ptr.numpy(), labels.numpy())
     assert_close(gT[:, :B].t().cpu().numpy()[finite], g_ref[finite], 5e-5, 2e-7 / (B * L), "gradient")
+
+
+def test_waits_that_run_out_end_the_kernel(cuda_device):
+    """With a limit below what a tile takes every warp gives up, at its own time, while tiles still need further rounds: the
+    launch ends, the event is counted, and the next call is right again."""
+    import ctypes
+    import time
+
+    import cases
+    from ecml23_sparse_b200 import _lib
+
+    dev, lib = cuda_device, _lib.load()
+    B, N, L, K = 256, 768, 20_000, 32
+    xd, idd, Wd, x, idx, W = bf16_case(dev, B, N, L, K, 47, "all")
+
+    def given_up():
+        n = ctypes.c_int(-1)
+        _lib.check(lib.ffi_wait_timeouts(ctypes.byref(n)))
+        return n.value
+
+    before = given_up()
+    _lib.check(lib.ffi_set_wait_limit_ticks(1_000))
+    try:
+        t0 = time.perf_counter()
+        ops._forward(xd, idd, Wd, None, False)
+        torch.cuda.synchronize()
+        assert time.perf_counter() - t0 < 1.0
+    finally:
+        _lib.check(lib.ffi_set_wait_limit_ticks(4_000_000_000))
+    after = given_up()
+    assert after > before
+    cases.EXPECTED_WAIT_TIMEOUTS += after - before
+    assert_close(ops._forward(xd, idd, Wd, None, False).cpu().numpy(), oracle.forward_f64(x, idx, W), RTOL, ATOL, "y")
+    assert given_up() == after
