@@ -31,6 +31,7 @@ int set_dense_forward_wait_limit(long long ticks);
 namespace {
 __device__ int g_wait_timeouts = 0;  // bounded waits of this file's kernels that gave up
 __device__ long long g_wait_limit = 4000000000ll;  // clock64 ticks a wait may last (about two seconds)
+constexpr long long kDrainLimit = 4000000000ll;    // ... and one for a copy that has to end before the CTA does
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
@@ -174,11 +175,12 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
         : "memory");
     return ok != 0;
 }
-// Waits for the phase with the given parity, at most about two seconds; false if it gave up.
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity) {
+// Waits for the phase with the given parity, at most g_wait_limit (or, for a copy that nobody will use, kDrainLimit) ticks;
+// false if it gave up.
+__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity, bool drain = false) {
     if (mbar_try_wait(bar, parity)) return true;
     const long long start = clock64();
-    const long long limit = g_wait_limit;
+    const long long limit = drain ? kDrainLimit : g_wait_limit;
     while (!mbar_try_wait(bar, parity))
         if (clock64() - start > limit) return false;
     return true;
@@ -731,9 +733,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
     }
 
-    // A thread that gave up waits once more, again bounded, for the copy it abandoned (the chunk it recorded
-    // when the copy was issued) before the CTA releases its shared memory.
-    if (pending >= 0) mbar_wait_bounded(g_bar, static_cast<unsigned>(pending - c_begin) & 1u);
+    // A thread that gave up waits once more for the copy it abandoned (the chunk it recorded when the copy was
+    // issued) before the CTA releases its shared memory: again bounded, but not by a limit that a caller has lowered.
+    if (pending >= 0) mbar_wait_bounded(g_bar, static_cast<unsigned>(pending - c_begin) & 1u, true);
     tmem_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, kTmemCols);
