@@ -96,7 +96,7 @@ int check_plan_device(const ffi_plan* plan) {
 int launch_forward_bf16(const void* xT, int64_t ldx, const int32_t* idx, const void* W, const float* bias, float* y,
                         int64_t B, int64_t N, int64_t L, int64_t K, const Bf16LossEpilogue* loss, cudaStream_t stream,
                         bool* handled);
-bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss);
+bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, const void* W, const int32_t* idx, bool loss);
 int launch_forward_dense(const void* xT, int64_t ldx, const int32_t* idx, const void* W, const float* bias, float* y, int64_t B,
                          int64_t N, int64_t L, int64_t K, const Bf16LossEpilogue* loss, cudaStream_t stream);
 bool forward_bf16_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss_epilogue);
@@ -277,7 +277,7 @@ extern "C" int ffi_forward(const void* x, const int32_t* idx, const void* W, con
         if (rc != FFI_OK || handled) return rc;
     }
     if (dtype == FFI_BF16) {
-        if (forward_dense_applicable(B, N, L, K, false)) {  // tensor cores on densified tiles of W
+        if (forward_dense_applicable(B, N, L, K, W, idx, false)) {  // tensor cores on densified tiles of W
             const void* xT = nullptr;
             int64_t ldx = 0;
             rc = stage_x_bf16(x, workspace, workspace_bytes, B, N, x_transposed, stream, &xT, &ldx);
@@ -622,7 +622,7 @@ extern "C" int ffi_forward_loss(int loss_kind, const void* x, const int32_t* idx
         return fail(FFI_ERR_WORKSPACE, "ffi_forward_loss needs %zu bytes of %zu-byte aligned workspace",
                     ffi_forward_bce_workspace_bytes(B, N, L, K, x_transposed, dtype), kAlign);
     unsigned char* ws = static_cast<unsigned char*>(workspace);
-    const bool dense = dtype == FFI_BF16 && forward_dense_applicable(B, N, L, K, true);
+    const bool dense = dtype == FFI_BF16 && forward_dense_applicable(B, N, L, K, W, idx, true);
     const bool bf16_native = dtype == FFI_BF16 && forward_bf16_applicable(B, N, L, K, true) &&
                              reinterpret_cast<uintptr_t>(W) % 16 == 0 && reinterpret_cast<uintptr_t>(idx) % 16 == 0;
     const bool bf16_tiled = !dense && dtype == FFI_BF16 && !bf16_native && bf16_takes_tiled_forward(B, N, K);

@@ -14,20 +14,22 @@
 //   * the batch tile of x is the A operand and stays in tensor memory, lane = sample, 32-bit column = two inputs
 //     (N / 2 <= 384 columns); D is [128 samples][64 outputs] fp32, two buffers of 64 columns;
 //   * B is a tile of 64 rows of Wd, [64][N] bf16 in shared memory (128-byte swizzled panels of 64 inputs), two buffers.  It
-//     is never cleared as a whole: a warp owns four rows, remembers where it wrote and puts zeros back there, so a row of
-//     K entries costs 2K two-byte stores instead of a row of N;
+//     is never cleared as a whole: a warp owns eight rows (four with K > 32), remembers where it wrote and puts zeros back there,
+//     so a row of K entries costs 2K two-byte stores instead of a row of N;
 //   * entries of a row with the same input cannot share a cell (their sum is no bf16): one of them is written, the others
-//     go to a short list that is added to the results with fp32 FMAs (x read from L2); what does not fit the list waits
-//     for another round of the same tile that accumulates.  Tables without repeated inputs never do either;
-//   * the warps specialise: 8 build tiles, one issues the N / 16 MMAs of a tile (M = 128, N = 64, K = 16), 8 turn D into y
-//     or the loss gradient; mbarriers hand the buffers on, so the three stages of consecutive tiles overlap.  (With all
-//     warps building and emitting in turn, one CTA barrier per tile, the stages' latencies added up: 214 us for y, 310 with
-//     the BCE epilogue.)
-// What bounds it: an MMA of M = 128 takes 62 clocks for any N up to 128 (measured), so the N = 64 that fits beside x costs
-// 48 x 62 clocks per tile at N = 768 (110 us at L = 670,091); the building warps' chain of stores and the results' stores
-// are about as long and overlap only in part.  Measured at B = 128, L = 670,091, against the gather kernels:
-// N = 768, K = 32: y 234 (408) us, loss gradient 249 (284) us; K = 64: 325 (590) and 360 (468) us; inputs drawn with
-// replacement: 296 (403) and 325 (286) us; B = 256, N = 512, L = 65,536, K = 64: y 66 (196) us.
+//     go to a list per 16 rows that is added to the results with fp32 FMAs, x read back from tensor memory; what does not fit
+//     the list waits for another round of the same tile that accumulates.  Tables without repeated inputs never do either;
+//   * the warps specialise: 8 build tiles, one issues the N / 16 MMAs of a tile (M = 128, N = 64, K = 16), 16 turn D into y
+//     or the loss gradient (16 and 8 with K > 32: building, two entries a lane, is the longest stage there); mbarriers hand the
+//     buffers on, so the three stages of consecutive tiles overlap.  (With all warps building and emitting in turn, one CTA
+//     barrier per tile, the stages' latencies added up: 214 us for y, 310 with the BCE epilogue.)
+// What bounds it: at N = 768 and K = 32 the thread that issues the MMAs is busy for 0.92 of the time, the
+// tensor pipe for 0.4 (tiles of 64 rows are what fits beside x); with repeated inputs the emitting warps,
+// about 80 clocks an entry (its square of results is read, added to and written in shared memory).
+// Measured at B = 128, L = 670,091, tables of distinct inputs / drawn with replacement, against the gather kernel:
+// N = 768, K = 32: y 232/261 (379) us, loss gradient 245/288 (289) us; K = 64: 274/430 (594) and 294/493 (474) us;
+// B = 256, N = 512, L = 65,536, K = 64: y 62/113 (113) us.  With the lists read by 16 warps from L2, one entry after the other, and
+// 8 building warps: y 239/299 and 331/905, loss gradient 253/327 and 364/986, 71/220 us.
 #include <type_traits>
 
 #include "tcgen05.cuh"
@@ -39,11 +41,10 @@ __device__ int g_dense_timeouts = 0;                // bounded waits of this ker
 __device__ long long g_dense_limit = 4000000000ll;  // clock64 ticks a wait may last (about two seconds)
 constexpr long long kDrainLimit = 4000000000ll;     // ... and the last one, for MMAs that are under way, whatever that is set to
 
-constexpr int kEmitWarps = 16, kBuildWarps = 8;  // warps 0..15 write results, 16..23 build tiles, 24 issues the MMAs
-constexpr int kMmaWarp = kEmitWarps + kBuildWarps;
+constexpr int kMmaWarp = 24;                  // the warps before it write results or build tiles, this one issues the MMAs
 constexpr int kThreads = 32 * (kMmaWarp + 1);
+constexpr int kMaxBuildWarps = 16;
 constexpr int kRows = 64;                     // outputs per tile
-constexpr int kWarpRows = kRows / kBuildWarps;
 constexpr int kMaxPanels = 12;                // 12 * 32 columns of x + 2 * 64 of D fill the tensor memory
 constexpr unsigned kPanelBytes = kRows * 128;
 
@@ -56,6 +57,7 @@ struct DenseFwdParams {
     float* y;
     int B, N, L, K;
     int panels;  // ceil(N / 64)
+    int cap;     // entries a building warp may add to a list of repeated inputs, a multiple of 4
     // loss epilogue (MODE 1), as in forward_stream.cu
     float* gT;
     long long ldg;
@@ -86,8 +88,6 @@ __device__ __forceinline__ bool bf16_finite(unsigned low_half) { return (low_hal
 __device__ __forceinline__ __nv_bfloat162 as_bf162(unsigned w) { return *reinterpret_cast<const __nv_bfloat162*>(&w); }
 __device__ __forceinline__ unsigned as_word(__nv_bfloat162 v) { return *reinterpret_cast<const unsigned*>(&v); }
 
-constexpr int kExtras = 19;  // per building warp and tile (8 rows): the shared memory that N = 768 leaves
-
 struct DenseBarriers {
     unsigned long long full[2];    // a tile is built (one arrival per building warp)
     unsigned long long done[2];    // its MMAs are done: the tile buffer is free
@@ -96,11 +96,28 @@ struct DenseBarriers {
     unsigned long long idle;       // all MMAs of the CTA are done
     unsigned tmem;
     int more[2];                   // another round of this tile follows
-    int extras[2][kBuildWarps];    // entries in the lists below
-    uint2 extra[2][kBuildWarps][kExtras];  // (input | row of the tile << 16, weight) of repeated inputs
+    int listed[2][kMaxBuildWarps]; // entries each building warp has in the lists of repeated inputs
     int bad;                       // a wait gave up: everybody runs through without waiting, the results are void
     unsigned nonfinite[2 * kMaxPanels];  // inputs with a sample of this tile that is infinite or NaN
 };
+// Behind the barriers: the lists of repeated inputs, one per buffer and 16 rows.  An entry is laid out so that the emitting warps
+// need few instructions for it: the weight in the half of a word that its input has in a column of x, and
+// column << 23 | square_row(row of the 16).
+constexpr size_t kListsAt = (sizeof(DenseBarriers) + 15) / 16 * 16;
+
+// Offset of output j's row in an emitting warp's square of [16 outputs][32 samples], with the key of its samples' order
+// (sample s stands at place s ^ 2j: conflict-free by rows and by columns).
+__host__ __device__ constexpr unsigned square_row(unsigned j) { return j << 7 | j << 3; }
+
+// z + x.lo * w.lo + x.hi * w.hi, exact products of bf16
+__device__ __forceinline__ float fma_pair(unsigned x, unsigned w, float z) {
+    unsigned short xl, xh, wl, wh;
+    asm("mov.b32 {%0, %1}, %2;" : "=h"(xl), "=h"(xh) : "r"(x));
+    asm("mov.b32 {%0, %1}, %2;" : "=h"(wl), "=h"(wh) : "r"(w));
+    asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(z) : "h"(xl), "h"(wl));
+    asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(z) : "h"(xh), "h"(wh));
+    return z;
+}
 
 // z plus the products of row o with the infinite and NaN inputs of sample b.  Called by whole warps, where a tile has any.
 __device__ __forceinline__ float add_nonfinite(const DenseFwdParams& p, const unsigned* flags, long long o, int b, float z) {
@@ -122,16 +139,20 @@ __device__ __forceinline__ float add_nonfinite(const DenseFwdParams& p, const un
     return z;
 }
 
-// MODE 0 writes y, 1 the loss gradient.  KG: entries of a row per lane (K <= 32 * KG).
-template <int MODE, int KG>
+// MODE 0 writes y, 1 the loss gradient.  KG: entries of a row per lane (K <= 32 * KG).  EMIT: warps that write results (8 or 16).
+template <int MODE, int KG, int EMIT>
 __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdParams p) {
+    constexpr int kEmitWarps = EMIT, kBuildWarps = kMmaWarp - EMIT;
+    constexpr int kWarpRows = kRows / kBuildWarps;  // rows of a tile that a building warp has
+    constexpr int kListWarps = 16 / kWarpRows;      // building warps that share a list
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b0 = blockIdx.y * 128;
     const int K = p.K, L = p.L;
     const unsigned tileBytes = p.panels * kPanelBytes;
-    float* ys = reinterpret_cast<float*>(smem + 2 * tileBytes);  // [warp][32 samples][16 outputs]
+    unsigned char* squares = smem + 2 * tileBytes;  // one of 2 KB per emitting warp
     DenseBarriers* bars = reinterpret_cast<DenseBarriers*>(smem + 2 * tileBytes + kEmitWarps * 2048);
+    uint2* lists = reinterpret_cast<uint2*>(reinterpret_cast<unsigned char*>(bars) + kListsAt);
     volatile int* bad = &bars->bad;
 
     if (warp == kMmaWarp) tc::alloc(&bars->tmem);
@@ -146,8 +167,8 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
         *bad = 0;
     }
     // After a wait that gave up the lists are read before or while they are written: what stands there is always a list.
-    for (unsigned e = tid; e < sizeof(bars->extra) / 4; e += kThreads) reinterpret_cast<unsigned*>(bars->extra)[e] = 0;
-    if (tid < 2 * kBuildWarps) bars->extras[0][tid] = 0;
+    for (int e = tid; e < 2 * kBuildWarps * p.cap; e += kThreads) lists[e] = make_uint2(0u, 0u);
+    if (tid < 2 * kMaxBuildWarps) (&bars->listed[0][0])[tid] = 0;
     if (tid < 2) bars->more[tid] = 0;
     if (tid < 2 * kMaxPanels) bars->nonfinite[tid] = 0;
     tc::fence_before_sync();
@@ -235,10 +256,14 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                 const bool more = __shfl_sync(0xffffffffu, *static_cast<volatile int*>(&bars->more[buf]) != 0 && !*bad, 0);
                 if (lane == 0) {
                     tc::fence_after_sync();
-                    const unsigned base = tc::smem_addr(smem) + buf * tileBytes;
-                    for (int m = 0; m < 4 * p.panels; ++m)
-                        tc::mma(tmem_d + buf * kRows, tmem + m * 8, tc::panel_desc(base + (m >> 2) * kPanelBytes + (m & 3) * 32),
-                                tc::instr_desc(kRows), !first || m > 0);
+                    // (a descriptor from scratch for each MMA took this thread 113 clocks a step)
+                    const unsigned long long b = tc::panel_desc(tc::smem_addr(smem) + buf * tileBytes);
+                    const unsigned d = tmem_d + buf * kRows;
+                    for (int panel = 0; panel < p.panels; ++panel)
+#pragma unroll
+                        for (int m = 0; m < 4; ++m)
+                            tc::mma(d, tmem + panel * 32 + m * 8, tc::desc_at(b, panel * kPanelBytes + m * 32), tc::instr_desc(kRows),
+                                    !first || panel + m > 0);
                     tc::commit(bars->done + buf);
                     if (!more) tc::commit(bars->ready + buf);
                 }
@@ -284,7 +309,6 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
             auto set_cell = [&](int r, int g, unsigned c) {
                 cells[buf][r / 2][g] = (r & 1) ? ((cells[buf][r / 2][g] & 0xffffu) | (c << 16)) : ((cells[buf][r / 2][g] & 0xffff0000u) | c);
             };
-            int extras = 0;
             for (bool wait = use > 0, first = true;; wait = true, first = false) {
                 if (wait) {  // the last MMAs on this buffer
                     await(bars->done + buf, done_ph[buf]);
@@ -330,28 +354,24 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                             set_cell(r, g, kNone);
                         }
                     }
-                bool left = false;
-                // the list of this buffer's tile before has been read
-                if (first && use > 0) await(bars->dfree + buf, (use - 1) & 1);
-                if (__any_sync(0xffffffffu, lost != 0)) {
+                // The entries that found another's number go to the list of their sixteen rows, in a fixed order: the warps that
+                // share it tell each other their counts across the barrier.  What a warp has no room for waits for another
+                // round, in which nothing is listed any more.
+                unsigned who[kWarpRows * KG];
+                int found = 0;
+                bool left = lost != 0;
+                if (first) {
+                    if (use > 0) await(bars->dfree + buf, (use - 1) & 1);  // the lists of this buffer's tile before have been read
+                    if (__any_sync(0xffffffffu, lost != 0)) {
 #pragma unroll
-                    for (int r = 0; r < kWarpRows; ++r)
-#pragma unroll
-                        for (int g = 0; g < KG; ++g) {
-                            const bool mine_lost = lost >> (r * KG + g) & 1u;
-                            const unsigned who = __ballot_sync(0xffffffffu, mine_lost);
-                            const int slot = extras + __popc(who & ((1u << lane) - 1u));
-                            if (mine_lost && slot < kExtras) {
-                                bars->extra[buf][bw][slot] = make_uint2(static_cast<unsigned>(ir[r][g]) | (bw * kWarpRows + r) << 16,
-                                                                        static_cast<unsigned>(wr[r][g]) << 16);
-                                wr[r][g] = 0;
-                            } else if (mine_lost) {
-                                left = true;
-                            }
-                            extras = min(kExtras, extras + __popc(who));
+                        for (int j = 0; j < kWarpRows * KG; ++j) {
+                            who[j] = __ballot_sync(0xffffffffu, lost >> j & 1u);
+                            found += __popc(who[j]);
                         }
+                        left = lost != 0 && found > p.cap;
+                    }
+                    if (lane == 0) bars->listed[buf][bw] = min(found, p.cap);
                 }
-                if (lane == 0) bars->extras[buf][bw] = extras;
                 tc::fence_smem();
                 unsigned again;
                 asm volatile(
@@ -360,11 +380,38 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                     : "=r"(again)
                     : "r"(static_cast<unsigned>(left && !*bad)), "n"(32 * kBuildWarps)
                     : "memory");
+                if (first) {
+                    const int part = bw % kListWarps;
+                    int at = 0, total = 0;
+#pragma unroll
+                    for (int w = 0; w < kListWarps; ++w) {
+                        const int n = *static_cast<volatile int*>(&bars->listed[buf][bw - part + w]);
+                        if (w < part) at += n;
+                        total += n;
+                    }
+                    uint2* list = lists + (buf * kBuildWarps + bw - part) * p.cap;
+                    if (found > 0) {
+                        int before = 0;
+#pragma unroll
+                        for (int j = 0; j < kWarpRows * KG; ++j) {
+                            const int slot = before + __popc(who[j] & ((1u << lane) - 1u));
+                            before += __popc(who[j]);
+                            if ((lost >> j & 1u) && slot < p.cap) {
+                                const unsigned i = static_cast<unsigned>(ir[j / KG][j % KG]), w = wr[j / KG][j % KG];
+                                list[at + slot] = make_uint2(i & 1u ? w << 16 : w, (i >> 1) << 23 | square_row(part * kWarpRows + j / KG));
+                                wr[j / KG][j % KG] = 0;
+                            }
+                        }
+                    }
+                    // a step of the emitting warps takes four entries
+                    if (part == kListWarps - 1 && lane < (-total & 3)) list[total + lane] = make_uint2(0u, 0u);
+                    __syncwarp();
+                }
                 if (lane == 0) {
                     if (bw == 0) *static_cast<volatile int*>(&bars->more[buf]) = static_cast<int>(again);
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_addr(bars->full + buf)) : "memory");
                 }
-                if (!again) break;  // one answer for the eight warps, which meet at the barrier above
+                if (!again) break;  // one answer for the building warps, which meet at the barrier above
             }
             const int next = t + static_cast<int>(gridDim.x);
             if (next < tiles) fetch(next);
@@ -380,49 +427,55 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
         }
     } else {
         // ---- results -----------------------------------------------------------------------------------------------------
-        const int q = warp & 3, c0 = (warp >> 2) * 16;  // this warp's samples and outputs within the tile
+        const int q = warp & 3, col = lane & 15;  // this warp's samples are 32 q ...; its outputs the 64 / EMIT groups of 16 below
         const int b = b0 + q * 32 + lane;
-        float* sq = ys + warp * 512;  // its [32 samples][16 outputs] square, rows rotated (conflict-free both ways)
-        auto sq_at = [&](int row, int col) -> float& { return sq[row * 16 + ((col + (row >> 1)) & 15)]; };
+        unsigned char* sq = squares + warp * 2048;
+        auto sq_at = [&](int j, int sample) -> float& { return *reinterpret_cast<float*>(sq + ((4 * sample) ^ square_row(j))); };
         const bool nonfinite = __any_sync(0xffffffffu, lane < 2 * kMaxPanels && bars->nonfinite[lane] != 0);
-        int it = 0;
-        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
-            const int buf = it & 1;
+        auto emit = [&](int t, int buf, int c0, bool last) {  // outputs c0 .. c0 + 15 of tile t
             const long long o0 = static_cast<long long>(t) * kRows + c0;
-            const int col = lane & 15;
             const float bias_l = p.bias && o0 + col < L ? __ldg(p.bias + o0 + col) : 0.f;
-            await(bars->ready + buf, (it >> 1) & 1);
             tc::fence_after_sync();
             float v[16];
             tc::load16(tmem_d + buf * kRows + c0 + lane_base, v);
-            tc::fence_before_sync();
-            // repeated inputs of these 16 outputs (two building warps)
-            const int n0 = bars->extras[buf][(c0 >> 3)], n1 = bars->extras[buf][(c0 >> 3) + 1];
-            const bool extra = n0 + n1 > 0 || nonfinite;
+            int total = 0;  // repeated inputs of these outputs
+#pragma unroll
+            for (int w = 0; w < kListWarps; ++w) total += bars->listed[buf][c0 / kWarpRows + w];
+            total = min(total, kListWarps * p.cap);
+            const bool extra = total > 0 || nonfinite;
             if (MODE == 0 || extra) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) sq_at(lane, j) = v[j];
+                for (int j = 0; j < 16; ++j) sq_at(j, lane) = v[j];
             }
             if (extra) {
-                for (int e = 0; e < n0 + n1; ++e) {
-                    const uint2 x = e < n0 ? bars->extra[buf][c0 >> 3][e] : bars->extra[buf][(c0 >> 3) + 1][e - n0];
-                    const float xv = b < p.B ? widen(p.xT[static_cast<size_t>(x.x & 0xffffu) * p.ldx + b]) : 0.f;
-                    float& z = sq_at(lane, static_cast<int>(x.x >> 16) - c0);
-                    z = fmaf(__uint_as_float(x.y), xv, z);
+                // x of the input is in tensor memory, in this warp's lanes
+                const uint4* list = reinterpret_cast<const uint4*>(lists + (buf * kBuildWarps + c0 / kWarpRows) * p.cap);
+#pragma unroll 1
+                for (int e = 0; e < total; e += 4) {
+                    const uint4 lo = list[e / 2], hi = list[e / 2 + 1];
+                    const unsigned w[4] = {lo.x, lo.z, hi.x, hi.z}, at[4] = {lo.y, lo.w, hi.y, hi.w};
+                    unsigned x[4];
+                    tc::load_columns(tmem + lane_base, at[0] >> 23, at[1] >> 23, at[2] >> 23, at[3] >> 23, x);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        float& z = *reinterpret_cast<float*>(sq + ((4 * lane) ^ (at[u] & 0x7f8u)));
+                        z = fma_pair(x[u], w[u], z);
+                    }
                 }
                 if (nonfinite) {
 #pragma unroll 1
                     for (int j = 0; j < 16 && o0 + j < L; ++j)
-                        sq_at(lane, j) = add_nonfinite(p, bars->nonfinite, o0 + j, b, sq_at(lane, j));
+                        sq_at(j, lane) = add_nonfinite(p, bars->nonfinite, o0 + j, b, sq_at(j, lane));
                 }
             }
+            tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0)
+            if (last && lane == 0)
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_addr(bars->dfree + buf)) : "memory");
             if constexpr (MODE == 1) {
                 if (extra) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = sq_at(lane, j);
+                    for (int j = 0; j < 16; ++j) v[j] = sq_at(j, lane);
                 }
                 const float scale = b < p.B ? p.scale : 0.f;
                 const int rows = static_cast<int>(L - o0 < 16 ? (L - o0 < 0 ? 0 : L - o0) : 16);
@@ -457,12 +510,18 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
                 const int left = o < L ? p.B - (b0 + q * 32 + (lane >> 4)) : 0;
 #pragma unroll
                 for (int rr = 0; rr < 16; ++rr) {
-                    const float z = sq_at(2 * rr + (lane >> 4), col) + bias_l;
+                    const float z = sq_at(col, 2 * rr + (lane >> 4)) + bias_l;
                     if (2 * rr < left) *dst = z;
                     dst += 2 * static_cast<long long>(L);
                 }
                 __syncwarp();
             }
+        };
+        int it = 0;
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
+            await(bars->ready + (it & 1), (it >> 1) & 1);
+#pragma unroll 1
+            for (int part = 0; part < 16 / EMIT; ++part) emit(t, it & 1, (warp >> 2) * (256 / EMIT) + part * 16, part == 16 / EMIT - 1);
         }
         if (MODE == 1 && b >= p.B) loss_local = 0.f;
     }
@@ -489,16 +548,25 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdPara
 
 }  // namespace
 
-// Where launch_forward_dense is the faster kernel.  Its time hardly depends on K or the batch, the gather kernel's
-// (forward_bf16.cu) is proportional to K and, in tiles of 32, 64 or 128 columns, to the batch:
-//   * more than 64 samples (128: y 236 against 370 us and loss gradient 242 against 272 at N=768, L=670,091, K=32, y 30 against
-//     53 at N=256, L=100,000; 64: 87 against 58 and 31 against 32);
-//   * a fan-in of at least 16 for y and 24 for the loss gradient (16: 43 against 51 and 50 against 47 us at B=256, N=512,
-//     L=65,536; 8: y 45 against 41);
-//   * a fan-in of at most 64 (registers of the building warps) and a quarter of the inputs: beyond, repeated inputs in a row
-//     are so frequent that their list overflows (N=150, K=40 drawn with replacement: 602 against 215 us).
-bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, bool loss) {
-    return N <= 64 * kMaxPanels && K <= 64 && 4 * K <= N && B > 64 && K >= (loss ? 24 : 16) && L > 0;
+// Where launch_forward_dense is the faster kernel.  Its time hardly depends on the batch or, in steps of 32, on K, that of the gather
+// kernel (forward_bf16.cu) is proportional to K and, in tiles of 32, 64 or 128 columns, to the batch.  How often a row repeats
+// an input is not known here: a table drawn with replacement (as FFILayer draws it and ffi_rewire edits it) has K*K / 2N
+// repeats a row, one of distinct inputs none, and a line is drawn where both kinds are served.  Times are
+// distinct / with replacement against the gather kernel, us:
+//   * more than 64 samples (64: y 87 against 58 at N=768, L=670,091, K=32; 72 at L=300,000: 121/133 against 147);
+//   * a fan-in of at most 64 (registers of the building warps) and a quarter of the inputs;
+//   * at least 16 for y, 24 for the loss gradient (16: 53/59 against 60 and 62 against 62 at B=256, N=512, L=65,536);
+//   * where the gather kernel cannot run (a fan-in off the multiples of 8, rows off the 16-byte boundaries) nothing else: the
+//     alternatives widen x and W first (N=512, L=200,000, K=36: y 88/109 against 196; N=256, L=100,000, K=60: loss 62/136 against 142);
+//   * else y up to a fan-in of an eighth of the inputs (B=256, N=512, L=65,536, K=64: 62/113 against 113; N=384, L=300,000, K=48: 117/201
+//     against 192; beyond, N=256, L=100,000, K=48: 47/92 against 74),
+//   * and the loss gradient, whose epilogue already fills the emitting warps, up to a twelfth, with K at 32 or not far below 64
+//     (N=768, L=670,091: K=32 245/288 against 289, K=64 294/493 against 474, but K=24 245/278 against 251 and K=48 292/407 against
+//     385; N=512, L=200,000: K=32 83/101 against 105, but K=40 103/140 against 118).
+bool forward_dense_applicable(int64_t B, int64_t N, int64_t L, int64_t K, const void* W, const int32_t* idx, bool loss) {
+    if (N > 64 * kMaxPanels || K > 64 || 4 * K > N || B <= 64 || K < (loss ? 24 : 16) || L <= 0) return false;
+    if (K % 8 != 0 || reinterpret_cast<uintptr_t>(W) % 16 != 0 || reinterpret_cast<uintptr_t>(idx) % 16 != 0) return true;
+    return loss ? 12 * K <= N && K >= 32 && round_up(K, 32) - K <= 8 : 8 * K <= N;
 }
 
 // y (or, with `loss`, the loss gradient and one loss partial per CTA) from bf16 x as [N][ldx] and bf16 W.
@@ -524,19 +592,24 @@ int launch_forward_dense(const void* xT, int64_t ldx, const int32_t* idx, const 
     p.scale = loss ? loss->scale : 0.f;
     p.loss_partials = loss ? loss->loss_partials : nullptr;
     p.loss_kind = loss ? loss->loss_kind : 0;
-    const size_t smem = 2 * static_cast<size_t>(p.panels) * kPanelBytes + kEmitWarps * 2048 + sizeof(DenseBarriers);
     const int64_t nBT = ceil_div(B, 128), tiles = ceil_div(L, kRows);
     const int64_t per_bt = dev.sm_count / nBT > 0 ? dev.sm_count / nBT : 1;
     const dim3 grid(static_cast<unsigned>(tiles < per_bt ? tiles : per_bt), static_cast<unsigned>(nBT));
     if (loss) *loss->ctas = static_cast<int>(grid.x * grid.y);
-    auto go = [&](auto kern) -> int {
+    auto go = [&](auto kern, int emit) -> int {
+        // lists as long as a building warp's rows could need, or what is left of the shared memory
+        const int build = kMmaWarp - emit;
+        const size_t used = 2 * static_cast<size_t>(p.panels) * kPanelBytes + emit * 2048 + kListsAt;
+        const int64_t longest = round_up(kRows / build * K, 4), room = (dev.max_smem_optin - static_cast<int64_t>(used)) / (2 * build * 32) * 4;
+        p.cap = static_cast<int>(longest < room ? longest : room);
+        const size_t smem = used + 2 * build * 8 * static_cast<size_t>(p.cap);
         FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
         kern<<<grid, kThreads, smem, stream>>>(p);
         FFI_LAUNCH_CHECK("ffi_fwd_dense_kernel");
         return FFI_OK;
     };
-    if (loss) return K <= 32 ? go(ffi_fwd_dense_kernel<1, 1>) : go(ffi_fwd_dense_kernel<1, 2>);
-    return K <= 32 ? go(ffi_fwd_dense_kernel<0, 1>) : go(ffi_fwd_dense_kernel<0, 2>);
+    if (loss) return K <= 32 ? go(ffi_fwd_dense_kernel<1, 1, 16>, 16) : go(ffi_fwd_dense_kernel<1, 2, 8>, 8);
+    return K <= 32 ? go(ffi_fwd_dense_kernel<0, 1, 16>, 16) : go(ffi_fwd_dense_kernel<0, 2, 8>, 8);
 }
 
 int dense_forward_timeouts(int* out) {

@@ -46,6 +46,18 @@ __device__ __forceinline__ void load16(unsigned taddr, float (&v)[16]) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
+// One column each, at base + c0 ... base + c3, complete on return
+__device__ __forceinline__ void load_columns(unsigned base, unsigned c0, unsigned c1, unsigned c2, unsigned c3, unsigned (&r)[4]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%4];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x1.b32 {%1}, [%5];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x1.b32 {%2}, [%6];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x1.b32 {%3}, [%7];\n"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3])
+        : "r"(base + c0), "r"(base + c1), "r"(base + c2), "r"(base + c3)
+        : "memory");
+}
 
 // Shared-memory descriptor of a K-major panel with the 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes
 // apart; the panel starts on a 1024-byte boundary and K advances by 32 bytes per MMA inside a row.
@@ -53,6 +65,8 @@ __device__ __forceinline__ unsigned long long panel_desc(unsigned addr) {
     return static_cast<unsigned long long>((addr & 0x3ffffu) >> 4) | (1ull << 16) | (static_cast<unsigned long long>(1024 >> 4) << 32) |
            (1ull << 46) | (2ull << 61);
 }
+// The descriptor of what lies `bytes` (a multiple of 16) behind it
+__device__ __forceinline__ unsigned long long desc_at(unsigned long long desc, unsigned bytes) { return desc + (bytes >> 4); }
 // Byte offset of element (row, k) of a panel, k < 64.
 __device__ __forceinline__ unsigned panel_offset(unsigned row, unsigned k) { return row * 128u + ((2u * k) ^ ((row & 7u) << 4)); }
 

@@ -23,8 +23,8 @@ def bf16_case(dev, B, N, L, K, seed, repeats):
     return xd, to_cuda(idx, dev), Wd, xd.float().cpu().numpy(), idx, Wd.float().cpu().numpy()
 
 
-@pytest.mark.parametrize("shape", [(65, 128, 64, 32), (128, 768, 1_001, 32), (100, 300, 130, 40), (256, 512, 777, 64),
-                                   (130, 129, 20_003, 8), (33, 64, 1, 4), (97, 700, 300, 31)],
+@pytest.mark.parametrize("shape", [(65, 256, 64, 32), (128, 768, 1_001, 32), (100, 320, 130, 40), (256, 512, 777, 64),
+                                   (130, 129, 20_003, 16), (70, 128, 37, 16), (97, 700, 300, 31), (128, 768, 130, 64)],
                          ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
 @pytest.mark.parametrize("repeats", ["none", "some", "all"])
 def test_dense_forward_matches_the_oracle(cuda_device, shape, repeats):
@@ -40,7 +40,7 @@ def test_dense_forward_matches_the_oracle(cuda_device, shape, repeats):
         assert torch.equal(y, ops._forward(xin, idd, Wd, to_cuda(bias, dev), transposed))
 
 
-@pytest.mark.parametrize("shape", [(65, 128, 64, 32), (128, 768, 1_001, 32), (100, 300, 130, 40), (256, 512, 777, 64)],
+@pytest.mark.parametrize("shape", [(65, 384, 64, 32), (128, 768, 1_001, 32), (100, 300, 37, 41), (256, 768, 777, 64)],
                          ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
 @pytest.mark.parametrize("repeats", ["none", "some"])
 @pytest.mark.parametrize("loss_name", ["bce", "squared_hinge"])
@@ -62,7 +62,7 @@ def test_dense_forward_loss_matches_the_oracle(cuda_device, shape, repeats, loss
     assert not gT[:, B:].any()
 
 
-@pytest.mark.parametrize("shape", [(65, 128, 64, 32), (130, 768, 1_001, 32), (100, 300, 130, 40)],
+@pytest.mark.parametrize("shape", [(65, 384, 64, 32), (130, 768, 1_001, 32), (100, 300, 130, 41)],
                          ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
 @pytest.mark.parametrize("repeats", ["none", "some", "all"])
 def test_non_finite_inputs_reach_only_the_rows_that_read_them(cuda_device, shape, repeats):
