@@ -137,7 +137,7 @@ def load(rebuild_if_stale: bool = True):
     if rebuild_if_stale:
         try:
             path = _build.build()
-        except Exception as exc:  # no nvcc on this machine: use the shipped library if there is one
+        except _build.CompilerMissing as exc:  # use the shipped library if there is one
             if not os.path.exists(path):
                 raise ImportError(f"libffi_b200.so is missing and could not be built: {exc}") from exc
     if not os.path.exists(path):
@@ -158,9 +158,12 @@ def binding():
         load()
         try:
             _build.build_binding()
-        except Exception as exc:  # no compiler on this machine: use the shipped module if there is one
-            if not os.path.exists(_build.BINDING_PATH):
-                raise ImportError(f"_native.so is missing and could not be built: {exc}") from exc
+        except _build.CompilerMissing as exc:  # use the shipped module if there is one for this torch
+            import torch
+
+            if _build.binding_torch() != torch.__version__:
+                raise ImportError(f"_native.so was built for torch {_build.binding_torch()}, this is torch {torch.__version__}: "
+                                  f"{exc}") from exc
         from . import _native
 
         _binding = _native

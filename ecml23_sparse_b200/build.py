@@ -2,7 +2,7 @@
 binding of its hot entry points over torch tensors, with the host compiler.
 
 ``python -m ecml23_sparse_b200.build`` or :func:`build`.  Each is rebuilt when a source file is newer
-than it.  nvcc cross-compiles without a GPU.
+than it, the binding also when it was built for another torch.  nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -27,10 +27,14 @@ NVCC_FLAGS = [
 ]
 
 
+class CompilerMissing(RuntimeError):
+    """This machine has no compiler; what was built elsewhere may be used."""
+
+
 def _nvcc() -> str:
     exe = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(exe):
-        raise RuntimeError("nvcc not found; the FFI library cannot be built")
+        raise CompilerMissing("nvcc not found; the FFI library cannot be built")
     return exe
 
 
@@ -85,8 +89,22 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     return LIB_PATH
 
 
-def _binding_stale() -> bool:
+_TORCH_MARK = b"ffi-binding-torch="
+
+
+def binding_torch() -> str | None:
+    """The torch version ``_native.so`` was compiled against (None: there is no module)."""
     if not os.path.exists(BINDING_PATH):
+        return None
+    with open(BINDING_PATH, "rb") as f:
+        after = f.read().partition(_TORCH_MARK)[2]
+    return after.partition(b"\0")[0].decode("ascii", "replace")
+
+
+def _binding_stale() -> bool:
+    import torch
+
+    if binding_torch() != torch.__version__:
         return True
     deps = [BINDING_SRC, os.path.join(INCLUDE, "ffi_b200.h")]
     return any(os.path.getmtime(d) > os.path.getmtime(BINDING_PATH) for d in deps)
@@ -105,8 +123,11 @@ def build_binding(force: bool = False, verbose: bool = False) -> str:
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include"), INCLUDE]
     libs = [p for p in cpp_extension.library_paths()]
-    cmd = [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-isystem{i}" for i in includes),
+    gxx = shutil.which("g++")
+    if not gxx:
+        raise CompilerMissing("g++ not found; the binding cannot be built")
+    cmd = [gxx, "-std=c++17", "-O2", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DFFI_TORCH_VERSION="{torch.__version__}"', *(f"-isystem{i}" for i in includes),
            BINDING_SRC, "-o", BINDING_PATH, f"-L{PKG_DIR}", "-lffi_b200", "-Wl,-rpath,$ORIGIN",
            *(f"-L{p}" for p in libs), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
     if verbose:

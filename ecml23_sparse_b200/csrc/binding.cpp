@@ -22,6 +22,9 @@
 
 #include "ffi_b200.h"
 
+// read from the file by build.py: a module built for another torch is stale
+extern "C" __attribute__((used, visibility("default"))) const char ffi_binding_torch[] = "ffi-binding-torch=" FFI_TORCH_VERSION;
+
 namespace py = pybind11;
 using at::Tensor;
 using OptTensor = std::optional<Tensor>;
