@@ -544,7 +544,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 
         // grad_bias of the chunk's rows: the slices of a range take turns, each row is one group's sum
         if (p.gbias && static_cast<int>(c % gridDim.y) == static_cast<int>(blockIdx.y)) {
-            // (T is a multiple of 8: with more groups the last rows leave some of a warp's lanes without one)
+            // (T is a multiple of 8: with more groups the last rows leave some of a warp's lanes without one.  The form for
+            // them, used throughout, costs 961.5 -> 969.7 us at B=128, N=768, L=670,091, K=32, three runs each within 0.1.)
             for (int rr = G * warp + grp; G <= 8 ? rr < T : rr - grp < T; rr += G * kWarps) {
                 LaneT v;
                 if constexpr (G > 8) v.zero();

@@ -333,9 +333,12 @@ struct DeviceBuffer {
 // Rows per chunk of the chunked lists: the one-pass backward keeps, per chunk, a g tile of T x 128 floats and twice the
 // (weight, code) pairs of a slice of the inputs in shared memory, and a chunk's positions fit 14 bits.
 //   * T is the largest multiple of 8 for which that fits (long runs per input and chunk are cheap runs) into what leaves
-//     60 KB of L1 to the gathers of W: with 28 KB the kernel slows down by a tenth (B=128, N=768, K=32: 903 us with T=264,
-//     917 with 256, 995 with 288).  Where the runs would be shorter than six entries their length counts for more, and the
-//     whole shared memory is used (N=1024, K=8: 322 us with T=352, 352 with 296; N=2000, K=32: 223 and 235).
+//     60 KB of L1 to the gathers of W (28 KB slow those down), or, where the runs are short, into the whole shared memory: a run's
+//     cost of its own then counts for more.  Backward at B=128, L=200,000, us with 60 KB / with the whole, by the
+//     entries of a run (264 K / N): 2.1 (N=1024, K=8) 202/187; 4.1 (N=1024, K=16) 249/233; 5.5 (N=1536, K=32) 405/392; 6.6 (N=1280, K=32)
+//     382/380; 8.2 (N=1024, K=32) 337/349; 11 (N=768, K=32) 306/316; 16.5 (N=768, K=48) 409/431; 33 (N=512, K=64) 484/519.  The
+//     line is between 6.6 and 8.2.  (Fan-ins of 8 and 16 gain 2 to 5 % from the whole also above it, a batch of 32, whose tile
+//     leaves L1 room in either case, up to 8 %; the plan does not know the batch.)
 //   * it is lowered until the chunks fill the SMs: the kernel runs R = SMs / slices ranges of chunks, so the chunks are cut
 //     to a whole number per range; a short L (down to 16 rows per chunk) is cut to one chunk per range, or two where they
 //     keep 64 rows, for the ranges of a batch of 64 are twice as many.  Before, a table of fewer than R * 256 rows left most
@@ -346,7 +349,7 @@ int plan_chunk_rows(int64_t L, int64_t K, int64_t N) {
     const FusedSlices sl = fused_slices(N, false);
     const double share = sl.parts > 1 ? 16.0 * sl.ni / static_cast<double>(N) : 1.0;
     int64_t T = 512;
-    const double budget = 264.0 * K >= 6.0 * N ? 160700.0 : 190464.0;
+    const double budget = 264.0 * K >= 7.0 * N ? 160700.0 : 190464.0;
     for (; T > 8; T -= 8) {
         const double entries = static_cast<double>(T) * K * share;
         const double spread = sl.parts > 1 ? 4.0 * std::sqrt(entries) : 0.0;  // a random table's fullest slice
