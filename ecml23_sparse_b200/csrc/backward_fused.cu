@@ -21,7 +21,7 @@
 
 #include <type_traits>
 
-#include "ffi_common.cuh"
+#include "tcgen05.cuh"
 
 namespace ffi {
 int peer_wait_timeouts(int* out);  // peer_reduce.cu
@@ -101,30 +101,9 @@ struct BwdFusedParams {
 // tcgen05.ld of the 16 columns and ends with one tcgen05.st of the sums, so the loop over the
 // warp's inputs needs no unrolling and few registers.
 // =====================================================================================
-constexpr int kTmemCols = 512;            // per lane quarter: 4 warps x 8 inputs x 16 columns
 constexpr unsigned kPadCode = 0xffffffffu;  // code of the missing second entry of an odd run's last step
 
-__device__ __forceinline__ void tmem_alloc(void* smem_dst, unsigned ncols) {
-    const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(a), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(unsigned taddr, unsigned ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_fence_before_sync() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_fence_after_sync() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// 8 consecutive 32-bit columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_store8(unsigned taddr, const unsigned (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// 8 consecutive 32-bit columns of this thread's TMEM lane; tmem_wait_load comes before their first use
 __device__ __forceinline__ void tmem_load8(unsigned taddr, unsigned (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -142,46 +121,28 @@ __device__ __forceinline__ void tmem_wait_load(unsigned (&r)[8], unsigned (&s)[8
 
 // ---- mbarrier + TMA (one tiled bulk copy per g tile, no multicast) ------------------------------
 
-__device__ __forceinline__ unsigned smem_u32(const void* ptr) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(ptr));
-}
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-// Orders this thread's earlier generic-proxy accesses to shared memory before later async-proxy ones.
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_addr(bar)), "r"(bytes) : "memory");
 }
 // Box of the 2-D tensor `map` with first element (x, y) -> dst; completion is signalled on `bar`.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_u32(dst)),
-        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+            tc::smem_addr(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(tc::smem_addr(bar))
         : "memory");
 }
 // The same box into L2 only.
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // Waits for the phase with the given parity, at most g_wait_limit (or, for a copy that nobody will use, kDrainLimit) ticks;
 // false if it gave up.
 __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity, bool drain = false) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (tc::bar_try_wait(bar, parity)) return true;
     const long long start = clock64();
     const long long limit = drain ? kDrainLimit : g_wait_limit;
-    while (!mbar_try_wait(bar, parity))
+    while (!tc::bar_try_wait(bar, parity))
         if (clock64() - start > limit) return false;
     return true;
 }
@@ -291,7 +252,7 @@ __device__ __forceinline__ void tmem_store_sums(unsigned taddr, const Lane4& sum
 template <int VPL>
 __device__ __forceinline__ void tmem_store_cols(unsigned taddr, const unsigned (&r)[VPL]) {
     if constexpr (VPL == 8) {
-        tmem_store8(taddr, r);
+        tc::store8(taddr, r);
     } else {
         asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
                      "r"(r[2]), "r"(r[3])
@@ -358,7 +319,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int ni = FULL ? NI : p.ni;  // inputs per warp: the slices of a range split the inputs evenly
     const int CPN = kWarps * ni + 1;
     constexpr unsigned kRowMask = (1u << kKShift) - 1u;
-    static_assert((THREADS / 128) * NI * COLS <= kTmemCols, "the warps of a lane quarter share the TMEM columns");
+    static_assert((THREADS / 128) * NI * COLS <= tc::kCols, "the warps of a lane quarter share the TMEM columns");
     static_assert(SLOTS * G == 32, "the lane reduction maps the 32 lanes to (buffered step, group)");
     static_assert(32 + G <= kDRow, "a dot-buffer row holds 32 dots and G entry codes");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -382,11 +343,11 @@ __global__ void __launch_bounds__(THREADS, 1)
     const long long c_begin = p.nChunks * r / p.R;
     const long long c_end = p.nChunks * (r + 1) / p.R;
 
-    if (warp == 0) tmem_alloc(tmem_base_p, kTmemCols);
-    if (tid == 32) mbar_init(g_bar, 1);
-    tmem_fence_before_sync();
+    if (warp == 0) tc::alloc(tmem_base_p);
+    if (tid == 32) tc::bar_init(g_bar, 1);
+    tc::fence_before_sync();
     __syncthreads();
-    tmem_fence_after_sync();
+    tc::fence_after_sync();
     const unsigned tmem_base = *tmem_base_p;
     // lanes 32*(warp % 4) .. +31 are the ones this warp may touch; its inputs take NI*COLS columns
     const unsigned taddr0 = tmem_base + ((static_cast<unsigned>(warp & 3) * 32u) << 16) +
@@ -416,7 +377,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 tmem_store_cols<VPL>(taddr0 + (j0 + jj) * COLS + VPL, xv[jj]);
             }
     }
-    tmem_wait_store();
+    tc::wait_store();
 
     auto slice_bounds = [&](long long c, int& e_lo, int& cnt) {
         const int* cptr_c = p.cptr + c * (N + 1);
@@ -514,7 +475,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         // (A second tile buffer filled one chunk ahead was measured: it needs T <= 168 to fit, and the
         // shorter runs cost more than the hidden copy saves.)
         if (tid == 0) {
-            fence_proxy_async();
+            tc::fence_smem();
             mbar_expect_tx(g_bar, tileBytes);
             for (int h = 0; h < p.boxes; ++h) {
                 const int rows = T / p.boxes;
@@ -646,7 +607,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             tmem_store_sums(taddr0 + j * COLS, acc);
         }
         if (dptr != dlane) reduce_slots();
-        tmem_wait_store();
+        tc::wait_store();
 
         __pipeline_wait_prior(0);  // this thread's staged weights of the next chunk are in place
         widen_staged(buf ^ 1, staged_cnt);
@@ -663,7 +624,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     #pragma unroll
                     for (int m = 0; m < 8; ++m) zero[m] = 0u;
                     tmem_wait_load(av, zero);
-                    tmem_store8(taddr0 + j * 16, zero);
+                    tc::store8(taddr0 + j * 16, zero);
                     float out[8];
     #pragma unroll
                     for (int m = 0; m < 8; ++m) {
@@ -718,7 +679,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                 }
             }
-            tmem_wait_store();
+            tc::wait_store();
         }
     }
 
@@ -737,9 +698,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     // A thread that gave up waits once more for the copy it abandoned (the chunk it recorded when the copy was
     // issued) before the CTA releases its shared memory: again bounded, but not by a limit that a caller has lowered.
     if (pending >= 0) mbar_wait_bounded(g_bar, static_cast<unsigned>(pending - c_begin) & 1u, true);
-    tmem_fence_before_sync();
+    tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_base, kTmemCols);
+    if (warp == 0) tc::dealloc(tmem_base);
 }
 
 struct FusedConfig {

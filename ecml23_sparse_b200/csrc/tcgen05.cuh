@@ -1,5 +1,6 @@
-// Thin wrappers of the fifth-generation tensor core instructions (tcgen05, TMEM, mbarrier) for the kernels that densify
-// tiles of the weight table (forward_dense.cu, backward_dense.cu).  All of them use one form of the MMA:
+// Thin wrappers of the fifth-generation tensor core instructions (tcgen05, TMEM, mbarrier): for the forward that densifies tiles
+// of the weight table (forward_dense.cu), and for the one-pass backward, which keeps sums and inputs in tensor memory
+// (backward_fused.cu).  The MMA has one form here:
 //   D[128][n] (+)= A[128][16] * B[n][16]^T,  bf16 operands, fp32 accumulation,
 // A and D in tensor memory, B in shared memory, K-major in panels of 64 elements (128 bytes) with the 128-byte swizzle.
 #pragma once
@@ -24,7 +25,7 @@ __device__ __forceinline__ void dealloc(unsigned base) {
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// Orders this thread's generic-proxy writes to shared memory before the tensor core's reads.
+// Orders this thread's generic-proxy accesses to shared memory before later reads of the tensor core or copies of the TMA unit.
 __device__ __forceinline__ void fence_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // 8 consecutive columns of this thread's TMEM lane
