@@ -153,7 +153,8 @@ __device__ __forceinline__ void store_lane_f32(float* base, int lane, const floa
 // xT is x in [N][ldx] layout (batch contiguous); xT and W are fp32, or bf16 when `bf16` is set (only the
 // tiled kernels take bf16; the callers see to that).
 // loss and d(loss)/dz of one logit whose target is 0 (ffi_loss_kind: BCE, squared hinge, hinge);
-// shared by the loss epilogues of all forward kernels, so that they agree bit for bit
+// shared by the loss epilogues of the forward kernels, so that they agree bit for bit (all but BCE in the tensor-core forward, which
+// has the same formulas for sixteen logits at once and takes one logarithm of a product: there the last bits may differ)
 __device__ __forceinline__ void loss_for_negative(int kind, float z, float& value, float& grad) {
     if (kind == 0) {
         // one exponential serves both: s = exp(-|z|), softplus(z) = max(z,0) + log(1+s),

@@ -41,19 +41,6 @@ struct FwdBf16Params {
     int loss_kind;
 };
 
-__device__ __forceinline__ void loss_negative_bf(int kind, float z, float& value, float& grad) {
-    if (kind == 0) {
-        const float s = __expf(-fabsf(z));
-        const float r = __fdividef(1.f, 1.f + s);
-        value = fmaxf(z, 0.f) + __logf(1.f + s);
-        grad = z >= 0.f ? r : s * r;
-    } else {
-        const float h = fmaxf(1.f + z, 0.f);
-        value = kind == 1 ? h * h : h;
-        grad = kind == 1 ? 2.f * h : (h > 0.f ? 1.f : 0.f);
-    }
-}
-
 // VPL bf16 of one lane, as 32-bit words
 template <int VPL>
 struct LaneWords;
@@ -218,7 +205,7 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
                     for (int j = 0; j < VPL; ++j) {
                         const bool live = b + j < p.B;
                         float v, g;
-                        loss_negative_bf(p.loss_kind, z[j] + bias, v, g);
+                        loss_for_negative(p.loss_kind, z[j] + bias, v, g);
                         if (live && mine) loss_local += v;
                         gv[j] = live ? p.scale * g : 0.f;
                     }
