@@ -23,7 +23,6 @@ import torch
 
 from . import _lib
 
-_workspaces: dict = {}
 _plan_cache: dict = {}
 _PLAN_CACHE_MAX = 8
 
@@ -41,16 +40,10 @@ def _native():
     return mod
 
 
-def _workspace(device, nbytes: int) -> Optional[torch.Tensor]:
-    """A cached scratch buffer of at least nbytes on `device` (grown, never shrunk)."""
-    if nbytes <= 0:
-        return None
-    key = (device.index, _stream_ptr(device))
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(int(nbytes * 1.25) + 256, dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
+def _workspace(device, nbytes: int) -> torch.Tensor:
+    """Scratch of a call that goes over ctypes, in stream order from torch's allocator (a few kilobytes; the hot entry points
+    keep one buffer per stream, csrc/binding.cpp)."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 def _check_cuda(name: str, t: torch.Tensor, dtypes) -> torch.Tensor:
@@ -155,7 +148,6 @@ def get_plan(lookup: torch.Tensor, n_in: int) -> FFIPlan:
 
 def clear_caches():
     _plan_cache.clear()
-    _workspaces.clear()
     _native().clear_scratch()
 
 
