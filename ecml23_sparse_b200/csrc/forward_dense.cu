@@ -23,9 +23,10 @@
 //     or the loss gradient (16 and 8 with K > 32: building, two entries a lane, is the longest stage there); mbarriers hand the
 //     buffers on, so the three stages of consecutive tiles overlap.  (With all warps building and emitting in turn, one CTA
 //     barrier per tile, the stages' latencies added up: 214 us for y, 310 with the BCE epilogue.)
-// What bounds it: at N = 768 and K = 32 the thread that issues the MMAs is busy for 0.92 of the time, the
-// tensor pipe for 0.4 (tiles of 64 rows are what fits beside x); with repeated inputs the emitting warps,
-// about 80 clocks an entry (its square of results is read, added to and written in shared memory).
+// What bounds it, by the share of the time that a stage does not wait for another (N = 768, distinct inputs / with replacement): at
+// K = 32 the thread that issues the MMAs 0.88 / 0.86 (the tensor core's part is active for 0.46 / 0.42; tiles of 64 rows are
+// what fits beside x), the building warps 0.84 / 0.95, the emitting ones 0.43 / 0.56; at K = 64 the thread 0.90 / 0.59, building
+// 0.82 / 0.68, emitting 0.59 / 0.97 (about 80 clocks per repeated input: its sum is read, added to and written in shared memory).
 // Measured at B = 128, L = 670,091, tables of distinct inputs / drawn with replacement, against the gather kernel:
 // N = 768, K = 32: y 232/261 (379) us, loss gradient 245/288 (289) us; K = 64: 274/430 (594) and 294/493 (474) us;
 // B = 256, N = 512, L = 65,536, K = 64: y 62/113 (113) us.  With the lists read by 16 warps from L2, one entry after the other, and
