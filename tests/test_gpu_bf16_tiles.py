@@ -11,7 +11,8 @@ from cases import ATOL, RTOL, assert_close, config_style_inputs, to_cuda
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(16, 80, 3_001, 72), (9, 2_900, 501, 8), (32, 768, 5, 72), (59, 455, 2_973, 72), (64, 1_500, 777, 16), (33, 96, 40_001, 80),
-          (128, 768, 1_001, 72), (130, 384, 515, 16), (203, 384, 7_210, 16), (500, 80, 1_111, 72), (97, 1_100, 333, 24)]
+          (128, 768, 1_001, 72), (130, 384, 515, 16), (203, 384, 7_210, 16), (500, 80, 1_111, 72), (97, 1_100, 333, 24),
+          (130, 384, 515, 64)]  # the last: gathers where the rows start on 16 bytes, the tensor cores where not
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "B{}_N{}_L{}_K{}".format(*s))
