@@ -381,7 +381,8 @@ extern "C" size_t ffi_backward_workspace_bytes(const ffi_plan* plan, int64_t B, 
     if (want_grad_x && plan) {
         const size_t sep = grad_x_workspace_bytes(plan, B), fus = backward_fused_workspace_bytes(plan, B);
         total += align_up(sep > fus ? sep : fus);
-        total += align_up(static_cast<size_t>(N) * round_up(B, 128) * 4);  // xT copy of the fused kernel
+        total += align_up(static_cast<size_t>(N) * round_up(B, 128) * 4);  // xT copy of the fused kernel, grad_x as [N][B] of the wide one
+        if (want_grad_w && backward_wide_applicable(plan)) total += align_up(static_cast<size_t>(N) * 4);  // its cursors
     }
     // the transposed upstream gradient gT[L][ldg], shared by grad_x and the barrier-free grad_W kernel
     if (want_grad_x || (want_grad_w && K % 4 == 0))
@@ -450,7 +451,13 @@ static int backward_impl(const void* x, const int32_t* idx, const void* W, const
 
     // One pass for grad_x and grad_W when the shape allows it, else one kernel each.
     const bool fused = grad_x && grad_w && backward_fused_applicable(plan, B);
-    const bool sep_w = !fused && (grad_w || grad_bias);
+    // Wide inputs: the one-pass kernel of backward_wide.cu, unless a caller that sized its workspace by itself left no room
+    // for the cursors and copies.
+    const size_t wide_gT = gT_in ? 0 : align_up(static_cast<size_t>(L) * transposed_g_stride(B) * 4);
+    const size_t wide_x = x_transposed ? 0 : align_up(static_cast<size_t>(N) * round_up(B, 128) * esize) + align_up(static_cast<size_t>(N) * B * 4);
+    const bool wide = !fused && grad_x && grad_w && backward_wide_applicable(plan) && (x_transposed || N <= 65535 * 32) &&
+                      workspace && workspace_bytes >= wide_gT + wide_x + align_up(static_cast<size_t>(N) * 4);
+    const bool sep_w = !fused && !wide && (grad_w || grad_bias);
     const bool gw_stream = sep_w && grad_w_stream_applicable(Bi, Ni, Ki, idx);
 
     // g transposed to [L][ldg] once, for the kernels that read whole batch rows of g; the same
@@ -510,6 +517,30 @@ static int backward_impl(const void* x, const int32_t* idx, const void* W, const
         ax.workspace = part;
         ax.workspace_bytes = workspace_bytes - (static_cast<unsigned char*>(part) - ws);
         return launch_backward_fused(ax, xT, ldx, grad_w, bias_done ? nullptr : grad_bias, stream);
+    }
+
+    if (wide) {
+        const void* xT = x;
+        int64_t ldx = B;
+        void* cursor = nullptr;
+        rc = take(static_cast<size_t>(N) * 4, "the cursors", &cursor);
+        if (rc != FFI_OK) return rc;
+        float* gxT = grad_x;
+        if (!x_transposed) {
+            ldx = round_up(B, 128);
+            void *dst = nullptr, *gdst = nullptr;
+            rc = take(static_cast<size_t>(N) * ldx * esize, "the transposed x", &dst);
+            if (rc == FFI_OK) rc = take(static_cast<size_t>(N) * B * 4, "the transposed grad_x", &gdst);
+            if (rc != FFI_OK) return rc;
+            rc = bf16 ? launch_transpose_pad_bf16(x, dst, Bi, Ni, ldx, stream)
+                      : launch_transpose_pad(static_cast<const float*>(x), static_cast<float*>(dst), Bi, Ni, ldx, stream);
+            if (rc != FFI_OK) return rc;
+            xT = dst;
+            gxT = static_cast<float*>(gdst);
+        }
+        rc = launch_backward_wide(ax, xT, ldx, gxT, grad_w, bias_done ? nullptr : grad_bias, static_cast<int*>(cursor), stream);
+        if (rc != FFI_OK || x_transposed) return rc;
+        return launch_transpose_pad(gxT, grad_x, Ni, Bi, N, stream);
     }
 
     if (grad_w || (grad_bias && !bias_done)) {

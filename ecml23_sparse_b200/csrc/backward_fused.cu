@@ -21,6 +21,7 @@
 
 #include <type_traits>
 
+#include "packed.cuh"
 #include "tcgen05.cuh"
 
 namespace ffi {
@@ -39,27 +40,6 @@ constexpr int kWarps = kThreads / 32;
 __host__ __device__ constexpr int dot_row(int groups) { return groups <= 4 ? 36 : 32 + groups; }
 constexpr int kStageUnroll = 4;       // staged entries per thread kept in flight
 constexpr int kKShift = 18;           // entry code = byte offset of the g row (with its swizzle key) | k << 18
-
-// ---- packed fp32 pairs: sm_100 issues two IEEE fp32 operations per lane and instruction -----------
-using u64 = unsigned long long;
-__device__ __forceinline__ u64 pack2(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 
 struct BwdFusedParams {
     const void* W;   // fp32; the group kernel also takes bf16 (its TX)

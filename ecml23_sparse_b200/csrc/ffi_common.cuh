@@ -318,5 +318,9 @@ size_t backward_fused_workspace_bytes(const ffi_plan* plan, int64_t B);
 // xT (x as [N][ldx]) has the element type of a.W: fp32, or bf16 when a.w_bf16 is set.
 int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float* gW, float* gbias,
                           cudaStream_t stream);
+// The same for wide inputs; grad_x leaves as gxT[N][B], cursor is scratch of N ints.
+bool backward_wide_applicable(const ffi_plan* plan);
+int launch_backward_wide(const GradXArgs& a, const void* xT, int64_t ldx, float* gxT, float* gW, float* gbias, int* cursor,
+                         cudaStream_t stream);
 
 }  // namespace ffi

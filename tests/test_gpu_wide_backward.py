@@ -1,0 +1,104 @@
+"""One-pass backward for wide inputs (csrc/backward_wide.cu) against fp64 sums: edges of its tiles, batches and chunks."""
+import pytest
+import torch
+
+from ecml23_sparse_b200 import ops
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -24
+
+# B, N, L, K, storage, x given as [N,B]
+SHAPES = [
+    (1, 2049, 70, 3, "f32", True),             # one column, runs of a handful of entries
+    (33, 3001, 517, 33, "f32", False),         # odd batch: tile of 64 columns, ragged rows of x, x given as [B,N]
+    (64, 20000, 31, 8, "bf16", True),          # most inputs have no entry
+    (85, 2500, 4099, 36, "bf16", False),
+    (128, 16384, 2000, 32, "f32", True),
+    (130, 4096, 1500, 63, "f32", True),        # 256 columns allocated, the second half nearly empty
+    (300, 2200, 900, 17, "bf16", True),        # three tiles of 128 columns
+    (32, 2111, 400000, 4, "f32", True),        # two chunks of one narrow tile
+    (256, 3000, 50021, 8, "bf16", True),       # two chunks of one tile of 256 columns
+    (512, 3000, 50021, 5, "f32", False),       # two chunks of two tiles each
+]
+
+
+def _inputs(B, N, L, K, storage, seed=3):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    dt = torch.bfloat16 if storage == "bf16" else torch.float32
+    x = torch.randn((B, N), generator=gen, device="cuda").to(dt)
+    idx = torch.randint(0, N, (L, K), generator=gen, dtype=torch.int32, device="cuda")
+    idx[:, 0] = idx[:, 0] % 5          # long runs: several batches of 32 entries per chunk
+    W = torch.randn((L, K), generator=gen, device="cuda").to(dt)
+    g = torch.randn((B, L), generator=gen, device="cuda")
+    return x, idx, W, g
+
+
+def _reference(x, idx, W, g):
+    """fp64 values and the sums of magnitudes that bound the rounding of any order of fp32 additions."""
+    xT, gT, W = x.double().t().contiguous(), g.double().t().contiguous(), W.double()
+    gx, gx_abs = torch.zeros_like(xT), torch.zeros_like(xT)
+    gw, gw_abs = torch.empty_like(W), torch.empty_like(W)
+    for k in range(idx.shape[1]):
+        i = idx[:, k].long()
+        t = W[:, k, None] * gT
+        gx.index_add_(0, i, t)
+        gx_abs.index_add_(0, i, t.abs())
+        t = xT[i] * gT
+        gw[:, k], gw_abs[:, k] = t.sum(1), t.abs().sum(1)
+    return gx, gx_abs, gw, gw_abs, gT.sum(1), gT.abs().sum(1)
+
+
+@pytest.mark.parametrize("B,N,L,K,storage,tp", SHAPES)
+def test_matches_fp64(B, N, L, K, storage, tp):
+    x, idx, W, g = _inputs(B, N, L, K, storage)
+    gx, gx_abs, gw, gw_abs, gb, gb_abs = _reference(x, idx, W, g)
+    ldg = 32 if B <= 32 else 64 if B <= 64 else (B + 127) // 128 * 128
+    gT = torch.zeros((L, ldg), device="cuda")
+    gT[:, :B] = g.t()
+    xs = x.t().contiguous() if tp else x
+    plan = ops.FFIPlan(idx, N)
+    # a sum of n products in fp32, in any order, is off by at most n * 2^-24 times the sum of magnitudes
+    runs = torch.bincount(idx.flatten().long(), minlength=N).double()[:, None] + 8
+    for from_transposed in (True, False):
+        def call():
+            return ops._backward(xs, idx, W, gT if from_transposed else g, tp, plan=plan, want_bias_grad=True,
+                                 grad_is_transposed=from_transposed)
+        ox, ow, ob = call()
+        oxT = (ox if tp else ox.t()).double()
+        assert ((oxT - gx).abs() <= runs * EPS * gx_abs + 1e-30).all()
+        assert ((ow.double() - gw).abs() <= (B + 8) * EPS * gw_abs).all()
+        assert ((ob.double() - gb).abs() <= (B + 8) * EPS * gb_abs).all()
+        for a, b in zip((ox, ow, ob), call()):
+            assert torch.equal(a, b)
+
+
+def test_captured_and_with_special_values():
+    B, N, L, K = 256, 3000, 50021, 8
+    x, idx, W, g = _inputs(B, N, L, K, "f32")
+    g[7, 49999] = float("nan")
+    g[9, 3] = float("inf")
+    xs, gT = x.t().contiguous(), g.t().contiguous()
+    plan = ops.FFIPlan(idx, N)
+
+    def call():
+        return ops._backward(xs, idx, W, gT, True, plan=plan, want_bias_grad=True, grad_is_transposed=True)
+
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        want = call()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = call()
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    bad_rows = torch.zeros(L, dtype=torch.bool, device="cuda")
+    bad_rows[[49999, 3]] = True
+    assert not torch.isfinite(want[1][bad_rows]).any() and torch.isfinite(want[1][~bad_rows]).all()
+    bad = torch.zeros((N, B), dtype=torch.bool, device="cuda")
+    bad[idx[49999].long(), 7] = True
+    bad[idx[3].long(), 9] = True
+    assert torch.equal(~torch.isfinite(want[0]), bad)
