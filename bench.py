@@ -767,7 +767,7 @@ def run_ours(args):
     names = {"forward": ("ffi_fwd_dense_kernel" if args.storage == "bf16" else "ffi_fwd_pair_kernel") if narrow
              else "ffi_fwd_gather_kernel",
              "transpose_g": "transpose_g_kernel",
-             "backward_fused": "ffi_bwd_pairs_kernel" if narrow else "ffi_grad_w_gather_kernel + ffi_grad_x_wide_kernel"}
+             "backward_fused": "ffi_bwd_runs_kernel" if narrow else "ffi_bwd_wide_kernel"}
     kernels = {}
     for name, ms in kernel_ms.items():
         nbytes, fmas = work[name]

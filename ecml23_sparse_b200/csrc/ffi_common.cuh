@@ -259,6 +259,10 @@ int launch_transpose_pad(const float* src, float* dst, int rows, int cols, int64
 
 }  // namespace ffi
 
+namespace ffi {
+constexpr int kFusedWarps = 16;  // walking warps of the one-pass backward
+}  // namespace ffi
+
 // The plan object (defined in plan.cu, used by backward.cu and api.cu).
 struct ffi_plan {
     int64_t L = 0, K = 0, N = 0;
@@ -266,8 +270,10 @@ struct ffi_plan {
     int chunk_rows = 0;     // T: outputs per chunk of the chunked lists
     int64_t n_chunks = 0;   // ceil(L / T)
     bool has_chunks = false;
-    // largest number of entries any (chunk, slice) holds, for the slicings fused_slices(N, 0 / 1)
-    int max_slice_entries[2] = {0, 0};
+    // where the entries of each warp of a slice start in a staging buffer of the one-pass backward: the gaps hold the largest number
+    // that the warp has in any chunk and slice
+    int fused_entries[ffi::kFusedWarps + 1] = {};
+    int fused_ni = 0;  // inputs per warp of the one-pass backward
     void* arrays = nullptr;     // the allocation that holds the four index arrays
     int32_t* rowptr = nullptr;  // [N+1]   canonical CSR-by-input
     int32_t* perm = nullptr;    // [L*K]   positions sorted by (idx[p], p)
@@ -301,15 +307,16 @@ size_t grad_x_workspace_bytes(const ffi_plan* plan, int64_t B);
 bool grad_x_narrow_applicable(const ffi_plan* plan, int64_t B);
 int launch_grad_x(const GradXArgs& a, cudaStream_t stream);
 
-// How the one-pass backward splits the inputs: `parts` slices of 16 warps x `ni` inputs, as even as possible; at most
-// kFusedNI inputs per warp with a batch tile of 65..128 columns, twice that with up to 64 (narrow).
-constexpr int kFusedNI = 8;
-struct FusedSlices {
-    int parts, ni;
-};
-inline FusedSlices fused_slices(int64_t N, bool narrow) {
-    const int64_t parts = ceil_div(N, 16 * kFusedNI * (narrow ? 2 : 1));
-    return {static_cast<int>(parts), static_cast<int>(ceil_div(N, 16 * parts))};
+// How the one-pass backward splits the inputs: slices of 16 warps x `ni` inputs, as even as possible.
+constexpr int kFusedNI = 16;
+inline int fused_inputs_per_warp(int64_t N) {
+    const int64_t parts = ceil_div(N, kFusedWarps * kFusedNI);
+    return static_cast<int>(ceil_div(N, kFusedWarps * parts));
+}
+// Shared memory of its CTA: the g tiles, a row of zeros, two staging buffers of `entries` (weight, code) pairs, 32 / groups rows of 36 partial dots and
+// 2 x 36 bounds per warp, barriers.
+inline size_t fused_smem_bytes(int64_t tile_bytes, int64_t entries, int groups) {
+    return static_cast<size_t>(tile_bytes) + 16 * static_cast<size_t>(entries) + kFusedWarps * (32 / groups * 36 + 2 * 36) * 4 + 48 + 512;
 }
 
 // grad_x and grad_W in one pass over the transposed index (narrow inputs).

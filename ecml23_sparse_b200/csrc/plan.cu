@@ -267,18 +267,14 @@ __global__ void chunk_fill_kernel(const int* __restrict__ perm, const int* __res
     }
 }
 
-// stats[j] = max over chunks c and slices s of the entries of chunk c whose input lies in slice s (w0 or w1 inputs wide).
-// Integer max is order independent.
-__global__ void slice_stats_kernel(const int* __restrict__ cptr, int N, long long nChunks, int w0, int w1, int* __restrict__ stats) {
-    const long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (c >= nChunks) return;
-    const int* row = cptr + c * (N + 1);
-    for (int j = 0; j < 2; ++j) {
-        const int w = j ? w1 : w0;
-        int best = 0;
-        for (int lo = 0; lo < N; lo += w) best = max(best, row[min(N, lo + w)] - row[lo]);
-        atomicMax(stats + j, best);
-    }
+// most[w] = largest number of entries that warp w of a slice has in any chunk and slice (zeroed by the caller); a slice is kFusedWarps
+// warps of ni inputs.  One block per warp of all slices.
+__global__ void warp_stats_kernel(const int* __restrict__ cptr, int N, long long nChunks, int ni, int* __restrict__ most) {
+    const int lo = min(N, static_cast<int>(blockIdx.x) * ni), hi = min(N, lo + ni);
+    int best = 0;
+    for (long long c = threadIdx.x; c < nChunks; c += blockDim.x) best = max(best, cptr[c * (N + 1) + hi] - cptr[c * (N + 1) + lo]);
+    best = __reduce_max_sync(0xffffffffu, best);
+    if (threadIdx.x % 32 == 0) atomicMax(most + blockIdx.x % kFusedWarps, best);
 }
 
 // Self-check export: rebuild the canonical form from (cptr, cperm).
@@ -330,38 +326,39 @@ struct DeviceBuffer {
 
 }  // namespace
 
-// Rows per chunk of the chunked lists: the one-pass backward keeps, per chunk, a g tile of T x 128 floats and twice the
-// (weight, code) pairs of a slice of the inputs in shared memory, and a chunk's positions fit 14 bits.
-//   * T is the largest multiple of 8 for which that fits (long runs per input and chunk are cheap runs) into what leaves
-//     60 KB of L1 to the gathers of W (28 KB slow those down), or, where the runs are short, into the whole shared memory: a run's
-//     cost of its own then counts for more.  Backward at B=128, L=200,000, us with 60 KB / with the whole, by the
-//     entries of a run (264 K / N): 2.1 (N=1024, K=8) 202/187; 4.1 (N=1024, K=16) 249/233; 5.5 (N=1536, K=32) 405/392; 6.6 (N=1280, K=32)
-//     382/380; 8.2 (N=1024, K=32) 337/349; 11 (N=768, K=32) 306/316; 16.5 (N=768, K=48) 409/431; 33 (N=512, K=64) 484/519.  The
-//     line is between 6.6 and 8.2.  (Fan-ins of 8 and 16 gain 2 to 5 % from the whole also above it, a batch of 32, whose tile
-//     leaves L1 room in either case, up to 8 %; the plan does not know the batch.)
+// Rows per chunk of the chunked lists and inputs per warp of the one-pass backward, which keeps, per chunk, g tiles of T x 128 floats
+// in all and twice the (weight, code) pairs of a slice of the inputs in shared memory; a chunk's positions fit 14 bits.
+//   * T is the largest multiple of 8 for which that fits: long runs per input and chunk are cheap runs, and what they gain
+//     is more than the L1 that is left loses in the gathers of W (backward at N=768, L=670,091, K=32, us, by T: 272, 248, 224, 200,
+//     176; B=128 828, 833, 839, 874, 909; B=32 368, 373, 386, 402, 424).
 //   * it is lowered until the chunks fill the SMs: the kernel runs R = SMs / slices ranges of chunks, so the chunks are cut
 //     to a whole number per range; a short L (down to 16 rows per chunk) is cut to one chunk per range, or two where they
-//     keep 64 rows, for the ranges of a batch of 64 are twice as many.  Before, a table of fewer than R * 256 rows left most
-//     SMs idle: 513 rows ran on 3 of 148 (B=127, N=254, K=73: backward 73 -> 18 us).
-int plan_chunk_rows(int64_t L, int64_t K, int64_t N) {
+//     keep 64 rows.
+//   * where even so there are fewer chunks than ranges, the warps take fewer inputs each, so that more slices fill the SMs
+//     (backward of 513 rows, B=127, N=254, K=73: 23 -> 16 us).
+struct PlanShape {
+    int rows, ni;
+};
+PlanShape plan_shape(int64_t L, int64_t K, int64_t N) {
     DeviceInfo dev;
     const int64_t sms = get_device_info(&dev) == FFI_OK ? dev.sm_count : 148;
-    const FusedSlices sl = fused_slices(N, false);
-    const double share = sl.parts > 1 ? 16.0 * sl.ni / static_cast<double>(N) : 1.0;
+    const int64_t smem = dev.max_smem_optin > 0 ? dev.max_smem_optin : 232448;
+    int ni = fused_inputs_per_warp(N);
     int64_t T = 512;
-    const double budget = 264.0 * K >= 7.0 * N ? 160700.0 : 190464.0;
     for (; T > 8; T -= 8) {
-        const double entries = static_cast<double>(T) * K * share;
-        const double spread = sl.parts > 1 ? 4.0 * std::sqrt(entries) : 0.0;  // a random table's fullest slice
-        if (T * K <= 16384 && T * 512 + 16 * (entries + spread + 16) <= budget) break;
+        // a random table's warp with the most entries
+        const double entries = static_cast<double>(T) * K * ni / static_cast<double>(N), most = entries + 5.0 * std::sqrt(entries) + 4.0;
+        if (T * K <= 16384 && fused_smem_bytes(T * 512, static_cast<int64_t>(kFusedWarps * most), 4) <= static_cast<size_t>(smem)) break;
     }
-    if (T * K > 16384) return 0;  // K in the thousands: no chunked lists
-    const int64_t R = sms / sl.parts > 0 ? sms / sl.parts : 1;
+    if (T * K > 16384) return {0, ni};  // K in the thousands: no chunked lists
+    const int64_t parts = ceil_div(N, kFusedWarps * ni), R = sms / parts > 0 ? sms / parts : 1;
     const int64_t n = ceil_div(L, T);
     const int64_t want = n > R ? round_up(n, R) : (L >= 2 * R * 64 ? 2 * R : R);
     const int64_t even = round_up(ceil_div(L, want), 8);
     if (even < T) T = even < 16 ? (T < 16 ? T : 16) : even;
-    return static_cast<int>(T);
+    const int64_t chunks = ceil_div(L, T);
+    while (ni > 4 && chunks * ceil_div(N, kFusedWarps * (ni - 4)) <= sms) ni -= 4;
+    return {static_cast<int>(T), ni};
 }
 
 constexpr int64_t kNarrowMaxN = 2048;  // inputs the register-accumulator grad_x kernel covers
@@ -379,7 +376,7 @@ size_t scratch_up(size_t v) { return (v + kScratchAlign - 1) / kScratchAlign * k
 // Geometry of a plan and the carving of its build scratch (one allocation).
 struct PlanLayout {
     long long n, nTiles, scan_segs, nChunks, cptrBytes;
-    int T;
+    int T, ni;
     bool chunks;
     size_t off_kA, off_vA, off_kB, off_vB, off_counts, off_bad, off_segs, off_lb, off_stats, total;
 };
@@ -389,7 +386,8 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     g.n = L * K;
     g.nTiles = ceil_div(g.n, kTile);
     g.scan_segs = ceil_div(256 * g.nTiles > N + 1 ? 256 * g.nTiles : N + 1, kScanSeg);
-    g.T = plan_chunk_rows(L, K, N);
+    const PlanShape shape = plan_shape(L, K, N);
+    g.T = shape.rows, g.ni = shape.ni;
     g.nChunks = ceil_div(L, g.T > 0 ? g.T : 1);
     g.cptrBytes = g.nChunks * (N + 1) * 4;
     g.chunks = g.T >= 8 && N <= kNarrowMaxN && g.cptrBytes <= (512LL << 20) && static_cast<long long>(g.T) * K <= 65536;
@@ -407,7 +405,7 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     g.off_bad = take(4);
     g.off_segs = take(g.scan_segs * 8);
     g.off_lb = take(g.chunks ? (g.nChunks + 1) * N * 4 : 4);
-    g.off_stats = take(4 * sizeof(int));
+    g.off_stats = take(kFusedWarps * sizeof(int));
     g.total = off;
     return g;
 }
@@ -427,6 +425,7 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
     long long* segs = reinterpret_cast<long long*>(scratch + g.off_segs);
     int* lb = reinterpret_cast<int*>(scratch + g.off_lb);
     int* stats = reinterpret_cast<int*>(scratch + g.off_stats);
+    int most[kFusedWarps] = {};
 
     FFI_CUDA_CHECK(cudaMemsetAsync(bad, 0, 4, stream));
     validate_idx_kernel<<<1024, 256, 0, stream>>>(idx, n, static_cast<int>(N), bad);
@@ -468,17 +467,19 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
         chunk_fill_kernel<<<static_cast<unsigned>(g.nChunks), 256, (N + 1) * sizeof(int), stream>>>(
             plan->perm, lb, static_cast<int>(N), chunkEntries, plan->cptr, plan->cperm);
         FFI_LAUNCH_CHECK("chunk kernels");
-        // slice statistics for the kernels that stage one slice of a chunk in shared memory
-        FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, 4 * sizeof(int), stream));
-        slice_stats_kernel<<<static_cast<unsigned>(ceil_div(g.nChunks, 256)), 256, 0, stream>>>(
-            plan->cptr, static_cast<int>(N), g.nChunks, 16 * fused_slices(N, false).ni, 16 * fused_slices(N, true).ni, stats);
-        FFI_LAUNCH_CHECK("slice_stats_kernel");
-        FFI_CUDA_CHECK(cudaMemcpyAsync(plan->max_slice_entries, stats, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+        // entries per warp, for the kernel that stages them in shared memory
+        FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, kFusedWarps * sizeof(int), stream));
+        plan->fused_ni = g.ni;
+        warp_stats_kernel<<<static_cast<unsigned>(ceil_div(N, g.ni)), 256, 0, stream>>>(plan->cptr, static_cast<int>(N), g.nChunks, g.ni, stats);
+        FFI_LAUNCH_CHECK("warp_stats_kernel");
+        FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, kFusedWarps * sizeof(int), cudaMemcpyDeviceToHost, stream));
         plan->chunk_rows = g.T;
         plan->n_chunks = g.nChunks;
         plan->has_chunks = true;
     }
     FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
+    plan->fused_entries[0] = 0;
+    for (int w = 0; w < kFusedWarps; ++w) plan->fused_entries[w + 1] = plan->fused_entries[w] + (most[w] + 1) / 2 * 2;
     return FFI_OK;
 }
 
