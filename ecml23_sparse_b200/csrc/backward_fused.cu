@@ -61,6 +61,7 @@ struct BwdFusedParams {
     int ni;         // inputs per warp
     int boxes;      // TMA boxes per tile (at most 256 rows each)
     int lastHalf;   // bf16 W of an odd number of elements: position of the last one, which has no whole word; else -1
+    bool xVec;      // rows of x start on 8 bytes; what lies behind an odd B in them is zero
     int entOff[kWarps + 1];  // where each warp's entries start in a staging buffer
 };
 
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
     const long long c_end = p.nChunks * (r + 1) / p.R;
     const bool turns = p.gbias != nullptr;  // the fetching warp reads tiles, too
 
+    chain_wait();
     if (warp == 0) tc::alloc(tmem_base_p);
     if (threadIdx.x == 32) {
         for (int b = 0; b < 2; ++b) tc::bar_init(full + b, 1), tc::bar_init(empty + b, kWarps + (turns ? 1 : 0));
@@ -356,9 +358,16 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                 for (int m = 0; m < VPL; m += 2) {
                     const int b = (m / 4) * (4 * LG) + 4 * q + (m & 3);
                     float f[2];
+                    if (VPL == 16 && !kBf16 && p.xVec) {  // two neighbours at a time
+                        const float2 w = k < ni && i < N && b < p.B
+                                             ? *reinterpret_cast<const float2*>(static_cast<const float*>(p.xT) + static_cast<size_t>(i) * p.ldx + b)
+                                             : make_float2(0.f, 0.f);
+                        f[0] = w.x, f[1] = w.y;
+                    } else {
 #pragma unroll
-                    for (int u = 0; u < 2; ++u)
-                        f[u] = (k < ni && i < N && b + u < p.B) ? widen(xT[static_cast<size_t>(i) * p.ldx + b + u]) : 0.f;
+                        for (int u = 0; u < 2; ++u)
+                            f[u] = (k < ni && i < N && b + u < p.B) ? widen(xT[static_cast<size_t>(i) * p.ldx + b + u]) : 0.f;
+                    }
                     x[j].v[m / 2] = pack2(f[0], f[1]);
                 }
             }
@@ -631,6 +640,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
             }
         }
     }
+    chain_release();
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::dealloc(*tmem_base_p);
@@ -776,6 +786,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         p.gT = a.gT + b0;
         p.xT = static_cast<const unsigned char*>(xT) + b0 * (a.w_bf16 ? 2 : 4);
         p.B = cols;
+        p.xVec = ldx % 2 == 0 && reinterpret_cast<uintptr_t>(p.xT) % 8 == 0;
         p.R = c.R;
         p.Bpad = c.Bpad;
         p.segChunks = c.segChunks;
@@ -789,7 +800,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         dim3 grid(static_cast<unsigned>(c.R), static_cast<unsigned>(c.iparts), 1);
         auto launch_kernel = [&](auto kern) -> int {
             FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, c.smem, nullptr));
-            kern<<<grid, kThreads, c.smem, stream>>>(p, g_map);
+            FFI_CUDA_CHECK(launch_chained(kern, grid, dim3(kThreads), c.smem, stream, p, g_map));
             return FFI_OK;
         };
         auto launch_typed = [&](auto tx, auto acc) -> int {

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kThreads, 4) ffi_bwd_wide_kernel(const __grid_
 
     // The launch after this one may start its CTAs while this one's last warps finish: grad_bias needs nothing of the chunks
     // before, and reading the chunk's rows for it brings them into L2.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    chain_release();
     if (p.gbias) {  // four rows at a time
         for (long long o = p.o0 + i0; o < p.o1; o += 4ll * stride) {
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 4) ffi_bwd_wide_kernel(const __grid_
                 if (lane == 0 && o + j * stride < p.o1) p.gbias[o + j * stride] = sum[j];
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    chain_wait();
     if (i0 >= p.N) return;
 
     // A batch is up to 32 entries of one run.  While one is worked on, the weights of the next and the positions of the one
@@ -358,15 +358,11 @@ int launch_wide(BwdWideParams p, long long L, const DeviceInfo& dev, cudaStream_
             p.addW = t > 0;
             p.cursor = t + 1 == tiles && p.o1 < L ? cursor : nullptr;
             p.gbias = t == 0 ? gbias : nullptr;
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(static_cast<unsigned>(ctas)), cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = smem, cfg.stream = stream;
-            cudaLaunchAttribute overlap{};
-            overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            overlap.val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = &overlap, cfg.numAttrs = o0 > 0 || t > 0 ? 1 : 0;
-            FFI_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, p));
+            if (o0 > 0 || t > 0) FFI_CUDA_CHECK(launch_chained(kern, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), smem, stream, p));
+            else kern<<<static_cast<unsigned>(ctas), kThreads, smem, stream>>>(p);  // (reads gT before it waits)
         }
     }
+    FFI_LAUNCH_CHECK("ffi_bwd_wide_kernel");
     return FFI_OK;
 }
 

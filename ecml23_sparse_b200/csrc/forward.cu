@@ -56,6 +56,7 @@ struct FwdKernelParams {
 // MODE 0 writes y, 1 the loss gradient (see FwdKernelParams), 2 the top-k lists.
 template <int BPL, bool XSMEM, int MODE, typename TX>
 __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_kernel(FwdKernelParams p) {
+    chain_wait();
     constexpr int BT = 32 * BPL;
     constexpr bool LOSS = MODE == 1;
     constexpr int PARTS = kThreads / BT;  // top-k: threads per batch element
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_kernel(FwdKernelParams p)
 
 __global__ void transpose_pad_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                      int rows, int cols, long long ld_dst) {
+    chain_begin();
     // src [rows][cols] -> dst [cols][ld_dst], dst[c][r] = src[r][c]; r in [rows, ld_dst) zero.
     __shared__ float tile[32][33];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -328,7 +330,7 @@ int launch_fwd_t(const FwdKernelParams& p, size_t smem, int nBT, const DeviceInf
         return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %d per-CTA partials; this batch needs %u",
                     kMaxLossPartials, grid.x * grid.y);
     if (ctas_out) *ctas_out = static_cast<int>(grid.x * grid.y);
-    kern<<<grid, kThreads, smem, stream>>>(p);
+    FFI_CUDA_CHECK(launch_chained(kern, grid, dim3(kThreads), smem, stream, p));
     FFI_LAUNCH_CHECK("ffi_fwd_kernel");
     return FFI_OK;
 }
@@ -480,7 +482,7 @@ int launch_transpose_pad(const float* src, float* dst, int rows, int cols, int64
                          cudaStream_t stream) {
     dim3 block(32, 8);
     dim3 grid(static_cast<unsigned>(ceil_div(cols, 32)), static_cast<unsigned>(ceil_div(ld_dst, 32)));
-    transpose_pad_kernel<<<grid, block, 0, stream>>>(src, dst, rows, cols, ld_dst);
+    FFI_CUDA_CHECK(launch_chained(transpose_pad_kernel, grid, block, 0, stream, src, dst, rows, cols, static_cast<long long>(ld_dst)));
     FFI_LAUNCH_CHECK("transpose_pad_kernel");
     return FFI_OK;
 }

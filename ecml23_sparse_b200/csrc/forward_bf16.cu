@@ -62,6 +62,7 @@ struct LaneWords<2> {
 // VPL batch elements per lane, so a batch tile has 16 * VPL columns: 128, 64 or 32.
 template <int MODE, int VPL>
 __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
+    chain_wait();
     constexpr int BT = 16 * VPL;
     constexpr int S = result_stride(BT);
     using XV = typename LaneWords<VPL>::type;
@@ -268,6 +269,7 @@ __global__ void __launch_bounds__(512, 1) ffi_fwd_bf16_kernel(FwdBf16Params p) {
 template <typename T>
 __global__ void transpose_pad_any_kernel(const T* __restrict__ src, T* __restrict__ dst, int rows, int cols,
                                          long long ld_dst) {
+    chain_begin();
     // src [rows][cols] -> dst [cols][ld_dst], dst[c][r] = src[r][c]; r in [rows, ld_dst) zero
     __shared__ T tile[32][33];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -285,6 +287,7 @@ __global__ void transpose_pad_any_kernel(const T* __restrict__ src, T* __restric
 // src [rows][cols] -> dst [rows][ld_dst], zero padded; one thread per 16 bytes of dst (ld_dst a multiple of 16 bytes)
 template <typename T>
 __global__ void pad_rows_kernel(const T* __restrict__ src, uint4* __restrict__ dst, long long rows, int cols, int vecs) {
+    chain_begin();
     constexpr int E = 16 / sizeof(T);
     const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (id >= rows * vecs) return;
@@ -305,12 +308,12 @@ __global__ void pad_rows_kernel(const T* __restrict__ src, uint4* __restrict__ d
 int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int64_t ld_dst, int esize, cudaStream_t stream) {
     const int vecs = static_cast<int>(ld_dst * esize / 16);
     const unsigned blocks = static_cast<unsigned>(ceil_div(rows * vecs, 256));
-    if (esize == 2)
-        pad_rows_kernel<<<blocks, 256, 0, stream>>>(static_cast<const unsigned short*>(src), static_cast<uint4*>(dst), rows,
-                                                    static_cast<int>(cols), vecs);
-    else
-        pad_rows_kernel<<<blocks, 256, 0, stream>>>(static_cast<const unsigned*>(src), static_cast<uint4*>(dst), rows,
-                                                    static_cast<int>(cols), vecs);
+    auto launch = [&](auto kern, auto* from) {
+        return launch_chained(kern, dim3(blocks), dim3(256), 0, stream, from, static_cast<uint4*>(dst), static_cast<long long>(rows),
+                              static_cast<int>(cols), vecs);
+    };
+    FFI_CUDA_CHECK(esize == 2 ? launch(pad_rows_kernel<unsigned short>, static_cast<const unsigned short*>(src))
+                              : launch(pad_rows_kernel<unsigned>, static_cast<const unsigned*>(src)));
     FFI_LAUNCH_CHECK("pad_rows_kernel");
     return FFI_OK;
 }
@@ -319,8 +322,8 @@ int launch_pad_rows(const void* src, void* dst, int64_t rows, int64_t cols, int6
 int launch_transpose_pad_bf16(const void* src, void* dst, int rows, int cols, int64_t ld_dst, cudaStream_t stream) {
     dim3 block(32, 8);
     dim3 grid(static_cast<unsigned>(ceil_div(cols, 32)), static_cast<unsigned>(ceil_div(ld_dst, 32)));
-    transpose_pad_any_kernel<__nv_bfloat16><<<grid, block, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(src), static_cast<__nv_bfloat16*>(dst), rows, cols, ld_dst);
+    FFI_CUDA_CHECK(launch_chained(transpose_pad_any_kernel<__nv_bfloat16>, grid, block, 0, stream, static_cast<const __nv_bfloat16*>(src),
+                                  static_cast<__nv_bfloat16*>(dst), rows, cols, static_cast<long long>(ld_dst)));
     FFI_LAUNCH_CHECK("transpose_pad_any_kernel");
     return FFI_OK;
 }
@@ -361,7 +364,7 @@ template <int MODE, int VPL>
 static int launch_bf16_t(const FwdBf16Params& p, dim3 grid, int warps, size_t smem, cudaStream_t stream) {
     auto kern = ffi_fwd_bf16_kernel<MODE, VPL>;
     FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
-    kern<<<grid, warps * 32, smem, stream>>>(p);
+    FFI_CUDA_CHECK(launch_chained(kern, grid, dim3(warps * 32), smem, stream, p));
     FFI_LAUNCH_CHECK("ffi_fwd_bf16_kernel");
     return FFI_OK;
 }

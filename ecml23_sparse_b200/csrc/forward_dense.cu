@@ -143,6 +143,7 @@ __device__ __forceinline__ float add_nonfinite(const DenseFwdParams& p, const un
 // MODE 0 writes y, 1 the loss gradient.  KG: entries of a row per lane (K <= 32 * KG).  EMIT: warps that write results (8 or 16).
 template <int MODE, int KG, int EMIT>
 __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_dense_kernel(DenseFwdParams p) {
+    chain_wait();
     constexpr int kEmitWarps = EMIT, kBuildWarps = kMmaWarp - EMIT;
     constexpr int kWarpRows = kRows / kBuildWarps;  // rows of a tile that a building warp has
     constexpr int kListWarps = 16 / kWarpRows;      // building warps that share a list
@@ -605,7 +606,7 @@ int launch_forward_dense(const void* xT, int64_t ldx, const int32_t* idx, const 
         p.cap = static_cast<int>(longest < room ? longest : room);
         const size_t smem = used + 2 * build * 8 * static_cast<size_t>(p.cap);
         FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), 0, smem, nullptr));
-        kern<<<grid, kThreads, smem, stream>>>(p);
+        FFI_CUDA_CHECK(launch_chained(kern, grid, dim3(kThreads), smem, stream, p));
         FFI_LAUNCH_CHECK("ffi_fwd_dense_kernel");
         return FFI_OK;
     };

@@ -75,6 +75,7 @@ __host__ __device__ constexpr int staged_w_words(int K) {
 
 template <int BPL, int MODE, typename TX, bool ODD>
 __global__ void __launch_bounds__(kThreads, 2) ffi_fwd_gather_kernel(FwdGatherParams p) {
+    chain_wait();
     constexpr int BT = 32 * BPL;
     constexpr int S = BT + 4;  // row stride of the result tile
     constexpr int kRows = ResultRows<BPL>::value;
@@ -249,7 +250,7 @@ int launch_fwd_gather_t(FwdGatherParams p, int nBT, int max_partials, const Devi
         return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %d per-CTA partials; this batch needs %u",
                     max_partials, grid.x * grid.y);
     if (ctas_out) *ctas_out = static_cast<int>(grid.x * grid.y);
-    kern<<<grid, kThreads, smem, stream>>>(p);
+    FFI_CUDA_CHECK(launch_chained(kern, grid, dim3(kThreads), smem, stream, p));
     FFI_LAUNCH_CHECK("ffi_fwd_gather_kernel");
     return FFI_OK;
 }

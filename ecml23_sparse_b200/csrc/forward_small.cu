@@ -60,6 +60,7 @@ __device__ __forceinline__ void load_samples(const float* x_s, int i, float (&ou
 
 template <int BP, typename TX>
 __global__ void __launch_bounds__(kThreads) ffi_fwd_small_kernel(SmallParams p) {
+    chain_begin();
     constexpr bool kBf16 = !std::is_same<TX, float>::value;
     constexpr int U = BP <= 4 ? 4 : 2;  // rows per lane group in flight
     extern __shared__ __align__(16) float x_s[];  // [N][BP]
@@ -148,7 +149,7 @@ int launch_small_t(const SmallParams& p, size_t smem, const DeviceInfo& dev, cud
     if (occ < 1) return fail(FFI_ERR_CUDA, "small-batch forward kernel does not fit on an SM (smem %zu)", smem);
     const int tileRows = (BP <= 4 ? 4 : 2) * (32 >> p.lgG);
     const int64_t want = ceil_div(ceil_div(p.L, tileRows), kWarps), cap = static_cast<int64_t>(dev.sm_count) * occ;
-    kern<<<static_cast<unsigned>(want < cap ? want : cap), kThreads, smem, stream>>>(p);
+    FFI_CUDA_CHECK(launch_chained(kern, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(kThreads), smem, stream, p));
     FFI_LAUNCH_CHECK("ffi_fwd_small_kernel");
     return FFI_OK;
 }

@@ -71,6 +71,7 @@ __device__ __forceinline__ int pair_column(int q, int j) {
 // turn an infinite x into a NaN.  Such shapes went to the kernel with CTA-wide tiles before.
 template <int VPL, int MODE, bool ODD>
 __global__ void __launch_bounds__(kThreads, 1) ffi_fwd_pair_kernel(FwdStreamParams p) {
+    chain_wait();
     constexpr bool BCE = MODE == 1;  // 0: write y; 1: loss epilogue; 2: running top-k of the logits
     constexpr int BT = 16 * VPL;
     constexpr int S = BT + 8;  // result-tile row stride: 16-byte rows, conflict-free for both access patterns
@@ -372,7 +373,7 @@ int launch_pair_t(const FwdStreamParams& p, size_t smem, int nBT, const DeviceIn
         return fail(FFI_ERR_UNSUPPORTED, "the fused loss keeps at most %d per-CTA partials; this batch needs %u",
                     kMaxLossPartials, grid.x * grid.y);
     if (ctas_out) *ctas_out = static_cast<int>(grid.x * grid.y);
-    kern<<<grid, kThreads, smem, stream>>>(p);
+    FFI_CUDA_CHECK(launch_chained(kern, grid, dim3(kThreads), smem, stream, p));
     FFI_LAUNCH_CHECK("ffi_fwd_pair_kernel");
     return FFI_OK;
 }

@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_grad_x_narrow_kernel(GxNarrow
 // the 8 sums are added in warp order.  (One thread per column with a chain of R loads took 13 us at R=148, N=128; this 4.)
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ gx,
                                                               int R, int N, int cols, int Bpad, int B, int x_transposed) {
+    chain_begin();
     // blockIdx.y: batch tile, each with R partials of its own and `cols` columns (the last one what is left of them)
     partial += static_cast<size_t>(blockIdx.y) * R * N * Bpad;
     const int b0 = blockIdx.y * Bpad;
@@ -397,6 +398,7 @@ template <int BS>
 __global__ void __launch_bounds__(256, kTrResident) transpose_g_kernel(const float* __restrict__ g, float* __restrict__ gT,
                                                                     float* __restrict__ gbias, int B, long long L,
                                                                     long long ldg, int tro) {
+    chain_begin();
     __shared__ float tile[BS][kTrO + 1];
     const int tid = threadIdx.x;
     const int tx = tid & (kTrO - 1), ty = tid / kTrO;  // load: tx = output, ty = batch row within a group of 4
@@ -450,7 +452,8 @@ int launch_transpose_g(const float* g, float* gT, float* gbias, int B, int64_t L
     const long long blocks_o = ceil_div(L, tro);
     if (blocks_o > 2147483647LL) return fail(FFI_ERR_UNSUPPORTED, "L too large");
     auto kern = ldg == 32 ? transpose_g_kernel<32> : (ldg == 64 ? transpose_g_kernel<64> : transpose_g_kernel<128>);
-    kern<<<static_cast<unsigned>(blocks_o), 256, 0, stream>>>(g, gT, gbias, B, L, ldg, static_cast<int>(tro));
+    FFI_CUDA_CHECK(launch_chained(kern, dim3(static_cast<unsigned>(blocks_o)), dim3(256), 0, stream, g, gT, gbias, B, static_cast<long long>(L),
+                                  static_cast<long long>(ldg), static_cast<int>(tro)));
     FFI_LAUNCH_CHECK("transpose_g_kernel");
     return FFI_OK;
 }
@@ -484,7 +487,7 @@ size_t grad_x_min_workspace_bytes(const ffi_plan* plan, int64_t B) {
 int reduce_range_partials(const float* partial, float* gx, int R, int N, int cols, int Bpad, int tiles, int B,
                           int x_transposed, cudaStream_t stream) {
     const dim3 grid(static_cast<unsigned>(ceil_div(static_cast<long long>(N) * Bpad, 32)), static_cast<unsigned>(tiles));
-    reduce_partials_kernel<<<grid, 256, 0, stream>>>(partial, gx, R, N, cols, Bpad, B, x_transposed);
+    FFI_CUDA_CHECK(launch_chained(reduce_partials_kernel, grid, dim3(256), 0, stream, partial, gx, R, N, cols, Bpad, B, x_transposed));
     FFI_LAUNCH_CHECK("reduce_partials_kernel");
     return FFI_OK;
 }

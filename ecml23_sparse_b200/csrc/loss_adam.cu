@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(256) bce_positive_fix_kernel(
     float* __restrict__ gT, long long ldg, double* pos_partials, float scale, long long L, int K,
     long long label_offset, int loss_kind, const double* __restrict__ partials, int nPartials, unsigned* ticket,
     float* __restrict__ loss) {
+    chain_begin();
     __shared__ double sh[32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -213,6 +214,7 @@ __device__ __forceinline__ float adam_update(float g, float& m, float& v, const 
 }
 
 __global__ void __launch_bounds__(256) adam_kernel(const __grid_constant__ AdamParams p) {
+    chain_begin();
     int block = blockIdx.x, j = 0;
     while (block >= p.t[j].blocks) block -= p.t[j].blocks, ++j;
     const AdamTensor& t = p.t[j];
@@ -263,6 +265,7 @@ namespace ffi {
 namespace {
 __global__ void __launch_bounds__(256) widen_bf16_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ dst,
                                                          long long n) {
+    chain_begin();
     const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
     for (long long e = tid; e < n; e += stride) dst[e] = __bfloat162float(src[e]);
@@ -272,8 +275,9 @@ __global__ void __launch_bounds__(256) widen_bf16_kernel(const __nv_bfloat16* __
 // bf16 -> fp32 (exact).
 int launch_widen_bf16(const void* src, float* dst, int64_t n, cudaStream_t stream) {
     const long long blocks = (n + 255) / 256;
-    widen_bf16_kernel<<<static_cast<unsigned>(blocks < 1184 * 4 ? (blocks < 1 ? 1 : blocks) : 1184 * 4), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(src), dst, n);
+    const dim3 grid(static_cast<unsigned>(blocks < 1184 * 4 ? (blocks < 1 ? 1 : blocks) : 1184 * 4));
+    FFI_CUDA_CHECK(launch_chained(widen_bf16_kernel, grid, dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(src), dst,
+                                  static_cast<long long>(n)));
     FFI_LAUNCH_CHECK("widen_bf16_kernel");
     return FFI_OK;
 }
@@ -284,14 +288,13 @@ int launch_bce_positive_fix(const void* xT, int64_t ldx, const int* idx, const v
                             const double* partials, int nPartials, double* pos_partials, float scale, int B,
                             int64_t L, int K, int64_t label_offset, int loss_kind, bool bf16, cudaStream_t stream) {
     unsigned* ticket = loss_ticket(const_cast<double*>(partials));
-    if (bf16)
-        bce_positive_fix_kernel<__nv_bfloat16><<<static_cast<unsigned>(B), 256, 0, stream>>>(
-            static_cast<const __nv_bfloat16*>(xT), ldx, idx, static_cast<const __nv_bfloat16*>(W), bias, row_ptr, labels,
-            gT, ldg, pos_partials, scale, L, K, label_offset, loss_kind, partials, nPartials, ticket, loss);
-    else
-        bce_positive_fix_kernel<float><<<static_cast<unsigned>(B), 256, 0, stream>>>(
-            static_cast<const float*>(xT), ldx, idx, static_cast<const float*>(W), bias, row_ptr, labels, gT, ldg,
-            pos_partials, scale, L, K, label_offset, loss_kind, partials, nPartials, ticket, loss);
+    auto launch = [&](auto kern, const auto* x, const auto* w) {
+        return launch_chained(kern, dim3(static_cast<unsigned>(B)), dim3(256), 0, stream, x, static_cast<long long>(ldx), idx, w, bias, row_ptr,
+                              labels, gT, static_cast<long long>(ldg), pos_partials, scale, static_cast<long long>(L), K,
+                              static_cast<long long>(label_offset), loss_kind, partials, nPartials, ticket, loss);
+    };
+    FFI_CUDA_CHECK(bf16 ? launch(bce_positive_fix_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(xT), static_cast<const __nv_bfloat16*>(W))
+                        : launch(bce_positive_fix_kernel<float>, static_cast<const float*>(xT), static_cast<const float*>(W)));
     FFI_LAUNCH_CHECK("bce_positive_fix_kernel");
     return FFI_OK;
 }
@@ -377,7 +380,7 @@ extern "C" int ffi_adam_step_group(const ffi_adam_tensor* tensors, int count, fl
             out.blocks = static_cast<int>(share < most ? share : most);
             grid += out.blocks;
         }
-        adam_kernel<<<static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream_v)>>>(p);
+        FFI_CUDA_CHECK(launch_chained(adam_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream_v), p));
         FFI_LAUNCH_CHECK("adam_kernel");
     }
     return FFI_OK;

@@ -84,6 +84,7 @@ __device__ __forceinline__ void gather_lists(const uint2* lists, int n, size_t s
 __global__ void __launch_bounds__(kThreads) topk_merge_kernel(const uint2* __restrict__ lists, int listsPerTile, int BT,
                                                               int kk, int label_offset, float* __restrict__ out_val,
                                                               int* __restrict__ out_idx) {
+    chain_begin();
     const int b = blockIdx.x;
     const int tile = b / BT, bl = b - tile * BT;
     float tv[kTopK];
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(kThreads) topk_merge_kernel(const uint2* __res
 __global__ void __launch_bounds__(kThreads) topk_rows_kernel(const float* __restrict__ y, int L, int segRows, int kk, uint2* lists,
                                                              unsigned* tickets, int label_offset, float* __restrict__ out_val,
                                                              int* __restrict__ out_idx) {
+    chain_begin();
     __shared__ int wmax[kWarps];
     __shared__ bool last;
     const int o0 = blockIdx.x * segRows, o1 = min(L, o0 + segRows);
@@ -159,8 +161,8 @@ int64_t row_segments(int64_t B, int64_t L, const DeviceInfo& dev) {
 
 int launch_topk_merge(const uint2* lists, int lists_per_tile, int bt, int B, int kk, int label_offset, float* top_val,
                       int* top_idx, cudaStream_t stream) {
-    topk_merge_kernel<<<static_cast<unsigned>(B), kThreads, 0, stream>>>(lists, lists_per_tile, bt, kk, label_offset, top_val,
-                                                                         top_idx);
+    FFI_CUDA_CHECK(launch_chained(topk_merge_kernel, dim3(static_cast<unsigned>(B)), dim3(kThreads), 0, stream, lists, lists_per_tile, bt, kk,
+                                  label_offset, top_val, top_idx));
     FFI_LAUNCH_CHECK("topk_merge_kernel");
     return FFI_OK;
 }
@@ -184,8 +186,8 @@ int launch_topk_rows(const float* y, int64_t B, int64_t L, uint2* lists, int kk,
     if (rc != FFI_OK) return rc;
     const int64_t segs = row_segments(B, L, dev);
     const int segRows = static_cast<int>(ceil_div(L, segs));
-    topk_rows_kernel<<<dim3(static_cast<unsigned>(segs), static_cast<unsigned>(B)), kThreads, 0, stream>>>(
-        y, static_cast<int>(L), segRows, kk, lists, topk_rows_tickets(lists, B, L), label_offset, top_val, top_idx);
+    FFI_CUDA_CHECK(launch_chained(topk_rows_kernel, dim3(static_cast<unsigned>(segs), static_cast<unsigned>(B)), dim3(kThreads), 0, stream, y,
+                                  static_cast<int>(L), segRows, kk, lists, topk_rows_tickets(lists, B, L), label_offset, top_val, top_idx));
     FFI_LAUNCH_CHECK("topk_rows_kernel");
     return FFI_OK;
 }
