@@ -4,7 +4,7 @@
 //
 // Replaces the reference's backward_weights_vector / backward_weights_scalar kernels
 // (tfsparse/cc/kernels/backward.cu.h:62-105,269-292) for the output layers of the stacked configurations
-// (hidden widths of 32,768 ... 100,000).
+// (hidden widths of 32,768 ... 100,000) where grad_x is not wanted as well (both at once: backward_wide.cu).
 //
 // What bounds this shape is the number of gathered bytes in flight per SM (B*L*K*e bytes cross the L2-to-SM
 // fabric, every load takes about a microsecond), so the kernel is built to keep many loads in flight with few

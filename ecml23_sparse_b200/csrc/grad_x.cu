@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
 // ---- wide inputs -------------------------------------------------------------------
 
 // One warp per (input i, batch tile of 32*VEC): walks row i of the canonical index and gathers
-// one row of the transposed gradient gT[L][ldg] per entry.
+// one row of the transposed gradient gT[L][ldg] per entry.  For grad_x alone (with grad_W: backward_wide.cu).
 //
 // What bounds it: 4*B*L*K gathered bytes through the L2-to-SM fabric (20 TB/s for 512-byte rows that hit L2, 9 TB/s for
 // a table of three times L2, by a bare gather loop), so the rows have to hit L2.  All resident warps start at output 0
