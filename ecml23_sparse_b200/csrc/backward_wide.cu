@@ -30,6 +30,7 @@
 // moving window (965, 2,077 and 1,239 us); rows asked for two steps ahead in a ring of registers instead of two at a time (1,003,
 // 1,554, 1,133); outputs and weights of both steps read before the gathers (858, 1,553, 1,127); bulk copies of the rows to shared
 // memory (3 to 6 TB/s).
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 
@@ -41,9 +42,12 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-// Bytes of a chunk's rows of gT, of the tile's columns (us at the three shapes above with 32, 40, 48, 56, 64 MB: 874, 848, 842, 898,
-// 944; 1,551, 1,478, 1,511, 1,549, 1,609; no difference where one or two chunks hold all rows).
-constexpr long long kChunkBytes = 48ll << 20;
+// A chunk's rows of gT, of the tile's columns, take at most kChunkBytes (whole steps, us, with 32, 40, 48, 56, 64 MB at the three shapes
+// above: 1,476, 1,455, 1,456, 1,513, 1,589; 2,061, 1,953, 1,946, 1,971, 2,043; 1,425, 1,421, 1,404, 1,438, 1,447), and together with the
+// chunk's W, positions and grad_W, which pass through L2 besides, at most kChunkAll: with 64 columns and fewer those are the larger
+// part (without that limit, with 112 MB, with 88 MB: B=64, N=78,400, L=558,266, K=48 bf16 1,831, 1,521, 1,453; B=32, N=30,000, L=600,000,
+// K=32 fp32 848, 772, 770; B=20, N=20,000, L=700,000, K=72 fp32 1,915, 1,847, 1,852).
+constexpr long long kChunkBytes = 48ll << 20, kChunkAll = 96ll << 20;
 constexpr int kRow = 36;  // floats per buffered step: 32 partial dots + padding (16-byte rows, conflict-free both ways)
 
 struct BwdWideParams {
@@ -337,7 +341,9 @@ int launch_wide(BwdWideParams p, long long L, const DeviceInfo& dev, cudaStream_
     FFI_CUDA_CHECK(prepare_kernel(reinterpret_cast<const void*>(kern), kThreads, smem, &occ));
     if (occ < 1) return fail(FFI_ERR_CUDA, "one-pass backward for wide inputs does not fit on an SM");
     const int B = p.B, tiles = static_cast<int>(ceil_div(B, BT));
-    const long long rows = kChunkBytes / (BT * 4);
+    const long long perRow = BT * 4 + static_cast<long long>(p.K) * (4 + 4 + sizeof(TX));
+    long long rows = std::min(kChunkBytes / (BT * 4), kChunkAll / perRow);
+    if (rows < 1) rows = 1;
     const long long nChunks = ceil_div(L, rows), T = ceil_div(L, nChunks);
     // as many warps as give each the same number of inputs
     const long long cap = static_cast<long long>(dev.sm_count) * occ * kWarps;
