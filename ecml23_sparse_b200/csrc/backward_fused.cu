@@ -517,18 +517,21 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                         // row of zeros (weight 0), where that costs the pipe less than branches cost the rest: with 4 columns per lane
                         // throughout (374 against 388 us at B=32, N=768, L=670,091, K=32 with zeroed registers and a branch), with 16 in the
                         // steps that some groups do not have, one at a time (820 against 836 at B=128); with 8 the branch (501, 518).
+                        // (A run's end is not the buffer's: the longest run of a bundle may have thousands of entries more than another, whose
+                        // group must not read on, past the end of shared memory in the last warp's.)
+                        auto entry = [](const uint2* at, bool there) { return there ? *at : make_uint2(0u, 0u); };
                         auto row = [&](uint2 en_s, bool there) { return there ? gs_lane + (en_s.y & kRowMask) : zero_lane; };
                         int s = 0;
                         if constexpr (VPL == 4) {
                             for (; s < steps; s += 2) {  // (SLOTS is even: the row after an odd last step is the buffer's)
-                                const uint2 en0 = en[s], en1 = en[s + 1];
                                 const bool p0 = s0 + s < n, p1 = s0 + s + 1 < n;
+                                const uint2 en0 = entry(en + s, p0), en1 = entry(en + s + 1, p1);
                                 LaneT g0, g1;
                                 g0.load_shared(row(en0, p0));
                                 g1.load_shared(row(en1, p1));
-                                acc.axpy(p0 ? __uint_as_float(en0.x) : 0.f, g0);
+                                acc.axpy(__uint_as_float(en0.x), g0);
                                 d[0] = xr.dot(g0);
-                                acc.axpy(p1 ? __uint_as_float(en1.x) : 0.f, g1);
+                                acc.axpy(__uint_as_float(en1.x), g1);
                                 d[kDRow] = xr.dot(g1);
                                 d += 2 * kDRow;
                             }
@@ -550,9 +553,9 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                                 LaneT g0;
                                 float w = 0.f;
                                 if constexpr (VPL == 16) {
-                                    const uint2 en0 = en[s];
+                                    const uint2 en0 = entry(en + s, there);
                                     g0.load_shared(row(en0, there));
-                                    if (there) w = __uint_as_float(en0.x);
+                                    w = __uint_as_float(en0.x);
                                 } else {
                                     g0.zero();
                                     if (there) {
