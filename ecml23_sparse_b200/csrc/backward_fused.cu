@@ -38,7 +38,11 @@ constexpr int kDRow = 36;                   // row stride of the per-warp dot bu
 constexpr int kPosRegs = 8;                 // positions per lane kept in registers ahead of their staging
 constexpr int kKShift = 18;                 // entry code = byte offset of the g row in its tile | position in the chunk << 18
 constexpr int kBounds = 36;                 // ints per warp and staging buffer: where its runs (or their halves) start
-static_assert(kFusedNI * 2 + 1 <= kBounds && kFusedWarps == kWarps, "bounds of the halves of a warp's runs");
+// The kernel of uneven tables: in a chunk where the longest run of a bundle has more than twice the average and kLongRun entries, what
+// it has more than the others is walked by all lane groups.  No run walked side by side exceeds kSideBySide: a group whose run has
+// ended fetches on, unused, and must stay inside shared memory (see dbuf and bounds, which follow the entries).
+constexpr int kLongRun = 16, kSideBySide = kFusedLongestRun;
+static_assert(kFusedNI * 2 + 1 < kBounds && kFusedWarps == kWarps, "bounds of the halves of a warp's runs");
 
 struct BwdFusedParams {
     const void* W;   // fp32 or bf16 (TX)
@@ -132,6 +136,18 @@ struct LaneVec {
             unpack2(s, lo, hi);
         }
         return lo + hi;
+    }
+    // what lane `src` holds
+    __device__ __forceinline__ void from_lane(int src) {
+#pragma unroll
+        for (int j = 0; j < kPairs; ++j) v[j] = __shfl_sync(0xffffffffu, v[j], src);
+    }
+    // the sum over the lane groups, in all of them
+    __device__ __forceinline__ void add_groups() {
+#pragma unroll
+        for (int j = 0; j < kPairs; ++j)
+#pragma unroll
+            for (int off = LG; off < 32; off *= 2) v[j] = fma2(pack2(1.f, 1.f), v[j], __shfl_xor_sync(0xffffffffu, v[j], off));
     }
     __device__ __forceinline__ float sum() const {
         float s = 0.f;
@@ -234,6 +250,14 @@ __device__ __forceinline__ void tmem_store(unsigned taddr, const LaneVec<VPL, LG
 // 8 436 -> 222; B=256, N=512, L=65,536, K=64, bf16 357 -> 313; 513 rows, B=127, N=254, K=73 18.3 -> 16.7.
 // Without the warp that fetches (the last warp done with a tile asks for the next; 128 instead of 96 registers): 882 to 921 at B=128.
 //
+// UNEVEN: a bundle lasts as long as its longest run, so a hot input, walked by one lane group, holds up its warp and the warp its CTA.
+// Tables with such inputs have a kernel that lets all groups walk what a run has more than the others of its bundle, every G-th entry
+// each (x of the input handed round by shuffles, the groups' sums added at the end), and that stages a warp's thousands of entries
+// with as many loads in flight as there are registers for.  Backward at N=768, L=670,091, K=32 with inputs drawn by Zipf's law in
+// shuffled order, us without -> with: exponent 0.4 B=128 1,312 -> 1,147, 64 905 -> 708, 16 600 -> 410; 0.8 B=32 2,197 -> 748, 16
+// 2,575 -> 568; 1.0 B=32 4,064 -> 1,081, 16 4,859 -> 816.  In one kernel with the flag looked up per chunk, even tables took 2 to
+// 6 % longer (registers).
+//
 // ACC: a batch tile after the first (as a run-time flag it cost 5 %), whose grad_W and grad_bias add to what the tiles
 // before stored.
 // TX is the storage type of x and W.  bf16 x is widened (exactly) on its way into tensor memory.  A bf16
@@ -242,12 +266,13 @@ __device__ __forceinline__ void tmem_store(unsigned taddr, const LaneVec<VPL, LG
 // which half: the chunk's first position is even, so the parity of the position within the chunk is the
 // parity of the flat position).  W has to start on a word; of the last element of an odd number two bytes are copied.
 // =====================================================================================
-template <int G, int VPL, int HALVES, typename TX, bool ACC>
+template <int G, int VPL, int HALVES, typename TX, bool ACC, bool UNEVEN>
 __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_constant__ BwdFusedParams p, const __grid_constant__ CUtensorMap g_map) {
     constexpr bool kBf16 = !std::is_same<TX, float>::value;
     constexpr int LG = 32 / G, BT = VPL * LG, COLS = 2 * VPL, NB = kFusedNI / G, SLOTS = 32 / G;
     constexpr unsigned kAll = 0xffffffffu, kRowMask = (1u << kKShift) - 1u;
     static_assert(kFusedNI % G == 0 && (kWarps / 4) * NB * COLS <= tc::kCols, "the warps of a lane quarter share the TMEM columns");
+    static_assert((kSideBySide + SLOTS) * 8 <= kWarps * (SLOTS * kDRow + 2 * kBounds) * 4, "fetches past the last run stay inside shared memory");
     using LaneT = LaneVec<VPL, LG>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int T = p.T, K = p.K, N = p.N, ni = p.ni;
@@ -424,16 +449,37 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                     if (pos[u] >= 0) stage_one(dst + lane + u * 32, pos[u], pos0);
                 // more entries than the registers cover: the rest is fetched here
                 const int* src = p.cperm + c * static_cast<long long>(T) * K + e_lo;
-                for (int e = lane + kRegs * 32; e < cnt; e += 32) stage_one(dst + e, __ldg(src + e), pos0);
+                if constexpr (UNEVEN) {  // thousands of them, maybe
+                    for (int e0 = kRegs * 32; e0 < cnt; e0 += kRegs * 32) {
+#pragma unroll
+                        for (int u = 0; u < kRegs; ++u) pos[u] = e0 + lane + u * 32 < cnt ? __ldg(src + e0 + lane + u * 32) : -1;
+#pragma unroll
+                        for (int u = 0; u < kRegs; ++u)
+                            if (pos[u] >= 0) stage_one(dst + e0 + lane + u * 32, pos[u], pos0);
+                    }
+                } else {
+                    for (int e = lane + kRegs * 32; e < cnt; e += 32) stage_one(dst + e, __ldg(src + e), pos0);
+                }
             } else {
                 __pipeline_wait_prior(0);  // (each lane reads what it copied)
                 for (int e = lane; e < cnt; e += 32) stage_one(dst + e, static_cast<int>(dst[e].y), pos0);
             }
             int* b = bnd_s + buf * kBounds;
             if (lane <= ni) b[lane * HALVES] = bnd - e_lo;
+            const int next = __shfl_down_sync(kAll, bnd, 1);
+            if constexpr (UNEVEN) {
+                // does the longest run of a bundle (lanes G*j ..) have far more entries than their average?
+                int most = lane < ni ? next - bnd : 0, sum = most;
+#pragma unroll
+                for (int off = 1; off < G; off *= 2) {
+                    most = max(most, __shfl_xor_sync(kAll, most, off));
+                    sum += __shfl_xor_sync(kAll, sum, off);
+                }
+                const bool far = __any_sync(kAll, most > kSideBySide || most > sum / G * 2 + kLongRun);
+                if (lane == 0) b[kBounds - 1] = far;
+            }
             if constexpr (HALVES == 2) {
                 // where the rows of the second half start in each run
-                const int next = __shfl_down_sync(kAll, bnd, 1);
                 __syncwarp();
                 if (lane < ni) {
                     int lo = bnd - e_lo, hi = next - e_lo;
@@ -497,18 +543,30 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                 }
                 const unsigned char* gs_lane = tiles_s + (t & 1) * tileBytes + q * 16;
                 const unsigned char* zero_lane = zero_s + q * 16;
-#pragma unroll 1
-                for (int j = 0; j < nb; ++j) {
-                    const int k = j * G + grp;
-                    int e = 0, n = 0;  // first entry of this group's run, its length
-                    if (k < ni) e = bounds[k * HALVES + half], n = bounds[k * HALVES + half + 1] - e;
-                    const int most = __reduce_max_sync(kAll, n);
-                    const int least = VPL == 4 ? 0 : __reduce_min_sync(kAll, n);  // (here: behind the load of the state it costs 10 %)
-                    if (most == 0) continue;
+                // Lane row*G + h adds the LG dots of group h's entry of buffered step `row` (fixed order) ...
+                auto dots_sum = [&]() -> float {
+                    if constexpr (LG == 2) {
+                        const float2 q0 = *reinterpret_cast<const float2*>(drow);
+                        return q0.x + q0.y;
+                    } else if constexpr (LG == 4) {
+                        return (drow[0].x + drow[0].y) + (drow[0].z + drow[0].w);
+                    } else {
+                        const float4 q0 = drow[0], q1 = drow[1];
+                        return ((q0.x + q0.y) + (q0.z + q0.w)) + ((q1.x + q1.y) + (q1.z + q1.w));
+                    }
+                };
+                // ... and stores grad_W of that entry.
+                auto store_grad_w = [&](int at, float sum) {
+                    if (!gWc) return;
+                    float* dst = gWc + (ent[at].y >> kKShift);
+                    // batch tiles after the first add to what the tile before stored: one addition per element and launch
+                    if (ACC) atomicAdd(dst, sum);
+                    else *dst = sum;
+                };
+                // The lane groups walk a run each: `n` entries from `e` on, at most `most`, at least `least`.
+                auto side_by_side = [&](LaneT& acc, const LaneT& xr, int e, int n, int most, int least) {
                     // the run this lane reduces dots of
                     const int re = __shfl_sync(kAll, e, myent * LG), rn = __shfl_sync(kAll, n, myent * LG);
-                    LaneT acc, xr;
-                    tmem_load_input(taddr0 + j * COLS, acc, xr);
                     for (int s0 = 0; s0 < most; s0 += SLOTS) {
                         const uint2* en = ent + e + s0;
                         const int steps = min(SLOTS, most - s0);
@@ -517,21 +575,18 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                         // row of zeros (weight 0), where that costs the pipe less than branches cost the rest: with 4 columns per lane
                         // throughout (374 against 388 us at B=32, N=768, L=670,091, K=32 with zeroed registers and a branch), with 16 in the
                         // steps that some groups do not have, one at a time (820 against 836 at B=128); with 8 the branch (501, 518).
-                        // (A run's end is not the buffer's: the longest run of a bundle may have thousands of entries more than another, whose
-                        // group must not read on, past the end of shared memory in the last warp's.)
-                        auto entry = [](const uint2* at, bool there) { return there ? *at : make_uint2(0u, 0u); };
                         auto row = [&](uint2 en_s, bool there) { return there ? gs_lane + (en_s.y & kRowMask) : zero_lane; };
                         int s = 0;
                         if constexpr (VPL == 4) {
                             for (; s < steps; s += 2) {  // (SLOTS is even: the row after an odd last step is the buffer's)
+                                const uint2 en0 = en[s], en1 = en[s + 1];
                                 const bool p0 = s0 + s < n, p1 = s0 + s + 1 < n;
-                                const uint2 en0 = entry(en + s, p0), en1 = entry(en + s + 1, p1);
                                 LaneT g0, g1;
                                 g0.load_shared(row(en0, p0));
                                 g1.load_shared(row(en1, p1));
-                                acc.axpy(__uint_as_float(en0.x), g0);
+                                acc.axpy(p0 ? __uint_as_float(en0.x) : 0.f, g0);
                                 d[0] = xr.dot(g0);
-                                acc.axpy(__uint_as_float(en1.x), g1);
+                                acc.axpy(p1 ? __uint_as_float(en1.x) : 0.f, g1);
                                 d[kDRow] = xr.dot(g1);
                                 d += 2 * kDRow;
                             }
@@ -553,9 +608,9 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                                 LaneT g0;
                                 float w = 0.f;
                                 if constexpr (VPL == 16) {
-                                    const uint2 en0 = entry(en + s, there);
+                                    const uint2 en0 = en[s];
                                     g0.load_shared(row(en0, there));
-                                    w = __uint_as_float(en0.x);
+                                    if (there) w = __uint_as_float(en0.x);
                                 } else {
                                     g0.zero();
                                     if (there) {
@@ -569,28 +624,93 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                                 d += kDRow;
                             }
                         }
-                        // Lane row*G + h adds the LG dots of group h's entry of buffered step `row` (fixed order) and stores
-                        // grad_W of that entry.
                         __syncwarp();
-                        float sum;
-                        if constexpr (LG == 2) {
-                            const float2 q0 = *reinterpret_cast<const float2*>(drow);
-                            sum = q0.x + q0.y;
-                        } else if constexpr (LG == 4) {
-                            sum = (drow[0].x + drow[0].y) + (drow[0].z + drow[0].w);
-                        } else {
-                            const float4 q0 = drow[0], q1 = drow[1];
-                            sum = ((q0.x + q0.y) + (q0.z + q0.w)) + ((q1.x + q1.y) + (q1.z + q1.w));
-                        }
-                        if (s0 + myrow < rn && gWc) {
-                            float* dst = gWc + (ent[re + s0 + myrow].y >> kKShift);
-                            // batch tiles after the first add to what the tile before stored: one addition per element and launch
-                            if (ACC) atomicAdd(dst, sum);
-                            else *dst = sum;
-                        }
+                        const float sum = dots_sum();
+                        if (s0 + myrow < rn) store_grad_w(re + s0 + myrow, sum);
                         __syncwarp();
                     }
-                    tmem_store(taddr0 + j * COLS, acc);
+                };
+                if (!UNEVEN || bounds[kBounds - 1] == 0) {
+#pragma unroll 1
+                    for (int j = 0; j < nb; ++j) {
+                        const int k = j * G + grp;
+                        int e = 0, n = 0;  // first entry of this group's run, its length
+                        if (k < ni) e = bounds[k * HALVES + half], n = bounds[k * HALVES + half + 1] - e;
+                        const int most = __reduce_max_sync(kAll, n);
+                        const int least = VPL == 4 ? 0 : __reduce_min_sync(kAll, n);  // (here: behind the load of the state it costs 10 %)
+                        if (most == 0) continue;
+                        LaneT acc, xr;
+                        tmem_load_input(taddr0 + j * COLS, acc, xr);
+                        side_by_side(acc, xr, e, n, most, least);
+                        tmem_store(taddr0 + j * COLS, acc);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int j = 0; j < nb; ++j) {
+                        const int k = j * G + grp;
+                        int e = 0, n = 0;  // first entry of this group's run, its length
+                        if (k < ni) e = bounds[k * HALVES + half], n = bounds[k * HALVES + half + 1] - e;
+                        const int most = __reduce_max_sync(kAll, n);
+                        const int least = VPL == 4 ? 0 : __reduce_min_sync(kAll, n);  // (here: behind the load of the state it costs 10 %)
+                        if (most == 0) continue;
+                        // what a run has more than the longest that is not much above the average is left for all groups together
+                        const int mean = __reduce_add_sync(kAll, q == 0 ? n : 0) / G;
+                        const int lim = min(kSideBySide, __reduce_max_sync(kAll, n <= mean + mean / 2 + kLongRun ? n : 0));
+                        LaneT acc, xr;
+                        tmem_load_input(taddr0 + j * COLS, acc, xr);
+                        if (lim > 0) side_by_side(acc, xr, e, min(n, lim), lim, min(least, lim));
+                        tmem_store(taddr0 + j * COLS, acc);
+                        // ... every G-th entry each; the run's sums come from tensor memory and go back there
+#pragma unroll 1
+                        for (int h = 0; h < G && lim < most; ++h) {
+                            constexpr int AT = VPL == 4 && SLOTS >= 4 ? 4 : 2;  // steps in flight
+                            const int first = __shfl_sync(kAll, e, h * LG) + lim, cnt = __shfl_sync(kAll, n, h * LG) - lim;
+                            if (cnt <= 0) continue;
+                            tc::wait_store();
+                            LaneT sums, xh;
+                            tmem_load_input(taddr0 + j * COLS, sums, xh);
+                            xh.from_lane(h * LG + q);
+                            if (grp != h) sums.zero();
+                            for (int s0 = 0; s0 < cnt; s0 += 32) {
+                                const uint2* en = ent + first + s0 + grp;
+                                const int left = cnt - s0;
+                                float* d = dlane;
+                                int s = 0;
+                                for (; s < SLOTS && (s + AT) * G <= left; s += AT) {
+                                    uint2 en_s[AT];
+                                    LaneT g_s[AT];
+#pragma unroll
+                                    for (int u = 0; u < AT; ++u) en_s[u] = en[(s + u) * G];
+#pragma unroll
+                                    for (int u = 0; u < AT; ++u) g_s[u].load_shared(gs_lane + (en_s[u].y & kRowMask));
+#pragma unroll
+                                    for (int u = 0; u < AT; ++u) {
+                                        sums.axpy(__uint_as_float(en_s[u].x), g_s[u]);
+                                        d[u * kDRow] = xh.dot(g_s[u]);
+                                    }
+                                    d += AT * kDRow;
+                                }
+                                for (; s < SLOTS && s * G < left; ++s) {
+                                    const bool there = s * G + grp < left;
+                                    const uint2 en0 = there ? en[s * G] : make_uint2(0u, 0u);
+                                    LaneT g0;
+                                    g0.load_shared(there ? gs_lane + (en0.y & kRowMask) : zero_lane);
+                                    sums.axpy(__uint_as_float(en0.x), g0);
+                                    d[0] = xh.dot(g0);
+                                    d += kDRow;
+                                }
+                                __syncwarp();
+                                const float sum = dots_sum();
+                                if (lane < left) store_grad_w(first + s0 + lane, sum);
+                                __syncwarp();
+                            }
+                            sums.add_groups();
+                            LaneT own;
+                            tmem_load_input(taddr0 + j * COLS, own, xh);
+                            if (grp == h) own = sums;
+                            tmem_store(taddr0 + j * COLS, own);
+                        }
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty + (t & 1));
@@ -806,16 +926,19 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
             FFI_CUDA_CHECK(launch_chained(kern, grid, dim3(kThreads), c.smem, stream, p, g_map));
             return FFI_OK;
         };
-        auto launch_typed = [&](auto tx, auto acc) -> int {
+        auto launch_typed = [&](auto tx, auto acc, auto uneven) -> int {
             using TX = decltype(tx);
-            constexpr bool ACC = decltype(acc)::value;
-            if (c.Bpad == 128) return launch_kernel(ffi_bwd_runs_kernel<4, 16, 2, TX, ACC>);
-            if (c.Bpad == 64) return launch_kernel(ffi_bwd_runs_kernel<4, 8, 1, TX, ACC>);
-            if (c.Bpad == 32) return launch_kernel(ffi_bwd_runs_kernel<4, 4, 1, TX, ACC>);
-            if (c.Bpad == 16) return launch_kernel(ffi_bwd_runs_kernel<8, 4, 1, TX, ACC>);
-            return launch_kernel(ffi_bwd_runs_kernel<16, 4, 1, TX, ACC>);
+            constexpr bool ACC = decltype(acc)::value, UNEVEN = decltype(uneven)::value;
+            if (c.Bpad == 128) return launch_kernel(ffi_bwd_runs_kernel<4, 16, 2, TX, ACC, UNEVEN>);
+            if (c.Bpad == 64) return launch_kernel(ffi_bwd_runs_kernel<4, 8, 1, TX, ACC, UNEVEN>);
+            if (c.Bpad == 32) return launch_kernel(ffi_bwd_runs_kernel<4, 4, 1, TX, ACC, UNEVEN>);
+            if (c.Bpad == 16) return launch_kernel(ffi_bwd_runs_kernel<8, 4, 1, TX, ACC, UNEVEN>);
+            return launch_kernel(ffi_bwd_runs_kernel<16, 4, 1, TX, ACC, UNEVEN>);
         };
-        auto launch_tile = [&](auto acc) { return a.w_bf16 ? launch_typed(__nv_bfloat16{}, acc) : launch_typed(float{}, acc); };
+        auto launch_table = [&](auto tx, auto acc) {
+            return a.plan->fused_uneven ? launch_typed(tx, acc, std::true_type{}) : launch_typed(tx, acc, std::false_type{});
+        };
+        auto launch_tile = [&](auto acc) { return a.w_bf16 ? launch_table(__nv_bfloat16{}, acc) : launch_table(float{}, acc); };
         rc = b0 > 0 ? launch_tile(std::true_type{}) : launch_tile(std::false_type{});
         if (rc != FFI_OK) return rc;
         FFI_LAUNCH_CHECK("ffi_bwd_runs_kernel");

@@ -286,6 +286,10 @@ int launch_transpose_pad(const float* src, float* dst, int rows, int cols, int64
 
 namespace ffi {
 constexpr int kFusedWarps = 16;  // walking warps of the one-pass backward
+// Its lane groups walk the runs of a chunk's entries side by side; tables with a run of more than three times the average and
+// kFusedFarRun entries go to a variant of the kernel (random tables stay below: average 11, longest 38 of 1.9 million runs at N=768,
+// L=670,091, K=32), and those with one of more than kFusedLongestRun have to (see backward_fused.cu).
+constexpr int kFusedFarRun = 32, kFusedLongestRun = 1024;
 }  // namespace ffi
 
 // The plan object (defined in plan.cu, used by backward.cu and api.cu).
@@ -299,6 +303,7 @@ struct ffi_plan {
     // that the warp has in any chunk and slice
     int fused_entries[ffi::kFusedWarps + 1] = {};
     int fused_ni = 0;  // inputs per warp of the one-pass backward
+    bool fused_uneven = false;  // some input has far more entries in a chunk than the average
     void* arrays = nullptr;     // the allocation that holds the four index arrays
     int32_t* rowptr = nullptr;  // [N+1]   canonical CSR-by-input
     int32_t* perm = nullptr;    // [L*K]   positions sorted by (idx[p], p)

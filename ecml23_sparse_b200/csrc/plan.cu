@@ -267,14 +267,27 @@ __global__ void chunk_fill_kernel(const int* __restrict__ perm, const int* __res
     }
 }
 
-// most[w] = largest number of entries that warp w of a slice has in any chunk and slice (zeroed by the caller); a slice is kFusedWarps
-// warps of ni inputs.  One block per warp of all slices.
+// most[w] = largest number of entries that warp w of a slice has in any chunk and slice, most[kFusedWarps] = largest number that an
+// input has in any chunk (zeroed by the caller); a slice is kFusedWarps warps of ni inputs.  One block per warp of all slices.
 __global__ void warp_stats_kernel(const int* __restrict__ cptr, int N, long long nChunks, int ni, int* __restrict__ most) {
     const int lo = min(N, static_cast<int>(blockIdx.x) * ni), hi = min(N, lo + ni);
-    int best = 0;
-    for (long long c = threadIdx.x; c < nChunks; c += blockDim.x) best = max(best, cptr[c * (N + 1) + hi] - cptr[c * (N + 1) + lo]);
+    int best = 0, longest = 0;
+    for (long long c = threadIdx.x; c < nChunks; c += blockDim.x) {
+        const int* at = cptr + c * (N + 1);
+        int before = at[lo];
+        best = max(best, at[hi] - before);
+        for (int i = lo + 1; i <= hi; ++i) {
+            const int here = at[i];
+            longest = max(longest, here - before);
+            before = here;
+        }
+    }
     best = __reduce_max_sync(0xffffffffu, best);
-    if (threadIdx.x % 32 == 0) atomicMax(most + blockIdx.x % kFusedWarps, best);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (threadIdx.x % 32 == 0) {
+        atomicMax(most + blockIdx.x % kFusedWarps, best);
+        atomicMax(most + kFusedWarps, longest);
+    }
 }
 
 // Self-check export: rebuild the canonical form from (cptr, cperm).
@@ -405,7 +418,7 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     g.off_bad = take(4);
     g.off_segs = take(g.scan_segs * 8);
     g.off_lb = take(g.chunks ? (g.nChunks + 1) * N * 4 : 4);
-    g.off_stats = take(kFusedWarps * sizeof(int));
+    g.off_stats = take((kFusedWarps + 1) * sizeof(int));
     g.total = off;
     return g;
 }
@@ -425,7 +438,7 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
     long long* segs = reinterpret_cast<long long*>(scratch + g.off_segs);
     int* lb = reinterpret_cast<int*>(scratch + g.off_lb);
     int* stats = reinterpret_cast<int*>(scratch + g.off_stats);
-    int most[kFusedWarps] = {};
+    int most[kFusedWarps + 1] = {};
 
     FFI_CUDA_CHECK(cudaMemsetAsync(bad, 0, 4, stream));
     validate_idx_kernel<<<1024, 256, 0, stream>>>(idx, n, static_cast<int>(N), bad);
@@ -468,11 +481,11 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
             plan->perm, lb, static_cast<int>(N), chunkEntries, plan->cptr, plan->cperm);
         FFI_LAUNCH_CHECK("chunk kernels");
         // entries per warp, for the kernel that stages them in shared memory
-        FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, kFusedWarps * sizeof(int), stream));
+        FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, (kFusedWarps + 1) * sizeof(int), stream));
         plan->fused_ni = g.ni;
         warp_stats_kernel<<<static_cast<unsigned>(ceil_div(N, g.ni)), 256, 0, stream>>>(plan->cptr, static_cast<int>(N), g.nChunks, g.ni, stats);
         FFI_LAUNCH_CHECK("warp_stats_kernel");
-        FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, kFusedWarps * sizeof(int), cudaMemcpyDeviceToHost, stream));
+        FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, (kFusedWarps + 1) * sizeof(int), cudaMemcpyDeviceToHost, stream));
         plan->chunk_rows = g.T;
         plan->n_chunks = g.nChunks;
         plan->has_chunks = true;
@@ -480,6 +493,8 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
     FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
     plan->fused_entries[0] = 0;
     for (int w = 0; w < kFusedWarps; ++w) plan->fused_entries[w + 1] = plan->fused_entries[w] + (most[w] + 1) / 2 * 2;
+    const long long average = ceil_div(static_cast<int64_t>(g.T) * K, N);
+    plan->fused_uneven = most[kFusedWarps] > 3 * average + kFusedFarRun || most[kFusedWarps] > kFusedLongestRun;
     return FFI_OK;
 }
 
