@@ -52,6 +52,7 @@ struct BwdFusedParams {
     long long ldx;
     const int* cperm;
     const int* cptr;
+    const int* order;  // UNEVEN: the input at each place of the chunked lists
     float* partial;  // [R][N][Bpad]
     float* gW;
     float* gbias;  // grad_bias[o] = sum_b gT[o][b], from the g tiles at hand anyway; or nullptr
@@ -251,12 +252,18 @@ __device__ __forceinline__ void tmem_store(unsigned taddr, const LaneVec<VPL, LG
 // Without the warp that fetches (the last warp done with a tile asks for the next; 128 instead of 96 registers): 882 to 921 at B=128.
 //
 // UNEVEN: a bundle lasts as long as its longest run, so a hot input, walked by one lane group, holds up its warp and the warp its CTA.
-// Tables with such inputs have a kernel that lets all groups walk what a run has more than the others of its bundle, every G-th entry
-// each (x of the input handed round by shuffles, the groups' sums added at the end), and that stages a warp's thousands of entries
-// with as many loads in flight as there are registers for.  Backward at N=768, L=670,091, K=32 with inputs drawn by Zipf's law in
-// shuffled order, us without -> with: exponent 0.4 B=128 1,312 -> 1,147, 64 905 -> 708, 16 600 -> 410; 0.8 B=32 2,197 -> 748, 16
-// 2,575 -> 568; 1.0 B=32 4,064 -> 1,081, 16 4,859 -> 816.  In one kernel with the flag looked up per chunk, even tables took 2 to
-// 6 % longer (registers).
+// Tables with such inputs have theirs dealt to slices and warps by count (plan_build) and a kernel that lets all groups walk what a
+// run has more than the others of its bundle, every G-th entry each (x of the input handed round by shuffles, the groups' sums added
+// at the end), and that stages a warp's thousands of entries with as many loads in flight as there are registers for.  What bounds
+// it is the chain of the warp that has the hottest input: 13.9 ns an entry at 64 columns, 6 at 8.  Backward at N=768, L=670,091, K=32,
+// us, before -> now; "two": grad_x and grad_W by a kernel each, because the entries of the warps did not fit:
+//   inputs drawn by Zipf's law, exponent 0.4: B=128 1,310 -> 1,029, 64 904 -> 620, 32 615 -> 462, 8 428 -> 280
+//   exponent 0.8: 128 1,973 (two) -> 1,373, 64 1,300 (two) -> 811, 32 2,194 -> 632, 8 1,968 -> 384
+//   exponent 1:   128 2,350 (two) -> 1,788, 64 1,375 (two) -> 1,110, 32 4,067 -> 889, 8 3,856 -> 548
+//   30 % of the links added to the leading quarter of the inputs: 128 1,974 (two) -> 862, 64 1,201 (two) -> 517
+// (An even table: 813, 499, 356, 224.)  Two kernels are faster again from about a fifth (33 to 64 columns, where the
+// chain is 1.6 times theirs at four fifths), a third (65 to 128 and 17 to 32) or more of all links to ONE input.  In one kernel with the even case and
+// a flag looked up per chunk, even tables took 2 to 6 % longer (registers).
 //
 // ACC: a batch tile after the first (as a run-time flag it cost 5 %), whose grad_W and grad_bias add to what the tiles
 // before stored.
@@ -367,7 +374,8 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
     } else {
         // ---- the warps that walk -------------------------------------------------------------
         const TX* xT = static_cast<const TX*>(p.xT);
-        const int iw = i_lo + warp * ni;                 // this warp's first input
+        const int iw = i_lo + warp * ni;                 // this warp's first input, or its place
+        auto input_at = [&](int i) { return UNEVEN ? __ldg(p.order + i) : i; };
         const int nb = (ni + G - 1) / G;                 // its bundles
         // lanes 32*(warp % 4) .. +31 are the ones this warp may touch; its bundles take NB*COLS columns
         const unsigned taddr0 = *tmem_base_p + ((static_cast<unsigned>(warp & 3) * 32u) << 16) + static_cast<unsigned>(warp >> 2) * (NB * COLS);
@@ -378,7 +386,9 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
             zero.zero();
 #pragma unroll
             for (int j = 0; j < NB; ++j) {
-                const int k = j * G + grp, i = iw + k;
+                const int k = j * G + grp;
+                int i = iw + k;
+                if (UNEVEN && k < ni && i < N) i = input_at(i);
 #pragma unroll
                 for (int m = 0; m < VPL; m += 2) {
                     const int b = (m / 4) * (4 * LG) + 4 * q + (m & 3);
@@ -663,7 +673,8 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                         // ... every G-th entry each; the run's sums come from tensor memory and go back there
 #pragma unroll 1
                         for (int h = 0; h < G && lim < most; ++h) {
-                            constexpr int AT = VPL == 4 && SLOTS >= 4 ? 4 : 2;  // steps in flight
+                            constexpr int AT = VPL <= 8 && SLOTS >= 4 ? 4 : 2;
+                            constexpr bool kRowsAhead = VPL == 4;
                             const int first = __shfl_sync(kAll, e, h * LG) + lim, cnt = __shfl_sync(kAll, n, h * LG) - lim;
                             if (cnt <= 0) continue;
                             tc::wait_store();
@@ -671,38 +682,51 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                             tmem_load_input(taddr0 + j * COLS, sums, xh);
                             xh.from_lane(h * LG + q);
                             if (grp != h) sums.zero();
-                            for (int s0 = 0; s0 < cnt; s0 += 32) {
-                                const uint2* en = ent + first + s0 + grp;
-                                const int left = cnt - s0;
-                                float* d = dlane;
-                                int s = 0;
-                                for (; s < SLOTS && (s + AT) * G <= left; s += AT) {
-                                    uint2 en_s[AT];
-                                    LaneT g_s[AT];
+                            // AT steps at a time.  A hot run is one warp's chain, so the next steps' entries, and where registers allow
+                            // their rows, are asked for before these are worked on; a group without an entry has a row of zeros.
+                            float w_n[AT];
+                            int row_n[AT];
+                            LaneT g_n[AT];
+                            auto fetch_entries = [&](int s) {
 #pragma unroll
-                                    for (int u = 0; u < AT; ++u) en_s[u] = en[(s + u) * G];
-#pragma unroll
-                                    for (int u = 0; u < AT; ++u) g_s[u].load_shared(gs_lane + (en_s[u].y & kRowMask));
-#pragma unroll
-                                    for (int u = 0; u < AT; ++u) {
-                                        sums.axpy(__uint_as_float(en_s[u].x), g_s[u]);
-                                        d[u * kDRow] = xh.dot(g_s[u]);
-                                    }
-                                    d += AT * kDRow;
+                                for (int u = 0; u < AT; ++u) {
+                                    const int at = (s + u) * G + grp;
+                                    const uint2 en = at < cnt ? ent[first + at] : make_uint2(0u, 0u);
+                                    w_n[u] = __uint_as_float(en.x);
+                                    row_n[u] = at < cnt ? static_cast<int>(en.y & kRowMask) : static_cast<int>(zero_lane - gs_lane);
                                 }
-                                for (; s < SLOTS && s * G < left; ++s) {
-                                    const bool there = s * G + grp < left;
-                                    const uint2 en0 = there ? en[s * G] : make_uint2(0u, 0u);
-                                    LaneT g0;
-                                    g0.load_shared(there ? gs_lane + (en0.y & kRowMask) : zero_lane);
-                                    sums.axpy(__uint_as_float(en0.x), g0);
-                                    d[0] = xh.dot(g0);
-                                    d += kDRow;
+                            };
+                            auto fetch_rows = [&]() {
+#pragma unroll
+                                for (int u = 0; u < AT; ++u) g_n[u].load_shared(gs_lane + row_n[u]);
+                            };
+                            fetch_entries(0);
+                            if constexpr (kRowsAhead) fetch_rows();
+                            float* d = dlane;
+                            const int total = (cnt + G - 1) / G;
+#pragma unroll 1
+                            for (int s = 0; s < total; s += AT) {
+                                if constexpr (!kRowsAhead) fetch_rows();
+                                float w[AT];
+                                LaneT g_s[AT];
+#pragma unroll
+                                for (int u = 0; u < AT; ++u) w[u] = w_n[u], g_s[u] = g_n[u];
+                                fetch_entries(s + AT);
+                                if constexpr (kRowsAhead) fetch_rows();
+#pragma unroll
+                                for (int u = 0; u < AT; ++u) {
+                                    sums.axpy(w[u], g_s[u]);
+                                    d[u * kDRow] = xh.dot(g_s[u]);
                                 }
-                                __syncwarp();
-                                const float sum = dots_sum();
-                                if (lane < left) store_grad_w(first + s0 + lane, sum);
-                                __syncwarp();
+                                d += AT * kDRow;
+                                if ((s + AT) % SLOTS == 0 || s + AT >= total) {
+                                    const int e0 = s / SLOTS * 32 + lane;
+                                    __syncwarp();
+                                    const float sum = dots_sum();
+                                    if (e0 < cnt) store_grad_w(first + e0, sum);
+                                    __syncwarp();
+                                    d = dlane;
+                                }
                             }
                             sums.add_groups();
                             LaneT own;
@@ -730,7 +754,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                         // One partial per range: the first segment stores, the later ones add to what this lane stored before
                         // (a handful of fp32 additions of segment sums; the long sums stay inside the segments, and the
                         // ranges are added in fp64 afterwards).
-                        float* dst = p.partial + (static_cast<size_t>(r) * N + i) * p.Bpad + 4 * q;
+                        float* dst = p.partial + (static_cast<size_t>(r) * N + input_at(i)) * p.Bpad + 4 * q;
 #pragma unroll
                         for (int m = 0; m < VPL / 4; ++m) {
                             float4 out;
@@ -788,7 +812,7 @@ bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedC
     c->iparts = static_cast<int>(ceil_div(plan->N, kWarps * c->ni));
     int R = dev.sm_count / c->iparts;
     if (R < 1) R = 1;
-    if (R > plan->n_chunks) R = static_cast<int>(plan->n_chunks);
+    if (R > plan->range_chunks) R = static_cast<int>(plan->range_chunks);
     c->R = R;
     // flush after about 128 summands per (input, batch) pair, and at least once on the way
     const double per_chunk = static_cast<double>(plan->chunk_rows) * plan->K / static_cast<double>(plan->N);
@@ -885,6 +909,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
     p.ldx = ldx;
     p.cperm = a.plan->cperm;
     p.cptr = a.plan->cptr;
+    p.order = a.plan->order;
     p.partial = static_cast<float*>(a.workspace);
     p.gW = gW;
     p.gbias = gbias;
@@ -936,7 +961,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
             return launch_kernel(ffi_bwd_runs_kernel<16, 4, 1, TX, ACC, UNEVEN>);
         };
         auto launch_table = [&](auto tx, auto acc) {
-            return a.plan->fused_uneven ? launch_typed(tx, acc, std::true_type{}) : launch_typed(tx, acc, std::false_type{});
+            return a.plan->order ? launch_typed(tx, acc, std::true_type{}) : launch_typed(tx, acc, std::false_type{});
         };
         auto launch_tile = [&](auto acc) { return a.w_bf16 ? launch_table(__nv_bfloat16{}, acc) : launch_table(float{}, acc); };
         rc = b0 > 0 ? launch_tile(std::true_type{}) : launch_tile(std::false_type{});

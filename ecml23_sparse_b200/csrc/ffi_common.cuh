@@ -287,8 +287,9 @@ int launch_transpose_pad(const float* src, float* dst, int rows, int cols, int64
 namespace ffi {
 constexpr int kFusedWarps = 16;  // walking warps of the one-pass backward
 // Its lane groups walk the runs of a chunk's entries side by side; tables with a run of more than three times the average and
-// kFusedFarRun entries go to a variant of the kernel (random tables stay below: average 11, longest 38 of 1.9 million runs at N=768,
-// L=670,091, K=32), and those with one of more than kFusedLongestRun have to (see backward_fused.cu).
+// kFusedFarRun entries have their inputs dealt to the warps by count and go to a variant of the kernel (random tables stay below:
+// average 11, longest 38 of 1.9 million runs at N=768, L=670,091, K=32), and those with one of more than kFusedLongestRun have to
+// (see plan_build and backward_fused.cu).
 constexpr int kFusedFarRun = 32, kFusedLongestRun = 1024;
 }  // namespace ffi
 
@@ -298,17 +299,19 @@ struct ffi_plan {
     int device = 0;
     int chunk_rows = 0;     // T: outputs per chunk of the chunked lists
     int64_t n_chunks = 0;   // ceil(L / T)
+    int64_t range_chunks = 0;  // the same for an even table: bounds the ranges of chunks, so that scratch does not depend on the table
     bool has_chunks = false;
     // where the entries of each warp of a slice start in a staging buffer of the one-pass backward: the gaps hold the largest number
     // that the warp has in any chunk and slice
     int fused_entries[ffi::kFusedWarps + 1] = {};
     int fused_ni = 0;  // inputs per warp of the one-pass backward
-    bool fused_uneven = false;  // some input has far more entries in a chunk than the average
     void* arrays = nullptr;     // the allocation that holds the four index arrays
     int32_t* rowptr = nullptr;  // [N+1]   canonical CSR-by-input
     int32_t* perm = nullptr;    // [L*K]   positions sorted by (idx[p], p)
     int32_t* cperm = nullptr;   // [L*K]   chunk-major: chunk c holds its T*K positions sorted by (idx[p], p)
     int32_t* cptr = nullptr;    // [n_chunks][N+1] offsets of each input's run inside its chunk
+    int32_t* order = nullptr;   // [N] uneven tables: the chunked lists hold the run of input order[s] at place s; else nullptr
+    int32_t* order_store = nullptr;  // where it lies then
     void* build_scratch = nullptr;  // sort scratch kept by ffi_plan_rebuild (none after ffi_plan_create alone)
     size_t device_bytes = 0;
 };

@@ -44,6 +44,7 @@ struct GxNarrowParams {
     long long ldg;
     const int* cperm;
     const int* cptr;
+    const int* order;  // the input at each place of the chunked lists, or nullptr: in order
     float* partial;  // [R * S][N][Bpad]
     int B, N, L, K;
     int T;           // rows per chunk
@@ -185,7 +186,8 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_grad_x_narrow_kernel(GxNarrow
             for (int j = 0; j < NI; ++j) {
                 const int i = i_lo + warp * NI + j;
                 if (i < N) {
-                    float* dst = p.partial + ((static_cast<size_t>(r) * p.S + seg) * N + i) * p.Bpad + b0 + lane * BPL;
+                    const int row = p.order ? __ldg(p.order + i) : i;
+                    float* dst = p.partial + ((static_cast<size_t>(r) * p.S + seg) * N + row) * p.Bpad + b0 + lane * BPL;
 #pragma unroll
                     for (int q = 0; q < BPL; ++q) {
                         dst[q] = acc[j][q];
@@ -353,7 +355,7 @@ bool narrow_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, Narro
     c->Bpad = c->nBT * BT;
     int R = dev.sm_count / (c->iparts * c->nBT);
     if (R < 1) R = 1;
-    if (R > plan->n_chunks) R = static_cast<int>(plan->n_chunks);
+    if (R > plan->range_chunks) R = static_cast<int>(plan->range_chunks);
     c->R = R;
     const size_t gbytes = static_cast<size_t>(plan->chunk_rows) * BT * 4;
     const size_t cpbytes = (kWarps * c->ni + 1) * 4 + 16;
@@ -518,6 +520,7 @@ int launch_grad_x(const GradXArgs& a, cudaStream_t stream) {
         p.ldg = a.ldg;
         p.cperm = plan->cperm;
         p.cptr = plan->cptr;
+        p.order = plan->order;
         p.partial = static_cast<float*>(a.workspace);
         p.B = a.B;
         p.N = a.N;

@@ -12,7 +12,9 @@
 // of T rows, and chunk c stores its T*K positions ordered by (key, position) in
 // cperm[c*T*K ...], with cptr[c][i] the offset of input i's run inside the chunk.
 // Concatenating, for each input i, its runs over the chunks in chunk order gives back
-// exactly row i of the canonical form (chunks are ascending ranges of p).
+// exactly row i of the canonical form (chunks are ascending ranges of p).  A chunk of an uneven table holds the runs in another
+// order of the inputs (`order`).
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -222,14 +224,15 @@ __global__ void rowptr_kernel(const int* __restrict__ sorted_keys, long long n, 
     rowptr[i] = static_cast<int>(lo);
 }
 
-// lb[c][i] = first position e in row i of the canonical form with perm[e] >= c*T*K.
-__global__ void chunk_bounds_kernel(const int* __restrict__ rowptr, const int* __restrict__ perm,
+// lb[c][s] = first position e in row i of the canonical form with perm[e] >= c*T*K, where i is the input at place s (order[s], or s).
+__global__ void chunk_bounds_kernel(const int* __restrict__ rowptr, const int* __restrict__ perm, const int* __restrict__ order,
                                     int N, long long chunkEntries, long long nChunks,
                                     int* __restrict__ lb) {
     const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (id >= (nChunks + 1) * N) return;
     const long long c = id / N;
-    const int i = static_cast<int>(id - c * N);
+    const int place = static_cast<int>(id - c * N);
+    const int i = order ? order[place] : place;
     const long long target = c * chunkEntries;
     int lo = rowptr[i], hi = rowptr[i + 1];
     while (lo < hi) {
@@ -291,7 +294,7 @@ __global__ void warp_stats_kernel(const int* __restrict__ cptr, int N, long long
 }
 
 // Self-check export: rebuild the canonical form from (cptr, cperm).
-__global__ void chunked_row_totals_kernel(const int* __restrict__ cptr, int N, long long nChunks,
+__global__ void chunked_row_totals_kernel(const int* __restrict__ cptr, const int* __restrict__ order, int N, long long nChunks,
                                           int* __restrict__ totals) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > N) return;
@@ -301,16 +304,16 @@ __global__ void chunked_row_totals_kernel(const int* __restrict__ cptr, int N, l
     }
     long long s = 0;
     for (long long c = 0; c < nChunks; ++c) s += cptr[c * (N + 1) + i + 1] - cptr[c * (N + 1) + i];
-    totals[i] = static_cast<int>(s);
+    totals[order ? order[i] : i] = static_cast<int>(s);
 }
 
 __global__ void chunked_gather_kernel(const int* __restrict__ cptr, const int* __restrict__ cperm,
-                                      const int* __restrict__ rowptr, int N, long long nChunks,
+                                      const int* __restrict__ order, const int* __restrict__ rowptr, int N, long long nChunks,
                                       long long chunkEntries, int* __restrict__ perm_out) {
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (i >= N) return;
-    long long run = rowptr[i];
+    long long run = rowptr[order ? order[i] : i];
     for (long long c = 0; c < nChunks; ++c) {
         const int s = cptr[c * (N + 1) + i], len = cptr[c * (N + 1) + i + 1] - s;
         const int* src = cperm + c * chunkEntries + s;
@@ -349,19 +352,30 @@ struct DeviceBuffer {
 //     keep 64 rows.
 //   * where even so there are fewer chunks than ranges, the warps take fewer inputs each, so that more slices fill the SMs
 //     (backward of 513 rows, B=127, N=254, K=73: 23 -> 16 us).
+// That is for tables whose inputs have about equally many entries.  For others see plan_build: their inputs are dealt to the warps
+// by count, and T is lowered, to half at the least, until the entries of the largest warps fit.
 struct PlanShape {
     int rows, ni;
 };
-PlanShape plan_shape(int64_t L, int64_t K, int64_t N) {
+int64_t device_sms() {
     DeviceInfo dev;
-    const int64_t sms = get_device_info(&dev) == FFI_OK ? dev.sm_count : 148;
-    const int64_t smem = dev.max_smem_optin > 0 ? dev.max_smem_optin : 232448;
+    return get_device_info(&dev) == FFI_OK ? dev.sm_count : 148;
+}
+int64_t device_smem() {
+    DeviceInfo dev;
+    return get_device_info(&dev) == FFI_OK && dev.max_smem_optin > 0 ? dev.max_smem_optin : 232448;
+}
+// Whether chunks of T rows fit whose warps' largest numbers of entries add up to `entries`.
+bool chunks_fit(int64_t T, int64_t entries) { return fused_smem_bytes(T * 512, entries, 4) <= static_cast<size_t>(device_smem()); }
+
+PlanShape plan_shape(int64_t L, int64_t K, int64_t N) {
+    const int64_t sms = device_sms();
     int ni = fused_inputs_per_warp(N);
     int64_t T = 512;
     for (; T > 8; T -= 8) {
         // a random table's warp with the most entries
         const double entries = static_cast<double>(T) * K * ni / static_cast<double>(N), most = entries + 5.0 * std::sqrt(entries) + 4.0;
-        if (T * K <= 16384 && fused_smem_bytes(T * 512, static_cast<int64_t>(kFusedWarps * most), 4) <= static_cast<size_t>(smem)) break;
+        if (T * K <= 16384 && chunks_fit(T, static_cast<int64_t>(kFusedWarps * most))) break;
     }
     if (T * K > 16384) return {0, ni};  // K in the thousands: no chunked lists
     const int64_t parts = ceil_div(N, kFusedWarps * ni), R = sms / parts > 0 ? sms / parts : 1;
@@ -372,6 +386,17 @@ PlanShape plan_shape(int64_t L, int64_t K, int64_t N) {
     const int64_t chunks = ceil_div(L, T);
     while (ni > 4 && chunks * ceil_div(N, kFusedWarps * (ni - 4)) <= sms) ni -= 4;
     return {static_cast<int>(T), ni};
+}
+
+// For an uneven table whose chunks of T rows have warps with `entries` entries (see chunks_fit): the most rows that may fit, cut
+// to a whole number of chunks per range like plan_shape's; at least `least`.
+int lower_rows(int64_t L, int64_t N, int ni, int T, int64_t entries, int least) {
+    int64_t t = T - 8;
+    while (t > least && !chunks_fit(t, entries * t / T)) t -= 8;
+    if (t <= least) return least;
+    const int64_t parts = ceil_div(N, kFusedWarps * ni), R = device_sms() / parts > 0 ? device_sms() / parts : 1;
+    const int64_t n = ceil_div(L, t), even = n > R ? round_up(ceil_div(L, round_up(n, R)), 8) : t;
+    return static_cast<int>(std::max<int64_t>(least, std::min(t, even)));
 }
 
 constexpr int64_t kNarrowMaxN = 2048;  // inputs the register-accumulator grad_x kernel covers
@@ -388,8 +413,9 @@ size_t scratch_up(size_t v) { return (v + kScratchAlign - 1) / kScratchAlign * k
 
 // Geometry of a plan and the carving of its build scratch (one allocation).
 struct PlanLayout {
-    long long n, nTiles, scan_segs, nChunks, cptrBytes;
-    int T, ni;
+    long long n, nTiles, scan_segs, nChunks, mostChunks, cptrBytes;
+    int T, ni;   // rows per chunk of an even table, inputs per warp
+    int leastT;  // rows per chunk that an uneven table is cut down to, at most: cptr and lb hold its mostChunks chunks
     bool chunks;
     size_t off_kA, off_vA, off_kB, off_vB, off_counts, off_bad, off_segs, off_lb, off_stats, total;
 };
@@ -402,8 +428,10 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     const PlanShape shape = plan_shape(L, K, N);
     g.T = shape.rows, g.ni = shape.ni;
     g.nChunks = ceil_div(L, g.T > 0 ? g.T : 1);
-    g.cptrBytes = g.nChunks * (N + 1) * 4;
-    g.chunks = g.T >= 8 && N <= kNarrowMaxN && g.cptrBytes <= (512LL << 20) && static_cast<long long>(g.T) * K <= 65536;
+    g.leastT = std::max(8, g.T / 2 / 8 * 8);
+    g.mostChunks = ceil_div(L, std::min(g.T, g.leastT) > 0 ? std::min(g.T, g.leastT) : 1);
+    g.cptrBytes = g.mostChunks * (N + 1) * 4;
+    g.chunks = g.T >= 8 && N <= kNarrowMaxN && g.nChunks * (N + 1) * 4 <= (512LL << 20) && static_cast<long long>(g.T) * K <= 65536;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t at = off;
@@ -417,10 +445,39 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     g.off_counts = take(256 * g.nTiles * 4);
     g.off_bad = take(4);
     g.off_segs = take(g.scan_segs * 8);
-    g.off_lb = take(g.chunks ? (g.nChunks + 1) * N * 4 : 4);
+    g.off_lb = take(g.chunks ? (g.mostChunks + 1) * N * 4 : 4);
     g.off_stats = take((kFusedWarps + 1) * sizeof(int));
     g.total = off;
     return g;
+}
+
+// Deals the inputs to the places of the chunked lists: place s is input order[s], a warp has ni places, a slice kFusedWarps warps.  By
+// descending count, each to the slice and there to the warp with the fewest entries that has a place left, so that slices and warps
+// have about the same number of entries and neighbours, which the lane groups of a warp walk side by side, about the same counts.
+void deal_inputs(const int* rowptr, int N, int ni, int* order) {
+    int by_count[kNarrowMaxN];
+    for (int i = 0; i < N; ++i) by_count[i] = i;
+    std::sort(by_count, by_count + N, [&](int a, int b) {
+        const int na = rowptr[a + 1] - rowptr[a], nb = rowptr[b + 1] - rowptr[b];
+        return na != nb ? na > nb : a < b;
+    });
+    const int warps = static_cast<int>(ceil_div(N, ni)), slices = static_cast<int>(ceil_div(warps, kFusedWarps));
+    long long load[kNarrowMaxN] = {}, slice_load[kNarrowMaxN] = {};  // (ni >= 1)
+    int used[kNarrowMaxN] = {};
+    auto room = [&](int w) { return used[w] < std::min(ni, N - w * ni); };
+    for (int r = 0; r < N; ++r) {
+        int best = -1;
+        for (int s = 0; s < slices; ++s) {
+            if (best >= 0 && slice_load[s] >= slice_load[best / kFusedWarps]) continue;
+            int w = -1;
+            for (int v = s * kFusedWarps; v < std::min(warps, (s + 1) * kFusedWarps); ++v)
+                if (room(v) && (w < 0 || load[v] < load[w])) w = v;
+            if (w >= 0) best = w;
+        }
+        const int i = by_count[r], n = rowptr[i + 1] - rowptr[i];
+        order[best * ni + used[best]++] = i;
+        load[best] += n, slice_load[best / kFusedWarps] += n;
+    }
 }
 
 // Fills the (already allocated) arrays of `plan` from `idx`; `scratch` holds plan_layout(...).total bytes.
@@ -471,30 +528,58 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
     FFI_CUDA_CHECK(cudaMemcpyAsync(plan->perm, vin, n * 4, cudaMemcpyDeviceToDevice, stream));
     FFI_LAUNCH_CHECK("rowptr_kernel");
 
-    // Chunked lists for the narrow-input grad_x kernel.
-    if (g.chunks) {
-        const long long chunkEntries = static_cast<long long>(g.T) * K;
-        const long long nb = (g.nChunks + 1) * N;
+    plan->order = nullptr;
+    if (!g.chunks) {
+        FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
+        return FFI_OK;
+    }
+
+    // Chunked lists for the narrow-input kernels, of T rows a chunk, and what the kernel that stages them in shared memory has to
+    // know: the entries per warp, the longest run.
+    int T = g.T, longest = 0;
+    auto chunk_lists = [&]() -> int {
+        const long long chunkEntries = static_cast<long long>(T) * K, nChunks = ceil_div(L, T), nb = (nChunks + 1) * N;
         chunk_bounds_kernel<<<static_cast<unsigned>(ceil_div(nb, 256)), 256, 0, stream>>>(
-            plan->rowptr, plan->perm, static_cast<int>(N), chunkEntries, g.nChunks, lb);
-        chunk_fill_kernel<<<static_cast<unsigned>(g.nChunks), 256, (N + 1) * sizeof(int), stream>>>(
+            plan->rowptr, plan->perm, plan->order, static_cast<int>(N), chunkEntries, nChunks, lb);
+        chunk_fill_kernel<<<static_cast<unsigned>(nChunks), 256, (N + 1) * sizeof(int), stream>>>(
             plan->perm, lb, static_cast<int>(N), chunkEntries, plan->cptr, plan->cperm);
         FFI_LAUNCH_CHECK("chunk kernels");
-        // entries per warp, for the kernel that stages them in shared memory
         FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, (kFusedWarps + 1) * sizeof(int), stream));
-        plan->fused_ni = g.ni;
-        warp_stats_kernel<<<static_cast<unsigned>(ceil_div(N, g.ni)), 256, 0, stream>>>(plan->cptr, static_cast<int>(N), g.nChunks, g.ni, stats);
+        warp_stats_kernel<<<static_cast<unsigned>(ceil_div(N, g.ni)), 256, 0, stream>>>(plan->cptr, static_cast<int>(N), nChunks, g.ni, stats);
         FFI_LAUNCH_CHECK("warp_stats_kernel");
         FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, (kFusedWarps + 1) * sizeof(int), cudaMemcpyDeviceToHost, stream));
-        plan->chunk_rows = g.T;
-        plan->n_chunks = g.nChunks;
-        plan->has_chunks = true;
+        FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
+        plan->chunk_rows = T;
+        plan->n_chunks = nChunks;
+        plan->fused_entries[0] = 0;
+        for (int w = 0; w < kFusedWarps; ++w) plan->fused_entries[w + 1] = plan->fused_entries[w] + (most[w] + 1) / 2 * 2;
+        longest = most[kFusedWarps];
+        return FFI_OK;
+    };
+    int rc = chunk_lists();
+    if (rc != FFI_OK) return rc;
+    const long long average = ceil_div(static_cast<int64_t>(T) * K, N);
+    if (longest > 3 * average + kFusedFarRun || longest > kFusedLongestRun || !chunks_fit(T, plan->fused_entries[kFusedWarps])) {
+        // An uneven table: the inputs are dealt anew, and the chunks get shorter until the entries of the largest warps fit (each try
+        // takes the kernels above and a round trip to the device: a rebuild at N=768, L=670,091, K=32 takes 1.26 ms for an even table,
+        // 1.75 with inputs drawn by Zipf's law of exponent 0.6, 2.3 of 1, 2.9 of 1.3).  Dealt, nearly all fit the chunks of an even
+        // table: T stays 272 up to exponent 0.8, 264 at 1, 240 at 1.3.
+        int rowptr[kNarrowMaxN + 1], order[kNarrowMaxN];
+        FFI_CUDA_CHECK(cudaMemcpyAsync(rowptr, plan->rowptr, (N + 1) * sizeof(int), cudaMemcpyDeviceToHost, stream));
+        FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
+        deal_inputs(rowptr, static_cast<int>(N), g.ni, order);
+        plan->order = plan->order_store;
+        FFI_CUDA_CHECK(cudaMemcpyAsync(plan->order, order, N * sizeof(int), cudaMemcpyHostToDevice, stream));
+        while (true) {
+            rc = chunk_lists();
+            if (rc != FFI_OK) return rc;
+            if (T <= g.leastT || chunks_fit(T, plan->fused_entries[kFusedWarps])) break;
+            T = lower_rows(L, N, g.ni, T, plan->fused_entries[kFusedWarps], g.leastT);
+        }
     }
-    FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
-    plan->fused_entries[0] = 0;
-    for (int w = 0; w < kFusedWarps; ++w) plan->fused_entries[w + 1] = plan->fused_entries[w] + (most[w] + 1) / 2 * 2;
-    const long long average = ceil_div(static_cast<int64_t>(g.T) * K, N);
-    plan->fused_uneven = most[kFusedWarps] > 3 * average + kFusedFarRun || most[kFusedWarps] > kFusedLongestRun;
+    plan->fused_ni = g.ni;
+    plan->range_chunks = g.nChunks;
+    plan->has_chunks = true;
     return FFI_OK;
 }
 
@@ -564,7 +649,8 @@ extern "C" int ffi_plan_create(const int32_t* idx, int64_t L, int64_t K, int64_t
 
     // the index arrays are one allocation: a cudaMalloc and a cudaFree of this size take about a millisecond each
     const size_t rowptr_at = 0, perm_at = rowptr_at + scratch_up((N + 1) * sizeof(int)), cptr_at = perm_at + scratch_up(g.n * 4);
-    const size_t cperm_at = cptr_at + (g.chunks ? scratch_up(g.cptrBytes) : 0), total = cperm_at + (g.chunks ? scratch_up(g.n * 4) : 0);
+    const size_t cperm_at = cptr_at + (g.chunks ? scratch_up(g.cptrBytes) : 0), order_at = cperm_at + (g.chunks ? scratch_up(g.n * 4) : 0),
+                 total = order_at + (g.chunks ? scratch_up(N * sizeof(int)) : 0);
     if (cudaMalloc(&plan->arrays, total) != cudaSuccess) {
         cudaGetLastError();
         plan->arrays = nullptr;
@@ -576,6 +662,7 @@ extern "C" int ffi_plan_create(const int32_t* idx, int64_t L, int64_t K, int64_t
     if (g.chunks) {
         plan->cptr = reinterpret_cast<int32_t*>(base + cptr_at);
         plan->cperm = reinterpret_cast<int32_t*>(base + cperm_at);
+        plan->order_store = reinterpret_cast<int32_t*>(base + order_at);
     }
     plan->device_bytes = total;
     DeviceBuffer scratch;
@@ -642,10 +729,10 @@ extern "C" int ffi_plan_export_chunked(const ffi_plan* plan, int32_t* rowptr, in
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const int N = static_cast<int>(plan->N);
     chunked_row_totals_kernel<<<static_cast<unsigned>(ceil_div(N + 1, 256)), 256, 0, stream>>>(
-        plan->cptr, N, plan->n_chunks, rowptr);
+        plan->cptr, plan->order, N, plan->n_chunks, rowptr);
     small_exclusive_scan_kernel<<<1, 1024, 0, stream>>>(rowptr, N + 1);
     chunked_gather_kernel<<<static_cast<unsigned>(ceil_div(N, 4)), 128, 0, stream>>>(
-        plan->cptr, plan->cperm, rowptr, N, plan->n_chunks,
+        plan->cptr, plan->cperm, plan->order, rowptr, N, plan->n_chunks,
         static_cast<long long>(plan->chunk_rows) * plan->K, perm);
     FFI_LAUNCH_CHECK("chunked export");
     return FFI_OK;

@@ -104,6 +104,8 @@ int ffi_plan_create(const int32_t* idx, int64_t L, int64_t K, int64_t N, void* s
  * step): same result as destroying it and calling ffi_plan_create, without allocating or freeing the
  * index arrays.  The first rebuild of a plan allocates its sort scratch (about 17 bytes per connection)
  * and keeps it until ffi_plan_destroy; later rebuilds allocate nothing.  Synchronises `stream`.
+ * The launches of a call depend on the table (rows per chunk, entries per warp): a CUDA graph that holds
+ * calls with this plan has to be captured again before it is replayed.
  * FFI_ERR_INDEX_RANGE leaves the plan unusable until a rebuild succeeds.
  */
 int ffi_plan_rebuild(ffi_plan* plan, const int32_t* idx, void* stream);

@@ -114,3 +114,81 @@ def test_hot_inputs_do_not_serialise(B):
         plan = ops.FFIPlan(idx, N)
         times.append(_time(lambda: ops._backward(x, idx, W, gT, True, plan=plan, grad_is_transposed=True)))
     assert times[1] < 8 * times[0]
+
+
+def _weighted_table(weights, L, K, gen):
+    cdf = torch.cumsum(weights.double(), 0)
+    u = torch.rand((L, K), generator=gen, dtype=torch.float64, device="cuda") * cdf[-1]
+    return torch.searchsorted(cdf, u).clamp(max=len(weights) - 1).int()
+
+
+def _weights(kind, N, gen):
+    ranks = torch.arange(1, N + 1, device="cuda")
+    if kind == "uniform":
+        return torch.ones(N, device="cuda")
+    if kind == "leading quarter":  # 30 % of the links more
+        w = torch.ones(N, device="cuda")
+        w[:N // 4] += 0.3 / 0.7 * 4
+        return w
+    exponent, order = kind
+    w = ranks.double() ** -exponent
+    return w if order == "ordered" else w[torch.randperm(N, generator=gen, device="cuda")]
+
+
+def _kernels(f):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events()]
+
+
+@pytest.mark.parametrize("kind", [(0.6, "shuffled"), (1.0, "shuffled"), (0.5, "ordered"), "leading quarter", "uniform"], ids=str)
+def test_uneven_tables_take_the_one_pass_kernel(kind):
+    N, L, K = 768, 670091, 32
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    idx = _weighted_table(_weights(kind, N, gen), L, K, gen)
+    W = torch.randn((L, K), generator=gen, device="cuda")
+    plan = ops.FFIPlan(idx, N)
+    for B in (16, 64, 128):
+        x, gT = torch.randn((N, B), generator=gen, device="cuda"), torch.zeros((L, _stride(B)), device="cuda")
+        names = _kernels(lambda: ops._backward(x, idx, W, gT, True, plan=plan, grad_is_transposed=True))
+        assert any("ffi_bwd_runs_kernel" in n for n in names), names
+        assert not any("grad_x_narrow" in n for n in names), names
+
+
+@pytest.mark.parametrize("N,L,K", [(768, 20011, 32), (100, 3001, 7), (15, 900, 3), (513, 40000, 24), (2048, 9000, 16), (300, 33, 5)])
+@pytest.mark.parametrize("kind", [(0.8, "shuffled"), (1.2, "ordered"), "leading quarter"], ids=str)
+def test_dealt_plans(N, L, K, kind):
+    """Plans of uneven tables hold their inputs in another order, and shorter chunks where need be: the index they hold, all entry
+    points that read it, and rebuilds from even to uneven tables and back."""
+    gen, x, W, g = _inputs(70, N, L, K, torch.float32, 3)
+    idx = _weighted_table(_weights(kind, N, gen), L, K, gen)
+    even = torch.randint(0, N, (L, K), generator=gen, dtype=torch.int32, device="cuda")
+    _check(x, idx, W, g)
+    plan = ops.FFIPlan(idx, N)
+    for a, b in zip(plan.export(), plan.export(chunked=True)):
+        assert torch.equal(a, b)
+    gT = torch.zeros((L, 128), device="cuda")
+    gT[:, :70] = g
+
+    def grads(plan, idx):
+        both = ops._backward(x, idx, W, gT, True, plan=plan, grad_is_transposed=True)
+        alone = ops._backward(x, idx, W, gT, True, plan=plan, want_weight_grad=False, grad_is_transposed=True)
+        return both[0], both[1], alone[0]
+
+    want, want_even = grads(plan, idx), grads(ops.FFIPlan(even, N), even)
+    n = torch.bincount(idx.flatten().long(), minlength=N).double()[:, None] + 8
+    size = torch.zeros((N, 70), dtype=torch.float64, device="cuda")
+    for k in range(K):
+        size.index_add_(0, idx[:, k].long(), (W[:, k, None] * g).abs().double())
+    assert ((want[0].double() - want[2].double()).abs() <= 2 * n * EPS * size + 1e-30).all()
+    plan.rebuild(even)
+    held = plan.info()["device_bytes"]
+    for table, values in ((even, want_even), (idx, want), (even, want_even)):
+        plan.rebuild(table)
+        assert plan.info()["device_bytes"] == held
+        for a, b in zip(grads(plan, table), values):
+            assert torch.equal(a, b)
+        for a, b in zip(plan.export(), plan.export(chunked=True)):
+            assert torch.equal(a, b)
