@@ -284,7 +284,10 @@ __global__ void __launch_bounds__(kThreads, 4) ffi_bwd_wide_kernel(const __grid_
             if (LPE == 2) s[0] += __shfl_xor_sync(kAll, s[0], 1);
             if (lane % LPE == 0 && el < n) {
                 float* dst = p.gW + ws.pos[slot][h + el];
-                *dst = p.addW ? *dst + s[0] : s[0];
+                // (a batch tile after the first adds to what the one before stored, once per element: a reduction in L2 that nobody waits
+                // for; loading the old value took 158 to 187 % of the time at B=300, N=3,000 ... 4,000)
+                if (p.addW) atomicAdd(dst, s[0]);
+                else *dst = s[0];
             }
             __syncwarp();
         }
@@ -345,9 +348,10 @@ int launch_wide(BwdWideParams p, long long L, const DeviceInfo& dev, cudaStream_
     long long rows = std::min(kChunkBytes / (BT * 4), kChunkAll / perRow);
     if (rows < 1) rows = 1;
     const long long nChunks = ceil_div(L, rows), T = ceil_div(L, nChunks);
-    // as many warps as give each the same number of inputs
+    // as many warps as give each the same number of inputs, and as many CTAs on every SM: with 257 CTAs for 2,049 inputs some SMs had
+    // two and others one (B=300, L=200,000, K=32 1,334 -> 987 us; N=5,000 1,224 -> 1,007; from 16,384 inputs on no difference)
     const long long cap = static_cast<long long>(dev.sm_count) * occ * kWarps;
-    const long long ctas = ceil_div(ceil_div(p.N, ceil_div(p.N, cap)), kWarps);
+    const long long ctas = round_up(ceil_div(ceil_div(p.N, ceil_div(p.N, cap)), kWarps), dev.sm_count);
     int* cursor = p.cursor;
     const float* gT = p.gT;
     const TX* xT = static_cast<const TX*>(p.xT);
@@ -374,7 +378,9 @@ int launch_wide(BwdWideParams p, long long L, const DeviceInfo& dev, cudaStream_
 
 }  // namespace
 
-// Plans without chunked lists (wide inputs).
+// Plans without chunked lists (wide inputs).  Against a kernel each for grad_x and grad_W, at K=16 ... 64, L=20,000 and 200,000, by
+// number of inputs: 2,049 1.1 (B=390 bf16, two tiles of which the second is half empty) to 3.8 times as fast (B=20), 5,000 1.1 to
+// 2.4, 12,000 1.35 to 2.6, 65,536 1.2 to 2.1.
 bool backward_wide_applicable(const ffi_plan* plan) { return plan && !plan->has_chunks && plan->N > 2048; }
 
 // grad_x as [N][B] (always), grad_W and, when gbias != nullptr, grad_bias, from gT; xT is x as [N][ldx]; cursor: N ints.
