@@ -7,9 +7,12 @@ from ecml23_sparse_b200 import ops
 
 pytestmark = pytest.mark.gpu
 
-# B, N, L, K, storage, x given as [N,B]; small ones, whose kernels are shorter than a launch, and one with long kernels
+# B, N, L, K, storage, x given as [N,B]; small ones, whose kernels are shorter than a launch, and one with long kernels; the last three take the
+# one-pass backward for wide inputs, whose launches set each other up and read gT before they wait, in two chunks of one and of two
+# batch tiles
 SHAPES = [(127, 254, 513, 73, "f32", False), (5, 64, 40, 8, "f32", True), (20, 205, 900, 16, "bf16", True), (130, 300, 2000, 24, "bf16", False),
-          (33, 3000, 700, 8, "f32", False), (128, 768, 30000, 32, "f32", True), (256, 512, 9000, 64, "bf16", True)]
+          (33, 3000, 700, 8, "f32", False), (128, 768, 30000, 32, "f32", True), (256, 512, 9000, 64, "bf16", True),
+          (33, 2111, 250007, 4, "f32", True), (256, 3000, 50021, 8, "bf16", True), (512, 3000, 50021, 5, "f32", False)]
 
 
 @pytest.mark.parametrize("B,N,L,K,storage,tp", SHAPES)
