@@ -143,7 +143,8 @@ __global__ void __launch_bounds__(kThreads, 4) ffi_bwd_wide_kernel(const __grid_
     int i0 = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
 
     // The launch after this one may start its CTAs while this one's last warps finish: grad_bias needs nothing of the chunks
-    // before, and reading the chunk's rows for it brings them into L2.
+    // before, and reading the chunk's rows for it brings them into L2.  This comes before the wait, so gT has to be complete when the
+    // first launch of the sequence starts: that one is a plain launch (launch_wide), which starts after all that precedes it.
     chain_release();
     if (p.gbias) {  // four rows at a time
         for (long long o = p.o0 + i0; o < p.o1; o += 4ll * stride) {
@@ -369,7 +370,7 @@ int launch_wide(BwdWideParams p, long long L, const DeviceInfo& dev, cudaStream_
             p.cursor = t + 1 == tiles && p.o1 < L ? cursor : nullptr;
             p.gbias = t == 0 ? gbias : nullptr;
             if (o0 > 0 || t > 0) FFI_CUDA_CHECK(launch_chained(kern, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), smem, stream, p));
-            else kern<<<static_cast<unsigned>(ctas), kThreads, smem, stream>>>(p);  // (reads gT before it waits)
+            else kern<<<static_cast<unsigned>(ctas), kThreads, smem, stream>>>(p);  // not chained: the kernel reads gT and writes grad_bias before it waits
         }
     }
     FFI_LAUNCH_CHECK("ffi_bwd_wide_kernel");

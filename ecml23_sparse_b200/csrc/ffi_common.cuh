@@ -64,7 +64,9 @@ cudaError_t prepare_kernel(const void* kern, int threads, size_t smem, int* occ)
 // ---- kernels that start while the one before them in the stream ends ---------------
 // A kernel launched by launch_chained may be set up (its launch, CTAs on SMs that are free) while the kernel before it in the stream
 // still runs.  It calls chain_wait() before it touches global memory: this waits until all kernels before it are done and what
-// they wrote is visible.  chain_release() lets the kernel after it be set up, once all CTAs have called it or are done: short
+// they wrote is visible.  One kernel reads and writes before that, ffi_bwd_wide_kernel, which is launched several times in a row: what
+// it reads before the wait (gT) was written before the first of these launches, which is for that reason a plain one, and what it
+// writes there (grad_bias) no other of them touches.  chain_release() lets the kernel after it be set up, once all CTAs have called it or are done: short
 // kernels do so first thing, long ones towards their end or not at all (CTAs that sit beside a long kernel's and wait slow it down:
 // one-pass backward of B=32, N=768, L=670,091, K=32 371 -> 378 us).
 // 127 x 254 -> 513 (K=73) forward and backward, six kernels: 37.1 -> 25.7 us.
