@@ -64,6 +64,7 @@ struct BwdFusedParams {
     int Bpad;
     int segChunks;  // chunks per flushed partial
     int ni;         // inputs per warp
+    int longRun;    // uneven tables: kLongRun, or 0 where a bundle has fewer inputs than lane groups
     int boxes;      // TMA boxes per tile (at most 256 rows each)
     int lastHalf;   // bf16 W of an odd number of elements: position of the last one, which has no whole word; else -1
     bool xVec;      // rows of x start on 8 bytes; what lies behind an odd B in them is zero
@@ -261,6 +262,9 @@ __device__ __forceinline__ void tmem_store(unsigned taddr, const LaneVec<VPL, LG
 //   exponent 0.8: 128 1,973 (two) -> 1,373, 64 1,300 (two) -> 811, 32 2,194 -> 632, 8 1,968 -> 384
 //   exponent 1:   128 2,350 (two) -> 1,788, 64 1,375 (two) -> 1,110, 32 4,067 -> 889, 8 3,856 -> 548
 //   30 % of the links added to the leading quarter of the inputs: 128 1,974 (two) -> 862, 64 1,201 (two) -> 517
+// Fewer than kFusedFewInputs inputs per warp take this variant, too, and share all runs longer than one and a half times the average of a
+// full bundle (longRun = 0): side by side most groups had no input.  L=300,000, us, before -> now: N=10, K=8 B=128 263 -> 114,
+// 8 134 -> 45; N=32, K=16 128 246 -> 177, 8 119 -> 65.  (With longRun 4, 8, 12 and 15 over 112 such shapes 1, 2, 3 and 6 % slower.)
 // (An even table: 813, 499, 356, 224.)  Two kernels are faster again from about a fifth (33 to 64 columns, where the
 // chain is 1.6 times theirs at four fifths), a third (65 to 128 and 17 to 32) or more of all links to ONE input.  In one kernel with the even case and
 // a flag looked up per chunk, even tables took 2 to 6 % longer (registers).
@@ -485,7 +489,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                     most = max(most, __shfl_xor_sync(kAll, most, off));
                     sum += __shfl_xor_sync(kAll, sum, off);
                 }
-                const bool far = __any_sync(kAll, most > kSideBySide || most > sum / G * 2 + kLongRun);
+                const bool far = p.longRun == 0 || __any_sync(kAll, most > kSideBySide || most > sum / G * 2 + p.longRun);
                 if (lane == 0) b[kBounds - 1] = far;
             }
             if constexpr (HALVES == 2) {
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
                         if (most == 0) continue;
                         // what a run has more than the longest that is not much above the average is left for all groups together
                         const int mean = __reduce_add_sync(kAll, q == 0 ? n : 0) / G;
-                        const int lim = min(kSideBySide, __reduce_max_sync(kAll, n <= mean + mean / 2 + kLongRun ? n : 0));
+                        const int lim = min(kSideBySide, __reduce_max_sync(kAll, n <= mean + mean / 2 + p.longRun ? n : 0));
                         LaneT acc, xr;
                         tmem_load_input(taddr0 + j * COLS, acc, xr);
                         if (lim > 0) side_by_side(acc, xr, e, min(n, lim), lim, min(least, lim));
@@ -939,6 +943,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         p.Bpad = c.Bpad;
         p.segChunks = c.segChunks;
         p.ni = c.ni;
+        p.longRun = c.ni < kFusedFewInputs ? 0 : kLongRun;
         // gT as a 2-D tensor [L rows][BT columns] with row pitch ldg; one or two boxes = a g tile
         CUtensorMap g_map;
         const int rows = p.T / c.halves;  // (T is a multiple of 8)

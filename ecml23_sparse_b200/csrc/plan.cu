@@ -371,11 +371,12 @@ bool chunks_fit(int64_t T, int64_t entries) { return fused_smem_bytes(T * 512, e
 PlanShape plan_shape(int64_t L, int64_t K, int64_t N) {
     const int64_t sms = device_sms();
     int ni = fused_inputs_per_warp(N);
+    const int64_t warps = std::min<int64_t>(kFusedWarps, ceil_div(N, ni));  // that have inputs
     int64_t T = 512;
     for (; T > 8; T -= 8) {
         // a random table's warp with the most entries
         const double entries = static_cast<double>(T) * K * ni / static_cast<double>(N), most = entries + 5.0 * std::sqrt(entries) + 4.0;
-        if (T * K <= 16384 && chunks_fit(T, static_cast<int64_t>(kFusedWarps * most))) break;
+        if (T * K <= 16384 && chunks_fit(T, static_cast<int64_t>(warps * most))) break;
     }
     if (T * K > 16384) return {0, ni};  // K in the thousands: no chunked lists
     const int64_t parts = ceil_div(N, kFusedWarps * ni), R = sms / parts > 0 ? sms / parts : 1;
@@ -556,26 +557,32 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
         longest = most[kFusedWarps];
         return FFI_OK;
     };
-    int rc = chunk_lists();
-    if (rc != FFI_OK) return rc;
-    const long long average = ceil_div(static_cast<int64_t>(T) * K, N);
-    if (longest > 3 * average + kFusedFarRun || longest > kFusedLongestRun || !chunks_fit(T, plan->fused_entries[kFusedWarps])) {
-        // An uneven table: the inputs are dealt anew, and the chunks get shorter until the entries of the largest warps fit (each try
-        // takes the kernels above and a round trip to the device: a rebuild at N=768, L=670,091, K=32 takes 1.26 ms for an even table,
-        // 1.75 with inputs drawn by Zipf's law of exponent 0.6, 2.3 of 1, 2.9 of 1.3).  Dealt, nearly all fit the chunks of an even
-        // table: T stays 272 up to exponent 0.8, 264 at 1, 240 at 1.3.
+    auto deal = [&]() -> int {
         int rowptr[kNarrowMaxN + 1], order[kNarrowMaxN];
         FFI_CUDA_CHECK(cudaMemcpyAsync(rowptr, plan->rowptr, (N + 1) * sizeof(int), cudaMemcpyDeviceToHost, stream));
         FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
         deal_inputs(rowptr, static_cast<int>(N), g.ni, order);
         plan->order = plan->order_store;
         FFI_CUDA_CHECK(cudaMemcpyAsync(plan->order, order, N * sizeof(int), cudaMemcpyHostToDevice, stream));
-        while (true) {
-            rc = chunk_lists();
-            if (rc != FFI_OK) return rc;
-            if (T <= g.leastT || chunks_fit(T, plan->fused_entries[kFusedWarps])) break;
-            T = lower_rows(L, N, g.ni, T, plan->fused_entries[kFusedWarps], g.leastT);
-        }
+        return FFI_OK;
+    };
+    int rc = g.ni < kFusedFewInputs ? deal() : FFI_OK;  // (few inputs: shared by the lane groups, whatever the table)
+    if (rc == FFI_OK) rc = chunk_lists();
+    if (rc != FFI_OK) return rc;
+    const long long average = ceil_div(static_cast<int64_t>(T) * K, N);
+    if (!plan->order && (longest > 3 * average + kFusedFarRun || longest > kFusedLongestRun || !chunks_fit(T, plan->fused_entries[kFusedWarps]))) {
+        // An uneven table: the inputs are dealt anew, and the chunks get shorter until the entries of the largest warps fit (each try
+        // takes the kernels above and a round trip to the device: a rebuild at N=768, L=670,091, K=32 takes 1.26 ms for an even table,
+        // 1.75 with inputs drawn by Zipf's law of exponent 0.6, 2.3 of 1, 2.9 of 1.3).  Dealt, nearly all fit the chunks of an even
+        // table: T stays 272 up to exponent 0.8, 264 at 1, 240 at 1.3.
+        rc = deal();
+        if (rc == FFI_OK) rc = chunk_lists();
+        if (rc != FFI_OK) return rc;
+    }
+    while (plan->order && T > g.leastT && !chunks_fit(T, plan->fused_entries[kFusedWarps])) {
+        T = lower_rows(L, N, g.ni, T, plan->fused_entries[kFusedWarps], g.leastT);
+        rc = chunk_lists();
+        if (rc != FFI_OK) return rc;
     }
     plan->fused_ni = g.ni;
     plan->range_chunks = g.nChunks;

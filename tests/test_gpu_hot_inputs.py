@@ -116,6 +116,30 @@ def test_hot_inputs_do_not_serialise(B):
     assert times[1] < 8 * times[0]
 
 
+@pytest.mark.parametrize("B", [1, 9, 24, 64, 127, 200])
+@pytest.mark.parametrize("N,L,K,bf16", [(1, 5003, 3, False), (3, 9001, 2, True), (10, 20011, 8, False), (16, 4099, 7, True), (17, 4099, 16, False),
+                                        (33, 30001, 5, True), (48, 7001, 24, False), (49, 7001, 24, True), (65, 3001, 16, False)])
+def test_few_inputs(B, N, L, K, bf16):
+    """Fewer inputs per warp than lane groups, down to warps without any: the groups share the runs."""
+    gen, x, W, g = _inputs(B, N, L, K, torch.bfloat16 if bf16 else torch.float32, B)
+    _check(x, torch.randint(0, N, (L, K), generator=gen, dtype=torch.int32, device="cuda"), W, g)
+
+
+@pytest.mark.parametrize("B", [8, 64, 128])
+def test_few_inputs_do_not_idle_the_lane_groups(B):
+    """As many entries among 10 inputs as among 256: 1 to 1.2 times the time; 2 to 3 times when a group walked an input by itself."""
+    L, K = 300000, 8
+    times = []
+    for N in (256, 10):
+        gen, x, W, g = _inputs(B, N, L, K, torch.float32, B)
+        idx = torch.randint(0, N, (L, K), generator=gen, dtype=torch.int32, device="cuda")
+        gT = torch.zeros((L, _stride(B)), device="cuda")
+        gT[:, :B] = g
+        plan = ops.FFIPlan(idx, N)
+        times.append(min(_time(lambda: ops._backward(x, idx, W, gT, True, plan=plan, grad_is_transposed=True)) for _ in range(3)))
+    assert times[1] < 1.6 * times[0]
+
+
 def _weighted_table(weights, L, K, gen):
     cdf = torch.cumsum(weights.double(), 0)
     u = torch.rand((L, K), generator=gen, dtype=torch.float64, device="cuda") * cdf[-1]
