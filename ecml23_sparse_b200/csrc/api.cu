@@ -451,11 +451,12 @@ static int backward_impl(const void* x, const int32_t* idx, const void* W, const
 
     // One pass for grad_x and grad_W when the shape allows it, else one kernel each.
     const bool fused = grad_x && grad_w && backward_fused_applicable(plan, B);
-    // Wide inputs: the one-pass kernel of backward_wide.cu, unless a caller that sized its workspace by itself left no room
-    // for the cursors and copies.
+    // Wide inputs: the one-pass kernel of backward_wide.cu, unless a hot input would hold it up or a caller that sized its workspace
+    // by itself left no room for the cursors and copies.
     const size_t wide_gT = gT_in ? 0 : align_up(static_cast<size_t>(L) * transposed_g_stride(B) * 4);
     const size_t wide_x = x_transposed ? 0 : align_up(static_cast<size_t>(N) * round_up(B, 128) * esize) + align_up(static_cast<size_t>(N) * B * 4);
     const bool wide = !fused && grad_x && grad_w && backward_wide_applicable(plan) && (x_transposed || N <= 65535 * 32) &&
+                      backward_wide_pays(plan, B, gT_in ? ldg_in : transposed_g_stride(B), bf16) &&
                       workspace && workspace_bytes >= wide_gT + wide_x + align_up(static_cast<size_t>(N) * 4);
     const bool sep_w = !fused && !wide && (grad_w || grad_bias);
     const bool gw_stream = sep_w && grad_w_stream_applicable(Bi, Ni, Ki, idx);

@@ -384,6 +384,28 @@ int launch_wide(BwdWideParams p, long long L, const DeviceInfo& dev, cudaStream_
 // 2.4, 12,000 1.35 to 2.6, 65,536 1.2 to 2.1.
 bool backward_wide_applicable(const ffi_plan* plan) { return plan && !plan->has_chunks && plan->N > 2048; }
 
+namespace {
+// Columns of the batch tiles.
+int tile_columns(int64_t ldg) { return ldg % 256 == 0 ? 256 : ldg % 128 == 0 ? 128 : ldg % 64 == 0 ? 64 : 32; }
+}  // namespace
+
+// An input belongs to one warp, here and in the kernel for grad_x alone, so an input with very many entries holds up everything else.
+// Here the batch tiles come one after another, in kChain us an entry and tile; there all tiles are walked at once, in about 0.2 us an
+// entry (0.13 to 0.28).  So several tiles pay for what the hottest input has beyond the others as long as that stays below what one
+// gather less gains, 0.1 (bf16) or 0.2 (fp32) us for a million entries and columns.  Measured, both kernels against one, us, for the inputs drawn
+// by Zipf's law of the exponents 0, 0.2, 0.3, 0.4, 0.6: B=512, N=16,384, L=50,000, K=32 bf16 334, 369, 520, 886, 2,732 against 254, 374,
+// 588, 1,043, 4,003 (line at 0.3), fp32 425, 469, 620, 1,001, 2,974 against 256, 371, 575, 1,016, 3,912 (line between 0.3 and 0.4);
+// B=1,024, N=32,768, L=60,000, K=32 bf16 788, 816, 929, 1,276, 3,695 against 597, 705, 998, 1,753, 7,343 (line between 0.2 and 0.3);
+// B=384 fp32 line between 0.4 and 0.5.  One tile pays always: B=256, N=65,536, L=200,000 bf16 681, 784, 1,057, 1,874, 8,353 against 520,
+// 575, 737, 1,168, 4,963.
+bool backward_wide_pays(const ffi_plan* plan, int64_t B, int64_t ldg, bool bf16) {
+    const int columns = tile_columns(ldg);
+    const double kChain = columns == 256 ? 0.14 : columns == 128 ? 0.077 : columns == 64 ? 0.054 : 0.035;
+    const double more = ceil_div(B, columns) * kChain - 0.2;
+    const double entries = static_cast<double>(plan->L) * plan->K, beyond = plan->longest_input - 2.0 * entries / plan->N;
+    return more <= 0.0 || beyond * more <= (bf16 ? 1e-7 : 2e-7) * entries * B;
+}
+
 // grad_x as [N][B] (always), grad_W and, when gbias != nullptr, grad_bias, from gT; xT is x as [N][ldx]; cursor: N ints.
 int launch_backward_wide(const GradXArgs& a, const void* xT, int64_t ldx, float* gxT, float* gW, float* gbias, int* cursor,
                          cudaStream_t stream) {
@@ -397,10 +419,12 @@ int launch_backward_wide(const GradXArgs& a, const void* xT, int64_t ldx, float*
     p.B = a.B, p.N = a.N, p.K = a.K;
     auto typed = [&](auto tx) -> int {
         using TX = decltype(tx);
-        if (a.ldg % 256 == 0) return launch_wide<1, TX>(p, a.L, dev, stream);
-        if (a.ldg % 128 == 0) return launch_wide<2, TX>(p, a.L, dev, stream);
-        if (a.ldg % 64 == 0) return launch_wide<4, TX>(p, a.L, dev, stream);
-        return launch_wide<8, TX>(p, a.L, dev, stream);
+        switch (tile_columns(a.ldg)) {
+            case 256: return launch_wide<1, TX>(p, a.L, dev, stream);
+            case 128: return launch_wide<2, TX>(p, a.L, dev, stream);
+            case 64: return launch_wide<4, TX>(p, a.L, dev, stream);
+            default: return launch_wide<8, TX>(p, a.L, dev, stream);
+        }
     };
     return a.w_bf16 ? typed(__nv_bfloat16{}) : typed(float{});
 }

@@ -308,6 +308,7 @@ struct ffi_plan {
     // that the warp has in any chunk and slice
     int fused_entries[ffi::kFusedWarps + 1] = {};
     int fused_ni = 0;  // inputs per warp of the one-pass backward
+    int longest_input = 0;  // without chunked lists: most entries that an input has
     void* arrays = nullptr;     // the allocation that holds the four index arrays
     int32_t* rowptr = nullptr;  // [N+1]   canonical CSR-by-input
     int32_t* perm = nullptr;    // [L*K]   positions sorted by (idx[p], p)
@@ -363,6 +364,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
                           cudaStream_t stream);
 // The same for wide inputs; grad_x leaves as gxT[N][B], cursor is scratch of N ints.
 bool backward_wide_applicable(const ffi_plan* plan);
+bool backward_wide_pays(const ffi_plan* plan, int64_t B, int64_t ldg, bool bf16);  // for this table, against a kernel each
 int launch_backward_wide(const GradXArgs& a, const void* xT, int64_t ldx, float* gxT, float* gW, float* gbias, int* cursor,
                          cudaStream_t stream);
 

@@ -293,6 +293,13 @@ __global__ void warp_stats_kernel(const int* __restrict__ cptr, int N, long long
     }
 }
 
+// longest[0] = largest number of entries an input has (zeroed by the caller).
+__global__ void longest_row_kernel(const int* __restrict__ rowptr, int N, int* __restrict__ longest) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int most = __reduce_max_sync(0xffffffffu, i < N ? rowptr[i + 1] - rowptr[i] : 0);
+    if (threadIdx.x % 32 == 0) atomicMax(longest, most);
+}
+
 // Self-check export: rebuild the canonical form from (cptr, cperm).
 __global__ void chunked_row_totals_kernel(const int* __restrict__ cptr, const int* __restrict__ order, int N, long long nChunks,
                                           int* __restrict__ totals) {
@@ -531,7 +538,12 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
 
     plan->order = nullptr;
     if (!g.chunks) {
+        FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, sizeof(int), stream));
+        longest_row_kernel<<<static_cast<unsigned>(ceil_div(N, 256)), 256, 0, stream>>>(plan->rowptr, static_cast<int>(N), stats);
+        FFI_LAUNCH_CHECK("longest_row_kernel");
+        FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, sizeof(int), cudaMemcpyDeviceToHost, stream));
         FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
+        plan->longest_input = most[0];
         return FFI_OK;
     }
 
