@@ -265,9 +265,8 @@ __device__ __forceinline__ void tmem_store(unsigned taddr, const LaneVec<VPL, LG
 // Fewer than kFusedFewInputs inputs per warp take this variant, too, and share all runs longer than one and a half times the average of a
 // full bundle (longRun = 0): side by side most groups had no input.  L=300,000, us, before -> now: N=10, K=8 B=128 263 -> 114,
 // 8 134 -> 45; N=32, K=16 128 246 -> 177, 8 119 -> 65.  (With longRun 4, 8, 12 and 15 over 112 such shapes 1, 2, 3 and 6 % slower.)
-// (An even table: 813, 499, 356, 224.)  Two kernels are faster again from about a fifth (33 to 64 columns, where the
-// chain is 1.6 times theirs at four fifths), a third (65 to 128 and 17 to 32) or more of all links to ONE input.  In one kernel with the even case and
-// a flag looked up per chunk, even tables took 2 to 6 % longer (registers).
+// (An even table: 813, 499, 356, 224.)  With a fifth or more of all links to ONE input two kernels are faster again, see fused_pays.
+// In one kernel with the even case and a flag looked up per chunk, even tables took 2 to 6 % longer (registers).
 //
 // ACC: a batch tile after the first (as a run-time flag it cost 5 %), whose grad_W and grad_bias add to what the tiles
 // before stored.
@@ -804,8 +803,8 @@ struct FusedConfig {
     size_t smem;
 };
 
-// For one tile of at most 128 batch columns.
-bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedConfig* c) {
+// For one tile of at most 128 batch columns.  `table`: whether the plan's table has to fit, too (the scratch is that of a table that does).
+bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedConfig* c, bool table = true) {
     if (!plan || !plan->has_chunks || B > 128) return false;
     // the entry code holds the position within the chunk in 14 bits
     if (static_cast<long long>(plan->chunk_rows) * plan->K > (1 << (32 - kKShift))) return false;
@@ -828,7 +827,7 @@ bool fused_config(const ffi_plan* plan, int64_t B, const DeviceInfo& dev, FusedC
     const size_t T = static_cast<size_t>(plan->chunk_rows);
     if (T * c->Bpad * 4 > (size_t{1} << kKShift)) return false;
     const size_t total = fused_smem_bytes(static_cast<int64_t>(T) * (c->halves == 2 ? 1 : 2) * c->Bpad * 4, plan->fused_entries[kFusedWarps], c->groups);
-    if (total > static_cast<size_t>(dev.max_smem_optin)) return false;  // a very uneven table: separate kernels
+    if (table && total > static_cast<size_t>(dev.max_smem_optin)) return false;  // a very uneven table: separate kernels
     c->smem = total;
     return true;
 }
@@ -872,12 +871,26 @@ int encode_g_map(CUtensorMap* map, const float* gT, int64_t L, int64_t ldg, int6
 
 }  // namespace
 
+// An input belongs to one warp of a range, so what bounds a table with a very hot input is that warp's chain, kChain ns an entry: the
+// more slices, the fewer ranges the input's entries are spread over.  The kernels for grad_x and grad_W alone take, with such tables,
+// about kTwo ns for every link, and 30 us for the second launch, its partials and short tables in general.  One pass against two, us, with a
+// share of 0.2 and 0.8 of the links on ONE input: N=2,048, L=150,000, K=32 B=64 869, 2,956 against 610, 1,295; 128 1,293, 3,990 against
+// 1,187, 3,401; 32 709, 2,437 against 570, 825; 8 (0.4 and 0.8) 744, 1,399 against 620, 823; N=768, L=200,000 B=64 494, 1,489 against 519,
+// 943; 32 (0.4 and 0.8) 683, 1,236 against 527, 646; N=300, L=100,000 B=64 192, 490 against 192, 325.  With one slice the one-pass kernel is
+// the faster one throughout (N=128 at 0.8: 0.3 to 0.94 of the two).
+static bool fused_pays(const ffi_plan* plan, const FusedConfig& c, int64_t columns) {
+    const double kChain = columns > 64 ? 20.0 : columns > 32 ? 14.5 : columns > 16 ? 11.5 : columns > 8 ? 7.9 : 6.7;
+    const double kTwo = columns > 64 ? 0.176 : columns > 32 ? 0.065 : columns > 16 ? 0.08 : columns > 8 ? 0.091 : 0.1;
+    const double links = static_cast<double>(plan->L) * plan->K;
+    return c.iparts == 1 || plan->longest_input * kChain / c.R <= links * kTwo + 30e3;
+}
+
 bool backward_fused_applicable(const ffi_plan* plan, int64_t B) {
     DeviceInfo dev;
     if (get_device_info(&dev) != FFI_OK) return false;
     FusedConfig c;
     const int64_t first = tile_columns(B, 0), last = B - (B - 1) / 128 * 128;
-    return fused_config(plan, first, dev, &c) && fused_config(plan, last, dev, &c);
+    return fused_config(plan, first, dev, &c) && fused_config(plan, last, dev, &c) && fused_pays(plan, c, first);
 }
 
 size_t backward_fused_workspace_bytes(const ffi_plan* plan, int64_t B) {
@@ -886,7 +899,7 @@ size_t backward_fused_workspace_bytes(const ffi_plan* plan, int64_t B) {
     size_t total = 0;  // the partials of every batch tile, summed by one launch at the end
     for (int64_t b0 = 0; b0 < B; b0 += 128) {
         FusedConfig c;
-        if (!fused_config(plan, tile_columns(B, b0), dev, &c)) return 0;
+        if (!fused_config(plan, tile_columns(B, b0), dev, &c, false)) return 0;
         total += static_cast<size_t>(c.R) * plan->N * c.Bpad * 4;
     }
     return total;

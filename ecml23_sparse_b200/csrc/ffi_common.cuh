@@ -308,7 +308,7 @@ struct ffi_plan {
     // that the warp has in any chunk and slice
     int fused_entries[ffi::kFusedWarps + 1] = {};
     int fused_ni = 0;  // inputs per warp of the one-pass backward
-    int longest_input = 0;  // without chunked lists: most entries that an input has
+    int longest_input = 0;  // most entries that an input has
     void* arrays = nullptr;     // the allocation that holds the four index arrays
     int32_t* rowptr = nullptr;  // [N+1]   canonical CSR-by-input
     int32_t* perm = nullptr;    // [L*K]   positions sorted by (idx[p], p)

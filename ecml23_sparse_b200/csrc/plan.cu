@@ -454,7 +454,7 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     g.off_bad = take(4);
     g.off_segs = take(g.scan_segs * 8);
     g.off_lb = take(g.chunks ? (g.mostChunks + 1) * N * 4 : 4);
-    g.off_stats = take((kFusedWarps + 1) * sizeof(int));
+    g.off_stats = take((kFusedWarps + 2) * sizeof(int));
     g.total = off;
     return g;
 }
@@ -537,13 +537,13 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
     FFI_LAUNCH_CHECK("rowptr_kernel");
 
     plan->order = nullptr;
+    int* longest_row = stats + kFusedWarps + 1;
+    FFI_CUDA_CHECK(cudaMemsetAsync(longest_row, 0, sizeof(int), stream));
+    longest_row_kernel<<<static_cast<unsigned>(ceil_div(N, 256)), 256, 0, stream>>>(plan->rowptr, static_cast<int>(N), longest_row);
+    FFI_LAUNCH_CHECK("longest_row_kernel");
+    FFI_CUDA_CHECK(cudaMemcpyAsync(&plan->longest_input, longest_row, sizeof(int), cudaMemcpyDeviceToHost, stream));
     if (!g.chunks) {
-        FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, sizeof(int), stream));
-        longest_row_kernel<<<static_cast<unsigned>(ceil_div(N, 256)), 256, 0, stream>>>(plan->rowptr, static_cast<int>(N), stats);
-        FFI_LAUNCH_CHECK("longest_row_kernel");
-        FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, sizeof(int), cudaMemcpyDeviceToHost, stream));
         FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
-        plan->longest_input = most[0];
         return FFI_OK;
     }
 

@@ -75,7 +75,18 @@ def test_hot_input_of_the_last_warp(B, hot):
 ])
 def test_hot_inputs(B, bf16, shares):
     """What a run has more than the others of its bundle is walked by all lane groups: remainders of all kinds."""
-    N, L, K = 300, 9001, 24
+    _check_shares(300, B, bf16, shares)
+
+
+@pytest.mark.parametrize("B", [7, 16, 17, 64, 128, 150])
+@pytest.mark.parametrize("shares", [((31, 0.35), (30, 0.05)), ((249, 0.6),), ((5, 1.0),)])
+def test_hot_inputs_of_one_slice(B, shares):
+    """With more than one slice the hottest of these tables go to a kernel for each gradient."""
+    _check_shares(250, B, B % 2 == 0, shares)
+
+
+def _check_shares(N, B, bf16, shares):
+    L, K = 9001, 24
     gen, x, W, g = _inputs(B, N, L, K, torch.bfloat16 if bf16 else torch.float32, B)
     idx = torch.randint(0, N, (L, K), generator=gen, dtype=torch.int32, device="cuda")
     u = torch.rand((L, K), generator=gen, device="cuda")
@@ -114,6 +125,23 @@ def test_hot_inputs_do_not_serialise(B):
         plan = ops.FFIPlan(idx, N)
         times.append(_time(lambda: ops._backward(x, idx, W, gT, True, plan=plan, grad_is_transposed=True)))
     assert times[1] < 8 * times[0]
+
+
+@pytest.mark.parametrize("N,L,K,B,share", [(2048, 150000, 32, 64, 0.2), (2048, 150000, 32, 32, 0.4), (2048, 150000, 32, 8, 0.8),
+                                           (768, 200000, 32, 32, 0.8), (768, 200000, 32, 64, 0.4), (300, 100000, 32, 64, 0.8)])
+def test_very_hot_input_is_no_slower_than_two_kernels(N, L, K, B, share):
+    """One input with a large part of the links: 1.2 to 3 times the two gradients by themselves in the one-pass kernel."""
+    gen, x, W, g = _inputs(B, N, L, K, torch.float32, B)
+    idx = torch.randint(0, N, (L, K), generator=gen, dtype=torch.int32, device="cuda")
+    idx[torch.rand((L, K), generator=gen, device="cuda") < share] = 17
+    gT = torch.zeros((L, _stride(B)), device="cuda")
+    gT[:, :B] = g
+    plan = ops.FFIPlan(idx, N)
+
+    def time(**want):
+        return min(_time(lambda: ops._backward(x, idx, W, gT, True, plan=plan, grad_is_transposed=True, **want)) for _ in range(3))
+
+    assert time() < 1.08 * (time(want_weight_grad=False) + time(want_feature_grad=False))
 
 
 @pytest.mark.parametrize("B", [1, 9, 24, 64, 127, 200])
@@ -161,8 +189,9 @@ def _weights(kind, N, gen):
 
 def _kernels(f):
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        f()
-        torch.cuda.synchronize()
+        for _ in range(3):  # (the profiler may miss single short kernels)
+            f()
+            torch.cuda.synchronize()
     return [e.name for e in prof.events()]
 
 
