@@ -392,7 +392,7 @@ int tile_columns(int64_t ldg) { return ldg % 256 == 0 ? 256 : ldg % 128 == 0 ? 1
 // An input belongs to one warp, here and in the kernel for grad_x alone, so an input with very many entries holds up everything else.
 // Here the batch tiles come one after another, in kChain us an entry and tile; there all tiles are walked at once, in about 0.2 us an
 // entry (0.13 to 0.28).  So several tiles pay for what the hottest input has beyond the others as long as that stays below what one
-// gather less gains, 0.1 (bf16) or 0.2 (fp32) us for a million entries and columns.  Measured, both kernels against one, us, for the inputs drawn
+// gather less gains, 0.1 (bf16) or 0.2 (fp32) us for a million entries and columns, and 10 us for a kernel less.  Measured, both kernels against one, us, for the inputs drawn
 // by Zipf's law of the exponents 0, 0.2, 0.3, 0.4, 0.6: B=512, N=16,384, L=50,000, K=32 bf16 334, 369, 520, 886, 2,732 against 254, 374,
 // 588, 1,043, 4,003 (line at 0.3), fp32 425, 469, 620, 1,001, 2,974 against 256, 371, 575, 1,016, 3,912 (line between 0.3 and 0.4);
 // B=1,024, N=32,768, L=60,000, K=32 bf16 788, 816, 929, 1,276, 3,695 against 597, 705, 998, 1,753, 7,343 (line between 0.2 and 0.3);
@@ -403,7 +403,7 @@ bool backward_wide_pays(const ffi_plan* plan, int64_t B, int64_t ldg, bool bf16)
     const double kChain = columns == 256 ? 0.14 : columns == 128 ? 0.077 : columns == 64 ? 0.054 : 0.035;
     const double more = ceil_div(B, columns) * kChain - 0.2;
     const double entries = static_cast<double>(plan->L) * plan->K, beyond = plan->longest_input - 2.0 * entries / plan->N;
-    return more <= 0.0 || beyond * more <= (bf16 ? 1e-7 : 2e-7) * entries * B;
+    return more <= 0.0 || beyond * more <= (bf16 ? 1e-7 : 2e-7) * entries * B + 10.0;
 }
 
 // grad_x as [N][B] (always), grad_W and, when gbias != nullptr, grad_bias, from gT; xT is x as [N][ldx]; cursor: N ints.
