@@ -436,7 +436,9 @@ PlanLayout plan_layout(int64_t L, int64_t K, int64_t N) {
     const PlanShape shape = plan_shape(L, K, N);
     g.T = shape.rows, g.ni = shape.ni;
     g.nChunks = ceil_div(L, g.T > 0 ? g.T : 1);
-    g.leastT = std::max(8, g.T / 2 / 8 * 8);
+    // (chunks that leave most of shared memory free, those of short tables, need not get shorter, and their arrays stay small: plan creation
+    // at 513 x 73 took 0.9 ms instead of 0.17 where they had just outgrown the blocks that cudaMalloc keeps at hand)
+    g.leastT = g.T <= 8 || chunks_fit(g.T, 4 * static_cast<int64_t>(g.T) * K) ? std::max(8, g.T) : std::max(8, g.T / 2 / 8 * 8);
     g.mostChunks = ceil_div(L, std::min(g.T, g.leastT) > 0 ? std::min(g.T, g.leastT) : 1);
     g.cptrBytes = g.mostChunks * (N + 1) * 4;
     g.chunks = g.T >= 8 && N <= kNarrowMaxN && g.nChunks * (N + 1) * 4 <= (512LL << 20) && static_cast<long long>(g.T) * K <= 65536;
@@ -503,7 +505,7 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
     long long* segs = reinterpret_cast<long long*>(scratch + g.off_segs);
     int* lb = reinterpret_cast<int*>(scratch + g.off_lb);
     int* stats = reinterpret_cast<int*>(scratch + g.off_stats);
-    int most[kFusedWarps + 1] = {};
+    int most[kFusedWarps + 2] = {};
 
     FFI_CUDA_CHECK(cudaMemsetAsync(bad, 0, 4, stream));
     validate_idx_kernel<<<1024, 256, 0, stream>>>(idx, n, static_cast<int>(N), bad);
@@ -541,8 +543,8 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
     FFI_CUDA_CHECK(cudaMemsetAsync(longest_row, 0, sizeof(int), stream));
     longest_row_kernel<<<static_cast<unsigned>(ceil_div(N, 256)), 256, 0, stream>>>(plan->rowptr, static_cast<int>(N), longest_row);
     FFI_LAUNCH_CHECK("longest_row_kernel");
-    FFI_CUDA_CHECK(cudaMemcpyAsync(&plan->longest_input, longest_row, sizeof(int), cudaMemcpyDeviceToHost, stream));
     if (!g.chunks) {
+        FFI_CUDA_CHECK(cudaMemcpyAsync(&plan->longest_input, longest_row, sizeof(int), cudaMemcpyDeviceToHost, stream));
         FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
         return FFI_OK;
     }
@@ -560,13 +562,14 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
         FFI_CUDA_CHECK(cudaMemsetAsync(stats, 0, (kFusedWarps + 1) * sizeof(int), stream));
         warp_stats_kernel<<<static_cast<unsigned>(ceil_div(N, g.ni)), 256, 0, stream>>>(plan->cptr, static_cast<int>(N), nChunks, g.ni, stats);
         FFI_LAUNCH_CHECK("warp_stats_kernel");
-        FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, (kFusedWarps + 1) * sizeof(int), cudaMemcpyDeviceToHost, stream));
+        FFI_CUDA_CHECK(cudaMemcpyAsync(most, stats, sizeof(most), cudaMemcpyDeviceToHost, stream));
         FFI_CUDA_CHECK(cudaStreamSynchronize(stream));
         plan->chunk_rows = T;
         plan->n_chunks = nChunks;
         plan->fused_entries[0] = 0;
         for (int w = 0; w < kFusedWarps; ++w) plan->fused_entries[w + 1] = plan->fused_entries[w] + (most[w] + 1) / 2 * 2;
         longest = most[kFusedWarps];
+        plan->longest_input = most[kFusedWarps + 1];
         return FFI_OK;
     };
     auto deal = [&]() -> int {

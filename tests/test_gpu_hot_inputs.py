@@ -245,3 +245,12 @@ def test_dealt_plans(N, L, K, kind):
             assert torch.equal(a, b)
         for a, b in zip(plan.export(), plan.export(chunked=True)):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("N,L,K", [(254, 513, 73), (64, 1000, 16), (700, 2000, 40)])
+def test_plans_of_short_tables_hold_one_set_of_chunks(N, L, K):
+    """Their chunks never get shorter, so nothing is kept in hand for that: plan creation grows by jumps with what it allocates."""
+    idx = torch.randint(0, N, (L, K), dtype=torch.int32, device="cuda")
+    info = ops.FFIPlan(idx, N).info()
+    arrays = [(N + 1) * 4, L * K * 4, L * K * 4, info["n_chunks"] * (N + 1) * 4, N * 4]
+    assert info["device_bytes"] <= sum((b + 255) // 256 * 256 for b in arrays)
