@@ -52,7 +52,7 @@ struct BwdFusedParams {
     long long ldx;
     const int* cperm;
     const int* cptr;
-    const int* order;  // UNEVEN: the input at each place of the chunked lists
+    const int* order;  // UNEVEN: the input at each place of the chunked lists, or nullptr: in order
     float* partial;  // [R][N][Bpad]
     float* gW;
     float* gbias;  // grad_bias[o] = sum_b gT[o][b], from the g tiles at hand anyway; or nullptr
@@ -64,7 +64,7 @@ struct BwdFusedParams {
     int Bpad;
     int segChunks;  // chunks per flushed partial
     int ni;         // inputs per warp
-    int longRun;    // uneven tables: kLongRun, or 0 where a bundle has fewer inputs than lane groups
+    int longRun;    // UNEVEN: kLongRun, or 0 where the lane groups share all runs (shares_runs)
     int boxes;      // TMA boxes per tile (at most 256 rows each)
     int lastHalf;   // bf16 W of an odd number of elements: position of the last one, which has no whole word; else -1
     bool xVec;      // rows of x start on 8 bytes; what lies behind an odd B in them is zero
@@ -262,9 +262,9 @@ __device__ __forceinline__ void tmem_store(unsigned taddr, const LaneVec<VPL, LG
 //   exponent 0.8: 128 1,973 (two) -> 1,373, 64 1,300 (two) -> 811, 32 2,194 -> 632, 8 1,968 -> 384
 //   exponent 1:   128 2,350 (two) -> 1,788, 64 1,375 (two) -> 1,110, 32 4,067 -> 889, 8 3,856 -> 548
 //   30 % of the links added to the leading quarter of the inputs: 128 1,974 (two) -> 862, 64 1,201 (two) -> 517
-// Fewer than kFusedFewInputs inputs per warp take this variant, too, and share all runs longer than one and a half times the average of a
-// full bundle (longRun = 0): side by side most groups had no input.  L=300,000, us, before -> now: N=10, K=8 B=128 263 -> 114,
-// 8 134 -> 45; N=32, K=16 128 246 -> 177, 8 119 -> 65.  (With longRun 4, 8, 12 and 15 over 112 such shapes 1, 2, 3 and 6 % slower.)
+// Warps with fewer inputs than lane groups take this variant, too (see shares_runs), and share all runs longer than one and a half times
+// the average of a full bundle (longRun = 0): side by side most groups had no input.  L=300,000, us, before -> now: N=10, K=8 B=128
+// 263 -> 114, 8 134 -> 45; N=32, K=16 128 246 -> 177, 8 119 -> 65.  (With longRun 4, 8, 12 and 15 over 112 such shapes 1, 2, 3 and 6 % slower.)
 // (An even table: 813, 499, 356, 224.)  With a fifth or more of all links to ONE input two kernels are faster again, see fused_pays.
 // In one kernel with the even case and a flag looked up per chunk, even tables took 2 to 6 % longer (registers).
 //
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffi_bwd_runs_kernel(const __grid_
         // ---- the warps that walk -------------------------------------------------------------
         const TX* xT = static_cast<const TX*>(p.xT);
         const int iw = i_lo + warp * ni;                 // this warp's first input, or its place
-        auto input_at = [&](int i) { return UNEVEN ? __ldg(p.order + i) : i; };
+        auto input_at = [&](int i) { return UNEVEN && p.order ? __ldg(p.order + i) : i; };
         const int nb = (ni + G - 1) / G;                 // its bundles
         // lanes 32*(warp % 4) .. +31 are the ones this warp may touch; its bundles take NB*COLS columns
         const unsigned taddr0 = *tmem_base_p + ((static_cast<unsigned>(warp & 3) * 32u) << 16) + static_cast<unsigned>(warp >> 2) * (NB * COLS);
@@ -871,6 +871,15 @@ int encode_g_map(CUtensorMap* map, const float* gT, int64_t L, int64_t ldg, int6
 
 }  // namespace
 
+// Whether the lane groups share the runs of any table because a warp has too few inputs for them.  It pays where the runs are long: graph
+// of backwards, side by side against shared, us, by entries in a chunk's average run: one input per warp 8 7.4, 8.3; 20 8.7, 8.3; 32 9.4,
+// 8.4; 208 42, 14; two 18 8.1, 8.6; 40 10.5, 9.2; 104 29, 18 (all 8 columns); three, up to 16 columns 27 9.4, 9.5; 69 24, 19; more columns
+// of three inputs lose throughout (32 columns 27 9.8, 10.8; 69 24, 26).
+static bool shares_runs(const ffi_plan* plan, const FusedConfig& c, int64_t columns) {
+    const double run = static_cast<double>(plan->chunk_rows) * plan->K / static_cast<double>(plan->N);
+    return c.ni == 1 ? run >= 20.0 : c.ni == 2 ? run >= 32.0 : c.ni == 3 && columns <= 16 && run >= 32.0;
+}
+
 // An input belongs to one warp of a range, so what bounds a table with a very hot input is that warp's chain, kChain ns an entry: the
 // more slices, the fewer ranges the input's entries are spread over.  The kernels for grad_x and grad_W alone take, with such tables,
 // about kTwo ns for every link, and 30 us for the second launch, its partials and short tables in general.  One pass against two, us, with a
@@ -956,7 +965,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
         p.Bpad = c.Bpad;
         p.segChunks = c.segChunks;
         p.ni = c.ni;
-        p.longRun = c.ni < kFusedFewInputs ? 0 : kLongRun;
+        p.longRun = shares_runs(a.plan, c, cols) ? 0 : kLongRun;
         // gT as a 2-D tensor [L rows][BT columns] with row pitch ldg; one or two boxes = a g tile
         CUtensorMap g_map;
         const int rows = p.T / c.halves;  // (T is a multiple of 8)
@@ -979,7 +988,7 @@ int launch_backward_fused(const GradXArgs& a, const void* xT, int64_t ldx, float
             return launch_kernel(ffi_bwd_runs_kernel<16, 4, 1, TX, ACC, UNEVEN>);
         };
         auto launch_table = [&](auto tx, auto acc) {
-            return a.plan->order ? launch_typed(tx, acc, std::true_type{}) : launch_typed(tx, acc, std::false_type{});
+            return p.order || p.longRun == 0 ? launch_typed(tx, acc, std::true_type{}) : launch_typed(tx, acc, std::false_type{});
         };
         auto launch_tile = [&](auto acc) { return a.w_bf16 ? launch_table(__nv_bfloat16{}, acc) : launch_table(float{}, acc); };
         rc = b0 > 0 ? launch_tile(std::true_type{}) : launch_tile(std::false_type{});

@@ -291,9 +291,8 @@ constexpr int kFusedWarps = 16;  // walking warps of the one-pass backward
 // Its lane groups walk the runs of a chunk's entries side by side; tables with a run of more than three times the average and
 // kFusedFarRun entries have their inputs dealt to the warps by count and go to a variant of the kernel (random tables stay below:
 // average 11, longest 38 of 1.9 million runs at N=768, L=670,091, K=32), and those with one of more than kFusedLongestRun have to
-// (see plan_build and backward_fused.cu).  So do tables with fewer than kFusedFewInputs inputs per warp (48 inputs and fewer), whose lane
-// groups would for the greater part have none to walk.
-constexpr int kFusedFarRun = 32, kFusedLongestRun = 1024, kFusedFewInputs = 4;
+// (see plan_build and backward_fused.cu).
+constexpr int kFusedFarRun = 32, kFusedLongestRun = 1024;
 }  // namespace ffi
 
 // The plan object (defined in plan.cu, used by backward.cu and api.cu).

@@ -581,11 +581,10 @@ int plan_build(ffi_plan* plan, const int32_t* idx, unsigned char* scratch, cudaS
         FFI_CUDA_CHECK(cudaMemcpyAsync(plan->order, order, N * sizeof(int), cudaMemcpyHostToDevice, stream));
         return FFI_OK;
     };
-    int rc = g.ni < kFusedFewInputs ? deal() : FFI_OK;  // (few inputs: shared by the lane groups, whatever the table)
-    if (rc == FFI_OK) rc = chunk_lists();
+    int rc = chunk_lists();
     if (rc != FFI_OK) return rc;
     const long long average = ceil_div(static_cast<int64_t>(T) * K, N);
-    if (!plan->order && (longest > 3 * average + kFusedFarRun || longest > kFusedLongestRun || !chunks_fit(T, plan->fused_entries[kFusedWarps]))) {
+    if (longest > 3 * average + kFusedFarRun || longest > kFusedLongestRun || !chunks_fit(T, plan->fused_entries[kFusedWarps])) {
         // An uneven table: the inputs are dealt anew, and the chunks get shorter until the entries of the largest warps fit (each try
         // takes the kernels above and a round trip to the device: a rebuild at N=768, L=670,091, K=32 takes 1.26 ms for an even table,
         // 1.75 with inputs drawn by Zipf's law of exponent 0.6, 2.3 of 1, 2.9 of 1.3).  Dealt, nearly all fit the chunks of an even

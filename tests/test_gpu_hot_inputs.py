@@ -146,9 +146,10 @@ def test_very_hot_input_is_no_slower_than_two_kernels(N, L, K, B, share):
 
 @pytest.mark.parametrize("B", [1, 9, 24, 64, 127, 200])
 @pytest.mark.parametrize("N,L,K,bf16", [(1, 5003, 3, False), (3, 9001, 2, True), (10, 20011, 8, False), (16, 4099, 7, True), (17, 4099, 16, False),
-                                        (33, 30001, 5, True), (48, 7001, 24, False), (49, 7001, 24, True), (65, 3001, 16, False)])
+                                        (33, 30001, 5, True), (48, 7001, 24, False), (49, 7001, 24, True), (65, 3001, 16, False),
+                                        (32, 9001, 40, True), (48, 40001, 40, False), (100, 500, 72, False)])
 def test_few_inputs(B, N, L, K, bf16):
-    """Fewer inputs per warp than lane groups, down to warps without any: the groups share the runs."""
+    """Fewer inputs per warp than lane groups, down to warps without any: the groups share the runs where these are long."""
     gen, x, W, g = _inputs(B, N, L, K, torch.bfloat16 if bf16 else torch.float32, B)
     _check(x, torch.randint(0, N, (L, K), generator=gen, dtype=torch.int32, device="cuda"), W, g)
 
